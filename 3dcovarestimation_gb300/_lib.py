@@ -21,6 +21,9 @@ KERNEL_ES, KERNEL_LINEAR, KERNEL_NEAREST = 0, 1, 2
 GRID_CENTERED, GRID_FFT_NATIVE = 0, 1
 # epilogue flags
 APPLY_NYQUIST, APPLY_CTF, APPLY_CTF_PARAMS = 1, 2, 4
+# the grid is a real volume's transform (cov3d_interp); only the output's real part is used
+# (cov3d_backproject)
+GRID_HERMITIAN, REAL_OUTPUT = 8, 16
 # CTF parameters per image (pixel size, defocus u, v, astigmatism angle, kV, Cs, amplitude contrast,
 # phase shift)
 CTF_NPARAMS = 8

@@ -56,7 +56,7 @@ __device__ __forceinline__ void point_freq(const PointGeom &g, int64_t id, float
   }
 }
 
-// Fractional centered-grid index of a frequency.
+// Fractional centered-grid index of a frequency, in float32.
 __device__ __forceinline__ float freq_to_index(const PointGeom &g, float w) {
   if (g.mapping == kMapES) {
     return __fadd_rn(__fmul_rn(w, g.s_es), g.half_n);
@@ -75,12 +75,88 @@ __device__ __forceinline__ void point_index(const PointGeom &g, int64_t id, floa
   t[2] = freq_to_index(g, w[2]);
 }
 
-// First cell of a point's window along one axis.
+// Records of kSortHalf hold their indices as integers in units of 2^-frac cell, with as many
+// fraction bits as leave room for the grid (22 at n = 256): mirrored points then have exactly
+// mirrored indices, and a float index of a 256^3 grid is only good to 1.5e-5 cells (white volumes
+// project to 1e-6 of the 64-bit result with the integers, to 1.1e-5 with the floats).
+constexpr int kDeadIndex = -2147483647 - 1;  // NaN or outside the grid
+constexpr int kRotShift = 40;  // rotation coefficients: cells per pixel step, in units of 2^-40
+constexpr long long kDeadCoef = -9223372036854775807LL - 1;
+
+// Index of point `id` along axes 0..2.  Rotations: R @ [kx, ky, 0] n / Lp from the image's integer
+// coefficients, wrapped to [-n/2, n/2).  Explicit points: w n / (2 pi) with the product's rounding
+// error carried along, wrapped when the kernel is periodic or the plan says so.
+template <int KT>
+__device__ __forceinline__ void point_index_fix(const PointGeom &g, int64_t id, int t[3]) {
+  const int one = 1 << g.frac;
+  const int64_t b = id / g.P;
+  const int p = (int)(id - b * g.P);
+  const int N = g.n << g.frac, c = (g.n / 2) << g.frac;
+  if (g.kind == kPointsRotations) {
+    const long long *A = g.rotc + b * 6;
+    const int row = p / g.Lp;
+    const int kx = p - row * g.Lp - g.Lp / 2, ky = row - g.Lp / 2;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const long long ax = __ldg(A + 2 * d), ay = __ldg(A + 2 * d + 1);
+      long long u = ax * kx + ay * ky;
+      u = (u + (1LL << (kRotShift - g.frac - 1))) >> (kRotShift - g.frac);
+      if (u >= N / 2) u -= N;
+      if (u < -(N / 2)) u += N;
+      if (u >= N / 2 || u < -(N / 2)) {  // not a rotation: several turns
+        u = (u + N / 2) % N;
+        u = (u < 0 ? u + N : u) - N / 2;
+      }
+      t[d] = ax == kDeadCoef || ay == kDeadCoef ? kDeadIndex : (int)u + c;
+    }
+    return;
+  }
+  const float *base = g.pts + b * 3 * (int64_t)g.P + p;
+  const float fn = (float)g.n;
+  const bool wrap = KT == COV3D_KERNEL_ES || g.wrap;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const float w = __ldg(base + d * (int64_t)g.P);
+    float u = w * g.s_es;
+    float e = fmaf(w, g.s_es, -u) + w * g.s_es_lo;
+    if (wrap) {
+      if (fabsf(u) < 8.0f * fn) {
+        u = fmaf(-rintf(u / fn), fn, u);
+      } else {  // many turns (or NaN, infinite: dead below)
+        const double v = fmod((double)w * ((double)g.s_es + (double)g.s_es_lo), (double)g.n);
+        u = (float)v;
+        e = (float)(v - (double)u);
+        if (fabsf(u) > 0.5f * fn) u -= copysignf(fn, u);
+      }
+    }
+    const float ip = rintf(u);
+    e += u - ip;
+    if (!(fabsf(ip) <= 0.5f * fn + 4.0f) || !(fabsf(e) <= 2.0f)) {
+      t[d] = kDeadIndex;
+      continue;
+    }
+    int v = (int)ip * one + __float2int_rn(e * (float)one);
+    if (wrap) {
+      if (v >= N / 2) v -= N;
+      if (v < -(N / 2)) v += N;
+    }
+    t[d] = v + c;
+  }
+}
+
+// First cell of a point's window along one axis, from a float index ...
 template <int KT, int W>
 __device__ __forceinline__ int first_cell(float t) {
   if (KT == COV3D_KERNEL_NEAREST) return (int)rintf(t);
   if (KT == COV3D_KERNEL_LINEAR) return (int)floorf(t);
   return (int)ceilf(t - 0.5f * (float)W);
+}
+// ... and from an integer one
+template <int KT, int W>
+__device__ __forceinline__ int first_cell_fix(int t, int frac) {
+  if (KT != COV3D_KERNEL_ES) return t >> frac;
+  const int one = 1 << frac;
+  return W % 2 == 0 ? ((t + (one - 1)) >> frac) - W / 2 : ((t + (one / 2 - 1)) >> frac) - (W - 1) / 2;
 }
 
 // ES kernel value exp(beta * (sqrt(1 - (2x/W)^2) - 1)) for |x| < W/2, else 0, with the fast
@@ -93,16 +169,46 @@ __device__ __forceinline__ float es_weight(float x, float beta) {
   return u > 0.0f ? __expf(beta * (u * rsqrtf(u) - 1.0f)) : 0.0f;
 }
 
-// Sorted point record written by the sort: fractional grid indices along axes 0..2 and the
+// Sorted point record written by the sort: grid indices along axes 0..2 (floats, or the bits of
+// point_index_fix's integers in records of kSortHalf) and the
 // point id, with kNyquistBit set when the point lies on the Nyquist row / column of an
-// even-sized image (vol_forward zeroes those pixels, projection_funcs.py:355-358).
+// even-sized image (vol_forward zeroes those pixels, projection_funcs.py:355-358).  Records of
+// kSortHalf may also stand for the mirror pixel -k of the id's k (kPairBit; the values there are
+// the conjugates), or hold the position of -k instead of the id's own (kConjBit, also with
+// kPairBit clear); ids are below 2^29 there, and below 2^30 in kSortFull, which sets neither.
 struct SortedPoint {
   float t0, t1, t2;
-  int idf;
+  unsigned idf;
 };
-constexpr int kNyquistBit = 1 << 30;
-__device__ __forceinline__ int sp_id(int idf) { return idf & (kNyquistBit - 1); }
-__device__ __forceinline__ bool sp_nyquist(int idf) { return (idf & kNyquistBit) != 0; }
+constexpr unsigned kNyquistBit = 1u << 31;
+constexpr unsigned kPairBit = 1u << 30;
+constexpr unsigned kConjBit = 1u << 29;
+// kHalf: the records are of kSortHalf
+template <bool HALF>
+__device__ __forceinline__ int sp_id(unsigned idf) {
+  return (int)(idf & (HALF ? kConjBit - 1 : kPairBit - 1));
+}
+__device__ __forceinline__ bool sp_nyquist(unsigned idf) { return (idf & kNyquistBit) != 0; }
+template <bool HALF>
+__device__ __forceinline__ bool sp_pair(unsigned idf) {
+  return HALF && (idf & kPairBit) != 0;
+}
+template <bool HALF>
+__device__ __forceinline__ bool sp_conj(unsigned idf) {
+  return HALF && (idf & kConjBit) != 0;
+}
+
+// Pixel holding -k of pixel p's k on the Lp x Lp image lattice, or -1 (Nyquist row or column of an
+// even-sized image); p itself at the centre.
+__device__ __forceinline__ int mirror_pixel(int p, int Lp) {
+  if (Lp % 2 != 0) return Lp * Lp - 1 - p;
+  return (p < Lp || p % Lp == 0) ? -1 : Lp * (Lp + 1) - p;
+}
+// id of the mirror pixel of a pair's id
+__device__ __forceinline__ int mirror_id(const PointGeom &g, int id) {
+  const int p = id % g.P;
+  return id + (g.Lp % 2 != 0 ? g.P - 1 : g.P + g.Lp) - 2 * p;
+}
 
 __device__ __forceinline__ bool on_nyquist(const PointGeom &g, int64_t id) {
   if (g.Lp % 2 != 0) return false;
@@ -110,35 +216,33 @@ __device__ __forceinline__ bool on_nyquist(const PointGeom &g, int64_t id) {
   return p < g.Lp || (p % g.Lp) == 0;
 }
 
-// Kernel taps along one axis: window cells c0 .. c0+W-1 and their weights.
-template <int KT, int W>
-__device__ __forceinline__ int taps(float t, float beta, float *wt) {
-  if (KT == COV3D_KERNEL_NEAREST) {
-    wt[0] = 1.0f;
-    return (int)rintf(t);
-  } else if (KT == COV3D_KERNEL_LINEAR) {
-    const float f0 = floorf(t);
-    wt[0] = (f0 + 1.0f) - t;
-    wt[1] = t - f0;
-    return (int)f0;
-  } else {
-    const int c0 = (int)ceilf(t - 0.5f * (float)W);
-#pragma unroll
-    for (int j = 0; j < W; ++j) wt[j] = es_weight<W>(t - (float)(c0 + j), beta);
-    return c0;
-  }
+// First cell of the window of a record's index t, and the weight of its tap q (0 <= q < W).
+template <int KT, int W, bool HALF>
+__device__ __forceinline__ int record_cell(float t, int frac) {
+  return HALF ? first_cell_fix<KT, W>(__float_as_int(t), frac) : first_cell<KT, W>(t);
 }
-
-// Weight of tap q (0 <= q < W) of the window of a point at fractional index t.
-template <int KT, int W>
-__device__ __forceinline__ float tap_weight(float t, int q, float beta) {
+template <int KT, int W, bool HALF>
+__device__ __forceinline__ float record_weight(float t, int c0, int q, int frac, float beta) {
   if (KT == COV3D_KERNEL_NEAREST) return 1.0f;
+  if (HALF) {  // the offset is exact
+    const float x = (float)(__float_as_int(t) - (c0 << frac)) * __int_as_float((127 - frac) << 23);
+    if (KT == COV3D_KERNEL_LINEAR) return q == 0 ? 1.0f - x : x;
+    return es_weight<W>(x - (float)q, beta);
+  }
   if (KT == COV3D_KERNEL_LINEAR) {
     const float f0 = floorf(t);
     return q == 0 ? (f0 + 1.0f) - t : t - f0;
   }
-  const int c0 = (int)ceilf(t - 0.5f * (float)W);
   return es_weight<W>(t - (float)(c0 + q), beta);
+}
+
+// Kernel taps along one axis: window cells c0 .. c0+W-1 and their weights.
+template <int KT, int W, bool HALF>
+__device__ __forceinline__ int taps(float t, int frac, float beta, float *wt) {
+  const int c0 = record_cell<KT, W, HALF>(t, frac);
+#pragma unroll
+  for (int j = 0; j < W; ++j) wt[j] = record_weight<KT, W, HALF>(t, c0, j, frac, beta);
+  return c0;
 }
 
 // CTF at pixel offsets (ka, kb) (row, column) from the image centre: sqrt(1 - w^2) sin(gamma) -

@@ -39,6 +39,7 @@ void count_launches(long long n);
 
 // How a nonuniform point's fine-grid fractional index is obtained.
 enum PointKind { kPointsNone = 0, kPointsExplicit = 1, kPointsRotations = 2 };
+
 // How a frequency maps to a fractional centered-grid index.
 enum Mapping { kMapES = 0, kMapGridSample = 1 };
 
@@ -46,12 +47,14 @@ struct PointGeom {
   int kind;           // PointKind
   const float *pts;   // explicit: contiguous (N, 3, P) frequencies
   const float *rot;   // rotations: (N, 9) row-major
+  const long long *rotc;  // their coefficients (N, 6), see point_index_fix
   int Lp;             // image edge (points per image = Lp*Lp)
   int P;              // Lp*Lp
   int n;              // fine grid edge
-  int mapping;        // Mapping
   int wrap;           // wrap explicit points to [-pi, pi)
-  float s_es;         // n / (2 pi)
+  int mapping;        // Mapping
+  int frac;           // fraction bits of the integer grid indices (point_index_fix)
+  float s_es, s_es_lo;  // n / (2 pi) as a float pair
   float half_n;       // n / 2 (integer division) as float
   float gs_scale;     // float32((n/(n-1))/pi)
   float gs_off;       // float32(1/(n-1)) for even n, else 0
@@ -88,6 +91,26 @@ struct DevBuf {
 };
 int grow(DevBuf &b, int64_t bytes);
 void release(DevBuf &b);
+
+// Which records the sort makes of the plan's points.  kSortFull: one per point.  kSortHalf: for a
+// Hermitian grid G(-k) = conj G(k) (the transform of a real volume), one record per pair of
+// mirror pixels (k, -k) of an image, so interpolation, and spreading of which only the real part
+// of the inverse transform is kept, do half the work (points_sort.cu, half_point).
+enum SortMode { kSortFull = 0, kSortHalf = 1, kSortModes = 2 };
+
+// One sorted view of the plan's points: records in bin order and the subproblem table.
+struct SortSet {
+  DevBuf bin_count;     // int (nbins + 1), last = dead points
+  DevBuf bin_off;       // int (nbins + 2)
+  DevBuf sub_off;       // int (nbins + 1)
+  DevBuf pt_bin, pt_rank;  // int (M), scratch of the sort
+  DevBuf sorted;        // SortedPoint (M)
+  DevBuf sub_bin, sub_first, sub_count;  // int (max subproblems)
+  DevBuf nsub;          // int scalar
+  bool used = false;    // some operator has asked for it: sorted with every new point set
+  bool valid = false;   // holds the current points
+  bool every_use = false;  // points may change by the replay of a graph that does not sort this view
+};
 }  // namespace cov3d
 
 struct cov3d_plan {
@@ -109,17 +132,12 @@ struct cov3d_plan {
   int64_t n_points = 0;
   cov3d::DevBuf pts;           // explicit points copy (N, 3, P) float
   cov3d::DevBuf rot;           // rotations (N, 9) float
+  cov3d::DevBuf rotc;          // their index coefficients (N, 6) int64
 
   // sort / subproblems
   cov3d::Bins bins{};
   int max_sub = 288;
-  cov3d::DevBuf bin_count;     // int (nbins + 1), last = dead points
-  cov3d::DevBuf bin_off;       // int (nbins + 2)
-  cov3d::DevBuf sub_off;       // int (nbins + 1)
-  cov3d::DevBuf pt_bin, pt_rank;              // int (M)
-  cov3d::DevBuf sorted;        // SortedPoint (M), bin-sorted order
-  cov3d::DevBuf sub_bin, sub_first, sub_count;  // int (max subproblems)
-  cov3d::DevBuf nsub;          // int scalar
+  cov3d::SortSet sets[cov3d::kSortModes];     // bin-sorted records by SortMode
 
   // workspaces
   cov3d::DevBuf fine, fine2;   // complex fine grids (n^3 * channels)
@@ -180,14 +198,19 @@ int launch_axis0_diag(cov3d_plan *p, float2 *g, const float *diag, int L, int n,
 int cg_operator_lines(cov3d_plan *p, const float2 *in, float2 *fine, float2 *out, const float2 *dotp,
                       const float *diag, int divide, const int *stop, const int *stop_last, double *dot);
 int step_forward_lines(cov3d_plan *p, const float *vec, const float *logs, const float *gc, int r, float2 *stage,
-                       float2 *grid, const float *fr, int64_t fr_stride, double coef, double *cost);
-int step_inverse_lines(cov3d_plan *p, float2 *grad_grid, const float *vec, const float *logs, const float *gc, int r,
-                       float *gvec, double *glog);
+                       float2 *grid, const float *fr, int64_t fr_stride, double coef, double *cost, double *glog);
+int step_inverse_lines(cov3d_plan *p, float2 *grad_grid, const float *logs, const float *gc, int r, float *gvec);
 inline bool prunable(const cov3d_plan *p) { return p->L % 2 == 0 && p->n >= p->L + 2; }
 
 // points_sort.cu
-int sort_points(cov3d_plan *p);
-int reserve_sort(cov3d_plan *p, int64_t M);
+int new_points(cov3d_plan *p);
+int need_sorted(cov3d_plan *p, SortMode mode);
+int reserve_sort(cov3d_plan *p, int64_t M, SortMode mode);
+// The records an operator uses on a grid (or volume) it knows to be Hermitian (real): half of them
+// where the plan's kernel and point count allow.
+inline SortMode hermitian_mode(const cov3d_plan *p) {
+  return p->kernel != COV3D_KERNEL_NEAREST && p->n_points < (int64_t(1) << 29) ? kSortHalf : kSortFull;
+}
 // gram_tc.cu: the BF16 Gram's operand and sum buffers for B images of P pixels at rank r
 int reserve_gram_bf16(cov3d_plan *p, int B, int P, int r);
 
@@ -218,11 +241,11 @@ struct EpilogueArgs {
 // plan's workspace; *out receives the device pointer.
 int prepare_ctf_coef(cov3d_plan *p, const float *params, int64_t n_images, int L, const CtfCoef **out);
 int launch_interp(cov3d_plan *p, const GridArgs &g, int nchan, void *out, int64_t out_ps, int64_t out_cs,
-                  const EpilogueArgs &e);
+                  const EpilogueArgs &e, SortMode mode);
 
 // spread.cu
 int launch_spread(cov3d_plan *p, const void *values, int64_t in_ps, int64_t in_cs, int nchan, const EpilogueArgs &e,
-                  void *grid, int64_t cell_stride, int64_t chan_stride, int shift);
+                  void *grid, int64_t cell_stride, int64_t chan_stride, int shift, SortMode mode);
 int launch_spread_unaggregated(cov3d_plan *p, const void *values, int64_t in_ps, const EpilogueArgs &e,
                                void *grids);
 
@@ -230,14 +253,14 @@ int launch_spread_unaggregated(cov3d_plan *p, const void *values, int64_t in_ps,
 int launch_pack(cov3d_plan *p, const float *vol_real, const void *vol_cplx, const float *log_scale, int use_gc,
                 int nchan, void *fine);
 int launch_unpack_complex(cov3d_plan *p, const void *fine, int nchan, int use_gc, void *out);
-int launch_unpack_grad(cov3d_plan *p, const void *fine, const float *vectors, const float *log_scale, int use_gc,
-                       int nchan, float *grad_vec, double *grad_log_acc);
+int launch_unpack_grad(cov3d_plan *p, const void *fine, const float *log_scale, int use_gc, int nchan,
+                       float *grad_vec);
 int launch_ml_reg(cov3d_plan *p, const void *grid, void *ggrid, const float *fr, int64_t fr_stride, int nchan, double coef,
-                  double *cost_acc, int init);
+                  double *cost_acc, double *glog, int init);
 int launch_gc_volume(const cov3d_plan *p, float *out);
 int launch_zero(cov3d_plan *p, void *ptr, int64_t bytes);
 int launch_ls_reg(cov3d_plan *p, const void *grid, void *ggrid, const float *fr, int64_t fr_stride, int r, double s,
-                  double *cost_acc);
+                  double *cost_acc, double *glog);
 void release_blas(cov3d_plan *p);
 int reserve_ls_reg(cov3d_plan *p, int r);
 
@@ -251,7 +274,7 @@ int launch_wpass(cudaStream_t st, int B, int P, int r, const void *q, int64_t is
                  const void *images, const void *C, const void *u, void *w, int64_t wis, int64_t wps, int64_t wcs);
 int launch_solve(cudaStream_t st, int B, int r, int objective, const void *gram, const void *h, double s2,
                  const double *linv, double wscale, double cscale, void *C, void *u, double *cost_b, double *cost_sum,
-                 void *z, void *m, int *bad);
+                 void *z, void *m, int *bad, double *glog = nullptr);
 int covar_cost_grad(cov3d_plan *p, const cov3d_cost_args *a, double *h_cost, double *d_cost, float *d_grad_vectors,
                     float *d_grad_log_sqrt, double *d_per_image_cost);
 

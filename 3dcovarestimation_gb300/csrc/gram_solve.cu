@@ -342,6 +342,7 @@ struct SolveArgs {
   float2 *u;           // (B, r)
   double *cost_b;      // (B) or null
   double *cost_sum;    // scalar accumulator
+  double *glog;        // (r) accumulators of d cost / d log_sqrt, or null
   float2 *z_out;       // (B, r) latent coordinates or null
   float2 *m_out;       // (B, r, r) m or null
   int *bad;            // set to 1 if a factorisation failed
@@ -351,8 +352,12 @@ struct SolveArgs {
 // so the same bits) and solves for z; thread kc then writes column kc of C from column kc of
 // m^-1, and thread 0 the per-image outputs (cost, z, m, u).  RMAX sizes the per-thread
 // working arrays (local memory): the smallest class that holds r keeps them in L1.
+// *glog receives the image's d cost / d log s_kc (the projections' channel kc scaled by s_kc):
+// 2 Re sum_p conj(W_pk) Q_pk, which m z = b and m^-1 gram / s2 = I - m^-1 (identity prior) turn into
+// wscale (1 - (m^-1)_kk - |z_k|^2) for ML -- no cancellation -- and
+// wscale (4 sum_i |gram_ik|^2 + 4 s2 gram_kk - 4 |h_k|^2) for LS.
 template <int RMAX>
-__device__ double solve_one(const SolveArgs &a, const int b, const int kc) {
+__device__ double solve_one(const SolveArgs &a, const int b, const int kc, double *glog) {
   const int r = a.r;
   cd m[RMAX * RMAX];
   cd z[RMAX];
@@ -391,6 +396,7 @@ __device__ double solve_one(const SolveArgs &a, const int b, const int kc) {
       cd col[RMAX];
       for (int i = 0; i < r; ++i) col[i] = {i == kc ? 1.0 : 0.0, 0.0};
       chol_solve(m, r, col);
+      *glog = a.wscale * (1.0 - col[kc].x - (z[kc].x * z[kc].x + z[kc].y * z[kc].y));
       for (int i = 0; i < r; ++i) {
         const cd zz = cmul(cconj(z[i]), z[kc]);
         a.C[((int64_t)b * r + i) * r + kc] = make_float2((float)((col[i].x + zz.x) * f), (float)((-col[i].y + zz.y) * f));
@@ -400,7 +406,13 @@ __device__ double solve_one(const SolveArgs &a, const int b, const int kc) {
       }
     }
   } else {
-    // least squares (thread 0 of the image)
+    if (a.C) {
+      double g2 = 0.0;
+      for (int i = 0; i < r; ++i) g2 += (double)G[i * r + kc].x * G[i * r + kc].x + (double)G[i * r + kc].y * G[i * r + kc].y;
+      const double h2 = (double)hb[kc].x * hb[kc].x + (double)hb[kc].y * hb[kc].y;
+      *glog = 4.0 * a.wscale * (g2 + a.s2 * G[kc * r + kc].x - h2);
+    }
+    // the rest: thread 0 of the image
     if (kc != 0) return 0.0;
     double t2 = 0.0, fro = 0.0, tr = 0.0;
     for (int i = 0; i < r; ++i) {
@@ -437,8 +449,19 @@ __global__ void __launch_bounds__(kSolveThreads) solve_kernel(const SolveArgs a)
   const int ipb = kSolveThreads / a.r;
   const int b = blockIdx.x * ipb + threadIdx.x / a.r;
   const int kc = threadIdx.x - (threadIdx.x / a.r) * a.r;
-  double cost = (threadIdx.x < ipb * a.r && b < a.B) ? solve_one<RMAX>(a, b, kc) : 0.0;
+  double glog = 0.0;
+  double cost = (threadIdx.x < ipb * a.r && b < a.B) ? solve_one<RMAX>(a, b, kc, &glog) : 0.0;
   if (!a.cost_sum) return;
+  if (a.glog) {  // the block's images summed per channel
+    __shared__ double s_gl[kSolveThreads];
+    s_gl[threadIdx.x] = glog;
+    __syncthreads();
+    if ((int)threadIdx.x < a.r) {
+      double t = 0.0;
+      for (int i = 0; i < ipb; ++i) t += s_gl[i * a.r + threadIdx.x];
+      atomicAdd(a.glog + threadIdx.x, t);
+    }
+  }
   for (int o = 16; o > 0; o >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, o);
   __shared__ double wsum[kSolveThreads / 32];
   if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = cost;
@@ -592,7 +615,7 @@ int launch_wpass(cudaStream_t st, int B, int P, int r, const void *q, int64_t is
 
 int launch_solve(cudaStream_t st, int B, int r, int objective, const void *gram, const void *h, double s2,
                  const double *linv, double wscale, double cscale, void *C, void *u, double *cost_b, double *cost_sum,
-                 void *z, void *m, int *bad) {
+                 void *z, void *m, int *bad, double *glog) {
   if (r < 1 || r > kMaxRank) {
     set_error("rank %d out of range (1..%d)", r, kMaxRank);
     return COV3D_EINVAL;
@@ -611,6 +634,7 @@ int launch_solve(cudaStream_t st, int B, int r, int objective, const void *gram,
   sa.u = static_cast<float2 *>(u);
   sa.cost_b = cost_b;
   sa.cost_sum = cost_sum;
+  sa.glog = glog;
   sa.z_out = static_cast<float2 *>(z);
   sa.m_out = static_cast<float2 *>(m);
   sa.bad = bad;
@@ -701,7 +725,7 @@ int covar_cost_grad(cov3d_plan *p, const cov3d_cost_args *a, double *h_cost, dou
     PhaseScope ps(p, kPhaseFftFwd);
     COV3D_TRY(step_forward_lines(p, a->d_vectors, a->d_log_sqrt, gcp, r, p->fine2.as<float2>(), p->fine.as<float2>(),
                                  ml_reg ? a->d_fourier_reg : nullptr, fr_stride, a->reg_scale / (2.0 * a->noise_var),
-                                 acc + 1));
+                                 acc + 1, acc + 8));
   } else {
     PhaseScope ps(p, kPhasePack);
     COV3D_TRY(launch_pack(p, a->d_vectors, nullptr, a->d_log_sqrt, a->use_grid_correction, r,
@@ -728,7 +752,7 @@ int covar_cost_grad(cov3d_plan *p, const cov3d_cost_args *a, double *h_cost, dou
   if (a->ctf_params && a->d_ctf) COV3D_TRY(prepare_ctf_coef(p, a->d_ctf, B, L, &ep.ctfc));
   {
     PhaseScope ps(p, kPhaseInterp);
-    COV3D_TRY(launch_interp(p, ga, r, p->q.ptr, r, 1, ep));
+    COV3D_TRY(launch_interp(p, ga, r, p->q.ptr, r, 1, ep, kSortFull));
   }
   // 4. per-image Gram, 5. FP64 solve -> cost, C, u
   {
@@ -744,7 +768,7 @@ int covar_cost_grad(cov3d_plan *p, const cov3d_cost_args *a, double *h_cost, dou
     PhaseScope ps(p, kPhaseSolve);
     COV3D_TRY(launch_solve(p->stream, B, r, a->objective, gram, h, a->noise_var, nullptr,
                            a->objective == 0 ? 1.0 / B : 1.0 / (B * L4), a->objective == 0 ? 1.0 : 1.0 / L4, C, u,
-                           d_per_image_cost, acc, nullptr, nullptr, bad));
+                           d_per_image_cost, acc, nullptr, nullptr, bad, acc + 8));
   }
   // 6. dcost/dconj(Q) in place, 7. spread through the exact adjoint (CTF, Nyquist, 1/L prologue)
   {
@@ -757,24 +781,24 @@ int covar_cost_grad(cov3d_plan *p, const cov3d_cost_args *a, double *h_cost, dou
   if (ml_reg && !lines_fwd) {
     PhaseScope ps(p, kPhaseReg);
     COV3D_TRY(launch_ml_reg(p, p->fine.ptr, p->fine2.ptr, a->d_fourier_reg, fr_stride, r,
-                            a->reg_scale / (2.0 * a->noise_var), acc + 1, 1));
+                            a->reg_scale / (2.0 * a->noise_var), acc + 1, acc + 8, 1));
   }
   if (ls_reg) {  // value and derivative, onto the gradient grid (zero after the line transforms)
     PhaseScope ps(p, kPhaseReg);
     if (!lines_fwd) COV3D_TRY(launch_zero(p, p->fine2.ptr, n3 * r * 8));
     COV3D_TRY(launch_ls_reg(p, p->fine.ptr, p->fine2.ptr, a->d_fourier_reg, fr_stride, r, a->reg_scale / L4,
-                            acc + 1));
+                            acc + 1, acc + 8));
   }
   {
     PhaseScope ps(p, kPhaseSpread);
     if (!with_reg && !lines_fwd) COV3D_TRY(launch_zero(p, p->fine2.ptr, n3 * r * 8));
-    COV3D_TRY(launch_spread(p, p->q.ptr, r, 1, r, ep, p->fine2.ptr, 1, n3, shift));
+    // only the real part of the inverse transform is used: mirror pixels are spread together
+    COV3D_TRY(launch_spread(p, p->q.ptr, r, 1, r, ep, p->fine2.ptr, 1, n3, shift, hermitian_mode(p)));
   }
   // 9. adjoint FFT, 10. crop + deapodise + chain rule to the Covar parameters
   if (lines_inv) {
     PhaseScope ps(p, kPhaseFftInv);
-    COV3D_TRY(step_inverse_lines(p, p->fine2.as<float2>(), a->d_vectors, a->d_log_sqrt, gcp, r, d_grad_vectors,
-                                 acc + 8));
+    COV3D_TRY(step_inverse_lines(p, p->fine2.as<float2>(), a->d_log_sqrt, gcp, r, d_grad_vectors));
   } else {
     PhaseScope ps(p, kPhaseFftInv);
     if (pruned) {  // axis 0 over all lines, then 2D only on the support planes the crop reads
@@ -791,8 +815,7 @@ int covar_cost_grad(cov3d_plan *p, const cov3d_cost_args *a, double *h_cost, dou
   }
   if (!lines_inv) {
     PhaseScope ps(p, kPhaseUnpack);
-    COV3D_TRY(launch_unpack_grad(p, p->fine2.ptr, a->d_vectors, a->d_log_sqrt, a->use_grid_correction, r,
-                                 d_grad_vectors, acc + 8));
+    COV3D_TRY(launch_unpack_grad(p, p->fine2.ptr, a->d_log_sqrt, a->use_grid_correction, r, d_grad_vectors));
   }
   finalize_kernel<<<1, 64, 0, p->stream>>>(acc, r, 1.0 / B, d_cost, d_grad_log_sqrt);
   COV3D_LAUNCHED("finalize_kernel");

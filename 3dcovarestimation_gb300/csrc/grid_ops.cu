@@ -65,50 +65,39 @@ __global__ void unpack_complex_kernel(const float2 *__restrict__ fine, const flo
   }
 }
 
-// Gradient w.r.t. the Covar parameters from the inverse-FFT'd fine-grid gradient:
-// dcost/dV = 2 Re(.) / gc on the cropped voxels; d/dvectors = dV * exp(s);
-// d/dlog_sqrt = sum dV * V (accumulated in double).
-__global__ void unpack_grad_kernel(const float2 *__restrict__ fine, const float *__restrict__ vectors,
-                                   const float *__restrict__ logs, const float *__restrict__ gc, int nchan, int L,
-                                   int n, float *__restrict__ gvec, double *__restrict__ glog) {
-  // capped grid walking voxel rows; one FP64 atomic per block and channel for d/dlog_sqrt
+// Gradient w.r.t. the eigenvectors from the inverse-FFT'd fine-grid gradient: dcost/dV = 2 Re(.) / gc
+// on the cropped voxels; d/dvectors = dV * exp(s).
+__global__ void unpack_grad_kernel(const float2 *__restrict__ fine, const float *__restrict__ logs,
+                                   const float *__restrict__ gc, int nchan, int L, int n, float *__restrict__ gvec) {
+  // capped grid walking voxel rows
   const int64_t L3 = (int64_t)L * L * L;
   const int64_t n3 = (int64_t)n * n * n;
   for (int c = 0; c < nchan; ++c) {
     const float e = expf(__ldg(logs + c));
-    double part = 0.0;
     for (int64_t row = blockIdx.x; row < (int64_t)L * L; row += gridDim.x) {
       const int j0 = (int)(row / L), j1 = (int)(row - (int64_t)j0 * L);
       const float2 *src = fine + (int64_t)c * n3 + ((int64_t)voxel_to_storage(j0, L, n) * n + voxel_to_storage(j1, L, n)) * n;
       const float g01 = gc ? 1.0f / (__ldg(gc + j0) * __ldg(gc + j1)) : 1.0f;
       for (int j2 = threadIdx.x; j2 < L; j2 += blockDim.x) {
         const float g = gc ? g01 / __ldg(gc + j2) : 1.0f;
-        const int64_t v = row * L + j2;
         const float dV = 2.0f * src[voxel_to_storage(j2, L, n)].x * g;
-        const float vec = __ldg(vectors + c * L3 + v);
-        gvec[c * L3 + v] = dV * e;
-        part += (double)(dV * (vec * e));
+        gvec[c * L3 + row * L + j2] = dV * e;
       }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    __shared__ double wp[32];
-    if ((threadIdx.x & 31) == 0) wp[threadIdx.x >> 5] = part;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += wp[i];
-      if (t != 0.0) atomicAdd(glog + c, t);
-    }
-    __syncthreads();
   }
 }
 
 // ML Fourier regulariser reg_scale * sum |G|^2 fr / (2 s2) (covar_sgd.py:1373-1376): adds its
 // conjugate-Wirtinger derivative coef * fr * G to the fine-grid gradient (or, with `init`,
-// writes it there, so the grid needs no zeroing before the spread), accumulates its value.
+// writes it there, so the grid needs no zeroing before the spread), accumulates its value and, twice
+// that per channel, its derivative with respect to log_sqrt (each thread's terms of a channel in
+// shared memory).
 __global__ void ml_reg_kernel(const float2 *__restrict__ grid, float2 *__restrict__ gg, const float *__restrict__ fr,
-                              int64_t frs, int nchan, int n, double coef, double *__restrict__ cost, int init) {
+                              int64_t frs, int nchan, int n, double coef, double *__restrict__ cost,
+                              double *__restrict__ glog, int init) {
+  extern __shared__ float s_gl[];  // nchan * blockDim.x
+  float *gl = s_gl + threadIdx.x;
+  for (int c = 0; c < nchan; ++c) gl[c * blockDim.x] = 0.0f;
   // capped grid walking whole rows (no per-element division); the channel sum of one cell is
   // FP32, the running sum over cells FP64, one FP64 atomic per block
   const int64_t n3 = (int64_t)n * n * n;
@@ -148,6 +137,7 @@ __global__ void ml_reg_kernel(const float2 *__restrict__ grid, float2 *__restric
                                                fmaf(cfb, x[u].z, y[u].z), fmaf(cfb, x[u].w, y[u].w));
             pa = fmaf(x[u].x, x[u].x, fmaf(x[u].y, x[u].y, pa));
             pb = fmaf(x[u].z, x[u].z, fmaf(x[u].w, x[u].w, pb));
+            gl[(c + u) * blockDim.x] += wa * (x[u].x * x[u].x + x[u].y * x[u].y) + wb * (x[u].z * x[u].z + x[u].w * x[u].w);
           }
         }
         for (; c < nchan; ++c) {
@@ -156,6 +146,7 @@ __global__ void ml_reg_kernel(const float2 *__restrict__ grid, float2 *__restric
           dst[c * cstep] = make_float4(fmaf(cfa, x.x, y.x), fmaf(cfa, x.y, y.y), fmaf(cfb, x.z, y.z), fmaf(cfb, x.w, y.w));
           pa = fmaf(x.x, x.x, fmaf(x.y, x.y, pa));
           pb = fmaf(x.z, x.z, fmaf(x.w, x.w, pb));
+          gl[c * blockDim.x] += wa * (x.x * x.x + x.y * x.y) + wb * (x.z * x.z + x.w * x.w);
         }
         part += (double)(wa * pa) + (double)(wb * pb);
       }
@@ -174,6 +165,7 @@ __global__ void ml_reg_kernel(const float2 *__restrict__ grid, float2 *__restric
         y.y = fmaf(cf, x.y, y.y);
         gg[c * n3 + cell] = y;
         p32 = fmaf(w, fmaf(x.x, x.x, x.y * x.y), p32);
+        gl[c * blockDim.x] += w * (x.x * x.x + x.y * x.y);
       }
       part += (double)p32;
     }
@@ -187,6 +179,15 @@ __global__ void ml_reg_kernel(const float2 *__restrict__ grid, float2 *__restric
     double s = 0.0;
     for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += warp_part[i];
     if (s != 0.0) atomicAdd(cost, s * coef);
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, nw = (int)(blockDim.x >> 5);
+  for (int c = threadIdx.x >> 5; c < nchan; c += nw) {  // a warp per channel
+    double t = 0.0;
+    for (int i = lane; i < (int)blockDim.x; i += 32) t += (double)s_gl[c * blockDim.x + i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0 && t != 0.0) atomicAdd(glog + c, 2.0 * t * coef);
   }
 }
 
@@ -219,26 +220,24 @@ int launch_unpack_complex(cov3d_plan *p, const void *fine, int nchan, int use_gc
   return launched("unpack_complex_kernel");
 }
 
-int launch_unpack_grad(cov3d_plan *p, const void *fine, const float *vectors, const float *log_scale, int use_gc,
-                       int nchan, float *grad_vec, double *grad_log_acc) {
-  const int64_t L3 = (int64_t)p->L * p->L * p->L;
+int launch_unpack_grad(cov3d_plan *p, const void *fine, const float *log_scale, int use_gc, int nchan,
+                       float *grad_vec) {
   const int64_t rows = (int64_t)p->L * p->L;
-  (void)L3;
   const int threads = p->L >= 256 ? 256 : (p->L + 31) / 32 * 32;  // one voxel row per pass
-  unpack_grad_kernel<<<(unsigned)(rows < 2432 ? rows : 2432), threads, 0, p->stream>>>(static_cast<const float2 *>(fine), vectors, log_scale,
-                                                         use_gc ? p->gc1d.as<float>() : nullptr, nchan, p->L, p->n,
-                                                         grad_vec, grad_log_acc);
+  unpack_grad_kernel<<<(unsigned)(rows < 2432 ? rows : 2432), threads, 0, p->stream>>>(
+      static_cast<const float2 *>(fine), log_scale, use_gc ? p->gc1d.as<float>() : nullptr, nchan, p->L, p->n,
+      grad_vec);
   return launched("unpack_grad_kernel");
 }
 
 int launch_ml_reg(cov3d_plan *p, const void *grid, void *ggrid, const float *fr, int64_t fr_stride, int nchan,
-                  double coef, double *cost_acc, int init) {
+                  double coef, double *cost_acc, double *glog, int init) {
   const int64_t n3 = (int64_t)p->n * p->n * p->n;
   const int64_t rows = (int64_t)p->n * p->n;
   const unsigned blocks = (unsigned)(rows < 2432 ? rows : 2432);  // 16 blocks of 4 warps per SM
   (void)n3;
-  ml_reg_kernel<<<blocks, 128, 0, p->stream>>>(static_cast<const float2 *>(grid), static_cast<float2 *>(ggrid), fr,
-                                               fr_stride, nchan, p->n, coef, cost_acc, init);
+  ml_reg_kernel<<<blocks, 128, (size_t)nchan * 128 * sizeof(float), p->stream>>>(static_cast<const float2 *>(grid), static_cast<float2 *>(ggrid), fr,
+                                               fr_stride, nchan, p->n, coef, cost_acc, glog, init);
   return launched("ml_reg_kernel");
 }
 

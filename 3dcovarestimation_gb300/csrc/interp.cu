@@ -28,6 +28,7 @@ struct InterpParams {
   const CtfCoef *ctfc;
   int nyquist;
   float scale;
+  int half;  // records of kSortHalf
 };
 
 constexpr int kBin = 8;
@@ -54,7 +55,7 @@ struct InterpCP {
 // rows -- W*CP contiguous 16-byte values per row, no bank conflicts -- and accumulates
 // weight * value; the W partial sums of each pair are combined by a warp-shuffle tree and the
 // epilogue (Nyquist zeroing, CTF, scale) is applied.
-template <int KT, int W, int CP>
+template <int KT, int W, int CP, bool HALF>
 __global__ void __launch_bounds__(InterpWarps<W, CP>::value * 32) interp_kernel(const InterpParams a) {
   constexpr int T = kBin + W - 1;
   constexpr int CH = 2 * CP;
@@ -65,7 +66,8 @@ __global__ void __launch_bounds__(InterpWarps<W, CP>::value * 32) interp_kernel(
   extern __shared__ float4 tile4[];  // T^3 * CP float4 (= 2 complex), then the point records
   float2 *tile = reinterpret_cast<float2 *>(tile4);
   SortedPoint *s_sp = reinterpret_cast<SortedPoint *>(tile4 + T * T * T * CP);  // kInterpChunk
-  float *s_sc = reinterpret_cast<float *>(s_sp + kInterpChunk);                  // epilogue factor
+  // epilogue factors: of the id and, for kSortHalf, of its mirror pixel
+  float *s_sc = reinterpret_cast<float *>(s_sp + kInterpChunk);
   const int sub = blockIdx.x;
   if (sub >= *a.nsub) return;
   const int bin = a.sub_bin[sub];
@@ -117,13 +119,17 @@ __global__ void __launch_bounds__(InterpWarps<W, CP>::value * 32) interp_kernel(
   }
   __syncthreads();
   // the subproblem's point records and epilogue factors (Nyquist zeroing, CTF, scale)
-  for (int k = tid; k < cnt; k += blockDim.x) {
-    const SortedPoint sp = a.pts[first + k];
-    s_sp[k] = sp;
-    float sc = (a.nyquist && sp_nyquist(sp.idf)) ? 0.0f : a.scale;
-    sc *= ctf_factor(a.ctf, a.ctfc, a.g, sp_id(sp.idf));
-    s_sc[k] = sc;
-  }
+  auto stage_points = [&](int from) {
+    for (int k = tid; k < cnt; k += blockDim.x) {
+      const SortedPoint sp = a.pts[from + k];
+      s_sp[k] = sp;
+      const int id = sp_id<HALF>(sp.idf);
+      const float sc = (a.nyquist && sp_nyquist(sp.idf)) ? 0.0f : a.scale;
+      s_sc[k] = sc * ctf_factor(a.ctf, a.ctfc, a.g, id);
+      if (sp_pair<HALF>(sp.idf)) s_sc[kInterpChunk + k] = a.scale * ctf_factor(a.ctf, a.ctfc, a.g, mirror_id(a.g, id));
+    }
+  };
+  stage_points(first);
   const float2 *gbase = a.grid + (int64_t)a.ch0 * a.chs;
   // asynchronous copies global -> shared (8 bytes each, zero-filled outside the grid / past the
   // pass's channels), all in flight before one wait.  A warp copies RPW tile rows (channel,
@@ -168,15 +174,15 @@ __global__ void __launch_bounds__(InterpWarps<W, CP>::value * 32) interp_kernel(
       const bool pt_ok = pp < PPW && k < cnt;
       const SortedPoint sp = s_sp[pt_ok ? k : k0];
       int c0[3];
-      c0[0] = first_cell<KT, W>(sp.t0);
-      c0[1] = first_cell<KT, W>(sp.t1);
-      c0[2] = first_cell<KT, W>(sp.t2);
+      c0[0] = record_cell<KT, W, HALF>(sp.t0, a.g.frac);
+      c0[1] = record_cell<KT, W, HALF>(sp.t1, a.g.frac);
+      c0[2] = record_cell<KT, W, HALF>(sp.t2, a.g.frac);
       // one kernel weight per lane wl < 3W, then shared through the warp
       float myw = 0.0f;
       if (wl < 3 * W) {
         const int d = wl / W, tq = wl - (wl / W) * W;
         const float td = d == 0 ? sp.t0 : d == 1 ? sp.t1 : sp.t2;
-        myw = tap_weight<KT, W>(td, tq, a.k.beta);
+        myw = record_weight<KT, W, HALF>(td, d == 0 ? c0[0] : d == 1 ? c0[1] : c0[2], tq, a.g.frac, a.k.beta);
       }
       // through the warp's slot in shared memory (double-buffered by iteration): axis-0 taps at
       // 0, axis-1 at 8, axis-2 at 16, read back as broadcast 16-byte loads -- five loads and a
@@ -254,50 +260,59 @@ __global__ void __launch_bounds__(InterpWarps<W, CP>::value * 32) interp_kernel(
       }
       if (pt_ok && sl < CP) {
         // epilogue: vol_forward's Nyquist zeroing, CTF multiply and 1/L (projection_funcs.py:355-370)
-        const int64_t id = sp_id(sp.idf);
+        const int id = sp_id<HALF>(sp.idf);
+        auto put = [&](int64_t to, float sc, float si) {
+          float2 *o = a.out + to * a.ops + (int64_t)(a.ch0 + 2 * sl) * a.ocs;
+          if (2 * sl < a.nch) o[0] = make_float2(s.x * sc, s.y * si);
+          if (2 * sl + 1 < a.nch) o[a.ocs] = make_float2(s.z * sc, s.w * si);
+        };
         const float sc = s_sc[k];
-        float2 *o = a.out + id * a.ops + (int64_t)(a.ch0 + 2 * sl) * a.ocs;
-        if (2 * sl < a.nch) o[0] = make_float2(s.x * sc, s.y * sc);
-        if (2 * sl + 1 < a.nch) o[a.ocs] = make_float2(s.z * sc, s.w * sc);
+        put(id, sc, sp_conj<HALF>(sp.idf) ? -sc : sc);
+        if (sp_pair<HALF>(sp.idf)) {  // the mirror pixel's values are the conjugates
+          const float sm = s_sc[kInterpChunk + k];
+          put(mirror_id(a.g, id), sm, -sm);
+        }
       }
     }
     base += kInterpChunk;
     if (base >= last) break;
     cnt = min(kInterpChunk, last - base);
     __syncthreads();  // every warp is done with the previous points
-    for (int k = tid; k < cnt; k += blockDim.x) {
-      const SortedPoint sp = a.pts[base + k];
-      s_sp[k] = sp;
-      float sc = (a.nyquist && sp_nyquist(sp.idf)) ? 0.0f : a.scale;
-      sc *= ctf_factor(a.ctf, a.ctfc, a.g, sp_id(sp.idf));
-      s_sc[k] = sc;
-    }
+    stage_points(base);
     __syncthreads();
   }
 }
 
 // Points whose window lies entirely outside the grid (zero padding) get zero outputs.
 __global__ void interp_dead_kernel(const SortedPoint *__restrict__ pts, const int *__restrict__ off, int64_t nbins,
-                                   int nchan, float2 *__restrict__ out, int64_t ops, int64_t ocs) {
+                                   int nchan, float2 *__restrict__ out, int64_t ops, int64_t ocs, bool half) {
   const int lo = off[nbins], hi = off[nbins + 1];
   for (int k = lo + blockIdx.x * blockDim.x + threadIdx.x; k < hi; k += gridDim.x * blockDim.x) {
-    const int64_t id = sp_id(pts[k].idf);
+    const int64_t id = half ? sp_id<true>(pts[k].idf) : sp_id<false>(pts[k].idf);
     for (int c = 0; c < nchan; ++c) out[id * ops + c * ocs] = make_float2(0.f, 0.f);
   }
 }
 
-template <int KT, int W, int CP>
-int launch_cp(const InterpParams &a, int64_t max_blocks, cudaStream_t st) {
+template <int KT, int W, int CP, bool HALF>
+int launch_half(const InterpParams &a, int64_t max_blocks, cudaStream_t st) {
   constexpr int T = kBin + W - 1;
   const size_t smem =
-      (size_t)T * T * T * CP * sizeof(float4) + (size_t)kInterpChunk * (sizeof(SortedPoint) + 4);
+      (size_t)T * T * T * CP * sizeof(float4) + (size_t)kInterpChunk * (sizeof(SortedPoint) + (HALF ? 8 : 4));
   if (smem > 32 * 1024) {  // static shared arrays come on top of the dynamic size
-    cudaError_t e = cudaFuncSetAttribute(interp_kernel<KT, W, CP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(interp_kernel<KT, W, CP, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(interp_kernel)");
   }
-  interp_kernel<KT, W, CP><<<(unsigned)max_blocks, InterpWarps<W, CP>::value * 32, smem, st>>>(a);
+  interp_kernel<KT, W, CP, HALF><<<(unsigned)max_blocks, InterpWarps<W, CP>::value * 32, smem, st>>>(a);
   return launched("interp_kernel");
+}
+
+template <int KT, int W, int CP>
+int launch_cp(const InterpParams &a, int64_t max_blocks, cudaStream_t st) {
+  if constexpr (KT != COV3D_KERNEL_NEAREST) {
+    if (a.half) return launch_half<KT, W, CP, true>(a, max_blocks, st);
+  }
+  return launch_half<KT, W, CP, false>(a, max_blocks, st);
 }
 
 // Channel passes of at most 2*InterpCP<W> channels; a short last pass uses a smaller tile.
@@ -340,20 +355,22 @@ int launch_w(InterpParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
 }  // namespace
 
 int launch_interp(cov3d_plan *p, const GridArgs &ga, int nchan, void *out, int64_t out_ps, int64_t out_cs,
-                  const EpilogueArgs &e) {
+                  const EpilogueArgs &e, SortMode mode) {
   if (p->point_kind == kPointsNone || p->n_points == 0) {
     set_error("no points set");
     return COV3D_ESTATE;
   }
+  COV3D_TRY(need_sorted(p, mode));
+  const SortSet &ss = p->sets[mode];
   InterpParams a{};
   a.g = make_geom(p);
   a.k = make_kernel(p);
   a.bins = p->bins;
-  a.pts = p->sorted.as<SortedPoint>();
-  a.sub_bin = p->sub_bin.as<int>();
-  a.sub_first = p->sub_first.as<int>();
-  a.bin_off = p->bin_off.as<int>();
-  a.nsub = p->nsub.as<int>();
+  a.pts = ss.sorted.as<SortedPoint>();
+  a.sub_bin = ss.sub_bin.as<int>();
+  a.sub_first = ss.sub_first.as<int>();
+  a.bin_off = ss.bin_off.as<int>();
+  a.nsub = ss.nsub.as<int>();
   a.grid = static_cast<const float2 *>(ga.grid);
   a.cs = ga.cell_stride;
   a.chs = ga.chan_stride;
@@ -365,10 +382,11 @@ int launch_interp(cov3d_plan *p, const GridArgs &ga, int nchan, void *out, int64
   a.ctfc = e.ctfc;
   a.nyquist = e.nyquist;
   a.scale = e.scale;
+  a.half = mode == kSortHalf;
   const int64_t mb = p->bins.nbins + p->n_points / p->max_sub + 1;
   if (p->kernel != COV3D_KERNEL_ES) {
-    interp_dead_kernel<<<64, 256, 0, p->stream>>>(a.pts, p->bin_off.as<int>(), p->bins.nbins, nchan, a.out, out_ps,
-                                                  out_cs);
+    interp_dead_kernel<<<64, 256, 0, p->stream>>>(a.pts, ss.bin_off.as<int>(), p->bins.nbins, nchan, a.out, out_ps,
+                                                  out_cs, a.half != 0);
     COV3D_LAUNCHED("interp_dead_kernel");
   }
   switch (p->kernel) {

@@ -227,10 +227,11 @@ __device__ void block_add_pair(double x, double y, double *a, double *b) {
 //   kRowInv    CG: inverse along axis 2, the L support entries / n^3 to the volume (crop fused),
 //              <p, out> accumulated
 //   kUnpackRows step: inverse along axis 2, then d cost / d eigenvectors (2 Re(.) / grid
-//              correction * exp(log_sqrt)) and the per-channel d cost / d log_sqrt sum
+//              correction * exp(log_sqrt))
 //   kAxisFwd   step: forward along axis 0 over the support rows; G written whole to gout, and the
 //              gradient grid initialised in place: coef * fr * G (the Fourier regulariser's
-//              derivative) with its value coef * sum fr |G|^2 accumulated, or zero without fr
+//              derivative) with its value coef * sum fr |G|^2 and, twice that per channel, its
+//              derivative with respect to log_sqrt accumulated, or zero without fr
 //   kAxisInv   step: inverse along axis 0, support rows out
 enum { kRowFwd, kPackRows, kColFwd, kColInv, kRowInv, kUnpackRows, kAxisFwd, kAxisInv };
 
@@ -244,11 +245,11 @@ struct LineArgs {
   float2 *out;        // kRowInv: L^3 output
   const float2 *p;    // kRowInv: <p, out> operand or null
   double *dot;        // kRowInv: <p, out> (2 doubles)
-  const float *vec;   // kPackRows, kUnpackRows: (r, L^3) eigenvectors
+  const float *vec;   // kPackRows: (r, L^3) eigenvectors
   const float *logs;  // (r) log sqrt eigenvalues or null
   const float *gc;    // (L) grid correction or null
   float *gvec;        // kUnpackRows: (r, L^3) gradient
-  double *glog;       // kUnpackRows: (r) d cost / d log_sqrt accumulators
+  double *glog;       // kAxisFwd: (r) d cost / d log_sqrt accumulators
   float2 *gout;       // kAxisFwd: transformed grid (channel stride cs)
   const float *fr;    // kAxisFwd: regulariser weights (n^3, centred) or null
   int64_t frs;        // kAxisFwd: element stride between channels' weights (0: shared)
@@ -327,9 +328,7 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
     } else {  // kUnpackRows
       const float es = a.logs ? expf(__ldg(a.logs + c)) : 1.0f;
       const float g01 = a.gc ? 1.0f / (__ldg(a.gc + j0) * __ldg(a.gc + j1)) : 1.0f;
-      const float *vsrc = a.vec + c * L3 + vrow;
       float *gdst = a.gvec + c * L3 + vrow;
-      float part = 0.0f;  // this thread's terms in FP32, then one FP64 block sum
       line_dft<N1, N2, true>(
           ex, s_tw, role, [&](int i) { return row[i]; },
           [&](int k, float2 v) {
@@ -338,9 +337,7 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
             const float gj = a.gc ? g01 / __ldg(a.gc + j) : 1.0f;
             const float dV = 2.0f * v.x * gj;
             gdst[j] = dV * es;
-            part = fmaf(dV, __ldg(vsrc + j) * es, part);
           });
-      block_add_pair((double)part, 0.0, a.glog + c, nullptr);
     }
   } else if (KIND == kColFwd || KIND == kColInv) {
     const int t0 = (int)(line / n), s2 = (int)(line - (int64_t)(line / n) * n);
@@ -375,7 +372,7 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
             }
             ax[(int64_t)k * nn] = y;
           });
-      if (a.fr) block_add_pair((double)part * a.coef, 0.0, a.cost, nullptr);
+      if (a.fr) block_add_pair((double)part * a.coef, 2.0 * (double)part * a.coef, a.cost, a.glog + c);
     } else {  // kAxisInv
       line_dft<N1, N2, true>(
           ex, s_tw, role, [&](int i) { return ax[(int64_t)i * nn]; },
@@ -498,7 +495,7 @@ int cg_operator_lines(cov3d_plan *p, const float2 *in, float2 *fine, float2 *out
 }
 
 int step_forward_lines(cov3d_plan *p, const float *vec, const float *logs, const float *gc, int r, float2 *stage,
-                       float2 *grid, const float *fr, int64_t fr_stride, double coef, double *cost) {
+                       float2 *grid, const float *fr, int64_t fr_stride, double coef, double *cost, double *glog) {
   LineArgs a;
   COV3D_TRY(line_args(p, a));
   const int64_t n3 = (int64_t)p->n * p->n * p->n;
@@ -512,6 +509,7 @@ int step_forward_lines(cov3d_plan *p, const float *vec, const float *logs, const
   a.frs = fr_stride;
   a.coef = coef;
   a.cost = cost;
+  a.glog = glog;
   switch (p->n) {
     case 128: return step_forward_n<16, 8>(p, a, r);
     case 256: return step_forward_n<16, 16>(p, a, r);
@@ -519,17 +517,14 @@ int step_forward_lines(cov3d_plan *p, const float *vec, const float *logs, const
   }
 }
 
-int step_inverse_lines(cov3d_plan *p, float2 *grad_grid, const float *vec, const float *logs, const float *gc, int r,
-                       float *gvec, double *glog) {
+int step_inverse_lines(cov3d_plan *p, float2 *grad_grid, const float *logs, const float *gc, int r, float *gvec) {
   LineArgs a;
   COV3D_TRY(line_args(p, a));
   a.g = grad_grid;
   a.cs = (int64_t)p->n * p->n * p->n;
-  a.vec = vec;
   a.logs = logs;
   a.gc = gc;
   a.gvec = gvec;
-  a.glog = glog;
   switch (p->n) {
     case 128: return step_inverse_n<16, 8>(p, a, r);
     case 256: return step_inverse_n<16, 16>(p, a, r);

@@ -43,25 +43,41 @@ __global__ void ls_gather_kernel(const float2 *__restrict__ g, const float *__re
   }
 }
 
-// gg[c][cell] += coef * sqrt(fr) * Y[c][centered cell]
-__global__ void ls_scatter_kernel(const float2 *__restrict__ y, const float *__restrict__ fr, int64_t frs, int nchan,
-                                  int n, float coef, float2 *__restrict__ gg) {
+// gg[c][cell] += D = coef * sqrt(fr) * Y[c][centered cell], and its derivative with respect to
+// log_sqrt, 2 Re sum conj(D) G per channel (blockIdx.y), added to glog
+__global__ void ls_scatter_kernel(const float2 *__restrict__ y, const float2 *__restrict__ g,
+                                  const float *__restrict__ fr, int64_t frs, int n, float coef,
+                                  float2 *__restrict__ gg, double *__restrict__ glog) {
   const int64_t n2 = (int64_t)n * n, n3 = n2 * n;
-  for (int64_t row = blockIdx.x; row < nchan * n2; row += gridDim.x) {
-    const int c = (int)(row / n2);
-    const int64_t rr = row - c * n2;
+  const int c = blockIdx.y;
+  double part = 0.0;
+  for (int64_t rr = blockIdx.x; rr < n2; rr += gridDim.x) {
+    float dot = 0.0f;  // a thread's terms of one row in FP32
     const int s0 = (int)(rr / n), s1 = (int)(rr - (int64_t)s0 * n);
     const int64_t crow = ((int64_t)native_to_centered(s0, n) * n + native_to_centered(s1, n)) * n;
     const float2 *src = y + c * n3 + crow;
     const float *f = fr + c * frs + crow;
     float2 *dst = gg + c * n3 + rr * n;
+    const float2 *gr = g + c * n3 + rr * n;
     for (int s2 = threadIdx.x; s2 < n; s2 += blockDim.x) {
       const int c2 = native_to_centered(s2, n);
       const float w = coef * sqrtf(__ldg(f + c2));
       const float2 v = src[c2];
-      const float2 o = dst[s2];
+      const float2 o = dst[s2], x = gr[s2];
       dst[s2] = make_float2(fmaf(w, v.x, o.x), fmaf(w, v.y, o.y));
+      dot = fmaf(w, fmaf(v.x, x.x, v.y * x.y), dot);
     }
+    part += (double)dot;
+  }
+  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+  __shared__ double wsum[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) wsum[warp] = part;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += wsum[i];
+    atomicAdd(glog + c, 2.0 * t);
   }
 }
 
@@ -116,7 +132,7 @@ int reserve_ls_reg(cov3d_plan *p, int r) {
 }
 
 int launch_ls_reg(cov3d_plan *p, const void *grid, void *ggrid, const float *fr, int64_t fr_stride, int r, double s,
-                  double *cost_acc) {
+                  double *cost_acc, double *glog) {
   const int n = p->n;
   const int64_t n3 = (int64_t)n * n * n;
   const int64_t kdim = (int64_t)r * n * n;  // length of a row of X
@@ -147,8 +163,10 @@ int launch_ls_reg(cov3d_plan *p, const void *grid, void *ggrid, const float *fr,
                                    reinterpret_cast<const cuComplex *>(kmat), n, reinterpret_cast<const cuComplex *>(x),
                                    (int)kdim, &czero, reinterpret_cast<cuComplex *>(y), (int)kdim),
                        "cublasChemm"));
-  ls_scatter_kernel<<<rows, 128, 0, p->stream>>>(y, fr, fr_stride, r, n, (float)(2.0 * s),
-                                                  static_cast<float2 *>(ggrid));
+  const unsigned crows = (unsigned)((int64_t)n * n < 1216 ? (int64_t)n * n : 1216);
+  ls_scatter_kernel<<<dim3(crows, (unsigned)r), 128, 0, p->stream>>>(y, static_cast<const float2 *>(grid), fr,
+                                                                     fr_stride, n, (float)(2.0 * s),
+                                                                     static_cast<float2 *>(ggrid), glog);
   return launched("ls_scatter_kernel");
 }
 

@@ -468,7 +468,7 @@ int mean_accumulate(cov3d_plan *p, const void *d_images, const float *d_ctf, con
                                                    d_contrasts, p->n_images, p->L, vals);
   COV3D_LAUNCHED("mean_values_kernel");
   EpilogueArgs e{nullptr, 1, 1.0f / (float)p->L};
-  return launch_spread(p, vals, 1, M, 2, e, d_grids, 1, n3, 0);
+  return launch_spread(p, vals, 1, M, 2, e, d_grids, 1, n3, 0, kSortFull);
 }
 
 int regularize_lhs(cov3d_plan *p, const void *d_lhs, float *d_out) {

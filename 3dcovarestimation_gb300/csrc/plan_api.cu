@@ -105,13 +105,17 @@ PointGeom make_geom(const cov3d_plan *p) {
   g.kind = p->point_kind;
   g.pts = p->pts.as<float>();
   g.rot = p->rot.as<float>();
+  g.rotc = p->rotc.as<long long>();
   g.Lp = p->points_L;
   g.P = p->points_L * p->points_L;
   g.n = p->n;
-  g.mapping = p->kernel == COV3D_KERNEL_ES ? kMapES : kMapGridSample;
   g.wrap = p->wrap;
-  g.s_es = (float)((double)p->n / (2.0 * kPi));
+  g.mapping = p->kernel == COV3D_KERNEL_ES ? kMapES : kMapGridSample;
   g.half_n = (float)(p->n / 2);
+  for (g.frac = 0; ((int64_t)(p->n + 64) << (g.frac + 1)) < (int64_t(1) << 31); ++g.frac) {
+  }
+  g.s_es = (float)((double)p->n / (2.0 * kPi));
+  g.s_es_lo = (float)((double)p->n / (2.0 * kPi) - (double)g.s_es);
   g.gs_scale = (float)(((double)p->n / (double)(p->n - 1)) / kPi);
   g.gs_off = (p->n % 2 == 0) ? (float)(1.0 / (double)(p->n - 1)) : 0.0f;
   g.plane_half = 0.5f * (float)p->points_L;
@@ -197,7 +201,7 @@ void grid_correction_1d(const cov3d_plan *p, std::vector<double> &g) {
 int finish_points(cov3d_plan *p) {
   p->n_points = p->n_images * (int64_t)p->points_L * p->points_L;
   PhaseScope ps(p, kPhaseSort);
-  return sort_points(p);
+  return new_points(p);
 }
 
 bool valid(const cov3d_plan *p) { return p != nullptr && p->n > 0; }
@@ -333,8 +337,9 @@ int cov3d_plan_reserve(cov3d_plan *p, int64_t max_images, int points_L, int ncha
   const int64_t P = (int64_t)points_L * points_L;
   const int64_t M = max_images * P;
   const int64_t n3 = (int64_t)p->n * p->n * p->n;
-  COV3D_TRY(reserve_sort(p, M));
+  for (int m = 0; m < kSortModes; ++m) COV3D_TRY(reserve_sort(p, M, (SortMode)m));
   COV3D_TRY(grow(p->rot, max_images * 9 * 4));
+  COV3D_TRY(grow(p->rotc, max_images * 6 * 8));
   if (flags & COV3D_RESERVE_POINTS) COV3D_TRY(grow(p->pts, max_images * 3 * P * 4));
   // the covariance step: fine grid and its gradient, projections, per-image matrices
   COV3D_TRY(grow(p->fine, n3 * nchan * 8));
@@ -365,10 +370,14 @@ int cov3d_plan_destroy(cov3d_plan *p) {
     for (auto &kv : *p->ffts) cufftDestroy(kv.second);
     delete p->ffts;
   }
-  DevBuf *bufs[] = {&p->gc1d, &p->pts, &p->rot, &p->bin_count, &p->bin_off, &p->sub_off, &p->pt_bin, &p->pt_rank,
-                    &p->sorted, &p->sub_bin, &p->sub_first, &p->sub_count, &p->nsub, &p->fine, &p->fine2, &p->q,
+  DevBuf *bufs[] = {&p->gc1d, &p->pts, &p->rot, &p->rotc, &p->fine, &p->fine2, &p->q,
                     &p->small, &p->acc, &p->cgw, &p->xbf, &p->gsum, &p->fftw, &p->ctfc, &p->lsw};
   for (DevBuf *b : bufs) release(*b);
+  for (SortSet &ss : p->sets) {
+    DevBuf *sb[] = {&ss.pt_bin, &ss.pt_rank, &ss.bin_count, &ss.bin_off, &ss.sub_off, &ss.sorted, &ss.sub_bin, &ss.sub_first, &ss.sub_count,
+                    &ss.nsub};
+    for (DevBuf *b : sb) release(*b);
+  }
   release_blas(p);
   if (p->h_acc) cudaFreeHost(p->h_acc);
   if (p->ev_pool) {
@@ -464,7 +473,8 @@ int cov3d_interp(cov3d_plan *p, const void *d_grid, const cov3d_grid_layout *lay
   GridArgs g{d_grid, layout->cell_stride, layout->chan_stride, layout_shift(p, layout)};
   EpilogueArgs e;
   COV3D_TRY(epilogue_args(p, d_ctf, flags, scale, &e));
-  return launch_interp(p, g, nchan, d_out, out_point_stride, out_chan_stride, e);
+  const SortMode mode = (flags & COV3D_GRID_HERMITIAN) ? hermitian_mode(p) : kSortFull;
+  return launch_interp(p, g, nchan, d_out, out_point_stride, out_chan_stride, e, mode);
 }
 
 int cov3d_spread(cov3d_plan *p, const void *d_values, int64_t in_point_stride, int64_t in_chan_stride, int nchan,
@@ -491,7 +501,7 @@ int cov3d_spread(cov3d_plan *p, const void *d_values, int64_t in_point_stride, i
   EpilogueArgs e;
   COV3D_TRY(epilogue_args(p, d_ctf, flags, scale, &e));
   return launch_spread(p, d_values, in_point_stride, in_chan_stride, nchan, e, d_grid, layout->cell_stride,
-                       layout->chan_stride, layout_shift(p, layout));
+                       layout->chan_stride, layout_shift(p, layout), kSortFull);
 }
 
 int cov3d_spread_unaggregated(cov3d_plan *p, const void *d_values, int64_t in_point_stride, const float *d_ctf,
@@ -526,7 +536,8 @@ static int type2(cov3d_plan *p, const float *d_vol_real, const void *d_vol_compl
   COV3D_TRY(check_cufft(cufftExecC2C(fft, p->fine.as<cufftComplex>(), p->fine.as<cufftComplex>(), CUFFT_FORWARD),
                         "cufftExecC2C(forward)"));
   GridArgs g{p->fine.ptr, 1, n3, p->n - p->n / 2};
-  return launch_interp(p, g, nchan, d_out, ops, ocs, e);
+  // a real volume's transform is Hermitian
+  return launch_interp(p, g, nchan, d_out, ops, ocs, e, d_vol_real ? hermitian_mode(p) : kSortFull);
 }
 
 int cov3d_fine_grid(cov3d_plan *p, const float *d_vol_real, const void *d_vol_complex, int nchan, void *d_grid) {
@@ -564,7 +575,7 @@ int cov3d_project(cov3d_plan *p, const float *d_vol_real, const void *d_vol_comp
 
 // type 1 with the backprojection prologue, input (point, channel) at values[point * ips + ch * ics]
 static int type1(cov3d_plan *p, const void *d_values, int64_t ips, int64_t ics, int nchan, void *d_vol_out,
-                 const EpilogueArgs &e) {
+                 const EpilogueArgs &e, SortMode mode) {
   if (!valid(p) || !d_values || !d_vol_out || nchan < 1 || nchan > p->n_trans) {
     set_error("invalid type-1 arguments (nchan must be in 1..n_trans)");
     return COV3D_EINVAL;
@@ -572,7 +583,7 @@ static int type1(cov3d_plan *p, const void *d_values, int64_t ips, int64_t ics, 
   const int64_t n3 = (int64_t)p->n * p->n * p->n;
   COV3D_TRY(grow(p->fine, n3 * nchan * 8));
   COV3D_TRY(launch_zero(p, p->fine.ptr, n3 * nchan * 8));
-  COV3D_TRY(launch_spread(p, d_values, ips, ics, nchan, e, p->fine.ptr, 1, n3, p->n - p->n / 2));
+  COV3D_TRY(launch_spread(p, d_values, ips, ics, nchan, e, p->fine.ptr, 1, n3, p->n - p->n / 2, mode));
   cufftHandle fft;
   COV3D_TRY(get_fft(p, nchan, &fft));
   COV3D_TRY(check_cufft(cufftExecC2C(fft, p->fine.as<cufftComplex>(), p->fine.as<cufftComplex>(), CUFFT_INVERSE),
@@ -582,7 +593,7 @@ static int type1(cov3d_plan *p, const void *d_values, int64_t ips, int64_t ics, 
 
 int cov3d_execute_type1(cov3d_plan *p, const void *d_values, int nchan, void *d_vol_out) {
   EpilogueArgs e{nullptr, 0, 1.0f};
-  return type1(p, d_values, 1, p ? p->n_points : 0, nchan, d_vol_out, e);
+  return type1(p, d_values, 1, p ? p->n_points : 0, nchan, d_vol_out, e, kSortFull);
 }
 
 int cov3d_backproject(cov3d_plan *p, const void *d_values, int64_t in_point_stride, int64_t in_chan_stride, int nchan,
@@ -597,7 +608,8 @@ int cov3d_backproject(cov3d_plan *p, const void *d_values, int64_t in_point_stri
   }
   EpilogueArgs e;
   COV3D_TRY(epilogue_args(p, d_ctf, flags, scale, &e));
-  return type1(p, d_values, in_point_stride, in_chan_stride, nchan, d_vol_out, e);
+  return type1(p, d_values, in_point_stride, in_chan_stride, nchan, d_vol_out, e,
+               (flags & COV3D_REAL_OUTPUT) ? hermitian_mode(p) : kSortFull);
 }
 
 int cov3d_grid_correction(const cov3d_plan *p, float *d_out) {

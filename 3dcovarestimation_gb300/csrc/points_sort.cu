@@ -11,168 +11,385 @@ namespace cov3d {
 
 namespace {
 
+// The views being sorted by one launch sequence (blockIdx.y).
+struct SortView {
+  int half;
+  int *count, *off, *sub_off, *nsub;
+  int *pt_bin, *pt_rank;
+  SortedPoint *sorted;
+  int *sub_bin, *sub_first, *sub_count;
+};
+struct SortViews {
+  SortView v[kSortModes];
+};
+
+// Bin holding the window corner c0 (dead: outside the grid or without an index).
+template <int KT, int W>
+__device__ __forceinline__ int corner_bin(const PointGeom &g, const Bins &bins, int (&c0)[3], bool dead) {
+  int b[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    if (KT == COV3D_KERNEL_ES) {
+      c0[d] = pmod(c0[d], g.n);
+    } else {
+      if (c0[d] + W - 1 < 0 || c0[d] > g.n - 1) dead = true;
+      c0[d] = min(max(c0[d], 0), g.n - 1);
+    }
+    b[d] = c0[d] / bins.bs[d];
+  }
+  return dead ? (int)bins.nbins : (b[0] * bins.nb[1] + b[1]) * bins.nb[2] + b[2];
+}
+
+template <int KT, int W>
+__device__ __forceinline__ int bin_of(const PointGeom &g, const Bins &bins, const float *t) {
+  int c0[3];
+  bool dead = false;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    c0[d] = first_cell<KT, W>(t[d]);
+    if (!(t[d] == t[d])) {  // NaN coordinate: no contribution
+      dead = true;
+      c0[d] = 0;
+    }
+  }
+  return corner_bin<KT, W>(g, bins, c0, dead);
+}
+
+template <int KT, int W>
+__device__ __forceinline__ int bin_of_fix(const PointGeom &g, const Bins &bins, const int *t) {
+  int c0[3];
+  bool dead = false;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    dead = dead || t[d] == kDeadIndex;
+    c0[d] = t[d] == kDeadIndex ? 0 : first_cell_fix<KT, W>(t[d], g.frac);
+  }
+  return corner_bin<KT, W>(g, bins, c0, dead);
+}
+
 // Bin of every point (dead points, whose window misses the grid, go to bin nbins) and its
 // rank in the bin.  The lanes of a warp that share a bin (neighbouring pixels mostly do) take
 // their ranks from one atomic on the bin's counter, in lane order.
 template <int KT, int W>
-__global__ void bin_count_kernel(PointGeom g, KernelSpec k, Bins bins, int64_t M, int *__restrict__ count,
-                                 int *__restrict__ pt_bin, int *__restrict__ pt_rank) {
+__device__ __forceinline__ void count_full(const PointGeom &g, const Bins &bins, int64_t M, const SortView &v) {
   const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = id < M;
   int bin = -1;
   if (valid) {
     float t[3];
     point_index(g, id, t);
-    int b[3];
-    bool dead = false;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      int c0 = first_cell<KT, W>(t[d]);
-      if (!(t[d] == t[d])) {  // NaN coordinate: no contribution
-        dead = true;
-        c0 = 0;
-      }
-      if (k.periodic) {
-        c0 = pmod(c0, g.n);
-      } else {
-        if (c0 + W - 1 < 0 || c0 > g.n - 1) dead = true;
-        c0 = min(max(c0, 0), g.n - 1);
-      }
-      b[d] = c0 / bins.bs[d];
-    }
-    bin = dead ? (int)bins.nbins : (b[0] * bins.nb[1] + b[1]) * bins.nb[2] + b[2];
+    bin = bin_of<KT, W>(g, bins, t);
   }
   const unsigned grp = __match_any_sync(0xffffffffu, bin);
   const int lane = threadIdx.x & 31;
   const int leader = __ffs(grp) - 1;
   int base = 0;
-  if (valid && lane == leader) base = atomicAdd(count + bin, __popc(grp));
+  if (valid && lane == leader) base = atomicAdd(v.count + bin, __popc(grp));
   base = __shfl_sync(0xffffffffu, base, leader);
   if (!valid) return;
-  pt_bin[id] = bin;
-  pt_rank[id] = base + __popc(grp & ((1u << lane) - 1u));
+  v.pt_bin[id] = bin;
+  v.pt_rank[id] = base + __popc(grp & ((1u << lane) - 1u));
 }
 
-// Single-block exclusive scans over the bin counts: point offsets, and subproblem offsets
-// (ceil(count / max_sub) subproblems per live bin).
-__global__ void bin_scan_kernel(const int *__restrict__ count, int64_t nbins, int max_sub, int *__restrict__ off,
-                                int *__restrict__ sub_off, int *__restrict__ nsub) {
-  __shared__ long long s_pts[1024];
-  __shared__ long long s_sub[1024];
-  const int tid = threadIdx.x;
-  const int64_t total = nbins + 1;  // includes the dead bin
-  const int64_t per = (total + blockDim.x - 1) / blockDim.x;
-  const int64_t lo = tid * per;
-  const int64_t hi = min(total, lo + per);
-  long long sp = 0, ss = 0;
-  for (int64_t i = lo; i < hi; ++i) {
-    sp += count[i];
-    if (i < nbins) ss += (count[i] + max_sub - 1) / max_sub;
+// kSortHalf.  Pixels p and p' = mirror_pixel(p) of an image sample k and -k, where the transform
+// of a real volume holds conjugate values, so one record serves both when their indices mirror
+// each other about the grid's centre: exactly for points made from rotations, to within
+// 1.5e-7 n cells for explicit ones (the float rounding of two wrapped angles; any other pair of
+// points gets a record each).  The record holds the mean of the one index and the mirrored other,
+// in the half space t0 >= n / 2; its id is the pixel there.  Grid-sample kernels need both windows
+// inside the grid as well (zero padding does not mirror: cell 0 is stored, cell n is not).
+// Periodic kernels also fold single points into the half space (kConjBit).
+struct HalfRecord {
+  int t[3];
+  unsigned flags;  // kPairBit / kConjBit
+  bool swap;       // the pair's id is the mirror pixel
+};
+
+__device__ __forceinline__ void fold_single(const PointGeom &g, bool periodic, HalfRecord &r) {
+  const int c = (g.n / 2) << g.frac;
+  r.flags = 0;
+  r.swap = false;
+  if (periodic && r.t[0] < c && r.t[0] != kDeadIndex && r.t[1] != kDeadIndex && r.t[2] != kDeadIndex) {
+    r.flags = kConjBit;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) r.t[d] = 2 * c - r.t[d];
   }
-  s_pts[tid] = sp;
-  s_sub[tid] = ss;
-  __syncthreads();
-  for (int ofs = 1; ofs < (int)blockDim.x; ofs <<= 1) {
-    long long ap = tid >= ofs ? s_pts[tid - ofs] : 0;
-    long long as = tid >= ofs ? s_sub[tid - ofs] : 0;
-    __syncthreads();
-    s_pts[tid] += ap;
-    s_sub[tid] += as;
-    __syncthreads();
+}
+
+// The record of the pair whose first pixel has index ta and second tb; false when the two do not
+// mirror each other.
+template <int KT>
+__device__ __forceinline__ bool pair_record(const PointGeom &g, const int (&ta)[3], const int (&tb)[3],
+                                            HalfRecord &r) {
+  const int c = (g.n / 2) << g.frac, N = g.n << g.frac, tol = 2 + (int)(1.5e-7f * (float)N);
+  bool ok = true;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    ok = ok && ta[d] != kDeadIndex && tb[d] != kDeadIndex;
+    const int a = ta[d] - c;
+    long long s = (long long)a + (tb[d] - c);
+    if (KT == COV3D_KERNEL_ES) s = s > N / 2 ? s - N : (s < -(N / 2) ? s + N : s);
+    ok = ok && s <= tol && s >= -tol;
+    r.t[d] = a - (int)(s >> 1);
   }
-  long long rp = s_pts[tid] - sp;
-  long long rs = s_sub[tid] - ss;
-  for (int64_t i = lo; i < hi; ++i) {
-    off[i] = (int)rp;
-    rp += count[i];
-    if (i < nbins) {
-      sub_off[i] = (int)rs;
-      rs += (count[i] + max_sub - 1) / max_sub;
+  if (!ok) return false;
+  r.flags = kPairBit;
+  r.swap = r.t[0] < 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) r.t[d] = (r.swap ? -r.t[d] : r.t[d]) + c;
+  if (KT != COV3D_KERNEL_ES) {
+    const int lo = max(0, 2 * (g.n / 2) - g.n + 1), hi = min(g.n - 1, 2 * (g.n / 2));
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const int f = first_cell_fix<KT, 2>(r.t[d], g.frac);
+      ok = ok && f >= lo && f + 1 <= hi;
     }
   }
-  if (tid == blockDim.x - 1) {
-    off[total] = (int)s_pts[tid];
-    *nsub = (int)s_sub[tid];
+  return ok;
+}
+
+// count_full for kSortHalf: the thread of the first pixel of a mirror pair decides for both
+// (pt_bin -1: no record under that id); the threads of second pixels only keep their warp company.
+template <int KT, int W>
+__device__ __forceinline__ void count_half(const PointGeom &g, const Bins &bins, int64_t M, const SortView &v) {
+  const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int bin = -1;
+  int64_t rec = id;
+  if (id < M) {
+    const int p = (int)(id % g.P), m = mirror_pixel(p, g.Lp);
+    if (m < 0 || m >= p) {
+      HalfRecord a;
+      point_index_fix<KT>(g, id, a.t);
+      bool pair = false;
+      if (m > p) {
+        const int64_t other = id + (m - p);
+        HalfRecord b, r;
+        point_index_fix<KT>(g, other, b.t);
+        pair = pair_record<KT>(g, a.t, b.t, r);
+        if (pair) {
+          rec = r.swap ? other : id;
+          v.pt_bin[r.swap ? id : other] = -1;
+          a = r;
+        } else {
+          fold_single(g, KT == COV3D_KERNEL_ES, b);
+          const int ob = bin_of_fix<KT, W>(g, bins, b.t);
+          v.pt_bin[other] = ob;
+          v.pt_rank[other] = atomicAdd(v.count + ob, 1);
+        }
+      }
+      if (!pair) fold_single(g, KT == COV3D_KERNEL_ES, a);
+      bin = bin_of_fix<KT, W>(g, bins, a.t);
+    }
+  }
+  const unsigned grp = __match_any_sync(0xffffffffu, bin);
+  const int lane = threadIdx.x & 31;
+  const int leader = __ffs(grp) - 1;
+  int base = 0;
+  if (bin >= 0 && lane == leader) base = atomicAdd(v.count + bin, __popc(grp));
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if (bin < 0) return;
+  v.pt_bin[rec] = bin;
+  v.pt_rank[rec] = base + __popc(grp & ((1u << lane) - 1u));
+}
+
+template <int KT, int W>
+__global__ void bin_count_kernel(PointGeom g, Bins bins, int64_t M, SortViews views) {
+  const SortView &v = views.v[blockIdx.y];
+  if constexpr (KT != COV3D_KERNEL_NEAREST) {
+    if (v.half) return count_half<KT, W>(g, bins, M, v);
+  }
+  count_full<KT, W>(g, bins, M, v);
+}
+
+template <int KT>
+__device__ __forceinline__ void scatter_half(const PointGeom &g, int64_t M, const SortView &v) {
+  const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= M) return;
+  const int bin = v.pt_bin[id];
+  if (bin < 0) return;
+  const int pos = v.off[bin] + v.pt_rank[id];
+  const int p = (int)(id % g.P), m = mirror_pixel(p, g.Lp);
+  HalfRecord a;
+  point_index_fix<KT>(g, id, a.t);
+  bool pair = false;
+  if (m >= 0 && m != p) {
+    HalfRecord b, r;
+    point_index_fix<KT>(g, id + (m - p), b.t);
+    pair = m > p ? pair_record<KT>(g, a.t, b.t, r) : pair_record<KT>(g, b.t, a.t, r);
+    if (pair) a = r;
+  }
+  if (!pair) fold_single(g, KT == COV3D_KERNEL_ES, a);
+  SortedPoint sp;
+  sp.t0 = __int_as_float(a.t[0]);
+  sp.t1 = __int_as_float(a.t[1]);
+  sp.t2 = __int_as_float(a.t[2]);
+  sp.idf = (unsigned)id | a.flags | (on_nyquist(g, id) ? kNyquistBit : 0u);
+  v.sorted[pos] = sp;
+}
+
+// Exclusive scans over a view's bin counts, one block per view: point offsets, and subproblem
+// offsets (ceil(count / max_sub) subproblems per live bin).  Each pass takes four bins per thread
+// from one 16-byte load (a scan of contiguous per-thread chunks loaded 128 bytes apart took 53 us
+// for 32768 bins, this one 12).
+__global__ void __launch_bounds__(1024) bin_scan_kernel(int64_t nbins, int max_sub, SortViews views) {
+  const SortView &v = views.v[blockIdx.x];
+  __shared__ int s_pts[32], s_sub[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t total = nbins + 1;  // includes the dead bin
+  int carry_p = 0, carry_s = 0;
+  for (int64_t base = 0; base < total; base += 4 * 1024) {
+    const int64_t i0 = base + 4 * tid;
+    int c[4] = {0, 0, 0, 0}, sp = 0, ss = 0, sub[4];
+    if (i0 + 4 <= total) {
+      const int4 x = *reinterpret_cast<const int4 *>(v.count + i0);
+      c[0] = x.x; c[1] = x.y; c[2] = x.z; c[3] = x.w;
+    } else {
+      for (int k = 0; k < 4; ++k)
+        if (i0 + k < total) c[k] = v.count[i0 + k];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      sub[k] = i0 + k < nbins ? (c[k] + max_sub - 1) / max_sub : 0;
+      sp += c[k];
+      ss += sub[k];
+    }
+    int ip = sp, is = ss;  // inclusive within the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, ip, o), b = __shfl_up_sync(0xffffffffu, is, o);
+      if (lane >= o) {
+        ip += a;
+        is += b;
+      }
+    }
+    __syncthreads();  // the previous pass has read the warp totals
+    if (lane == 31) {
+      s_pts[warp] = ip;
+      s_sub[warp] = is;
+    }
+    __syncthreads();
+    int wp = s_pts[lane], ws = s_sub[lane];  // every warp scans the 32 warp totals
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, wp, o), b = __shfl_up_sync(0xffffffffu, ws, o);
+      if (lane >= o) {
+        wp += a;
+        ws += b;
+      }
+    }
+    const int before_p = __shfl_sync(0xffffffffu, wp, (warp + 31) & 31), before_s = __shfl_sync(0xffffffffu, ws, (warp + 31) & 31);
+    int rp = carry_p + (warp ? before_p : 0) + ip - sp, rs = carry_s + (warp ? before_s : 0) + is - ss;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i0 + k < total) v.off[i0 + k] = rp;
+      if (i0 + k < nbins) v.sub_off[i0 + k] = rs;
+      rp += c[k];
+      rs += sub[k];
+    }
+    carry_p += __shfl_sync(0xffffffffu, wp, 31);
+    carry_s += __shfl_sync(0xffffffffu, ws, 31);
+  }
+  if (tid == 0) {
+    v.off[total] = carry_p;
+    *v.nsub = carry_s;
   }
 }
 
-__global__ void scatter_kernel(PointGeom g, int64_t M, const int *__restrict__ pt_bin, const int *__restrict__ pt_rank,
-                               const int *__restrict__ off, SortedPoint *__restrict__ sorted) {
+__device__ __forceinline__ void scatter_full(const PointGeom &g, int64_t M, const SortView &v) {
   const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= M) return;
-  const int pos = off[pt_bin[id]] + pt_rank[id];
+  const int pos = v.off[v.pt_bin[id]] + v.pt_rank[id];
   float t[3];
   point_index(g, id, t);
   SortedPoint sp;
   sp.t0 = t[0];
   sp.t1 = t[1];
   sp.t2 = t[2];
-  sp.idf = (int)id | (on_nyquist(g, id) ? kNyquistBit : 0);
-  sorted[pos] = sp;
+  sp.idf = (unsigned)id | (on_nyquist(g, id) ? kNyquistBit : 0u);
+  v.sorted[pos] = sp;
 }
 
-__global__ void subproblem_kernel(int64_t nbins, int max_sub, const int *__restrict__ count,
-                                  const int *__restrict__ off, const int *__restrict__ sub_off,
-                                  int *__restrict__ sub_bin, int *__restrict__ sub_first, int *__restrict__ sub_count) {
-  const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void write_subproblems(int64_t b, int64_t nbins, int max_sub, const SortView &v) {
   if (b >= nbins) return;
-  const int c = count[b];
-  const int s0 = sub_off[b];
+  const int c = v.count[b];
+  const int s0 = v.sub_off[b];
   for (int s = 0; s * max_sub < c; ++s) {
-    sub_bin[s0 + s] = (int)b;
-    sub_first[s0 + s] = off[b] + s * max_sub;
-    sub_count[s0 + s] = min(max_sub, c - s * max_sub);
+    v.sub_bin[s0 + s] = (int)b;
+    v.sub_first[s0 + s] = v.off[b] + s * max_sub;
+    v.sub_count[s0 + s] = min(max_sub, c - s * max_sub);
+  }
+}
+
+// The records in bin order, and in the blocks after the points' the subproblem table.
+template <int KT>
+__global__ void scatter_kernel(PointGeom g, int64_t M, int64_t nbins, int max_sub, SortViews views) {
+  const SortView &v = views.v[blockIdx.y];
+  const int64_t pb = (M + blockDim.x - 1) / blockDim.x;
+  if (blockIdx.x >= pb) return write_subproblems((blockIdx.x - pb) * blockDim.x + threadIdx.x, nbins, max_sub, v);
+  if constexpr (KT != COV3D_KERNEL_NEAREST) {
+    if (v.half) return scatter_half<KT>(g, M, v);
+  }
+  scatter_full(g, M, v);
+}
+
+// Before the count: the views' counters to zero and, for new rotations, their index coefficients:
+// axis d (row 2 - d of R) moves by coefficient / 2^40 cells per pixel column and row, reduced modulo
+// the period n (the indices wrap anyway).
+__global__ void sort_begin_kernel(int64_t counters, SortViews views, int nviews, const float *__restrict__ rot,
+                                  int64_t n_images, int n, int Lp, long long *__restrict__ rotc) {
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+  for (int m = 0; m < nviews; ++m)
+    for (int64_t e = tid; e < counters; e += nt) views.v[m].count[e] = 0;
+  if (!rotc) return;
+  for (int64_t e = tid; e < n_images * 6; e += nt) {
+    const int64_t b = e / 6;
+    const int q = (int)(e - b * 6);
+    double v = (double)rot[b * 9 + (2 - q / 2) * 3 + (q & 1)] * (double)n / (double)Lp;
+    v -= (double)n * rint(v / (double)n);
+    rotc[e] = isfinite(v) ? __double2ll_rn(v * (double)(1LL << kRotShift)) : kDeadCoef;
   }
 }
 
 template <int KT, int W>
-void launch_count(cov3d_plan *p, const PointGeom &g, const KernelSpec &k, int blocks) {
-  bin_count_kernel<KT, W><<<blocks, 256, 0, p->stream>>>(g, k, p->bins, p->n_points, p->bin_count.as<int>(), p->pt_bin.as<int>(),
-                                                        p->pt_rank.as<int>());
+void launch_count(cov3d_plan *p, const PointGeom &g, dim3 grid, const SortViews &views) {
+  bin_count_kernel<KT, W><<<grid, 256, 0, p->stream>>>(g, p->bins, p->n_points, views);
 }
 
-}  // namespace
-
-// Every buffer the sort of M points uses (a no-op when they are large enough already).
-int reserve_sort(cov3d_plan *p, int64_t M) {
-  const int64_t nb = p->bins.nbins;
-  const int64_t max_subs = nb + M / p->max_sub + 1;
-  COV3D_TRY(grow(p->bin_count, (nb + 2) * 4));
-  COV3D_TRY(grow(p->bin_off, (nb + 2) * 4));
-  COV3D_TRY(grow(p->sub_off, (nb + 2) * 4));
-  COV3D_TRY(grow(p->pt_bin, M * 4));
-  COV3D_TRY(grow(p->pt_rank, M * 4));
-  COV3D_TRY(grow(p->sorted, M * (int64_t)sizeof(SortedPoint)));
-  COV3D_TRY(grow(p->sub_bin, max_subs * 4));
-  COV3D_TRY(grow(p->sub_first, max_subs * 4));
-  COV3D_TRY(grow(p->sub_count, max_subs * 4));
-  COV3D_TRY(grow(p->nsub, 16));
-  return COV3D_OK;
-}
-
-int sort_points(cov3d_plan *p) {
-  const int64_t M = p->n_points;
-  if (M <= 0) return COV3D_OK;
-  if (M >= (int64_t)(1 << 30)) {
-    set_error("too many points (%lld); the limit is 2^30-1 per plan", (long long)M);
-    return COV3D_EINVAL;
+// Sorts the points into the views of `modes` (bits 1 << SortMode) in one launch sequence.
+int sort_points(cov3d_plan *p, unsigned modes) {
+  const int64_t M = p->n_points, nb = p->bins.nbins;
+  SortViews views{};
+  int nv = 0;
+  bool half = false;
+  for (int m = 0; m < kSortModes; ++m) {
+    if (!(modes >> m & 1)) continue;
+    COV3D_TRY(reserve_sort(p, M, (SortMode)m));
+    SortSet &ss = p->sets[m];
+    half = half || m == kSortHalf;
+    views.v[nv++] = SortView{m == kSortHalf, ss.bin_count.as<int>(), ss.bin_off.as<int>(), ss.sub_off.as<int>(),
+                             ss.nsub.as<int>(), ss.pt_bin.as<int>(), ss.pt_rank.as<int>(), ss.sorted.as<SortedPoint>(),
+                             ss.sub_bin.as<int>(), ss.sub_first.as<int>(), ss.sub_count.as<int>()};
   }
-  COV3D_TRY(reserve_sort(p, M));
-  const int64_t nb = p->bins.nbins;
-
-  COV3D_CUDA(cudaMemsetAsync(p->bin_count.as<int>(), 0, (nb + 1) * sizeof(int), p->stream));
+  if (nv == 0) return COV3D_OK;
+  long long *rotc = nullptr;
+  if (half && p->point_kind == kPointsRotations) {
+    COV3D_TRY(grow(p->rotc, p->n_images * 6 * 8));
+    rotc = p->rotc.as<long long>();
+  }
   const PointGeom g = make_geom(p);
-  const KernelSpec k = make_kernel(p);
-  const int blocks = (int)((M + 255) / 256);
+  const int64_t work = nb + 1 > p->n_images * 6 ? nb + 1 : p->n_images * 6;
+  sort_begin_kernel<<<(unsigned)((work + 255) / 256 < 608 ? (work + 255) / 256 : 608), 256, 0, p->stream>>>(
+      nb + 1, views, nv, p->rot.as<float>(), p->n_images, p->n, p->points_L, rotc);
+  COV3D_LAUNCHED("sort_begin_kernel");
+  const dim3 blocks((unsigned)((M + 255) / 256), (unsigned)nv);
   switch (p->kernel) {
-    case COV3D_KERNEL_NEAREST: launch_count<COV3D_KERNEL_NEAREST, 1>(p, g, k, blocks); break;
-    case COV3D_KERNEL_LINEAR: launch_count<COV3D_KERNEL_LINEAR, 2>(p, g, k, blocks); break;
+    case COV3D_KERNEL_NEAREST: launch_count<COV3D_KERNEL_NEAREST, 1>(p, g, blocks, views); break;
+    case COV3D_KERNEL_LINEAR: launch_count<COV3D_KERNEL_LINEAR, 2>(p, g, blocks, views); break;
     default:
       switch (p->width) {
 #define COV3D_W(Wv) \
-  case Wv: launch_count<COV3D_KERNEL_ES, Wv>(p, g, k, blocks); break;
-        COV3D_W(2) COV3D_W(3) COV3D_W(4) COV3D_W(5) COV3D_W(6) COV3D_W(7) COV3D_W(8) COV3D_W(9) COV3D_W(10)
-        COV3D_W(11) COV3D_W(12) COV3D_W(13) COV3D_W(14) COV3D_W(15) COV3D_W(16)
+  case Wv: launch_count<COV3D_KERNEL_ES, Wv>(p, g, blocks, views); break;
+        COV3D_W(4) COV3D_W(5) COV3D_W(6) COV3D_W(7) COV3D_W(8)
 #undef COV3D_W
         default:
           set_error("unsupported ES width %d", p->width);
@@ -180,16 +397,80 @@ int sort_points(cov3d_plan *p) {
       }
   }
   COV3D_LAUNCHED("bin_count_kernel");
-  bin_scan_kernel<<<1, 1024, 0, p->stream>>>(p->bin_count.as<int>(), nb, p->max_sub, p->bin_off.as<int>(), p->sub_off.as<int>(), p->nsub.as<int>());
+  bin_scan_kernel<<<nv, 1024, 0, p->stream>>>(nb, p->max_sub, views);
   COV3D_LAUNCHED("bin_scan_kernel");
-  scatter_kernel<<<blocks, 256, 0, p->stream>>>(g, M, p->pt_bin.as<int>(), p->pt_rank.as<int>(), p->bin_off.as<int>(),
-                                                p->sorted.as<SortedPoint>());
+  const dim3 sblocks(blocks.x + (unsigned)((nb + 255) / 256), (unsigned)nv);
+  switch (p->kernel) {
+    case COV3D_KERNEL_NEAREST:
+      scatter_kernel<COV3D_KERNEL_NEAREST><<<sblocks, 256, 0, p->stream>>>(g, M, nb, p->max_sub, views);
+      break;
+    case COV3D_KERNEL_LINEAR:
+      scatter_kernel<COV3D_KERNEL_LINEAR><<<sblocks, 256, 0, p->stream>>>(g, M, nb, p->max_sub, views);
+      break;
+    default: scatter_kernel<COV3D_KERNEL_ES><<<sblocks, 256, 0, p->stream>>>(g, M, nb, p->max_sub, views);
+  }
   COV3D_LAUNCHED("scatter_kernel");
-  subproblem_kernel<<<(int)((nb + 255) / 256), 256, 0, p->stream>>>(nb, p->max_sub, p->bin_count.as<int>(), p->bin_off.as<int>(),
-                                                                    p->sub_off.as<int>(), p->sub_bin.as<int>(), p->sub_first.as<int>(),
-                                                                    p->sub_count.as<int>());
-  COV3D_LAUNCHED("subproblem_kernel");
+  for (int m = 0; m < kSortModes; ++m)
+    if (modes >> m & 1) p->sets[m].valid = true;
   return COV3D_OK;
+}
+
+}  // namespace
+
+// Every buffer the sort of M points uses (a no-op when they are large enough already).
+int reserve_sort(cov3d_plan *p, int64_t M, SortMode mode) {
+  const int64_t nb = p->bins.nbins;
+  const int64_t max_subs = nb + M / p->max_sub + 1;
+  SortSet &ss = p->sets[mode];
+  COV3D_TRY(grow(ss.pt_bin, M * 4));
+  COV3D_TRY(grow(ss.pt_rank, M * 4));
+  COV3D_TRY(grow(ss.bin_count, (nb + 2) * 4));
+  COV3D_TRY(grow(ss.bin_off, (nb + 2) * 4));
+  COV3D_TRY(grow(ss.sub_off, (nb + 2) * 4));
+  COV3D_TRY(grow(ss.sorted, M * (int64_t)sizeof(SortedPoint)));
+  COV3D_TRY(grow(ss.sub_bin, max_subs * 4));
+  COV3D_TRY(grow(ss.sub_first, max_subs * 4));
+  COV3D_TRY(grow(ss.sub_count, max_subs * 4));
+  COV3D_TRY(grow(ss.nsub, 16));
+  return COV3D_OK;
+}
+
+// The plan's points have changed: the views that operators have used so far are sorted now (so a
+// captured call that reads one finds the new points in it), the others on their first use.  Inside
+// a stream capture the others are sorted too where their buffers are large enough already; where
+// not, a replay of that graph would change the points unseen, so such a view is sorted on every use.
+int new_points(cov3d_plan *p) {
+  for (SortSet &ss : p->sets) ss.valid = false;
+  const int64_t M = p->n_points;
+  if (M <= 0) return COV3D_OK;
+  if (M >= (int64_t)(1 << 30)) {
+    set_error("too many points (%lld); the limit is 2^30-1 per plan", (long long)M);
+    return COV3D_EINVAL;
+  }
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  COV3D_CUDA(cudaStreamIsCapturing(p->stream, &cap));
+  const bool capturing = cap != cudaStreamCaptureStatusNone;
+  unsigned modes = 0;
+  for (int m = 0; m < kSortModes; ++m) {
+    SortSet &ss = p->sets[m];
+    if (m != kSortFull && hermitian_mode(p) != m) continue;  // no operator reads it
+    if (capturing && !ss.used) {
+      const bool fits = ss.sorted.cap >= M * (int64_t)sizeof(SortedPoint) && ss.pt_rank.cap >= M * 4 &&
+                        (m == kSortFull || p->point_kind != kPointsRotations || p->rotc.cap >= p->n_images * 6 * 8);
+      if (fits) ss.used = true;
+      else ss.every_use = true;
+    }
+    if (ss.used) modes |= 1u << m;
+  }
+  return sort_points(p, modes);
+}
+
+int need_sorted(cov3d_plan *p, SortMode mode) {
+  SortSet &ss = p->sets[mode];
+  ss.used = true;
+  if (ss.valid && !ss.every_use) return COV3D_OK;
+  PhaseScope ps(p, kPhaseSort);
+  return sort_points(p, 1u << mode);
 }
 
 }  // namespace cov3d

@@ -37,6 +37,7 @@ struct SpreadParams {
   int64_t cs, chs;
   int shift;
   int max_sub;
+  int half;  // records of kSortHalf
 };
 
 // Prologue factor of im_backward: CTF multiply, Nyquist zeroing, scale (projection_funcs.py:385-399).
@@ -77,15 +78,16 @@ struct PointRec {
 struct StageSmem {
   long long *rowoff;  // T * T
   void *rec;          // max_sub * F2 record elements (float2, or float for scalar weights)
-  int *key, *pid;     // max_sub each
-  float *sc;          // max_sub
+  int *key;           // max_sub
+  unsigned *pid;      // max_sub: the record's id with kPairBit and kConjBit
+  float *sc, *scm;    // max_sub each: factors of the id and of its mirror pixel
   int *cnt, *off;     // kKeys, kKeys + 1
   int *coloff;        // T
   int *task;          // 1
 };
 
 __host__ __device__ constexpr size_t stage_bytes(int max_sub, int T, int F2, size_t esize) {
-  return (size_t)T * T * sizeof(long long) + (size_t)max_sub * (F2 * esize + 3 * sizeof(int)) +
+  return (size_t)T * T * sizeof(long long) + (size_t)max_sub * (F2 * esize + 4 * sizeof(int)) +
          (size_t)(2 * kKeys + 2 + T) * sizeof(int);
 }
 
@@ -94,9 +96,10 @@ __device__ __forceinline__ StageSmem carve(void *base, int max_sub, int T, int F
   s.rowoff = static_cast<long long *>(base);
   s.rec = s.rowoff + T * T;
   s.key = reinterpret_cast<int *>(static_cast<char *>(s.rec) + (size_t)max_sub * F2 * esize);
-  s.pid = s.key + max_sub;
+  s.pid = reinterpret_cast<unsigned *>(s.key + max_sub);
   s.sc = reinterpret_cast<float *>(s.pid + max_sub);
-  s.cnt = reinterpret_cast<int *>(s.sc + max_sub);
+  s.scm = s.sc + max_sub;
+  s.cnt = reinterpret_cast<int *>(s.scm + max_sub);
   s.off = s.cnt + kKeys;
   s.coloff = s.off + kKeys + 1;
   s.task = s.coloff + T;
@@ -128,7 +131,7 @@ __device__ __forceinline__ SubTile sub_tile(const SpreadParams &a, int sub) {
 __device__ __forceinline__ void put_weight(float2 *e, float x) { *e = make_float2(x, x); }
 __device__ __forceinline__ void put_weight(float *e, float x) { *e = x; }
 
-template <int KT, int W, int ROWS, typename E>
+template <int KT, int W, int ROWS, typename E, bool HALF>
 __device__ __forceinline__ void stage_subproblem(const SpreadParams &a, const StageSmem &s, const SubTile &st) {
   using Rec = PointRec<W, ROWS>;
   constexpr int T = Rec::T;
@@ -140,7 +143,7 @@ __device__ __forceinline__ void stage_subproblem(const SpreadParams &a, const St
   // sort keys and ranks
   for (int k = tid; k < st.cnt; k += blockDim.x) {
     const SortedPoint sp = a.pts[st.first + k];
-    int c0 = first_cell<KT, W>(sp.t0), c1 = first_cell<KT, W>(sp.t1);
+    int c0 = record_cell<KT, W, HALF>(sp.t0, a.g.frac), c1 = record_cell<KT, W, HALF>(sp.t1, a.g.frac);
     if (KT == COV3D_KERNEL_ES) {
       c0 = wrap1(c0, n);
       c1 = wrap1(c1, n);
@@ -177,9 +180,9 @@ __device__ __forceinline__ void stage_subproblem(const SpreadParams &a, const St
     const int kr = s.key[k];
     const int slot = s.off[kr & 255] + (kr >> 8);
     float w0[W], w1[W], w2[W];
-    int c0 = taps<KT, W>(sp.t0, a.k.beta, w0);
-    taps<KT, W>(sp.t1, a.k.beta, w1);
-    int c2 = taps<KT, W>(sp.t2, a.k.beta, w2);
+    int c0 = taps<KT, W, HALF>(sp.t0, a.g.frac, a.k.beta, w0);
+    taps<KT, W, HALF>(sp.t1, a.g.frac, a.k.beta, w1);
+    int c2 = taps<KT, W, HALF>(sp.t2, a.g.frac, a.k.beta, w2);
     if (KT == COV3D_KERNEL_ES) {
       c0 = wrap1(c0, n);
       c2 = wrap1(c2, n);
@@ -203,11 +206,12 @@ __device__ __forceinline__ void stage_subproblem(const SpreadParams &a, const St
       if (l2 + r >= 0 && l2 + r < T) put_weight(rec + Rec::W2 + l2 + r, w2[r]);
       put_weight(rec + Rec::W1 + r, w1[r]);
     }
-    const int id = sp_id(sp.idf);
+    const int id = sp_id<HALF>(sp.idf);
     float sc = (a.nyquist && sp_nyquist(sp.idf)) ? 0.0f : a.scale;
     sc *= ctf_factor(a.ctf, a.ctfc, a.g, id);
-    s.pid[slot] = id;
+    s.pid[slot] = sp.idf & ~kNyquistBit;
     s.sc[slot] = sc;
+    if (sp_pair<HALF>(sp.idf)) s.scm[slot] = a.scale * ctf_factor(a.ctf, a.ctfc, a.g, mirror_id(a.g, id));
   }
   // global offsets of the tile's rows (axes 0, 1) and columns (axis 2)
   for (int e = tid; e < T * T; e += blockDim.x) {
@@ -238,6 +242,25 @@ __device__ __forceinline__ void stage_subproblem(const SpreadParams &a, const St
     m2 = m2 >= n ? m2 - n : m2;
     s.coloff[e] = ok ? m2 : -1;
   }
+}
+
+// The scaled value of one channel of a staged record: src = values + channel * channel stride.  A
+// record of kSortHalf that stands for a pair of mirror pixels takes the sum of the one's value
+// and the conjugate of the other's, which has the same real part after the inverse transform.
+template <bool HALF>
+__device__ __forceinline__ float2 record_value(const SpreadParams &a, const StageSmem &s, int slot, const float2 *src) {
+  const unsigned pid = s.pid[slot];
+  const float sc = s.sc[slot];
+  const int id = sp_id<HALF>(pid);
+  const float2 x = __ldg(src + (int64_t)id * a.ips);
+  float2 v = make_float2(x.x * sc, sp_conj<HALF>(pid) ? -(x.y * sc) : x.y * sc);
+  if (sp_pair<HALF>(pid)) {
+    const float sm = s.scm[slot];
+    const float2 m = __ldg(src + (int64_t)mirror_id(a.g, id) * a.ips);
+    v.x = fmaf(m.x, sm, v.x);
+    v.y = fmaf(-m.y, sm, v.y);
+  }
+  return v;
 }
 
 // TwoSum (Knuth) on both lanes of a float2: s + d = s' + e exactly, e added to the error sum
@@ -271,7 +294,7 @@ struct SpreadLanes {
 // of one short FP32 sum per group.  The finished row goes to the global grid with one complex
 // atomic per cell and channel.  Warps take tasks from a shared counter.  The block needs no
 // shared-memory tile: its shared memory is the staged points only.
-template <int KT, int W, int CPL, bool COMP>
+template <int KT, int W, int CPL, bool COMP, bool HALF>
 __global__ void __launch_bounds__(kSpreadWarps * 32, W < 8 ? 2 : 1) spread_kernel(const SpreadParams a) {
   constexpr int T = SpreadLanes<W>::T;
   constexpr int G = SpreadLanes<W>::G;  // lane groups over channel pairs
@@ -285,7 +308,7 @@ __global__ void __launch_bounds__(kSpreadWarps * 32, W < 8 ? 2 : 1) spread_kerne
   const int sub = blockIdx.x;
   if (sub >= *a.nsub) return;
   const SubTile st = sub_tile(a, sub);
-  stage_subproblem<KT, W, 1, float2>(a, s, st);
+  stage_subproblem<KT, W, 1, float2, HALF>(a, s, st);
 
   const int tid = threadIdx.x, lane = tid & 31;
   const int g = lane / T, c = lane - (lane / T) * T;
@@ -297,11 +320,10 @@ __global__ void __launch_bounds__(kSpreadWarps * 32, W < 8 ? 2 : 1) spread_kerne
     // this group's scaled channel pairs, in sorted order
     for (int e = tid; e < st.cnt * NP; e += blockDim.x) {
       const int slot = e / NP, pp = p0 + (e - (e / NP) * NP);
-      const float sc = s.sc[slot];
-      const float2 *src = a.vals + (int64_t)s.pid[slot] * a.ips + (int64_t)(a.ch0 + 2 * pp) * a.ics;
-      const float2 v0 = 2 * pp < a.nch ? __ldg(src) : make_float2(0.f, 0.f);
-      const float2 v1 = 2 * pp + 1 < a.nch ? __ldg(src + a.ics) : make_float2(0.f, 0.f);
-      s_val[e] = make_float4(v0.x * sc, v0.y * sc, v1.x * sc, v1.y * sc);
+      const float2 *src = a.vals + (int64_t)(a.ch0 + 2 * pp) * a.ics;
+      const float2 v0 = 2 * pp < a.nch ? record_value<HALF>(a, s, slot, src) : make_float2(0.f, 0.f);
+      const float2 v1 = 2 * pp + 1 < a.nch ? record_value<HALF>(a, s, slot, src + a.ics) : make_float2(0.f, 0.f);
+      s_val[e] = make_float4(v0.x, v0.y, v1.x, v1.y);
     }
     if (tid == 0) *s.task = 0;
     __syncthreads();
@@ -417,7 +439,7 @@ __global__ void __launch_bounds__(kSpreadWarps * 32, W < 8 ? 2 : 1) spread_kerne
 // task's ranges are those of the corners l1 in [b - W + 1, b + ROWS - 1]; the summation (FP32
 // groups of kRowsFold ranges, TwoSum folds with COMP) and the atomics are those of
 // spread_kernel.
-template <int KT, int W, int CH, int ROWS, bool COMP>
+template <int KT, int W, int CH, int ROWS, bool COMP, bool HALF>
 __global__ void __launch_bounds__(kRowsWarps * 32, kRowsBlocks) spread_rows_kernel(const SpreadParams a) {
   constexpr int T = kBin + W - 1;
   static_assert(2 * T <= 32, "two lane halves of T columns per warp");
@@ -433,7 +455,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, kRowsBlocks) spread_rows_kern
   const int sub = blockIdx.x;
   if (sub >= *a.nsub) return;
   const SubTile st = sub_tile(a, sub);
-  stage_subproblem<KT, W, ROWS, float>(a, s, st);
+  stage_subproblem<KT, W, ROWS, float, HALF>(a, s, st);
 
   const int tid = threadIdx.x, lane = tid & 31;
   const int h = lane / T;
@@ -447,13 +469,8 @@ __global__ void __launch_bounds__(kRowsWarps * 32, kRowsBlocks) spread_rows_kern
     for (int e = tid; e < st.cnt * 2 * CH; e += blockDim.x) {
       const int slot = e / (2 * CH), r = e - slot * (2 * CH);
       const int hh = r / CH, ch = r - hh * CH;
-      const float sc = s.sc[slot];
-      float2 v = make_float2(0.f, 0.f);
-      if (p0 + r < a.nch) {
-        const float2 x = __ldg(a.vals + (int64_t)s.pid[slot] * a.ips + (int64_t)(a.ch0 + p0 + r) * a.ics);
-        v = make_float2(x.x * sc, x.y * sc);
-      }
-      s_val[slot * PS + hh * HS + ch] = v;
+      s_val[slot * PS + hh * HS + ch] = p0 + r < a.nch ? record_value<HALF>(a, s, slot, a.vals + (int64_t)(a.ch0 + p0 + r) * a.ics)
+                                                       : make_float2(0.f, 0.f);
     }
     if (tid == 0) *s.task = 0;
     __syncthreads();
@@ -572,7 +589,7 @@ int launch_spread_kernel(Kernel kernel, const char *name, size_t smem, const Spr
 // and wider ones take row-group tasks over two lane halves of kRowGroupCH channels (groups of
 // 2 * kRowGroupCH channels), otherwise row tasks with the (at most two, G >= 2) pairs spread
 // over the lane groups.
-template <int KT, int W, bool COMP>
+template <int KT, int W, bool COMP, bool HALF>
 int launch_wc(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
   constexpr int T = kBin + W - 1;
   constexpr int G = SpreadLanes<W>::G;
@@ -588,7 +605,7 @@ int launch_wc(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
       constexpr int CPL = 2;
       const size_t smem = (size_t)a.max_sub * G * CPL * sizeof(float4) +
                           stage_bytes(a.max_sub, T, PointRec<W, 1>::F2, sizeof(float2));
-      return launch_spread_kernel(spread_kernel<KT, W, CPL, COMP>, "spread_kernel", smem, a, max_blocks, st);
+      return launch_spread_kernel(spread_kernel<KT, W, CPL, COMP, HALF>, "spread_kernel", smem, a, max_blocks, st);
     }
   }
   if constexpr (W > 2) {
@@ -596,19 +613,25 @@ int launch_wc(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
       constexpr int PS = 2 * ((kRowGroupCH + 1) / 2 * 2);
       const size_t smem = (size_t)a.max_sub * PS * sizeof(float2) +
                           stage_bytes(a.max_sub, T, PointRec<W, kRows>::F2, sizeof(float));
-      return launch_spread_kernel(spread_rows_kernel<KT, W, kRowGroupCH, kRows, COMP>, "spread_rows_kernel", smem,
+      return launch_spread_kernel(spread_rows_kernel<KT, W, kRowGroupCH, kRows, COMP, HALF>, "spread_rows_kernel", smem,
                                   a, max_blocks, st, kRowsWarps);
     }
   }
   static_assert(2 * G >= 2, "at most two channel pairs spread over the lane groups");
   const size_t smem =
       (size_t)a.max_sub * G * sizeof(float4) + stage_bytes(a.max_sub, T, PointRec<W, 1>::F2, sizeof(float2));
-  return launch_spread_kernel(spread_kernel<KT, W, 1, COMP>, "spread_kernel", smem, a, max_blocks, st);
+  return launch_spread_kernel(spread_kernel<KT, W, 1, COMP, HALF>, "spread_kernel", smem, a, max_blocks, st);
 }
 
 template <int KT, int W>
 int launch_w(SpreadParams a, int nchan, bool comp, int64_t max_blocks, cudaStream_t st) {
-  return comp ? launch_wc<KT, W, true>(a, nchan, max_blocks, st) : launch_wc<KT, W, false>(a, nchan, max_blocks, st);
+  if constexpr (KT != COV3D_KERNEL_NEAREST) {
+    if (a.half)
+      return comp ? launch_wc<KT, W, true, true>(a, nchan, max_blocks, st)
+                  : launch_wc<KT, W, false, true>(a, nchan, max_blocks, st);
+  }
+  return comp ? launch_wc<KT, W, true, false>(a, nchan, max_blocks, st)
+              : launch_wc<KT, W, false, false>(a, nchan, max_blocks, st);
 }
 
 // Per-image adjoint (no sum over images): direct global atomics, one thread per point.
@@ -626,7 +649,7 @@ __global__ void spread_unagg_kernel(PointGeom g, KernelSpec k, int64_t M, const 
   float wt[3][W];
   int c0[3];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) c0[d] = taps<KT, W>(t[d], k.beta, wt[d]);
+  for (int d = 0; d < 3; ++d) c0[d] = taps<KT, W, false>(t[d], g.frac, k.beta, wt[d]);
   const float2 x = vals[id * ips];
   const float2 v = make_float2(x.x * sc, x.y * sc);
   float2 *out = grids + (id / g.P) * (int64_t)n * n * n;
@@ -654,20 +677,22 @@ __global__ void spread_unagg_kernel(PointGeom g, KernelSpec k, int64_t M, const 
 }  // namespace
 
 int launch_spread(cov3d_plan *p, const void *values, int64_t in_ps, int64_t in_cs, int nchan, const EpilogueArgs &e,
-                  void *grid, int64_t cell_stride, int64_t chan_stride, int shift) {
+                  void *grid, int64_t cell_stride, int64_t chan_stride, int shift, SortMode mode) {
   if (p->point_kind == kPointsNone || p->n_points == 0) {
     set_error("no points set");
     return COV3D_ESTATE;
   }
+  COV3D_TRY(need_sorted(p, mode));
+  const SortSet &ss = p->sets[mode];
   SpreadParams a{};
   a.g = make_geom(p);
   a.k = make_kernel(p);
   a.bins = p->bins;
-  a.pts = p->sorted.as<SortedPoint>();
-  a.sub_bin = p->sub_bin.as<int>();
-  a.sub_first = p->sub_first.as<int>();
-  a.sub_count = p->sub_count.as<int>();
-  a.nsub = p->nsub.as<int>();
+  a.pts = ss.sorted.as<SortedPoint>();
+  a.sub_bin = ss.sub_bin.as<int>();
+  a.sub_first = ss.sub_first.as<int>();
+  a.sub_count = ss.sub_count.as<int>();
+  a.nsub = ss.nsub.as<int>();
   a.vals = static_cast<const float2 *>(values);
   a.ips = in_ps;
   a.ics = in_cs;
@@ -680,6 +705,7 @@ int launch_spread(cov3d_plan *p, const void *values, int64_t in_ps, int64_t in_c
   a.chs = chan_stride;
   a.shift = shift;
   a.max_sub = p->max_sub;
+  a.half = mode == kSortHalf;
   if (p->bins.bs[0] != kBin || p->bins.bs[1] != kBin || p->bins.bs[2] != kBin) {
     set_error("spreading requires %d^3-cell bins", kBin);
     return COV3D_EINVAL;

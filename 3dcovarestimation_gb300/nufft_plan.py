@@ -214,7 +214,8 @@ class _Plan:
 
     def interp_native(self, grid, ctf=None, flags=0, scale=1.0):
         """Interpolation of a :meth:`fine_grid` result with the projection epilogue, written
-        point-major: returns (n_points, C) complex64."""
+        point-major: returns (n_points, C) complex64.  ``flags`` may hold ``_lib.GRID_HERMITIAN``
+        when the volumes were real."""
         C = grid.shape[0]
         out = torch.empty((self.n_points, C), dtype=torch.complex64, device=self.device)
         layout = _lib.GridLayout(order=_lib.GRID_FFT_NATIVE, cell_stride=1, chan_stride=self.n**3)
@@ -292,25 +293,29 @@ class _ProjectFn(torch.autograd.Function):
     def backward(ctx, g):
         if not ctx.needs_input_grad[0]:
             return None, None, None, None, None
-        grad = ctx.plan.backproject(g, ctx.ctf, ctx.flags, ctx.scale)
-        return (grad if ctx.complex_input else grad.real), None, None, None, None
+        if ctx.complex_input:
+            return ctx.plan.backproject(g, ctx.ctf, ctx.flags, ctx.scale), None, None, None, None
+        return ctx.plan.backproject(g, ctx.ctf, ctx.flags | _lib.REAL_OUTPUT, ctx.scale).real, None, None, None, None
 
 
 class _BackprojectFn(torch.autograd.Function):
-    """Exact adjoint with im_backward's prologue; backward is the projection."""
+    """Exact adjoint with im_backward's prologue, or with ``real`` its real part alone; backward is
+    the projection (of a real volume then)."""
 
     @staticmethod
-    def forward(ctx, values, plan, ctf, flags, scale):
+    def forward(ctx, values, plan, ctf, flags, scale, real=False):
         ctx.plan, ctx.ctf, ctx.flags, ctx.scale = plan, ctf, flags, scale
         ctx.complex_input = values.is_complex()
+        if real:
+            return plan.backproject(values, ctf, flags | _lib.REAL_OUTPUT, scale).real
         return plan.backproject(values, ctf, flags, scale)
 
     @staticmethod
     def backward(ctx, g):
         if not ctx.needs_input_grad[0]:
-            return None, None, None, None, None
+            return None, None, None, None, None, None
         grad = ctx.plan.project(g, ctx.ctf, ctx.flags, ctx.scale)
-        return (grad if ctx.complex_input else grad.real), None, None, None, None
+        return (grad if ctx.complex_input else grad.real), None, None, None, None, None
 
 
 class BaseNufftPlan(ABC):

@@ -144,9 +144,9 @@ def im_backward(image: torch.Tensor, plan: BaseNufftPlan, filters: Optional[torc
         return out.real if not fourier_domain else out
     if isinstance(plan, NufftPlan) and plan._plan is not None and im_fft.is_cuda:
         # the exact adjoint with the prologue (CTF, Nyquist zeroing, 1/L) fused into the spreading
-        back = _BackprojectFn.apply(im_fft.reshape(1, -1), plan._plan, filters, _lib.APPLY_NYQUIST, 1.0 / L)
-        back = back.to(plan.complex_dtype)
-        return back.real if not fourier_domain else back
+        back = _BackprojectFn.apply(im_fft.reshape(1, -1), plan._plan, filters, _lib.APPLY_NYQUIST, 1.0 / L,
+                                    not fourier_domain)
+        return back.to(plan.dtype if not fourier_domain else plan.complex_dtype)
     im_fft = im_fft.clone()
     if filters is not None:
         im_fft = im_fft * filters

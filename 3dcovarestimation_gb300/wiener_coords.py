@@ -120,7 +120,8 @@ class _EigenProjector:
             self.grid = p.fine_grid(self.vols)
         L = self.vols.shape[-1]
         ctf = None if filters is None else filters.reshape(p.n_images, -1)
-        out = p.interp_native(self.grid, ctf, _lib.APPLY_NYQUIST, 1.0 / L)
+        flags = _lib.APPLY_NYQUIST | (0 if self.vols.is_complex() else _lib.GRID_HERMITIAN)
+        out = p.interp_native(self.grid, ctf, flags, 1.0 / L)
         q = out.view(p.n_images, L * L, -1).permute(0, 2, 1).reshape(p.n_images, -1, L, L)
         return q if fourier_domain else centered_ifft2(q).real
 

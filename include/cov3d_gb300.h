@@ -79,6 +79,12 @@ typedef struct {
 #define COV3D_APPLY_CTF 2     /* multiply by a per-pixel real filter (B, L*L) */
 #define COV3D_APPLY_CTF_PARAMS 4 /* multiply by the CTF computed from per-image parameters: the d_ctf
                                     argument then holds (B, COV3D_CTF_NPARAMS) floats */
+/* cov3d_interp: the caller's grid is the transform of a real volume, G(-k) = conj G(k); one value is
+ * interpolated per pair of mirror pixels (k, -k) of an image, the other is its conjugate. */
+#define COV3D_GRID_HERMITIAN 8
+/* cov3d_backproject: only the real part of d_vol_out is defined (the caller drops the imaginary
+ * part); mirror pixels are spread together. */
+#define COV3D_REAL_OUTPUT 16
 /* CTF parameters per image, in order: pixel size (A), defocus u (A), defocus v (A), astigmatism
  * angle (degrees), voltage (kV), spherical aberration Cs (mm), amplitude contrast, phase shift
  * (degrees) -- the columns of the reference's ctf_params (source.py:157-172), which it hands to
