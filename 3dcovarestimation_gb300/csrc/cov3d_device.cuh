@@ -17,7 +17,9 @@ __device__ __forceinline__ int wrap1(int a, int n) { return a < 0 ? a + n : (a >
 __device__ __forceinline__ float wrap_pi(float x) {
   const float two_pi = 6.28318530717958647692f;
   float a = __fadd_rn(x, kPiF);
-  float q = floorf(__fdiv_rn(a, two_pi));
+  // floor(a / (2 pi)) without the division for the one turn that central slices make
+  float q = a >= 0.0f && a < two_pi ? 0.0f : a >= two_pi && a < 12.0f ? 1.0f : a < 0.0f && a > -6.0f ? -1.0f
+                                                                              : floorf(__fdiv_rn(a, two_pi));
   float r = __fsub_rn(a, __fmul_rn(q, two_pi));
   return __fsub_rn(r, kPiF);
 }
@@ -30,9 +32,10 @@ __device__ __forceinline__ float plane_coord(int i, const PointGeom &g) {
 }
 
 // Frequency (radians) of point `id` along volume axes 0, 1, 2.
-__device__ __forceinline__ void point_freq(const PointGeom &g, int64_t id, float w[3]) {
-  const int64_t b = id / g.P;
-  const int p = (int)(id - b * g.P);
+// (ids are below 2^30: 32-bit divisions)
+__device__ __forceinline__ void point_freq(const PointGeom &g, int id, float w[3]) {
+  const int64_t b = (unsigned)id / (unsigned)g.P;
+  const int p = id - (int)b * g.P;
   if (g.kind == kPointsExplicit) {
     const float *base = g.pts + b * 3 * (int64_t)g.P + p;
     w[0] = __ldg(base);
@@ -45,7 +48,7 @@ __device__ __forceinline__ void point_freq(const PointGeom &g, int64_t id, float
     }
   } else {
     const float *R = g.rot + b * 9;
-    const int row = p / g.Lp;
+    const int row = (unsigned)p / (unsigned)g.Lp;
     const int col = p - row * g.Lp;
     const float x = plane_coord(col, g);
     const float y = plane_coord(row, g);
@@ -67,7 +70,7 @@ __device__ __forceinline__ float freq_to_index(const PointGeom &g, float w) {
   return __fmul_rn(__fmul_rn(__fadd_rn(x, 1.0f), 0.5f), (float)(g.n - 1));
 }
 
-__device__ __forceinline__ void point_index(const PointGeom &g, int64_t id, float t[3]) {
+__device__ __forceinline__ void point_index(const PointGeom &g, int id, float t[3]) {
   float w[3];
   point_freq(g, id, w);
   t[0] = freq_to_index(g, w[0]);
@@ -87,14 +90,14 @@ constexpr long long kDeadCoef = -9223372036854775807LL - 1;
 // coefficients, wrapped to [-n/2, n/2).  Explicit points: w n / (2 pi) with the product's rounding
 // error carried along, wrapped when the kernel is periodic or the plan says so.
 template <int KT>
-__device__ __forceinline__ void point_index_fix(const PointGeom &g, int64_t id, int t[3]) {
+__device__ __forceinline__ void point_index_fix(const PointGeom &g, int id, int t[3]) {
   const int one = 1 << g.frac;
-  const int64_t b = id / g.P;
-  const int p = (int)(id - b * g.P);
+  const int64_t b = (unsigned)id / (unsigned)g.P;
+  const int p = id - (int)b * g.P;
   const int N = g.n << g.frac, c = (g.n / 2) << g.frac;
   if (g.kind == kPointsRotations) {
     const long long *A = g.rotc + b * 6;
-    const int row = p / g.Lp;
+    const int row = (unsigned)p / (unsigned)g.Lp;
     const int kx = p - row * g.Lp - g.Lp / 2, ky = row - g.Lp / 2;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -202,18 +205,18 @@ __device__ __forceinline__ bool sp_conj(unsigned idf) {
 // even-sized image); p itself at the centre.
 __device__ __forceinline__ int mirror_pixel(int p, int Lp) {
   if (Lp % 2 != 0) return Lp * Lp - 1 - p;
-  return (p < Lp || p % Lp == 0) ? -1 : Lp * (Lp + 1) - p;
+  return (p < Lp || (unsigned)p % (unsigned)Lp == 0) ? -1 : Lp * (Lp + 1) - p;
 }
 // id of the mirror pixel of a pair's id
 __device__ __forceinline__ int mirror_id(const PointGeom &g, int id) {
-  const int p = id % g.P;
+  const int p = (unsigned)id % (unsigned)g.P;
   return id + (g.Lp % 2 != 0 ? g.P - 1 : g.P + g.Lp) - 2 * p;
 }
 
-__device__ __forceinline__ bool on_nyquist(const PointGeom &g, int64_t id) {
+__device__ __forceinline__ bool on_nyquist(const PointGeom &g, int id) {
   if (g.Lp % 2 != 0) return false;
-  const int p = (int)(id % g.P);
-  return p < g.Lp || (p % g.Lp) == 0;
+  const int p = (unsigned)id % (unsigned)g.P;
+  return p < g.Lp || ((unsigned)p % (unsigned)g.Lp) == 0;
 }
 
 // First cell of the window of a record's index t, and the weight of its tap q (0 <= q < W).
@@ -221,11 +224,16 @@ template <int KT, int W, bool HALF>
 __device__ __forceinline__ int record_cell(float t, int frac) {
   return HALF ? first_cell_fix<KT, W>(__float_as_int(t), frac) : first_cell<KT, W>(t);
 }
+// Offset of a record's index t from cell c, in cells.
+template <bool HALF>
+__device__ __forceinline__ float record_offset(float t, int c, int frac) {
+  return HALF ? (float)(__float_as_int(t) - (c << frac)) * __int_as_float((127 - frac) << 23) : t - (float)c;
+}
 template <int KT, int W, bool HALF>
 __device__ __forceinline__ float record_weight(float t, int c0, int q, int frac, float beta) {
   if (KT == COV3D_KERNEL_NEAREST) return 1.0f;
   if (HALF) {  // the offset is exact
-    const float x = (float)(__float_as_int(t) - (c0 << frac)) * __int_as_float((127 - frac) << 23);
+    const float x = record_offset<true>(t, c0, frac);
     if (KT == COV3D_KERNEL_LINEAR) return q == 0 ? 1.0f - x : x;
     return es_weight<W>(x - (float)q, beta);
   }
@@ -275,12 +283,12 @@ __device__ __forceinline__ float ctf_eval(const CtfCoef &c, int ka, int kb) {
 }
 
 // The CTF factor of point id: the per-pixel array, or the per-image coefficients, or 1.
-__device__ __forceinline__ float ctf_factor(const float *ctf, const CtfCoef *ctfc, const PointGeom &g, int64_t id) {
+__device__ __forceinline__ float ctf_factor(const float *ctf, const CtfCoef *ctfc, const PointGeom &g, int id) {
   if (ctf) return __ldg(ctf + id);
   if (!ctfc) return 1.0f;
-  const int64_t b = id / g.P;
-  const int p = (int)(id - b * g.P);
-  const int row = p / g.Lp, col = p - (p / g.Lp) * g.Lp;
+  const int b = (unsigned)id / (unsigned)g.P;
+  const int p = id - b * g.P;
+  const int row = (unsigned)p / (unsigned)g.Lp, col = p - row * g.Lp;
   return ctf_eval(ctfc[b], row - g.Lp / 2, col - g.Lp / 2);
 }
 

@@ -189,28 +189,30 @@ __device__ __forceinline__ void line_dft(float2 *ex, const float2 *s_tw, int rol
 __device__ __forceinline__ int support_index(int t, int L, int n) { return t < L / 2 ? t : n - L + t; }
 __device__ __forceinline__ bool in_support(int s, int L, int n) { return s < L / 2 || s >= n - L / 2; }
 
-// Block sums of two doubles added to a and b (either may be null); every thread calls it.
-__device__ void block_add_pair(double x, double y, double *a, double *b) {
+// Block sums of two doubles (PAIR), or of x alone, added to a and b (b += 2 x without PAIR; either
+// may be null); every thread calls it.
+template <bool PAIR>
+__device__ void block_add(double x, double y, double *a, double *b) {
   __shared__ double sx[8], sy[8];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     x += __shfl_xor_sync(0xffffffffu, x, o);
-    y += __shfl_xor_sync(0xffffffffu, y, o);
+    if (PAIR) y += __shfl_xor_sync(0xffffffffu, y, o);
   }
   const int w = threadIdx.x >> 5;
   if ((threadIdx.x & 31) == 0) {
     sx[w] = x;
-    sy[w] = y;
+    if (PAIR) sy[w] = y;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     double tx = 0.0, ty = 0.0;
     for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
       tx += sx[i];
-      ty += sy[i];
+      if (PAIR) ty += sy[i];
     }
     if (a) atomicAdd(a, tx);
-    if (b) atomicAdd(b, ty);
+    if (b) atomicAdd(b, PAIR ? ty : 2.0 * tx);
   }
 }
 
@@ -324,7 +326,7 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
               im += (double)q.x * y.y - (double)q.y * y.x;
             }
           });
-      if (a.p) block_add_pair(re, im, a.dot, a.dot + 1);
+      if (a.p) block_add<true>(re, im, a.dot, a.dot + 1);
     } else {  // kUnpackRows
       const float es = a.logs ? expf(__ldg(a.logs + c)) : 1.0f;
       const float g01 = a.gc ? 1.0f / (__ldg(a.gc + j0) * __ldg(a.gc + j1)) : 1.0f;
@@ -372,7 +374,7 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
             }
             ax[(int64_t)k * nn] = y;
           });
-      if (a.fr) block_add_pair((double)part * a.coef, 2.0 * (double)part * a.coef, a.cost, a.glog + c);
+      if (a.fr) block_add<false>((double)part * a.coef, 0.0, a.cost, a.glog + c);
     } else {  // kAxisInv
       line_dft<N1, N2, true>(
           ex, s_tw, role, [&](int i) { return ax[(int64_t)i * nn]; },

@@ -77,7 +77,7 @@ __device__ __forceinline__ void count_full(const PointGeom &g, const Bins &bins,
   int bin = -1;
   if (valid) {
     float t[3];
-    point_index(g, id, t);
+    point_index(g, (int)id, t);
     bin = bin_of<KT, W>(g, bins, t);
   }
   const unsigned grp = __match_any_sync(0xffffffffu, bin);
@@ -116,13 +116,19 @@ __device__ __forceinline__ void fold_single(const PointGeom &g, bool periodic, H
   }
 }
 
-// The record of the pair whose first pixel has index ta and second tb; false when the two do not
-// mirror each other.
+// The record of the pair of pixels with ids `first` < `second`, the first at index ta; false, with the
+// second's index in tb, when the two do not mirror each other.
 template <int KT>
-__device__ __forceinline__ bool pair_record(const PointGeom &g, const int (&ta)[3], const int (&tb)[3],
+__device__ __forceinline__ bool pair_record(const PointGeom &g, const int (&ta)[3], int second, int (&tb)[3],
                                             HalfRecord &r) {
   const int c = (g.n / 2) << g.frac, N = g.n << g.frac, tol = 2 + (int)(1.5e-7f * (float)N);
   bool ok = true;
+  if (g.kind == kPointsRotations) {  // the second's is the mirrored first, up to a tie's rounding
+#pragma unroll
+    for (int d = 0; d < 3; ++d) tb[d] = ta[d] == kDeadIndex ? kDeadIndex : 2 * c - ta[d];
+  } else {
+    point_index_fix<KT>(g, second, tb);
+  }
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     ok = ok && ta[d] != kDeadIndex && tb[d] != kDeadIndex;
@@ -156,16 +162,15 @@ __device__ __forceinline__ void count_half(const PointGeom &g, const Bins &bins,
   int bin = -1;
   int64_t rec = id;
   if (id < M) {
-    const int p = (int)(id % g.P), m = mirror_pixel(p, g.Lp);
+    const int p = (unsigned)id % (unsigned)g.P, m = mirror_pixel(p, g.Lp);
     if (m < 0 || m >= p) {
       HalfRecord a;
-      point_index_fix<KT>(g, id, a.t);
+      point_index_fix<KT>(g, (int)id, a.t);
       bool pair = false;
       if (m > p) {
         const int64_t other = id + (m - p);
         HalfRecord b, r;
-        point_index_fix<KT>(g, other, b.t);
-        pair = pair_record<KT>(g, a.t, b.t, r);
+        pair = pair_record<KT>(g, a.t, (int)other, b.t, r);
         if (pair) {
           rec = r.swap ? other : id;
           v.pt_bin[r.swap ? id : other] = -1;
@@ -208,22 +213,23 @@ __device__ __forceinline__ void scatter_half(const PointGeom &g, int64_t M, cons
   const int bin = v.pt_bin[id];
   if (bin < 0) return;
   const int pos = v.off[bin] + v.pt_rank[id];
-  const int p = (int)(id % g.P), m = mirror_pixel(p, g.Lp);
+  const int p = (unsigned)id % (unsigned)g.P, m = mirror_pixel(p, g.Lp);
   HalfRecord a;
-  point_index_fix<KT>(g, id, a.t);
+  const bool second = m >= 0 && m < p;
+  point_index_fix<KT>(g, (int)id + (second ? m - p : 0), a.t);
   bool pair = false;
   if (m >= 0 && m != p) {
     HalfRecord b, r;
-    point_index_fix<KT>(g, id + (m - p), b.t);
-    pair = m > p ? pair_record<KT>(g, a.t, b.t, r) : pair_record<KT>(g, b.t, a.t, r);
+    pair = pair_record<KT>(g, a.t, (int)id + (second ? 0 : m - p), b.t, r);
     if (pair) a = r;
+    else if (second) a = b;
   }
   if (!pair) fold_single(g, KT == COV3D_KERNEL_ES, a);
   SortedPoint sp;
   sp.t0 = __int_as_float(a.t[0]);
   sp.t1 = __int_as_float(a.t[1]);
   sp.t2 = __int_as_float(a.t[2]);
-  sp.idf = (unsigned)id | a.flags | (on_nyquist(g, id) ? kNyquistBit : 0u);
+  sp.idf = (unsigned)id | a.flags | (on_nyquist(g, (int)id) ? kNyquistBit : 0u);
   v.sorted[pos] = sp;
 }
 
@@ -300,12 +306,12 @@ __device__ __forceinline__ void scatter_full(const PointGeom &g, int64_t M, cons
   if (id >= M) return;
   const int pos = v.off[v.pt_bin[id]] + v.pt_rank[id];
   float t[3];
-  point_index(g, id, t);
+  point_index(g, (int)id, t);
   SortedPoint sp;
   sp.t0 = t[0];
   sp.t1 = t[1];
   sp.t2 = t[2];
-  sp.idf = (unsigned)id | (on_nyquist(g, id) ? kNyquistBit : 0u);
+  sp.idf = (unsigned)id | (on_nyquist(g, (int)id) ? kNyquistBit : 0u);
   v.sorted[pos] = sp;
 }
 

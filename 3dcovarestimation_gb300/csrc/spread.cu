@@ -10,11 +10,6 @@ namespace {
 
 constexpr int kBin = 8;
 constexpr int kSpreadWarps = 16;
-// Row-group kernel: two blocks of 8 warps per SM (128 registers), so one block's staging
-// (sort, records, values) overlaps the other's tasks; one block of 16 warps measured 20.1
-// against 18.0 ms at the cov-SGD workload
-constexpr int kRowsWarps = 8;
-constexpr int kRowsBlocks = 2;
 
 struct SpreadParams {
   PointGeom g;
@@ -41,7 +36,7 @@ struct SpreadParams {
 };
 
 // Prologue factor of im_backward: CTF multiply, Nyquist zeroing, scale (projection_funcs.py:385-399).
-__device__ __forceinline__ float prologue(const PointGeom &g, int64_t id, const float *ctf, const CtfCoef *ctfc,
+__device__ __forceinline__ float prologue(const PointGeom &g, int id, const float *ctf, const CtfCoef *ctfc,
                                           int nyquist, float scale) {
   float sc = scale;
   if (nyquist && on_nyquist(g, id)) sc = 0.0f;
@@ -51,9 +46,6 @@ __device__ __forceinline__ float prologue(const PointGeom &g, int64_t id, const 
 constexpr int kLMin = -8;   // window corners relative to the bin lie in [kLMin, kLMin + 16)
 constexpr int kKeys = 256;  // sort key (l1 - kLMin) * 16 + (l0 - kLMin)
 constexpr int kFoldRanges = 3;  // window-corner rows l1 summed in FP32 between compensated folds
-// spread_rows_kernel: a task's W + ROWS - 1 = 8 ranges (w = 6) in two groups of four, two
-// compensated folds instead of three (16.3 against 16.6 ms per cov-SGD step)
-constexpr int kRowsFold = 4;
 
 // Per-point record staged once per block, in elements of float2 (each weight twice, the operand
 // of a packed multiply: spread_kernel) or float (each weight once, splatted in a register:
@@ -427,147 +419,298 @@ __global__ void __launch_bounds__(kSpreadWarps * 32, W < 8 ? 2 : 1) spread_kerne
   }
 }
 
-// Row-group tasks with the channels split over two lane halves, for many channels (the
-// covariance gradient's r eigenvolumes).  Stage 1 as in spread_kernel; the channel values of a
-// group of 2 * CH channels are staged per point as two 16-byte-aligned halves of CH.  A task is
-// ROWS consecutive tile rows of one plane: lane (h, c) owns tile column c of those rows for the
-// channels of half h (26 of 32 lanes at W = 6), so every point of the task's ranges costs a lane
-// CH values, ROWS + 2 weight loads and ROWS * CH packed multiply-adds, and a point is visited by
-// the tasks of its W planes and the row groups its W rows meet (W = 6, ROWS = 3: 16 on
-// average).  Shared memory returns per point and lane 40 bytes of values where lanes owning all
-// channels of one cell would take 80: the loads, not the multiply-adds, bound this kernel.  The
-// task's ranges are those of the corners l1 in [b - W + 1, b + ROWS - 1]; the summation (FP32
-// groups of kRowsFold ranges, TwoSum folds with COMP) and the atomics are those of
-// spread_kernel.
-template <int KT, int W, int CH, int ROWS, bool COMP, bool HALF>
-__global__ void __launch_bounds__(kRowsWarps * 32, kRowsBlocks) spread_rows_kernel(const SpreadParams a) {
-  constexpr int T = kBin + W - 1;
-  static_assert(2 * T <= 32, "two lane halves of T columns per warp");
-  constexpr int HS = (CH + 1) / 2 * 2;       // float2 per half of a point's values (even)
-  constexpr int PS = 2 * HS;                 // float2 of values per point
-  constexpr int RG = (T + ROWS - 1) / ROWS;  // row groups per plane
-  using Rec = PointRec<W, ROWS>;
-  constexpr int F2 = Rec::F2;
+// Spreading for the ES windows (W = 4 .. 8), any number of channels.  One block per subproblem (a bin
+// of 8^3 cells and at most max_sub of its points); the cells it can reach are a tile of T^3,
+// T = 8 + W - 1.  The block sorts its points by (axis-2 group, l1, l0), l the bin-local corner of
+// their window and a group GS = 9 - W neighbouring l2, so that the windows of a group lie in the
+// same 8 tile columns, and stages a record per point (weights) and its channel values.
+//
+// A warp task is NPL tile planes of one group, all T rows: lane (q, c) owns column c of the group,
+// part q % NQ of the channels (F floats) and part q / NQ of the planes (PP of them), with
+// acc[PP][T][F / 2] in registers.  The points whose windows meet the planes are for each l1 the
+// contiguous range l0 in [first plane - W + 1, last plane] of the sorted order, and with l1 a
+// compile-time constant in the unrolled loop their W rows are fixed registers: a point costs a lane
+// F values, W + PP + 1 weights and PP * W * F multiply-adds.
+//
+// What bounds it: latency at twelve warps per SM (issue 47 %, FP32 pipe 32 %, shared wavefronts
+// 17 % of their peaks on the B = 256 capture).  At the covariance step's 10 channels, W = 6, a visit
+// is some 50 instructions and a point has 3.5 of them.  Its predecessor, lanes owning all 13 tile
+// columns of three rows of one plane, had 16 visits and 2.2x the multiply-adds.  Measured on the step at L = 128, B = 1024, r = 10: 8.6 -> 5.3 ms, of which staging
+// (sort, weights, gathered values) about 2.0, the flush 0.9; one channel at W = 7, 512 images of
+// 128^2: 6.2 -> 1.2 ms.
+//
+// Each cell's sum is plain FP32 over the points of one group of one subproblem (some 30 terms at
+// one point per cell, a third of what the predecessor summed before its first TwoSum fold; two or
+// three partial sums folded by TwoSum round to the float sum of the partials), and the partial sums
+// meet in FP32 global atomics, so `compensated` changes nothing here.
+template <int W>
+struct TileGroups {
+  static constexpr int T = kBin + W - 1;
+  static constexpr int GS = 9 - W;                   // l2 values per group
+  static constexpr int NG = (kBin + GS - 1) / GS;    // groups
+  __device__ static constexpr int base(int g) {      // first tile column of the group's eight
+    return g * GS < T - 8 ? g * GS : T - 8;
+  }
+};
+
+// per block, two blocks per SM (168 registers); 5 or 4 warps measured 5.8 and 6.8 ms against 5.3 (a
+// unrolled point loop is slower too: the ranges hold some ten points), 7 spill
+constexpr int kTileWarps = 6;
+
+// A point's record in floats: the W axis-1 weights twice each (operands of packed multiplies), the
+// axis-2 weights of the group's 8 columns, the axis-0 weights of up to 16 planes; a stride that keeps
+// 16-byte stores of consecutive records free of bank conflicts (4 modulo 8 words).
+template <int W>
+struct TileRec {
+  static constexpr int W2 = (2 * W + 3) / 4 * 4;
+  static constexpr int W0 = W2 + 8;
+  static constexpr int STRIDE = W <= 6 ? 36 : 44;
+  static_assert(W0 + 16 <= STRIDE, "plane weights");
+};
+
+template <int F>
+struct TileVals {  // floats of a channel part's values, padded to 16 bytes where loads are
+  static constexpr int STRIDE = F <= 2 ? F : (F + 3) / 4 * 4;
+};
+
+template <int W, int F>
+__host__ __device__ constexpr size_t tile_point_bytes(int NQ) {
+  return (TileRec<W>::STRIDE + NQ * TileVals<F>::STRIDE + 5) * 4;  // ... key, id, mirror id, two factors
+}
+__host__ __device__ constexpr size_t tile_fixed_bytes(int T, int NG) {
+  return (size_t)T * T * sizeof(long long) + (size_t)(2 * NG * 64 + 1 + T + 2) * sizeof(int);
+}
+
+// The points of corner row l1 = L1 .. 7 added to the lane's cells
+template <int W, int F, int NQ, int PP, int L1>
+struct TileRows {
+  template <typename Range>
+  __device__ __forceinline__ static void run(const Range &range, const float *recs, const float *vals, int cp, int col,
+                                             int plane, float2 (&acc)[PP][TileGroups<W>::T][F / 2]) {
+    using Rec = TileRec<W>;
+    int i, iend;
+    range(L1, i, iend);
+    const float *rec = recs + i * Rec::STRIDE;
+    const float *vp = vals + (i * NQ + cp) * TileVals<F>::STRIDE;
+#pragma unroll 1
+    for (; i < iend; ++i, rec += Rec::STRIDE, vp += NQ * TileVals<F>::STRIDE) {
+      const float w2 = rec[Rec::W2 + col];
+      float w0[PP];
+      if constexpr (PP == 2) {
+        const float2 x = *reinterpret_cast<const float2 *>(rec + Rec::W0 + plane);
+        w0[0] = x.x;
+        w0[1] = x.y;
+      } else {
+        w0[0] = rec[Rec::W0 + plane];
+      }
+      float2 w1[W];
+#pragma unroll
+      for (int j = 0; j + 1 < W; j += 2) {
+        const float4 x = *reinterpret_cast<const float4 *>(rec + 2 * j);
+        w1[j] = make_float2(x.x, x.y);
+        w1[j + 1] = make_float2(x.z, x.w);
+      }
+      if constexpr (W & 1) w1[W - 1] = *reinterpret_cast<const float2 *>(rec + 2 * (W - 1));
+      float2 v[F / 2];
+#pragma unroll
+      for (int f = 0; f + 1 < F / 2; f += 2) {
+        const float4 x = *reinterpret_cast<const float4 *>(vp + 2 * f);
+        v[f] = make_float2(x.x, x.y);
+        v[f + 1] = make_float2(x.z, x.w);
+      }
+      if constexpr ((F / 2) & 1) v[F / 2 - 1] = *reinterpret_cast<const float2 *>(vp + F - 2);
+#pragma unroll
+      for (int k = 0; k < PP; ++k) {
+        const float w02 = w0[k] * w2;
+        const float2 ww = make_float2(w02, w02);
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+          const float2 w = __fmul2_rn(ww, w1[j]);
+#pragma unroll
+          for (int f = 0; f < F / 2; ++f) acc[k][L1 + j][f] = __ffma2_rn(w, v[f], acc[k][L1 + j][f]);
+        }
+      }
+    }
+    if constexpr (L1 + 1 < kBin) TileRows<W, F, NQ, PP, L1 + 1>::run(range, recs, vals, cp, col, plane, acc);
+  }
+};
+
+// F / 2 channels per lane in NQ parts: 2 x 5 channels per pass, or one part of 5, 2 or 1.
+template <int W, int F, int NQ, int PP, bool HALF>
+__global__ void __launch_bounds__(kTileWarps * 32, 2) spread_tile_kernel(const SpreadParams a) {
+  constexpr int KT = COV3D_KERNEL_ES;
+  using G = TileGroups<W>;
+  using Rec = TileRec<W>;
+  constexpr int VS = TileVals<F>::STRIDE;
+  constexpr int T = G::T, NG = G::NG, NK = NG * 64;
+  constexpr int CH = NQ * F / 2;                 // channels per pass
+  constexpr int NPL = PP * (4 / NQ);             // planes per task
+  constexpr int PGS = (T + NPL - 1) / NPL;       // plane groups
+  static_assert(PGS * NPL <= 16, "plane weights of a record");
   extern __shared__ float4 smem4[];
-  float2 *s_val = reinterpret_cast<float2 *>(smem4);  // max_sub * PS
-  const StageSmem s = carve(s_val + a.max_sub * PS, a.max_sub, T, F2, sizeof(float));
-  const float *recs = static_cast<const float *>(s.rec);  // weights once each (scalar records)
+  float *recs = reinterpret_cast<float *>(smem4);                // max_sub * record stride
+  float *vals = recs + (size_t)a.max_sub * Rec::STRIDE;          // max_sub * NQ * VS
+  int *s_key = reinterpret_cast<int *>(vals + (size_t)a.max_sub * NQ * VS);
+  int *s_id = s_key + a.max_sub, *s_mid = s_id + a.max_sub;      // ids; mirror ids or -1
+  float *s_sc = reinterpret_cast<float *>(s_mid + a.max_sub), *s_scm = s_sc + a.max_sub;
+  long long *s_row = reinterpret_cast<long long *>((reinterpret_cast<uintptr_t>(s_scm + a.max_sub) + 7) & ~(uintptr_t)7);
+  int *s_cnt = reinterpret_cast<int *>(s_row + T * T), *s_off = s_cnt + NK, *s_col = s_off + NK + 1;
+  int *s_task = s_col + T;
   const int sub = blockIdx.x;
   if (sub >= *a.nsub) return;
   const SubTile st = sub_tile(a, sub);
-  stage_subproblem<KT, W, ROWS, float, HALF>(a, s, st);
+  const int n = a.g.n, tid = threadIdx.x, lane = tid & 31;
 
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int h = lane / T;
-  const bool lane_live = h < 2;
-  const int hv = lane_live ? h : 0;             // idle lanes read half 0 ...
-  const int c = lane_live ? lane - h * T : T;   // ... and the zero column weight
-  const float *w2c = recs + Rec::W2 + c;        // this lane's column weight, record 0
-  for (int p0 = 0; p0 < a.nch; p0 += 2 * CH) {  // channel groups of 2 * CH
-    __syncthreads();
-    // this group's scaled channel values, in sorted order: half hh holds p0 + hh * CH + ch
-    for (int e = tid; e < st.cnt * 2 * CH; e += blockDim.x) {
-      const int slot = e / (2 * CH), r = e - slot * (2 * CH);
-      const int hh = r / CH, ch = r - hh * CH;
-      s_val[slot * PS + hh * HS + ch] = p0 + r < a.nch ? record_value<HALF>(a, s, slot, a.vals + (int64_t)(a.ch0 + p0 + r) * a.ics)
-                                                       : make_float2(0.f, 0.f);
+  for (int e = tid; e < NK; e += blockDim.x) s_cnt[e] = 0;
+  __syncthreads();
+  auto corner = [&](float t, int ts) {  // bin-local window corner, 0 .. 7
+    return min(max(wrap1(record_cell<KT, W, HALF>(t, a.g.frac), n) - ts, 0), kBin - 1);
+  };
+  for (int k = tid; k < st.cnt; k += blockDim.x) {
+    const SortedPoint sp = a.pts[st.first + k];
+    const int key = (corner(sp.t2, st.ts2) / G::GS) * 64 + corner(sp.t1, st.ts1) * 8 + corner(sp.t0, st.ts0);
+    s_key[k] = key | (atomicAdd(s_cnt + key, 1) << 9);
+  }
+  __syncthreads();
+  if (tid < 32) {  // exclusive scan of the counters by one warp
+    int v[NK / 32], sum = 0;
+#pragma unroll
+    for (int u = 0; u < NK / 32; ++u) {
+      v[u] = s_cnt[tid * (NK / 32) + u];
+      sum += v[u];
     }
-    if (tid == 0) *s.task = 0;
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (tid >= o) incl += t;
+    }
+    int base = incl - sum;
+#pragma unroll
+    for (int u = 0; u < NK / 32; ++u) {
+      s_off[tid * (NK / 32) + u] = base;
+      base += v[u];
+    }
+    if (tid == 31) s_off[NK] = incl;
+  }
+  // global offsets of the tile's rows (axes 0, 1) and columns (axis 2), periodic
+  for (int e = tid; e < T * T; e += blockDim.x) {
+    const int ra = e / T, rb = e - (e / T) * T;
+    const int m0 = wrap1(wrap1(st.ts0 + ra, n) + a.shift, n), m1 = wrap1(wrap1(st.ts1 + rb, n) + a.shift, n);
+    s_row[e] = ((int64_t)m0 * n + m1) * n;
+  }
+  for (int e = tid; e < T; e += blockDim.x) s_col[e] = wrap1(wrap1(st.ts2 + e, n) + a.shift, n);
+  __syncthreads();
+  // records (a weight is zero outside its window), ids and prologue factors in sorted order
+  for (int k = tid; k < st.cnt; k += blockDim.x) {
+    const SortedPoint sp = a.pts[st.first + k];
+    const int kr = s_key[k];
+    const int slot = s_off[kr & 511] + (kr >> 9);
+    const int c0 = record_cell<KT, W, HALF>(sp.t0, a.g.frac), c1 = record_cell<KT, W, HALF>(sp.t1, a.g.frac),
+              c2 = record_cell<KT, W, HALF>(sp.t2, a.g.frac);
+    const int l0 = wrap1(c0, n) - st.ts0, l2 = wrap1(c2, n) - st.ts2;
+    const float x0 = record_offset<HALF>(sp.t0, c0, a.g.frac) + (float)l0;
+    const float x1 = record_offset<HALF>(sp.t1, c1, a.g.frac);
+    const float x2 = record_offset<HALF>(sp.t2, c2, a.g.frac) + (float)(l2 - G::base((kr & 511) >> 6));
+    float4 *rec = reinterpret_cast<float4 *>(recs + slot * Rec::STRIDE);
+    float w[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = j < W ? es_weight<W>(x1 - (float)j, a.k.beta) : 0.0f;
+#pragma unroll
+    for (int u = 0; u < Rec::W2 / 4; ++u) rec[u] = make_float4(w[2 * u], w[2 * u], w[2 * u + 1], w[2 * u + 1]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = es_weight<W>(x2 - (float)j, a.k.beta);
+    rec[Rec::W2 / 4] = make_float4(w[0], w[1], w[2], w[3]);
+    rec[Rec::W2 / 4 + 1] = make_float4(w[4], w[5], w[6], w[7]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = 4 * u + j < T ? es_weight<W>(x0 - (float)(4 * u + j), a.k.beta) : 0.0f;
+      rec[Rec::W0 / 4 + u] = make_float4(w[0], w[1], w[2], w[3]);
+    }
+    const int id = sp_id<HALF>(sp.idf);
+    const float sc = ((a.nyquist && sp_nyquist(sp.idf)) ? 0.0f : a.scale) * ctf_factor(a.ctf, a.ctfc, a.g, id);
+    const int mid = sp_pair<HALF>(sp.idf) ? mirror_id(a.g, id) : -1;
+    s_id[slot] = sp_conj<HALF>(sp.idf) ? ~id : id;  // a negative id: the value's conjugate
+    s_mid[slot] = mid;
+    s_sc[slot] = sc;
+    if (mid >= 0) s_scm[slot] = a.scale * ctf_factor(a.ctf, a.ctfc, a.g, mid);
+  }
+
+  const int q = lane >> 3, c = lane & 7;
+  const int cp = q % NQ;  // channel part
+  for (int p0 = 0; p0 < a.nch; p0 += CH) {
+    __syncthreads();
+    // this pass's channel values in sorted order.  A record of kSortHalf that stands for a pair of
+    // mirror pixels takes the sum of the one's value and the conjugate of the other's, which has
+    // the same real part after the inverse transform.
+    for (int e = tid; e < st.cnt * CH; e += blockDim.x) {
+      const int slot = e / CH, ch = e - slot * CH;
+      float2 v = make_float2(0.f, 0.f);
+      if (p0 + ch < a.nch) {
+        const float2 *src = a.vals + (int64_t)(a.ch0 + p0 + ch) * a.ics;
+        int id = s_id[slot];
+        const bool conj = HALF && id < 0;
+        if (conj) id = ~id;
+        const float2 x = __ldg(src + (int64_t)id * a.ips);
+        const float sc = s_sc[slot];
+        v = make_float2(x.x * sc, conj ? -(x.y * sc) : x.y * sc);
+        if (HALF) {
+          const int mid = s_mid[slot];
+          if (mid >= 0) {
+            const float2 m = __ldg(src + (int64_t)mid * a.ips);
+            const float sm = s_scm[slot];
+            v.x = fmaf(m.x, sm, v.x);
+            v.y = fmaf(-m.y, sm, v.y);
+          }
+        }
+      }
+      const int part = ch / (F / 2);
+      *reinterpret_cast<float2 *>(vals + (slot * NQ + part) * VS + 2 * (ch - part * (F / 2))) = v;
+    }
+    if (tid == 0) *s_task = 0;
     __syncthreads();
 
     for (;;) {
       int task = 0;
-      if (lane == 0) task = atomicAdd(s.task, 1);
+      if (lane == 0) task = atomicAdd(s_task, 1);
       task = __shfl_sync(0xffffffffu, task, 0);
-      if (task >= T * RG) break;
-      const int pa = task / RG;
-      const int rb = (task - pa * RG) * ROWS;  // first row of the task
-      const int b0lo = max(pa - W + 1 - kLMin, 0), b0hi = min(pa - kLMin, 15);
-      float2 hi[ROWS][CH], lo[ROWS][CH];  // cell sums and their TwoSum errors
+      if (task >= PGS * NG) break;
+      const int g = task / PGS, pa0 = (task - g * PGS) * NPL;
+      const int plane = pa0 + (q / NQ) * PP;  // this lane's first plane
+      const int lo = max(pa0 - W + 1, 0), hi = min(pa0 + NPL - 1, kBin - 1);
+      if (lo > hi || s_off[g * 64] == s_off[g * 64 + 64]) continue;
+      float2 acc[PP][T][F / 2];
 #pragma unroll
-      for (int q = 0; q < ROWS; ++q)
+      for (int k = 0; k < PP; ++k)
 #pragma unroll
-        for (int ch = 0; ch < CH; ++ch) hi[q][ch] = lo[q][ch] = make_float2(0.f, 0.f);
-      // the points of the task's ranges l1g, l1g - 1, ... (kRowsFold of them) multiplied into acc
-      // (packed FP32, FFMA2: the same rounding as fmaf); true if any range held a point
-      auto group = [&](const int l1g, float2(&acc)[ROWS][CH]) {
-        bool got = false;
-#pragma unroll  // 128 registers, 8 bytes of spills; not unrolled (126, none): 16.5 against 16.3 ms
-        for (int sr = 0; sr < kRowsFold; ++sr) {
-          const int l1 = l1g - sr;
-          const int b1 = l1 - kLMin;
-          if (l1 <= rb - W || b1 < 0 || b1 > 15 || b0lo > b0hi) continue;
-          const int ibeg = s.off[(b1 << 4) | b0lo], iend = s.off[((b1 << 4) | b0hi) + 1];
-          got |= ibeg < iend;
-          const int k1 = Rec::W1 + rb - l1;  // row rb + q reads the axis-1 weight k1 + q
-#pragma unroll 2  // two points' loads in flight (17.5 against 18.0 ms; four: no further gain)
-          for (int i = ibeg; i < iend; ++i) {
-            const float *rec = recs + i * F2;
-            const float w02 = rec[pa] * w2c[i * F2];
-            float2 w[ROWS];
+        for (int r = 0; r < T; ++r)
 #pragma unroll
-            for (int q = 0; q < ROWS; ++q) {
-              const float wq = w02 * rec[k1 + q];
-              w[q] = make_float2(wq, wq);
-            }
-            const float2 *vp = s_val + i * PS + hv * HS;
-            float2 v[CH];
-#pragma unroll
-            for (int ch = 0; ch + 1 < CH; ch += 2) {
-              const float4 x = *reinterpret_cast<const float4 *>(vp + ch);
-              v[ch] = make_float2(x.x, x.y);
-              v[ch + 1] = make_float2(x.z, x.w);
-            }
-            if (CH & 1) v[CH - 1] = vp[CH - 1];
-#pragma unroll
-            for (int q = 0; q < ROWS; ++q)
-#pragma unroll
-              for (int ch = 0; ch < CH; ++ch) acc[q][ch] = __ffma2_rn(w[q], v[ch], acc[q][ch]);
-          }
-        }
-        return got;
+          for (int f = 0; f < F / 2; ++f) acc[k][r][f] = make_float2(0.f, 0.f);
+      auto range = [&](int l1, int &i, int &iend) {
+        i = s_off[g * 64 + l1 * 8 + lo];
+        iend = s_off[g * 64 + l1 * 8 + hi + 1];
       };
-      // the first group straight into the cell sums (its fold, TwoSum(0, sum), is (sum, 0)
-      // exactly), each later one summed apart and folded in
-      bool any = group(rb + ROWS - 1, hi);
-      for (int l1g = rb + ROWS - 1 - kRowsFold; l1g > rb - W; l1g -= kRowsFold) {
-        float2 part[ROWS][CH];
-#pragma unroll
-        for (int q = 0; q < ROWS; ++q)
-#pragma unroll
-          for (int ch = 0; ch < CH; ++ch) part[q][ch] = make_float2(0.f, 0.f);
-        if (!group(l1g, part)) continue;
-        any = true;
-#pragma unroll
-        for (int q = 0; q < ROWS; ++q)
-#pragma unroll
-          for (int ch = 0; ch < CH; ++ch) {
-            if (!COMP) hi[q][ch] = __fadd2_rn(hi[q][ch], part[q][ch]);
-            else two_sum2(hi[q][ch], lo[q][ch], part[q][ch]);
-          }
-      }
+      TileRows<W, F, NQ, PP, 0>::run(range, recs, vals, cp, c, plane, acc);
       // the finished cells go to the global grid
-      if (!any || !lane_live) continue;
-      const int co = s.coloff[c];
-      if (co < 0) continue;
+      const int co = s_col[G::base(g) + c];
+      const int ch0 = p0 + cp * (F / 2);  // this lane's first channel
 #pragma unroll
-      for (int q = 0; q < ROWS; ++q) {
-        if (rb + q >= T) break;
-        const long long ro = s.rowoff[pa * T + rb + q];
-        if (ro < 0) continue;
-        float2 *dst = a.grid + (ro + co) * a.cs + (int64_t)(a.ch0 + p0 + hv * CH) * a.chs;
+      for (int k = 0; k < PP; ++k) {
+        if (plane + k >= T) break;
 #pragma unroll
-        for (int ch = 0; ch < CH; ++ch) {
-          const float2 x = COMP ? __fadd2_rn(hi[q][ch], lo[q][ch]) : hi[q][ch];
-          if (p0 + hv * CH + ch < a.nch && (x.x != 0.0f || x.y != 0.0f)) atomicAdd(dst + ch * a.chs, x);
+        for (int r = 0; r < T; ++r) {
+          float2 *dst = a.grid + (s_row[(plane + k) * T + r] + co) * a.cs + (int64_t)(a.ch0 + ch0) * a.chs;
+#pragma unroll
+          for (int f = 0; f < F / 2; ++f) {
+            const float2 x = acc[k][r][f];
+            if (ch0 + f < a.nch && (x.x != 0.0f || x.y != 0.0f)) atomicAdd(dst + f * a.chs, x);
+          }
         }
       }
     }
   }
 }
-
-constexpr int kRowGroupCH = 5;  // channels per lane half (row-group tasks)
-constexpr int kRows = 3;        // tile rows per lane (row-group tasks; 2 measured 12 % slower)
 
 template <typename Kernel>
 int launch_spread_kernel(Kernel kernel, const char *name, size_t smem, const SpreadParams &a, int64_t max_blocks,
@@ -585,9 +728,8 @@ int launch_spread_kernel(Kernel kernel, const char *name, size_t smem, const Spr
 }
 
 // One launch for all channels: the block sorts and stages its points once.  With three or more
-// channel pairs, narrow windows (W <= 2) take row tasks with two channel pairs per lane group
-// and wider ones take row-group tasks over two lane halves of kRowGroupCH channels (groups of
-// 2 * kRowGroupCH channels), otherwise row tasks with the (at most two, G >= 2) pairs spread
+// channel pairs a lane group takes two pairs of a row task (bilinear step: 4.6 against 7.4 ms with
+// tasks of three rows over two lane halves), otherwise the (at most two, G >= 2) pairs are spread
 // over the lane groups.
 template <int KT, int W, bool COMP, bool HALF>
 int launch_wc(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
@@ -596,26 +738,11 @@ int launch_wc(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
   a.ch0 = 0;
   a.nch = nchan;
   const int npairs = (nchan + 1) / 2;
-  if constexpr (W <= 2) {
-    // narrow windows: one-row tasks with two pairs per lane group (G * 2 pairs per channel group),
-    // small registers and shared memory, two blocks per SM; the row-group kernel's three-row
-    // tasks multiply by zero for all but two of a lane's columns (bilinear step: 4.6 against
-    // 7.4 ms)
-    if (npairs >= 3) {
-      constexpr int CPL = 2;
-      const size_t smem = (size_t)a.max_sub * G * CPL * sizeof(float4) +
-                          stage_bytes(a.max_sub, T, PointRec<W, 1>::F2, sizeof(float2));
-      return launch_spread_kernel(spread_kernel<KT, W, CPL, COMP, HALF>, "spread_kernel", smem, a, max_blocks, st);
-    }
-  }
-  if constexpr (W > 2) {
-    if (npairs >= 3) {
-      constexpr int PS = 2 * ((kRowGroupCH + 1) / 2 * 2);
-      const size_t smem = (size_t)a.max_sub * PS * sizeof(float2) +
-                          stage_bytes(a.max_sub, T, PointRec<W, kRows>::F2, sizeof(float));
-      return launch_spread_kernel(spread_rows_kernel<KT, W, kRowGroupCH, kRows, COMP, HALF>, "spread_rows_kernel", smem,
-                                  a, max_blocks, st, kRowsWarps);
-    }
+  if (npairs >= 3) {
+    constexpr int CPL = 2;
+    const size_t smem = (size_t)a.max_sub * G * CPL * sizeof(float4) +
+                        stage_bytes(a.max_sub, T, PointRec<W, 1>::F2, sizeof(float2));
+    return launch_spread_kernel(spread_kernel<KT, W, CPL, COMP, HALF>, "spread_kernel", smem, a, max_blocks, st);
   }
   static_assert(2 * G >= 2, "at most two channel pairs spread over the lane groups");
   const size_t smem =
@@ -623,15 +750,45 @@ int launch_wc(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
   return launch_spread_kernel(spread_kernel<KT, W, 1, COMP, HALF>, "spread_kernel", smem, a, max_blocks, st);
 }
 
+template <int W, int F, int NQ, int PP, bool HALF>
+int launch_tile(const SpreadParams &a, int64_t max_blocks, cudaStream_t st) {
+  const size_t smem = (size_t)a.max_sub * tile_point_bytes<W, F>(NQ) + 8 +
+                      tile_fixed_bytes(TileGroups<W>::T, TileGroups<W>::NG);
+  return launch_spread_kernel(spread_tile_kernel<W, F, NQ, PP, HALF>, "spread_tile_kernel", smem, a, max_blocks, st,
+                              kTileWarps);
+}
+
+// Passes of ten channels in one launch, then the rest in the layout that holds it.
+template <int W, bool HALF>
+int launch_tile_channels(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
+  const int rest = nchan % 10, whole = rest > 5 ? nchan : nchan - rest;
+  if (whole > 0) {
+    a.ch0 = 0;
+    a.nch = whole;
+    COV3D_TRY((launch_tile<W, 10, 2, 1, HALF>(a, max_blocks, st)));
+  }
+  a.ch0 = whole;
+  a.nch = nchan - whole;
+  if (a.nch >= 3) return launch_tile<W, 10, 1, 1, HALF>(a, max_blocks, st);
+  if (a.nch == 2) return launch_tile<W, 4, 1, 1, HALF>(a, max_blocks, st);
+  if (a.nch == 1) return launch_tile<W, 2, 1, 2, HALF>(a, max_blocks, st);
+  return COV3D_OK;
+}
+
 template <int KT, int W>
 int launch_w(SpreadParams a, int nchan, bool comp, int64_t max_blocks, cudaStream_t st) {
-  if constexpr (KT != COV3D_KERNEL_NEAREST) {
-    if (a.half)
-      return comp ? launch_wc<KT, W, true, true>(a, nchan, max_blocks, st)
-                  : launch_wc<KT, W, false, true>(a, nchan, max_blocks, st);
+  if constexpr (KT == COV3D_KERNEL_ES) {
+    return a.half ? launch_tile_channels<W, true>(a, nchan, max_blocks, st)
+                  : launch_tile_channels<W, false>(a, nchan, max_blocks, st);
+  } else {
+    if constexpr (KT != COV3D_KERNEL_NEAREST) {
+      if (a.half)
+        return comp ? launch_wc<KT, W, true, true>(a, nchan, max_blocks, st)
+                    : launch_wc<KT, W, false, true>(a, nchan, max_blocks, st);
+    }
+    return comp ? launch_wc<KT, W, true, false>(a, nchan, max_blocks, st)
+                : launch_wc<KT, W, false, false>(a, nchan, max_blocks, st);
   }
-  return comp ? launch_wc<KT, W, true, false>(a, nchan, max_blocks, st)
-              : launch_wc<KT, W, false, false>(a, nchan, max_blocks, st);
 }
 
 // Per-image adjoint (no sum over images): direct global atomics, one thread per point.
@@ -639,8 +796,9 @@ template <int KT, int W>
 __global__ void spread_unagg_kernel(PointGeom g, KernelSpec k, int64_t M, const float2 *__restrict__ vals,
                                     int64_t ips, const float *ctf, const CtfCoef *ctfc, int nyquist, float scale,
                                     float2 *grids) {
-  const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= M) return;
+  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid >= M) return;
+  const int id = (int)gid;
   const float sc = prologue(g, id, ctf, ctfc, nyquist, scale);
   if (sc == 0.0f) return;
   const int n = g.n;
@@ -650,7 +808,7 @@ __global__ void spread_unagg_kernel(PointGeom g, KernelSpec k, int64_t M, const 
   int c0[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) c0[d] = taps<KT, W, false>(t[d], g.frac, k.beta, wt[d]);
-  const float2 x = vals[id * ips];
+  const float2 x = vals[(int64_t)id * ips];
   const float2 v = make_float2(x.x * sc, x.y * sc);
   float2 *out = grids + (id / g.P) * (int64_t)n * n * n;
   for (int i0 = 0; i0 < W; ++i0) {
