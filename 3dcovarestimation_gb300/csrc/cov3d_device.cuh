@@ -253,6 +253,19 @@ __device__ __forceinline__ int taps(float t, int frac, float beta, float *wt) {
   return c0;
 }
 
+// Groups of neighbouring window corners along axis 2 for the ES windows (W = 4 .. 8): the windows of
+// the GS = 9 - W corners of a group lie in the same eight columns of a bin's tile (8 + W - 1 cells
+// per axis).
+template <int W>
+struct TileGroups {
+  static constexpr int T = 8 + W - 1;
+  static constexpr int GS = 9 - W;           // corners per group
+  static constexpr int NG = (8 + GS - 1) / GS;
+  __device__ static constexpr int base(int g) {  // first tile column of the group's eight
+    return g * GS < T - 8 ? g * GS : T - 8;
+  }
+};
+
 // CTF at pixel offsets (ka, kb) (row, column) from the image centre: sqrt(1 - w^2) sin(gamma) -
 // w cos(gamma) with gamma = c0 K + c1 D + c2 X + d K^2 - ps (see CtfCoef).  gamma reaches a few
 // hundred radians at high frequency, so its large terms are formed in double-float arithmetic

@@ -98,15 +98,19 @@ void release(DevBuf &b);
 // of the inverse transform is kept, do half the work (points_sort.cu, half_point).
 enum SortMode { kSortFull = 0, kSortHalf = 1, kSortModes = 2 };
 
-// One sorted view of the plan's points: records in bin order and the subproblem table.
+// One sorted view of the plan's points: records in bin order and the subproblem table, in one
+// allocation (reserve_sort).
+struct SortedPoint;
 struct SortSet {
-  DevBuf bin_count;     // int (nbins + 1), last = dead points
-  DevBuf bin_off;       // int (nbins + 2)
-  DevBuf sub_off;       // int (nbins + 1)
-  DevBuf pt_bin, pt_rank;  // int (M), scratch of the sort
-  DevBuf sorted;        // SortedPoint (M)
-  DevBuf sub_bin, sub_first, sub_count;  // int (max subproblems)
-  DevBuf nsub;          // int scalar
+  DevBuf mem;
+  int64_t cap = -1;     // points it has room for
+  int *bin_count = nullptr;  // (nbins + 1), last = dead points
+  int *bin_off = nullptr;    // (nbins + 2)
+  int *sub_off = nullptr;    // (nbins + 1)
+  int *pt_bin = nullptr, *pt_rank = nullptr;  // (M), scratch of the sort
+  SortedPoint *sorted = nullptr;              // (M)
+  int *sub_bin = nullptr, *sub_first = nullptr, *sub_count = nullptr;  // (max subproblems)
+  int *nsub = nullptr;  // scalar
   bool used = false;    // some operator has asked for it: sorted with every new point set
   bool valid = false;   // holds the current points
   bool every_use = false;  // points may change by the replay of a graph that does not sort this view
@@ -204,7 +208,7 @@ inline bool prunable(const cov3d_plan *p) { return p->L % 2 == 0 && p->n >= p->L
 
 // points_sort.cu
 int new_points(cov3d_plan *p);
-int need_sorted(cov3d_plan *p, SortMode mode);
+int need_sorted(cov3d_plan *p, unsigned modes);
 int reserve_sort(cov3d_plan *p, int64_t M, SortMode mode);
 // The records an operator uses on a grid (or volume) it knows to be Hermitian (real): half of them
 // where the plan's kernel and point count allow.

@@ -672,6 +672,7 @@ int covar_cost_grad(cov3d_plan *p, const cov3d_cost_args *a, double *h_cost, dou
     set_error("noise_var must be positive");
     return COV3D_EINVAL;
   }
+  COV3D_TRY(need_sorted(p, 1u << kSortFull | 1u << hermitian_mode(p)));  // interpolation | spreading
   const int B = (int)p->n_images;
   const int L = p->L;
   const int P = L * L;

@@ -373,11 +373,7 @@ int cov3d_plan_destroy(cov3d_plan *p) {
   DevBuf *bufs[] = {&p->gc1d, &p->pts, &p->rot, &p->rotc, &p->fine, &p->fine2, &p->q,
                     &p->small, &p->acc, &p->cgw, &p->xbf, &p->gsum, &p->fftw, &p->ctfc, &p->lsw};
   for (DevBuf *b : bufs) release(*b);
-  for (SortSet &ss : p->sets) {
-    DevBuf *sb[] = {&ss.pt_bin, &ss.pt_rank, &ss.bin_count, &ss.bin_off, &ss.sub_off, &ss.sorted, &ss.sub_bin, &ss.sub_first, &ss.sub_count,
-                    &ss.nsub};
-    for (DevBuf *b : sb) release(*b);
-  }
+  for (SortSet &ss : p->sets) release(ss.mem);
   release_blas(p);
   if (p->h_acc) cudaFreeHost(p->h_acc);
   if (p->ev_pool) {

@@ -372,9 +372,9 @@ int sort_points(cov3d_plan *p, unsigned modes) {
     COV3D_TRY(reserve_sort(p, M, (SortMode)m));
     SortSet &ss = p->sets[m];
     half = half || m == kSortHalf;
-    views.v[nv++] = SortView{m == kSortHalf, ss.bin_count.as<int>(), ss.bin_off.as<int>(), ss.sub_off.as<int>(),
-                             ss.nsub.as<int>(), ss.pt_bin.as<int>(), ss.pt_rank.as<int>(), ss.sorted.as<SortedPoint>(),
-                             ss.sub_bin.as<int>(), ss.sub_first.as<int>(), ss.sub_count.as<int>()};
+    views.v[nv++] = SortView{m == kSortHalf, ss.bin_count, ss.bin_off, ss.sub_off,
+                             ss.nsub, ss.pt_bin, ss.pt_rank, ss.sorted,
+                             ss.sub_bin, ss.sub_first, ss.sub_count};
   }
   if (nv == 0) return COV3D_OK;
   long long *rotc = nullptr;
@@ -423,21 +423,34 @@ int sort_points(cov3d_plan *p, unsigned modes) {
 
 }  // namespace
 
-// Every buffer the sort of M points uses (a no-op when they are large enough already).
+// Room for a sort of M points in a view (a no-op when there is enough already).
 int reserve_sort(cov3d_plan *p, int64_t M, SortMode mode) {
+  SortSet &ss = p->sets[mode];
+  if (M <= ss.cap) return COV3D_OK;
   const int64_t nb = p->bins.nbins;
   const int64_t max_subs = nb + M / p->max_sub + 1;
-  SortSet &ss = p->sets[mode];
-  COV3D_TRY(grow(ss.pt_bin, M * 4));
-  COV3D_TRY(grow(ss.pt_rank, M * 4));
-  COV3D_TRY(grow(ss.bin_count, (nb + 2) * 4));
-  COV3D_TRY(grow(ss.bin_off, (nb + 2) * 4));
-  COV3D_TRY(grow(ss.sub_off, (nb + 2) * 4));
-  COV3D_TRY(grow(ss.sorted, M * (int64_t)sizeof(SortedPoint)));
-  COV3D_TRY(grow(ss.sub_bin, max_subs * 4));
-  COV3D_TRY(grow(ss.sub_first, max_subs * 4));
-  COV3D_TRY(grow(ss.sub_count, max_subs * 4));
-  COV3D_TRY(grow(ss.nsub, 16));
+  auto align = [](int64_t bytes) { return (bytes + 255) & ~int64_t(255); };
+  const int64_t bins = align((nb + 2) * 4), pts = align(M * 4), subs = align(max_subs * 4);
+  ss.cap = -1;
+  ss.valid = false;
+  COV3D_TRY(grow(ss.mem, 3 * bins + 2 * pts + align(M * (int64_t)sizeof(SortedPoint)) + 3 * subs + 256));
+  char *m = ss.mem.as<char>();
+  auto take = [&](int64_t bytes) {
+    char *q = m;
+    m += bytes;
+    return q;
+  };
+  ss.bin_count = reinterpret_cast<int *>(take(bins));
+  ss.bin_off = reinterpret_cast<int *>(take(bins));
+  ss.sub_off = reinterpret_cast<int *>(take(bins));
+  ss.pt_bin = reinterpret_cast<int *>(take(pts));
+  ss.pt_rank = reinterpret_cast<int *>(take(pts));
+  ss.sorted = reinterpret_cast<SortedPoint *>(take(align(M * (int64_t)sizeof(SortedPoint))));
+  ss.sub_bin = reinterpret_cast<int *>(take(subs));
+  ss.sub_first = reinterpret_cast<int *>(take(subs));
+  ss.sub_count = reinterpret_cast<int *>(take(subs));
+  ss.nsub = reinterpret_cast<int *>(take(256));
+  ss.cap = M;
   return COV3D_OK;
 }
 
@@ -461,7 +474,7 @@ int new_points(cov3d_plan *p) {
     SortSet &ss = p->sets[m];
     if (m != kSortFull && hermitian_mode(p) != m) continue;  // no operator reads it
     if (capturing && !ss.used) {
-      const bool fits = ss.sorted.cap >= M * (int64_t)sizeof(SortedPoint) && ss.pt_rank.cap >= M * 4 &&
+      const bool fits = ss.cap >= M &&
                         (m == kSortFull || p->point_kind != kPointsRotations || p->rotc.cap >= p->n_images * 6 * 8);
       if (fits) ss.used = true;
       else ss.every_use = true;
@@ -471,12 +484,19 @@ int new_points(cov3d_plan *p) {
   return sort_points(p, modes);
 }
 
-int need_sorted(cov3d_plan *p, SortMode mode) {
-  SortSet &ss = p->sets[mode];
-  ss.used = true;
-  if (ss.valid && !ss.every_use) return COV3D_OK;
+// The views in `modes` (bits 1 << SortMode) hold the current points, sorted in one launch sequence
+// where they do not yet.
+int need_sorted(cov3d_plan *p, unsigned modes) {
+  unsigned todo = 0;
+  for (int m = 0; m < kSortModes; ++m) {
+    if (!(modes >> m & 1)) continue;
+    SortSet &ss = p->sets[m];
+    ss.used = true;
+    if (!ss.valid || ss.every_use) todo |= 1u << m;
+  }
+  if (!todo) return COV3D_OK;
   PhaseScope ps(p, kPhaseSort);
-  return sort_points(p, 1u << mode);
+  return sort_points(p, todo);
 }
 
 }  // namespace cov3d

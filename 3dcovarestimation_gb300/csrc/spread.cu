@@ -443,16 +443,6 @@ __global__ void __launch_bounds__(kSpreadWarps * 32, W < 8 ? 2 : 1) spread_kerne
 // one point per cell, a third of what the predecessor summed before its first TwoSum fold; two or
 // three partial sums folded by TwoSum round to the float sum of the partials), and the partial sums
 // meet in FP32 global atomics, so `compensated` changes nothing here.
-template <int W>
-struct TileGroups {
-  static constexpr int T = kBin + W - 1;
-  static constexpr int GS = 9 - W;                   // l2 values per group
-  static constexpr int NG = (kBin + GS - 1) / GS;    // groups
-  __device__ static constexpr int base(int g) {      // first tile column of the group's eight
-    return g * GS < T - 8 ? g * GS : T - 8;
-  }
-};
-
 // per block, two blocks per SM (168 registers); 5 or 4 warps measured 5.8 and 6.8 ms against 5.3 (a
 // unrolled point loop is slower too: the ranges hold some ten points), 7 spill
 constexpr int kTileWarps = 6;
@@ -840,17 +830,17 @@ int launch_spread(cov3d_plan *p, const void *values, int64_t in_ps, int64_t in_c
     set_error("no points set");
     return COV3D_ESTATE;
   }
-  COV3D_TRY(need_sorted(p, mode));
+  COV3D_TRY(need_sorted(p, 1u << mode));
   const SortSet &ss = p->sets[mode];
   SpreadParams a{};
   a.g = make_geom(p);
   a.k = make_kernel(p);
   a.bins = p->bins;
-  a.pts = ss.sorted.as<SortedPoint>();
-  a.sub_bin = ss.sub_bin.as<int>();
-  a.sub_first = ss.sub_first.as<int>();
-  a.sub_count = ss.sub_count.as<int>();
-  a.nsub = ss.nsub.as<int>();
+  a.pts = ss.sorted;
+  a.sub_bin = ss.sub_bin;
+  a.sub_first = ss.sub_first;
+  a.sub_count = ss.sub_count;
+  a.nsub = ss.nsub;
   a.vals = static_cast<const float2 *>(values);
   a.ips = in_ps;
   a.ics = in_cs;
