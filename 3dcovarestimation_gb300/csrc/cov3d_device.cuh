@@ -305,6 +305,45 @@ __device__ __forceinline__ float ctf_factor(const float *ctf, const CtfCoef *ctf
   return ctf_eval(ctfc[b], row - g.Lp / 2, col - g.Lp / 2);
 }
 
+// Sums of products of floats in a float pair (about 46 bits: the products' rounding errors and those
+// of the leading sum are carried along): a thread's few terms and a warp's partial sums of the CG's
+// inner products before they are added in FP64, whose pipe (two operations per clock and SM) took
+// most of the kernels that formed every term there.
+struct FloatPair {
+  float h = 0.0f, l = 0.0f;
+  __device__ __forceinline__ void add(float x) {  // TwoSum
+    const float s = __fadd_rn(h, x), b = __fsub_rn(s, h);
+    l = __fadd_rn(l, __fadd_rn(__fsub_rn(h, __fsub_rn(s, b)), __fsub_rn(x, b)));
+    h = s;
+  }
+  __device__ __forceinline__ void add_product(float a, float b) {
+    const float p = __fmul_rn(a, b);
+    const float e = __fmaf_rn(a, b, -p);
+    add(p);
+    l = __fadd_rn(l, e);
+  }
+  __device__ __forceinline__ double warp_sum() {  // every lane
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float xh = __shfl_xor_sync(0xffffffffu, h, o), xl = __shfl_xor_sync(0xffffffffu, l, o);
+      add(xh);
+      l = __fadd_rn(l, xl);
+    }
+    return (double)h + (double)l;
+  }
+};
+
+// The next iteration of the CG begins: its direction is formed, the sums of its inner products start.
+__device__ __forceinline__ void roll_scalars(CgState *st) {
+  st->rz = st->rz_new;
+  st->rr = st->rr_new;
+  st->rz_new = 0.0;
+  st->rr_new = 0.0;
+  st->pap[0] = 0.0;
+  st->pap[1] = 0.0;
+  st->running += 1;
+}
+
 // Index maps of the fine grid (FFT-native storage: frequency / voxel offset k at k mod n).
 // centered index of storage index s on a grid of size m (fftshift)
 __device__ __forceinline__ int native_to_centered(int s, int m) {

@@ -31,8 +31,6 @@ int check_cufft(cufftResult r, const char *what);
 #define COV3D_CUDA(expr) COV3D_TRY(::cov3d::check_cuda((expr), #expr))
 // Counts one kernel launch of this library and checks the launch error.
 int launched(const char *name);
-// adds n kernel launches to the library's count (each replay of a captured CUDA graph)
-void count_launches(long long n);
 #define COV3D_LAUNCHED(name) COV3D_TRY(::cov3d::launched(name))
 
 // ----------------------------------------------------------------------------- geometry
@@ -192,6 +190,20 @@ int get_fft_planes(cov3d_plan *p, cufftHandle *out);
 int get_fft_axis0(cov3d_plan *p, cufftHandle *out);
 int fft2(cufftHandle h, const float2 *in, float2 *out, int dir);
 
+// The mean CG's scalars, in device memory (mean_cg.cu).
+struct CgState {
+  double rz;      // <r, z> of the previous iteration (z = r without a preconditioner)
+  double rr;      // <r, r>
+  double b2;      // <b, b>
+  double pap[2];  // <p, A p>, complex
+  double rz_new;
+  double rr_new;
+  int done;       // 1 converged, 2 reached maxiter, 3 not finite
+  int iters;      // loop index at which the loop stopped (the reference's num_iter)
+  int running;    // current loop index
+  unsigned ticket;
+};
+
 // line_fft.cu: hand-written line DFTs of the fine grid.  `stop` points at a done flag (kernels
 // return once it is nonzero) or is null.
 bool axis0_fused_size(int n);
@@ -200,7 +212,8 @@ int ensure_twiddles(cov3d_plan *p, int n);
 int launch_axis0_diag(cov3d_plan *p, float2 *g, const float *diag, int L, int n, int divide, float scale,
                       const int *stop);
 int cg_operator_lines(cov3d_plan *p, const float2 *in, float2 *fine, float2 *out, const float2 *dotp,
-                      const float *diag, int divide, const int *stop, const int *stop_last, double *dot);
+                      const float *diag, int divide, const int *stop, const int *stop_last, double *dot,
+                      const float2 *z = nullptr, float2 *pdir = nullptr, CgState *st = nullptr);
 int step_forward_lines(cov3d_plan *p, const float *vec, const float *logs, const float *gc, int r, float2 *stage,
                        float2 *grid, const float *fr, int64_t fr_stride, double coef, double *cost, double *glog);
 int step_inverse_lines(cov3d_plan *p, float2 *grad_grid, const float *logs, const float *gc, int r, float *gvec);

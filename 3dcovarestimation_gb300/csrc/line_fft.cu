@@ -189,30 +189,38 @@ __device__ __forceinline__ void line_dft(float2 *ex, const float2 *s_tw, int rol
 __device__ __forceinline__ int support_index(int t, int L, int n) { return t < L / 2 ? t : n - L + t; }
 __device__ __forceinline__ bool in_support(int s, int L, int n) { return s < L / 2 || s >= n - L / 2; }
 
-// Block sums of two doubles (PAIR), or of x alone, added to a and b (b += 2 x without PAIR; either
-// may be null); every thread calls it.
-template <bool PAIR>
-__device__ void block_add(double x, double y, double *a, double *b) {
-  __shared__ double sx[8], sy[8];
+// Block sum of x added to a, and twice it to b (may be null); every thread calls it.
+__device__ void block_add_twice(double x, double *a, double *b) {
+  __shared__ double sx[8];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (PAIR) y += __shfl_xor_sync(0xffffffffu, y, o);
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  if ((threadIdx.x & 31) == 0) sx[threadIdx.x >> 5] = x;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += sx[i];
+    atomicAdd(a, t);
+    if (b) atomicAdd(b, 2.0 * t);
   }
-  const int w = threadIdx.x >> 5;
+}
+
+// Block sums of two float pairs added to a and b; every thread calls it.
+__device__ void block_add_pairs(FloatPair x, FloatPair y, double *a, double *b) {
+  __shared__ double sx[8], sy[8];
+  const double wx = x.warp_sum(), wy = y.warp_sum();
   if ((threadIdx.x & 31) == 0) {
-    sx[w] = x;
-    if (PAIR) sy[w] = y;
+    sx[threadIdx.x >> 5] = wx;
+    sy[threadIdx.x >> 5] = wy;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     double tx = 0.0, ty = 0.0;
     for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
       tx += sx[i];
-      if (PAIR) ty += sy[i];
+      ty += sy[i];
     }
-    if (a) atomicAdd(a, tx);
-    if (b) atomicAdd(b, PAIR ? ty : 2.0 * tx);
+    atomicAdd(a, tx);
+    atomicAdd(b, ty);
   }
 }
 
@@ -222,9 +230,11 @@ __device__ void block_add(double x, double y, double *a, double *b) {
 // axis 1) or n^2 (axis 0) put adjacent lines on adjacent lanes.  Pruning: only support planes
 // and rows of the zero-padded volume are transformed, and each kernel writes exactly what the
 // next one reads, so no grid is ever zeroed.
-//   kRowFwd    CG: the volume row zero-padded (pad fused), forward along axis 2, whole row out
+//   kRowFwd    CG: the volume row zero-padded (pad fused), forward along axis 2, whole row out; with
+//              z, the row is the new search direction p = z + (rz_new / rz) p, which it also stores
 //   kPackRows  step: eigenvector row * exp(log_sqrt) / grid correction, zero-padded, forward
-//   kColFwd    forward along axis 1 over the support entries of a support plane, whole column out
+//   kColFwd    forward along axis 1 over the support entries of a support plane, whole column out; in
+//              the CG one thread also rolls the iteration's scalars (after kRowFwd has used them)
 //   kColInv    inverse along axis 1, support entries out
 //   kRowInv    CG: inverse along axis 2, the L support entries / n^3 to the volume (crop fused),
 //              <p, out> accumulated
@@ -244,6 +254,9 @@ struct LineArgs {
   float2 *g;         // fine grid, channel stride cs
   int64_t cs;
   const float2 *vol;  // kRowFwd: L^3 input
+  const float2 *z;    // kRowFwd: preconditioned residual, or null
+  float2 *pdir;       // kRowFwd: search direction, updated
+  CgState *st;        // kRowFwd, kColFwd: scalars, or null
   float2 *out;        // kRowInv: L^3 output
   const float2 *p;    // kRowInv: <p, out> operand or null
   double *dot;        // kRowInv: <p, out> (2 doubles)
@@ -291,9 +304,24 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
     float2 *row = g + ((int64_t)voxel_store(j0, L, n) * n + voxel_store(j1, L, n)) * n;
     const int64_t vrow = ((int64_t)j0 * L + j1) * L;  // voxel row in the L^3 volume
     if (KIND == kRowFwd) {
-      const float2 *src = a.vol + vrow;
+      const float2 *src = (a.z ? a.z : a.vol) + vrow;
+      float2 *pd = a.pdir + vrow;
+      const float beta = a.z ? (float)(a.st->rz_new / a.st->rz) : 0.0f;
       line_dft<N1, N2, false>(
-          ex, s_tw, role, [&](int i) { const int j = pad_voxel(i, L, n); return j < 0 ? zero : src[j]; },
+          ex, s_tw, role,
+          [&](int i) {
+            const int j = pad_voxel(i, L, n);
+            if (j < 0) return zero;
+            float2 v = src[j];
+            if (a.z) {
+              if (beta != 0.0f) {  // (the first direction is z: p holds nothing yet)
+                const float2 q = pd[j];
+                v = make_float2(v.x + beta * q.x, v.y + beta * q.y);
+              }
+              pd[j] = v;
+            }
+            return v;
+          },
           [&](int k, float2 v) { row[k] = v; });
     } else if (KIND == kPackRows) {
       const float *src = a.vec + c * L3 + vrow;
@@ -312,7 +340,7 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
       float2 *dst = a.out + vrow;
       const float2 *pr = a.p ? a.p + vrow : nullptr;
       const float inv = 1.0f / ((float)n * (float)n * (float)n);
-      double re = 0.0, im = 0.0;
+      FloatPair re, im;
       line_dft<N1, N2, true>(
           ex, s_tw, role, [&](int i) { return row[i]; },
           [&](int k, float2 v) {
@@ -322,11 +350,13 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
             dst[j] = y;
             if (pr) {  // conj(p) * y
               const float2 q = pr[j];
-              re += (double)q.x * y.x + (double)q.y * y.y;
-              im += (double)q.x * y.y - (double)q.y * y.x;
+              re.add_product(q.x, y.x);
+              re.add_product(q.y, y.y);
+              im.add_product(q.x, y.y);
+              im.add_product(-q.y, y.x);
             }
           });
-      if (a.p) block_add<true>(re, im, a.dot, a.dot + 1);
+      if (a.p) block_add_pairs(re, im, a.dot, a.dot + 1);
     } else {  // kUnpackRows
       const float es = a.logs ? expf(__ldg(a.logs + c)) : 1.0f;
       const float g01 = a.gc ? 1.0f / (__ldg(a.gc + j0) * __ldg(a.gc + j1)) : 1.0f;
@@ -345,6 +375,7 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
     const int t0 = (int)(line / n), s2 = (int)(line - (int64_t)(line / n) * n);
     float2 *col = g + (int64_t)support_index(t0, L, n) * nn + s2;  // entry s1 at col[s1 * n]
     if (KIND == kColFwd) {
+      if (a.st && blockIdx.x == 0 && threadIdx.x == 0) roll_scalars(a.st);
       line_dft<N1, N2, false>(
           ex, s_tw, role, [&](int i) { return in_support(i, L, n) ? col[(int64_t)i * n] : zero; },
           [&](int k, float2 v) { col[(int64_t)k * n] = v; });
@@ -374,7 +405,7 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
             }
             ax[(int64_t)k * nn] = y;
           });
-      if (a.fr) block_add<false>((double)part * a.coef, 0.0, a.cost, a.glog + c);
+      if (a.fr) block_add_twice((double)part * a.coef, a.cost, a.glog + c);
     } else {  // kAxisInv
       line_dft<N1, N2, true>(
           ex, s_tw, role, [&](int i) { return ax[(int64_t)i * nn]; },
@@ -479,13 +510,17 @@ bool line_transforms_apply(const cov3d_plan *p) {
 }
 
 int cg_operator_lines(cov3d_plan *p, const float2 *in, float2 *fine, float2 *out, const float2 *dotp,
-                      const float *diag, int divide, const int *stop, const int *stop_last, double *dot) {
+                      const float *diag, int divide, const int *stop, const int *stop_last, double *dot, const float2 *z,
+                      float2 *pdir, CgState *st) {
   LineArgs a;
   COV3D_TRY(line_args(p, a));
   a.stop = stop;
   a.g = fine;
   a.cs = 0;
   a.vol = in;
+  a.z = z;
+  a.pdir = pdir;
+  a.st = st;
   a.out = out;
   a.p = dotp;
   a.dot = dot;

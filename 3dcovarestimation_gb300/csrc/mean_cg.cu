@@ -10,14 +10,16 @@
 // DFTs of line_fft.cu (pad, crop and the diagonal fused in); at n = 64 the axis-0 transform
 // and the diagonal are fused between cuFFT 2D transforms of the support planes; otherwise it is
 // pad + cuFFT + diagonal multiply + inverse cuFFT + crop.  The vector updates
-// are fused with their inner products, which accumulate in FP64.  The iteration scalars stay
-// in device memory and a convergence flag turns every kernel of later iterations into a
-// no-op, so the host polls the flag only every few iterations.  Preconditioners:
+// are fused with their inner products: exact products summed in float pairs within a warp, FP64 from
+// there.  The iteration scalars stay in device memory and a convergence flag turns every kernel of
+// later iterations into a no-op, so the host polls the flag only every few iterations, one poll
+// behind the launches.  Preconditioners:
 //   1: M r = crop(ifft3(fft3(pad r) / lhs))              (the Fourier-diagonal solve on the
 //      fine grid, the operator the reference uses for its starting point, mean.py:238-239)
 //   2: M r = ifft3_L(fft3_L(r) / s)                      (a Fourier diagonal on the L^3 grid:
 //      the optimal circulant approximation of A from cov3d_circulant_symbol, or a learned s)
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "cov3d_device.cuh"
@@ -25,19 +27,6 @@
 namespace cov3d {
 
 namespace {
-
-struct CgState {
-  double rz;      // <r, z>  (z = r without a preconditioner)
-  double rr;      // <r, r>
-  double b2;      // <b, b>
-  double pap[2];  // <p, A p>, complex
-  double rz_new;
-  double rr_new;
-  int done;       // 1 converged, 2 reached maxiter
-  int iters;      // loop index at which the loop stopped (the reference's num_iter)
-  int running;    // current loop index
-  int pad;
-};
 
 inline unsigned nb(int64_t n) { return (unsigned)((n + 255) / 256); }
 
@@ -193,25 +182,59 @@ __global__ void residual_kernel(const float2 *__restrict__ b, float2 *__restrict
   block_add2(rr, bb, &st->rr, &st->b2);
 }
 
+// Block sum of a float pair added to a global accumulator
+__device__ void block_add_pair(FloatPair v, double *out) {
+  __shared__ double sv[32];
+  const double w = v.warp_sum();
+  if ((threadIdx.x & 31) == 0) sv[threadIdx.x >> 5] = w;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += sv[i];
+    atomicAdd(out, t);
+  }
+}
+
 // Re <r, z> into st->rz_new
 __global__ void dot_rz_kernel(const float2 *__restrict__ r, const float2 *__restrict__ z, int64_t N, CgState *st) {
   if (stopped(st)) return;
-  double acc = 0.0;
+  FloatPair acc;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
     const float2 a = r[i], c = z[i];
-    acc += (double)a.x * c.x + (double)a.y * c.y;
+    acc.add_product(a.x, c.x);
+    acc.add_product(a.y, c.y);
   }
-  block_add2(acc, 0.0, &st->rz_new, nullptr);
+  block_add_pair(acc, &st->rz_new);
 }
 
-// alpha = rz / <p, Ap>;  x += alpha p;  r -= alpha Ap;  accumulate <r, r>
+// convergence test of loop index `running` (||r|| < rtol ||b||, mean.py:80-81)
+__device__ void check_convergence(CgState *st, double rtol, int preconditioned, double *hist, int maxiter) {
+  const int it = st->running;
+  const double rr = *(volatile double *)&st->rr_new;
+  if (hist) hist[it + 1] = sqrt(rr / st->b2);
+  if (!(rr == rr)) {  // NaN: stop, reported by the host
+    st->done = 3;
+    st->iters = it;
+  } else if (sqrt(rr) < rtol * sqrt(st->b2)) {
+    st->done = 1;
+    st->iters = it;
+  } else if (it + 1 >= maxiter) {
+    st->done = 2;
+    st->iters = it;
+  } else if (!preconditioned) {
+    st->rz_new = rr;
+  }
+}
+
+// alpha = rz / <p, Ap>;  x += alpha p;  r -= alpha Ap;  accumulate <r, r>, which the last block tests
 __global__ void update_kernel(float2 *__restrict__ x, float2 *__restrict__ r, const float2 *__restrict__ p,
-                              const float2 *__restrict__ ap, int64_t N, CgState *st) {
+                              const float2 *__restrict__ ap, int64_t N, CgState *st, double rtol, int preconditioned,
+                              double *hist, int maxiter) {
   if (stopped(st)) return;
   const double pr = st->pap[0], pi = st->pap[1];
   const double den = pr * pr + pi * pi;
   const float ar = (float)(st->rz * pr / den), ai = (float)(-st->rz * pi / den);
-  double rr = 0.0;
+  FloatPair rr;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
     const float2 pv = p[i], av = ap[i];
     float2 xv = x[i], rv = r[i];
@@ -221,49 +244,35 @@ __global__ void update_kernel(float2 *__restrict__ x, float2 *__restrict__ r, co
     rv.y -= ar * av.y + ai * av.x;
     x[i] = xv;
     r[i] = rv;
-    rr += (double)rv.x * rv.x + (double)rv.y * rv.y;
+    rr.add_product(rv.x, rv.x);
+    rr.add_product(rv.y, rv.y);
   }
-  block_add2(rr, 0.0, &st->rr_new, nullptr);
-}
-
-// convergence test of loop index `running` (||r|| < rtol ||b||, mean.py:80-81)
-__global__ void check_kernel(CgState *st, double rtol, int preconditioned, double *hist, int maxiter) {
-  if (st->done) return;
-  const int it = st->running;
-  if (hist) hist[it + 1] = sqrt(st->rr_new / st->b2);
-  if (!(st->rr_new == st->rr_new)) {  // NaN: stop, reported by the host
-    st->done = 3;
-    st->iters = it;
-  } else if (sqrt(st->rr_new) < rtol * sqrt(st->b2)) {
-    st->done = 1;
-    st->iters = it;
-  } else if (it + 1 >= maxiter) {
-    st->done = 2;
-    st->iters = it;
-  } else if (!preconditioned) {
-    st->rz_new = st->rr_new;
+  block_add_pair(rr, &st->rr_new);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicInc(&st->ticket, gridDim.x - 1) == gridDim.x - 1) {
+      __threadfence();
+      check_convergence(st, rtol, preconditioned, hist, maxiter);
+    }
   }
 }
 
-// p = z + (rz_new / rz) p
+// p = z + (rz_new / rz) p (the first time, rz infinite: z)
 __global__ void direction_kernel(float2 *__restrict__ p, const float2 *__restrict__ z, int64_t N, const CgState *st) {
   if (stopped(st)) return;
   const float beta = (float)(st->rz_new / st->rz);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-    const float2 zv = z[i], pv = p[i];
-    p[i] = make_float2(zv.x + beta * pv.x, zv.y + beta * pv.y);
+    float2 v = z[i];
+    if (beta != 0.0f) {
+      const float2 pv = p[i];
+      v = make_float2(v.x + beta * pv.x, v.y + beta * pv.y);
+    }
+    p[i] = v;
   }
 }
 
 __global__ void roll_kernel(CgState *st) {
-  if (st->done) return;
-  st->rz = st->rz_new;
-  st->rr = st->rr_new;
-  st->rz_new = 0.0;
-  st->rr_new = 0.0;
-  st->pap[0] = 0.0;
-  st->pap[1] = 0.0;
-  st->running += 1;
+  if (!st->done) roll_scalars(st);
 }
 
 __global__ void copy_kernel(const float2 *__restrict__ a, float2 *__restrict__ b, int64_t N) {
@@ -272,14 +281,13 @@ __global__ void copy_kernel(const float2 *__restrict__ a, float2 *__restrict__ b
 }
 
 __global__ void init_kernel(CgState *st, int preconditioned, double *hist) {
-  st->rz = preconditioned ? st->rz_new : st->rr;
-  st->rz_new = 0.0;
+  if (!preconditioned) st->rz_new = st->rr;
+  st->rz = INFINITY;  // the first direction is z
   st->rr_new = 0.0;
-  st->pap[0] = 0.0;
-  st->pap[1] = 0.0;
   st->done = 0;
   st->iters = -1;
-  st->running = 0;
+  st->running = -1;
+  st->ticket = 0;
   if (hist) hist[0] = sqrt(st->rr / st->b2);
 }
 
@@ -588,7 +596,7 @@ int cg_solve(cov3d_plan *p, const float *d_lhs, const void *d_b, void *d_x, doub
   // out = crop(ifft3(diag^(+-1) * fft3(pad(in)))), with <p, out> into st->pap when dotp is given
   auto apply_op = [&](const float2 *in, float2 *out, int divide, const float2 *dotp, const CgState *gate) -> int {
     const int *stop = gate ? &gate->done : nullptr;
-    if (lines3) return cg_operator_lines(p, in, fine, out, dotp, d_lhs, divide, stop, dotp ? &st->done : stop, st->pap);
+    if (lines3) return cg_operator_lines(p, in, fine, out, dotp, d_lhs, divide, stop, stop, st->pap);
     if (fused) {
       pad_support_kernel<<<capped((int64_t)L * n), 256, 0, s>>>(in, L, n, fine, gate);
       COV3D_LAUNCHED("pad_support_kernel");
@@ -652,11 +660,7 @@ int cg_solve(cov3d_plan *p, const float *d_lhs, const void *d_b, void *d_x, doub
     COV3D_TRY(apply_M(r, z, nullptr));
     dot_rz_kernel<<<capped(nb(L3)), 256, 0, s>>>(r, z, L3, st);
     COV3D_LAUNCHED("dot_rz_kernel");
-    copy_kernel<<<nb(L3), 256, 0, s>>>(z, pv, L3);
-  } else {
-    copy_kernel<<<nb(L3), 256, 0, s>>>(r, pv, L3);
   }
-  COV3D_LAUNCHED("copy_kernel");
   init_kernel<<<1, 1, 0, s>>>(st, precond ? 1 : 0, d_history);
   COV3D_LAUNCHED("init_kernel");
   CgState hs{};
@@ -670,65 +674,53 @@ int cg_solve(cov3d_plan *p, const float *d_lhs, const void *d_b, void *d_x, doub
   }
 
   // one iteration: every kernel is a no-op once the device state says done
+  const float2 *zz = precond ? z : r;
   auto iteration = [&]() -> int {
-    COV3D_TRY(apply_A(pv, ap, pv, st));
-    update_kernel<<<capped(nb(L3)), 256, 0, s>>>(x, r, pv, ap, L3, st);
+    if (lines3) {  // the direction and the roll of the scalars ride in the operator's first two kernels
+      COV3D_TRY(cg_operator_lines(p, nullptr, fine, ap, pv, d_lhs, 0, &st->done, &st->done, st->pap, zz, pv, st));
+    } else {
+      direction_kernel<<<capped(nb(L3)), 256, 0, s>>>(pv, zz, L3, st);
+      COV3D_LAUNCHED("direction_kernel");
+      roll_kernel<<<1, 1, 0, s>>>(st);
+      COV3D_LAUNCHED("roll_kernel");
+      COV3D_TRY(apply_A(pv, ap, pv, st));
+    }
+    update_kernel<<<capped(nb(L3)), 256, 0, s>>>(x, r, pv, ap, L3, st, rtol, precond ? 1 : 0, d_history, maxiter);
     COV3D_LAUNCHED("update_kernel");
-    check_kernel<<<1, 1, 0, s>>>(st, rtol, precond ? 1 : 0, d_history, maxiter);
-    COV3D_LAUNCHED("check_kernel");
-    const float2 *zz = r;
     if (precond) {
       COV3D_TRY(apply_M(r, z, st));
       dot_rz_kernel<<<capped(nb(L3)), 256, 0, s>>>(r, z, L3, st);
       COV3D_LAUNCHED("dot_rz_kernel");
-      zz = z;
     }
-    direction_kernel<<<capped(nb(L3)), 256, 0, s>>>(pv, zz, L3, st);
-    COV3D_LAUNCHED("direction_kernel");
-    roll_kernel<<<1, 1, 0, s>>>(st);
-    return launched("roll_kernel");
+    return COV3D_OK;
   };
-  // poll_every iterations captured once as a CUDA graph on a side stream (a capture cannot run
-  // on the legacy default stream), then replayed on the plan's stream until the state says done:
-  // one launch per poll_every iterations instead of about 14 per iteration (learned-PC solve at
-  // L = 128: 0.221 -> 0.194 s, plain CG 1.39 -> 1.25 s)
+  // poll_every iterations are launched at a time and the state is read one such batch behind, so the
+  // GPU never waits for the host (a captured graph of the batch, made in each call, cost a call about
+  // a millisecond and saves little now that an iteration has five kernels).  The host copies of the
+  // state live in the plan's pinned buffer, two slots in turn.
   {
-    const cudaStream_t s0 = s;
-    cudaStream_t cs = nullptr;
-    COV3D_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-    const cufftHandle hs_all[] = {h, hc, hp, h0, hcp};
-    auto set_streams = [&](cudaStream_t to) -> int {
-      p->stream = to;
-      s = to;
-      for (cufftHandle hh : hs_all)
-        if (hh) COV3D_TRY(check_cufft(cufftSetStream(hh, to), "cufftSetStream"));
-      return COV3D_OK;
-    };
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    const long long l0 = cov3d_launch_count();
-    int rc = set_streams(cs);
-    if (rc == COV3D_OK) rc = check_cuda(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "capture");
-    if (rc == COV3D_OK) {
-      for (int k = 0; k < poll_every && rc == COV3D_OK; ++k) rc = iteration();
-      const int rc2 = check_cuda(cudaStreamEndCapture(cs, &graph), "end capture");
-      if (rc == COV3D_OK) rc = rc2;
+    static_assert(sizeof(CgState) <= 16 * sizeof(double), "two states in the pinned buffer");
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    int rc = check_cuda(cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming), "event");
+    if (rc == COV3D_OK) rc = check_cuda(cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming), "event");
+    int batch = 0;
+    for (int it = 0; rc == COV3D_OK && it < maxiter; it += poll_every, ++batch) {
+      for (int k = 0; k < poll_every && it + k < maxiter && rc == COV3D_OK; ++k) rc = iteration();
+      void *slot = p->h_acc + 16 * (batch & 1);
+      if (rc == COV3D_OK) rc = check_cuda(cudaMemcpyAsync(slot, st, sizeof(CgState), cudaMemcpyDeviceToHost, s), "poll");
+      if (rc == COV3D_OK) rc = check_cuda(cudaEventRecord(ev[batch & 1], s), "poll event");
+      if (rc != COV3D_OK || batch == 0) continue;
+      rc = check_cuda(cudaEventSynchronize(ev[(batch - 1) & 1]), "poll sync");
+      CgState prev;
+      std::memcpy(&prev, p->h_acc + 16 * ((batch - 1) & 1), sizeof(CgState));
+      if (prev.done) break;
     }
-    const long long per_replay = cov3d_launch_count() - l0;
-    const int rc3 = set_streams(s0);
-    if (rc == COV3D_OK) rc = rc3;
-    if (rc == COV3D_OK) rc = check_cuda(cudaGraphInstantiate(&exec, graph, 0), "graph instantiate");
-    for (int it = 0; rc == COV3D_OK && it < maxiter; it += poll_every) {
-      rc = check_cuda(cudaGraphLaunch(exec, s0), "graph launch");
-      count_launches(per_replay);
-      if (rc == COV3D_OK) rc = check_cuda(cudaMemcpyAsync(&hs, st, sizeof(CgState), cudaMemcpyDeviceToHost, s0), "poll");
-      if (rc == COV3D_OK) rc = check_cuda(cudaStreamSynchronize(s0), "poll sync");
-      if (rc == COV3D_OK && hs.done) break;
+    for (cudaEvent_t e : ev)
+      if (e) cudaEventDestroy(e);
+    if (rc != COV3D_OK) {
+      cudaStreamSynchronize(s);  // the launched iterations use the plan's workspace
+      return rc;
     }
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-    cudaStreamDestroy(cs);
-    if (rc != COV3D_OK) return rc;
   }
 
   COV3D_CUDA(cudaMemcpyAsync(&hs, st, sizeof(CgState), cudaMemcpyDeviceToHost, s));
