@@ -446,6 +446,7 @@ __global__ void __launch_bounds__(kSpreadWarps * 32, W < 8 ? 2 : 1) spread_kerne
 // per block, two blocks per SM (168 registers); 5 or 4 warps measured 5.8 and 6.8 ms against 5.3 (a
 // unrolled point loop is slower too: the ranges hold some ten points), 7 spill
 constexpr int kTileWarps = 6;
+constexpr int kTileMaxSub = 448;  // largest subproblem of an ES plan (three points per thread)
 
 // A point's record in floats: the W axis-1 weights twice each (operands of packed multiplies), the
 // axis-2 weights of the group's 8 columns, the axis-0 weights of up to 16 planes; a stride that keeps
@@ -454,8 +455,8 @@ template <int W>
 struct TileRec {
   static constexpr int W2 = (2 * W + 3) / 4 * 4;
   static constexpr int W0 = W2 + 8;
-  static constexpr int STRIDE = W <= 6 ? 36 : 44;
-  static_assert(W0 + 16 <= STRIDE, "plane weights");
+  static constexpr int STRIDE = W <= 2 ? 28 : W <= 6 ? 36 : 44;
+  static_assert(W0 + 16 <= STRIDE && STRIDE % 8 == 4, "plane weights; conflict-free stores");
 };
 
 template <int F>
@@ -465,7 +466,7 @@ struct TileVals {  // floats of a channel part's values, padded to 16 bytes wher
 
 template <int W, int F>
 __host__ __device__ constexpr size_t tile_point_bytes(int NQ) {
-  return (TileRec<W>::STRIDE + NQ * TileVals<F>::STRIDE + 5) * 4;  // ... key, id, mirror id, two factors
+  return (TileRec<W>::STRIDE + NQ * TileVals<F>::STRIDE + 4) * 4;  // ... id, mirror id, two factors
 }
 __host__ __device__ constexpr size_t tile_fixed_bytes(int T, int NG) {
   return (size_t)T * T * sizeof(long long) + (size_t)(2 * NG * 64 + 1 + T + 2) * sizeof(int);
@@ -526,9 +527,9 @@ struct TileRows {
 };
 
 // F / 2 channels per lane in NQ parts: 2 x 5 channels per pass, or one part of 5, 2 or 1.
-template <int W, int F, int NQ, int PP, bool HALF>
+template <int KT, int W, int F, int NQ, int PP, bool HALF>
 __global__ void __launch_bounds__(kTileWarps * 32, 2) spread_tile_kernel(const SpreadParams a) {
-  constexpr int KT = COV3D_KERNEL_ES;
+  constexpr bool ES = KT == COV3D_KERNEL_ES;
   using G = TileGroups<W>;
   using Rec = TileRec<W>;
   constexpr int VS = TileVals<F>::STRIDE;
@@ -540,8 +541,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, 2) spread_tile_kernel(const S
   extern __shared__ float4 smem4[];
   float *recs = reinterpret_cast<float *>(smem4);                // max_sub * record stride
   float *vals = recs + (size_t)a.max_sub * Rec::STRIDE;          // max_sub * NQ * VS
-  int *s_key = reinterpret_cast<int *>(vals + (size_t)a.max_sub * NQ * VS);
-  int *s_id = s_key + a.max_sub, *s_mid = s_id + a.max_sub;      // ids; mirror ids or -1
+  int *s_id = reinterpret_cast<int *>(vals + (size_t)a.max_sub * NQ * VS);
+  int *s_mid = s_id + a.max_sub;      // ids; mirror ids or -1
   float *s_sc = reinterpret_cast<float *>(s_mid + a.max_sub), *s_scm = s_sc + a.max_sub;
   long long *s_row = reinterpret_cast<long long *>((reinterpret_cast<uintptr_t>(s_scm + a.max_sub) + 7) & ~(uintptr_t)7);
   int *s_cnt = reinterpret_cast<int *>(s_row + T * T), *s_off = s_cnt + NK, *s_col = s_off + NK + 1;
@@ -553,13 +554,34 @@ __global__ void __launch_bounds__(kTileWarps * 32, 2) spread_tile_kernel(const S
 
   for (int e = tid; e < NK; e += blockDim.x) s_cnt[e] = 0;
   __syncthreads();
-  auto corner = [&](float t, int ts) {  // bin-local window corner, 0 .. 7
-    return min(max(wrap1(record_cell<KT, W, HALF>(t, a.g.frac), n) - ts, 0), kBin - 1);
+  // bin-local window corner, 0 .. 7 (linear: a window that starts one cell before the grid counts
+  // from cell 0)
+  auto corner = [&](float t, int ts) {
+    const int c0 = record_cell<KT, W, HALF>(t, a.g.frac);
+    return min(max((ES ? wrap1(c0, n) : c0) - ts, 0), kBin - 1);
   };
-  for (int k = tid; k < st.cnt; k += blockDim.x) {
-    const SortedPoint sp = a.pts[st.first + k];
-    const int key = (corner(sp.t2, st.ts2) / G::GS) * 64 + corner(sp.t1, st.ts1) * 8 + corner(sp.t0, st.ts0);
-    s_key[k] = key | (atomicAdd(s_cnt + key, 1) << 9);
+  // each thread keeps its points until their place in the sorted order is known, and asks for their
+  // values (point-major ones) ahead of the gather
+  constexpr int PPT = (kTileMaxSub + kTileWarps * 32 - 1) / (kTileWarps * 32);
+  SortedPoint pt[PPT];
+  int pkey[PPT];
+#pragma unroll
+  for (int u = 0; u < PPT; ++u) {
+    const int k = tid + u * kTileWarps * 32;
+    pkey[u] = -1;
+    if (k < st.cnt) pt[u] = a.pts[st.first + k];
+  }
+#pragma unroll
+  for (int u = 0; u < PPT; ++u) {
+    if (tid + u * kTileWarps * 32 >= st.cnt) continue;
+    const int key = (corner(pt[u].t2, st.ts2) / G::GS) * 64 + corner(pt[u].t1, st.ts1) * 8 + corner(pt[u].t0, st.ts0);
+    pkey[u] = key | (atomicAdd(s_cnt + key, 1) << 9);
+    if (a.ics == 1) {
+      const int id = sp_id<HALF>(pt[u].idf);
+      const float2 *v = a.vals + a.ch0;
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(v + (int64_t)id * a.ips));
+      if (sp_pair<HALF>(pt[u].idf)) asm volatile("prefetch.global.L2 [%0];" ::"l"(v + (int64_t)mirror_id(a.g, id) * a.ips));
+    }
   }
   __syncthreads();
   if (tid < 32) {  // exclusive scan of the counters by one warp
@@ -583,39 +605,61 @@ __global__ void __launch_bounds__(kTileWarps * 32, 2) spread_tile_kernel(const S
     }
     if (tid == 31) s_off[NK] = incl;
   }
-  // global offsets of the tile's rows (axes 0, 1) and columns (axis 2), periodic
+  // global offsets of the tile's rows (axes 0, 1) and columns (axis 2): periodic, or (linear) -1
+  // outside the grid
   for (int e = tid; e < T * T; e += blockDim.x) {
     const int ra = e / T, rb = e - (e / T) * T;
     const int m0 = wrap1(wrap1(st.ts0 + ra, n) + a.shift, n), m1 = wrap1(wrap1(st.ts1 + rb, n) + a.shift, n);
-    s_row[e] = ((int64_t)m0 * n + m1) * n;
+    s_row[e] = ES || (st.ts0 + ra < n && st.ts1 + rb < n) ? ((int64_t)m0 * n + m1) * n : -1;
   }
-  for (int e = tid; e < T; e += blockDim.x) s_col[e] = wrap1(wrap1(st.ts2 + e, n) + a.shift, n);
+  for (int e = tid; e < T; e += blockDim.x) s_col[e] = ES || st.ts2 + e < n ? wrap1(wrap1(st.ts2 + e, n) + a.shift, n) : -1;
   __syncthreads();
   // records (a weight is zero outside its window), ids and prologue factors in sorted order
-  for (int k = tid; k < st.cnt; k += blockDim.x) {
-    const SortedPoint sp = a.pts[st.first + k];
-    const int kr = s_key[k];
+#pragma unroll
+  for (int u = 0; u < PPT; ++u) {
+    const SortedPoint sp = pt[u];
+    const int kr = pkey[u];
+    if (kr < 0) continue;
     const int slot = s_off[kr & 511] + (kr >> 9);
     const int c0 = record_cell<KT, W, HALF>(sp.t0, a.g.frac), c1 = record_cell<KT, W, HALF>(sp.t1, a.g.frac),
               c2 = record_cell<KT, W, HALF>(sp.t2, a.g.frac);
-    const int l0 = wrap1(c0, n) - st.ts0, l2 = wrap1(c2, n) - st.ts2;
-    const float x0 = record_offset<HALF>(sp.t0, c0, a.g.frac) + (float)l0;
-    const float x1 = record_offset<HALF>(sp.t1, c1, a.g.frac);
-    const float x2 = record_offset<HALF>(sp.t2, c2, a.g.frac) + (float)(l2 - G::base((kr & 511) >> 6));
+    const int l0 = (ES ? wrap1(c0, n) : c0) - st.ts0, l2 = (ES ? wrap1(c2, n) : c2) - st.ts2;
+    const int b2 = G::base((kr & 511) >> 6);
     float4 *rec = reinterpret_cast<float4 *>(recs + slot * Rec::STRIDE);
+    // the axes' weights at offset i from the window's first cell, zero outside the window
+    float x0, x1, x2, y0 = 0.f, y1 = 0.f, y2 = 0.f;
+    if (ES) {
+      x0 = record_offset<HALF>(sp.t0, c0, a.g.frac);
+      x1 = record_offset<HALF>(sp.t1, c1, a.g.frac);
+      x2 = record_offset<HALF>(sp.t2, c2, a.g.frac);
+    } else {
+      x0 = record_weight<KT, W, HALF>(sp.t0, c0, 0, a.g.frac, 0.f);
+      y0 = record_weight<KT, W, HALF>(sp.t0, c0, 1, a.g.frac, 0.f);
+      x1 = record_weight<KT, W, HALF>(sp.t1, c1, 0, a.g.frac, 0.f);
+      y1 = record_weight<KT, W, HALF>(sp.t1, c1, 1, a.g.frac, 0.f);
+      x2 = record_weight<KT, W, HALF>(sp.t2, c2, 0, a.g.frac, 0.f);
+      y2 = record_weight<KT, W, HALF>(sp.t2, c2, 1, a.g.frac, 0.f);
+      if (c1 < st.ts1) {  // the window's first row is before the grid
+        x1 = y1;
+        y1 = 0.f;
+      }
+    }
+    auto weight = [&](float x, float y, int i) {
+      return ES ? es_weight<W>(x - (float)i, a.k.beta) : i == 0 ? x : i == 1 ? y : 0.0f;
+    };
     float w[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) w[j] = j < W ? es_weight<W>(x1 - (float)j, a.k.beta) : 0.0f;
+    for (int j = 0; j < 8; ++j) w[j] = j < W ? weight(x1, y1, j) : 0.0f;
 #pragma unroll
     for (int u = 0; u < Rec::W2 / 4; ++u) rec[u] = make_float4(w[2 * u], w[2 * u], w[2 * u + 1], w[2 * u + 1]);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) w[j] = es_weight<W>(x2 - (float)j, a.k.beta);
+    for (int j = 0; j < 8; ++j) w[j] = weight(x2, y2, b2 + j - l2);
     rec[Rec::W2 / 4] = make_float4(w[0], w[1], w[2], w[3]);
     rec[Rec::W2 / 4 + 1] = make_float4(w[4], w[5], w[6], w[7]);
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = 4 * u + j < T ? es_weight<W>(x0 - (float)(4 * u + j), a.k.beta) : 0.0f;
+      for (int j = 0; j < 4; ++j) w[j] = 4 * u + j < T ? weight(x0, y0, 4 * u + j - l0) : 0.0f;
       rec[Rec::W0 / 4 + u] = make_float4(w[0], w[1], w[2], w[3]);
     }
     const int id = sp_id<HALF>(sp.idf);
@@ -634,29 +678,43 @@ __global__ void __launch_bounds__(kTileWarps * 32, 2) spread_tile_kernel(const S
     // this pass's channel values in sorted order.  A record of kSortHalf that stands for a pair of
     // mirror pixels takes the sum of the one's value and the conjugate of the other's, which has
     // the same real part after the inverse transform.
-    for (int e = tid; e < st.cnt * CH; e += blockDim.x) {
-      const int slot = e / CH, ch = e - slot * CH;
-      float2 v = make_float2(0.f, 0.f);
-      if (p0 + ch < a.nch) {
-        const float2 *src = a.vals + (int64_t)(a.ch0 + p0 + ch) * a.ics;
-        int id = s_id[slot];
-        const bool conj = HALF && id < 0;
-        if (conj) id = ~id;
-        const float2 x = __ldg(src + (int64_t)id * a.ips);
-        const float sc = s_sc[slot];
-        v = make_float2(x.x * sc, conj ? -(x.y * sc) : x.y * sc);
-        if (HALF) {
-          const int mid = s_mid[slot];
-          if (mid >= 0) {
-            const float2 m = __ldg(src + (int64_t)mid * a.ips);
-            const float sm = s_scm[slot];
-            v.x = fmaf(m.x, sm, v.x);
-            v.y = fmaf(-m.y, sm, v.y);
+    // Four elements' loads in flight per thread: the gathers' latency is most of the staging.
+    constexpr int GU = 4;
+    const int total = st.cnt * CH;
+    for (int e0 = tid; e0 < total; e0 += GU * kTileWarps * 32) {
+      float2 x[GU], m[GU];
+      int sl[GU];
+#pragma unroll
+      for (int u = 0; u < GU; ++u) {
+        const int e = e0 + u * kTileWarps * 32;
+        const int slot = e / CH, ch = e - slot * CH;
+        sl[u] = e < total ? slot : -1;
+        x[u] = m[u] = make_float2(0.f, 0.f);
+        if (e < total && p0 + ch < a.nch) {
+          const float2 *src = a.vals + (int64_t)(a.ch0 + p0 + ch) * a.ics;
+          const int id = s_id[slot];
+          x[u] = __ldg(src + (int64_t)(HALF && id < 0 ? ~id : id) * a.ips);
+          if (HALF) {
+            const int mid = s_mid[slot];
+            if (mid >= 0) m[u] = __ldg(src + (int64_t)mid * a.ips);
           }
         }
       }
-      const int part = ch / (F / 2);
-      *reinterpret_cast<float2 *>(vals + (slot * NQ + part) * VS + 2 * (ch - part * (F / 2))) = v;
+#pragma unroll
+      for (int u = 0; u < GU; ++u) {
+        const int slot = sl[u];
+        if (slot < 0) continue;
+        const int ch = e0 + u * kTileWarps * 32 - slot * CH;
+        const float sc = s_sc[slot];
+        float2 v = make_float2(x[u].x * sc, HALF && s_id[slot] < 0 ? -(x[u].y * sc) : x[u].y * sc);
+        if (HALF && s_mid[slot] >= 0) {
+          const float sm = s_scm[slot];
+          v.x = fmaf(m[u].x, sm, v.x);
+          v.y = fmaf(-m[u].y, sm, v.y);
+        }
+        const int part = ch / (F / 2);
+        *reinterpret_cast<float2 *>(vals + (slot * NQ + part) * VS + 2 * (ch - part * (F / 2))) = v;
+      }
     }
     if (tid == 0) *s_task = 0;
     __syncthreads();
@@ -684,13 +742,16 @@ __global__ void __launch_bounds__(kTileWarps * 32, 2) spread_tile_kernel(const S
       TileRows<W, F, NQ, PP, 0>::run(range, recs, vals, cp, c, plane, acc);
       // the finished cells go to the global grid
       const int co = s_col[G::base(g) + c];
+      if (!ES && co < 0) continue;
       const int ch0 = p0 + cp * (F / 2);  // this lane's first channel
 #pragma unroll
       for (int k = 0; k < PP; ++k) {
         if (plane + k >= T) break;
 #pragma unroll
         for (int r = 0; r < T; ++r) {
-          float2 *dst = a.grid + (s_row[(plane + k) * T + r] + co) * a.cs + (int64_t)(a.ch0 + ch0) * a.chs;
+          const long long ro = s_row[(plane + k) * T + r];
+          if (!ES && ro < 0) continue;
+          float2 *dst = a.grid + (ro + co) * a.cs + (int64_t)(a.ch0 + ch0) * a.chs;
 #pragma unroll
           for (int f = 0; f < F / 2; ++f) {
             const float2 x = acc[k][r][f];
@@ -740,42 +801,37 @@ int launch_wc(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
   return launch_spread_kernel(spread_kernel<KT, W, 1, COMP, HALF>, "spread_kernel", smem, a, max_blocks, st);
 }
 
-template <int W, int F, int NQ, int PP, bool HALF>
+template <int KT, int W, int F, int NQ, int PP, bool HALF>
 int launch_tile(const SpreadParams &a, int64_t max_blocks, cudaStream_t st) {
   const size_t smem = (size_t)a.max_sub * tile_point_bytes<W, F>(NQ) + 8 +
                       tile_fixed_bytes(TileGroups<W>::T, TileGroups<W>::NG);
-  return launch_spread_kernel(spread_tile_kernel<W, F, NQ, PP, HALF>, "spread_tile_kernel", smem, a, max_blocks, st,
+  return launch_spread_kernel(spread_tile_kernel<KT, W, F, NQ, PP, HALF>, "spread_tile_kernel", smem, a, max_blocks, st,
                               kTileWarps);
 }
 
 // Passes of ten channels in one launch, then the rest in the layout that holds it.
-template <int W, bool HALF>
+template <int KT, int W, bool HALF>
 int launch_tile_channels(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
   const int rest = nchan % 10, whole = rest > 5 ? nchan : nchan - rest;
   if (whole > 0) {
     a.ch0 = 0;
     a.nch = whole;
-    COV3D_TRY((launch_tile<W, 10, 2, 1, HALF>(a, max_blocks, st)));
+    COV3D_TRY((launch_tile<KT, W, 10, 2, 1, HALF>(a, max_blocks, st)));
   }
   a.ch0 = whole;
   a.nch = nchan - whole;
-  if (a.nch >= 3) return launch_tile<W, 10, 1, 1, HALF>(a, max_blocks, st);
-  if (a.nch == 2) return launch_tile<W, 4, 1, 1, HALF>(a, max_blocks, st);
-  if (a.nch == 1) return launch_tile<W, 2, 1, 2, HALF>(a, max_blocks, st);
+  if (a.nch >= 3) return launch_tile<KT, W, 10, 1, 1, HALF>(a, max_blocks, st);
+  if (a.nch == 2) return launch_tile<KT, W, 4, 1, 1, HALF>(a, max_blocks, st);
+  if (a.nch == 1) return launch_tile<KT, W, 2, 1, 2, HALF>(a, max_blocks, st);
   return COV3D_OK;
 }
 
 template <int KT, int W>
 int launch_w(SpreadParams a, int nchan, bool comp, int64_t max_blocks, cudaStream_t st) {
-  if constexpr (KT == COV3D_KERNEL_ES) {
-    return a.half ? launch_tile_channels<W, true>(a, nchan, max_blocks, st)
-                  : launch_tile_channels<W, false>(a, nchan, max_blocks, st);
+  if constexpr (KT != COV3D_KERNEL_NEAREST) {
+    return a.half ? launch_tile_channels<KT, W, true>(a, nchan, max_blocks, st)
+                  : launch_tile_channels<KT, W, false>(a, nchan, max_blocks, st);
   } else {
-    if constexpr (KT != COV3D_KERNEL_NEAREST) {
-      if (a.half)
-        return comp ? launch_wc<KT, W, true, true>(a, nchan, max_blocks, st)
-                    : launch_wc<KT, W, false, true>(a, nchan, max_blocks, st);
-    }
     return comp ? launch_wc<KT, W, true, false>(a, nchan, max_blocks, st)
                 : launch_wc<KT, W, false, false>(a, nchan, max_blocks, st);
   }
