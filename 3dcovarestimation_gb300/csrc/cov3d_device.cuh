@@ -305,6 +305,30 @@ __device__ __forceinline__ float ctf_factor(const float *ctf, const CtfCoef *ctf
   return ctf_eval(ctfc[b], row - g.Lp / 2, col - g.Lp / 2);
 }
 
+// The mean's two spread values of a pixel: y * exp(-i (gx sx + gy sy)) * c * ctf (the image
+// phase-shifted by -offset, mean.py:201-204) and (c * ctf)^2 / L (the kernel, whose extra 1/L is
+// mean.py:215); gx, gy = ceil(k - L/2) 2 pi / L (poses.py:70-89).
+__device__ __forceinline__ void mean_value(const MeanSource &s, int id, int P, int L, float2 &v0, float &v1) {
+  const int b = (unsigned)id / (unsigned)P;
+  const int p = id - b * P;
+  float f = s.ctf ? __ldg(s.ctf + id) : 1.0f;
+  if (s.contrasts) f *= __ldg(s.contrasts + b);
+  float2 y = __ldg(s.images + id);
+  if (s.offsets) {
+    const int row = (unsigned)p / (unsigned)L, col = p - row * L;
+    const float half = 0.5f * (float)L;
+    const float gx = __fdiv_rn(__fmul_rn(__fmul_rn(ceilf((float)col - half), 2.0f), kPiF), (float)L);
+    const float gy = __fdiv_rn(__fmul_rn(__fmul_rn(ceilf((float)row - half), 2.0f), kPiF), (float)L);
+    const float sx = -__ldg(s.offsets + 2 * b), sy = -__ldg(s.offsets + 2 * b + 1);
+    const float arg = __fadd_rn(__fmul_rn(gx, sx), __fmul_rn(gy, sy));
+    float sn, cs;
+    sincosf(arg, &sn, &cs);
+    y = make_float2(y.x * cs - y.y * sn, y.x * sn + y.y * cs);
+  }
+  v0 = make_float2(y.x * f, y.y * f);
+  v1 = f * f / (float)L;
+}
+
 // Sums of products of floats in a float pair (about 46 bits: the products' rounding errors and those
 // of the leading sum are carried along): a thread's few terms and a warp's partial sums of the CG's
 // inner products before they are added in FP64, whose pipe (two operations per clock and SM) took

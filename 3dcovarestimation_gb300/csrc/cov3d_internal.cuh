@@ -263,6 +263,15 @@ int launch_interp(cov3d_plan *p, const GridArgs &g, int nchan, void *out, int64_
 // spread.cu
 int launch_spread(cov3d_plan *p, const void *values, int64_t in_ps, int64_t in_cs, int nchan, const EpilogueArgs &e,
                   void *grid, int64_t cell_stride, int64_t chan_stride, int shift, SortMode mode);
+// Inputs of the mean's backprojection (all but the images may be null)
+struct MeanSource {
+  const float2 *images;     // (n_images, P)
+  const float *ctf;         // (n_images, P)
+  const float *offsets;     // (n_images, 2)
+  const float *contrasts;   // (n_images)
+};
+int launch_spread_mean_nearest(cov3d_plan *p, const MeanSource &src, const EpilogueArgs &e, void *grids,
+                               int64_t chan_stride);
 int launch_spread_unaggregated(cov3d_plan *p, const void *values, int64_t in_ps, const EpilogueArgs &e,
                                void *grids);
 

@@ -399,34 +399,15 @@ __global__ void regularize_kernel(const float2 *__restrict__ lhs, int n, int nsh
 
 // ---------------------------------------------------------------------------- backprojection
 
-// Values spread for the mean: channel 0 = y * exp(-i (gx sx + gy sy)) * c * ctf (the image
-// phase-shifted by -offset, mean.py:201-204), channel 1 = (c * ctf)^2 / L (the kernel, whose
-// extra 1/L is mean.py:215); gx, gy = ceil(k - L/2) 2 pi / L (poses.py:70-89).
-__global__ void mean_values_kernel(const float2 *__restrict__ images, const float *__restrict__ ctf,
-                                   const float *__restrict__ offsets, const float *__restrict__ contrasts,
-                                   int64_t n_images, int L, float2 *__restrict__ vals) {
-  const int P = L * L;
-  const int64_t M = n_images * P;
+// The mean's values (mean_value) as two planar channels, for the plans whose spreading takes arrays
+__global__ void mean_values_kernel(const MeanSource src, int64_t M, int L, float2 *__restrict__ vals) {
   const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= M) return;
-  const int64_t b = id / P;
-  const int p = (int)(id - b * P);
-  float f = ctf ? __ldg(ctf + id) : 1.0f;
-  if (contrasts) f *= __ldg(contrasts + b);
-  float2 y = images[id];
-  if (offsets) {
-    const int row = p / L, col = p - row * L;
-    const float half = 0.5f * (float)L;
-    const float gx = __fdiv_rn(__fmul_rn(__fmul_rn(ceilf((float)col - half), 2.0f), kPiF), (float)L);
-    const float gy = __fdiv_rn(__fmul_rn(__fmul_rn(ceilf((float)row - half), 2.0f), kPiF), (float)L);
-    const float sx = -__ldg(offsets + 2 * b), sy = -__ldg(offsets + 2 * b + 1);
-    const float arg = __fadd_rn(__fmul_rn(gx, sx), __fmul_rn(gy, sy));
-    float sn, cs;
-    sincosf(arg, &sn, &cs);
-    y = make_float2(y.x * cs - y.y * sn, y.x * sn + y.y * cs);
-  }
-  vals[id] = make_float2(y.x * f, y.y * f);
-  vals[M + id] = make_float2(f * f / (float)L, 0.0f);
+  float2 v0;
+  float v1;
+  mean_value(src, (int)id, L * L, L, v0, v1);
+  vals[id] = v0;
+  vals[M + id] = make_float2(v1, 0.0f);
 }
 
 }  // namespace
@@ -469,13 +450,14 @@ int mean_accumulate(cov3d_plan *p, const void *d_images, const float *d_ctf, con
     return COV3D_EINVAL;
   }
   const int64_t M = p->n_points, n3 = (int64_t)p->n * p->n * p->n;
+  const MeanSource src{static_cast<const float2 *>(d_images), d_ctf, d_offsets, d_contrasts};
+  EpilogueArgs e{nullptr, 1, 1.0f / (float)p->L};
+  if (!accumulate) COV3D_TRY(launch_zero(p, d_grids, 2 * n3 * 8));
+  if (p->kernel == COV3D_KERNEL_NEAREST) return launch_spread_mean_nearest(p, src, e, d_grids, n3);
   COV3D_TRY(grow(p->q, M * 16));
   float2 *vals = p->q.as<float2>();
-  if (!accumulate) COV3D_TRY(launch_zero(p, d_grids, 2 * n3 * 8));
-  mean_values_kernel<<<nb(M), 256, 0, p->stream>>>(static_cast<const float2 *>(d_images), d_ctf, d_offsets,
-                                                   d_contrasts, p->n_images, p->L, vals);
+  mean_values_kernel<<<nb(M), 256, 0, p->stream>>>(src, M, p->L, vals);
   COV3D_LAUNCHED("mean_values_kernel");
-  EpilogueArgs e{nullptr, 1, 1.0f / (float)p->L};
   return launch_spread(p, vals, 1, M, 2, e, d_grids, 1, n3, 0, kSortFull);
 }
 

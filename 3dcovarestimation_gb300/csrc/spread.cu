@@ -9,7 +9,6 @@ namespace cov3d {
 namespace {
 
 constexpr int kBin = 8;
-constexpr int kSpreadWarps = 16;
 
 struct SpreadParams {
   PointGeom g;
@@ -19,6 +18,7 @@ struct SpreadParams {
   const int *sub_bin;
   const int *sub_first;
   const int *sub_count;
+  const int *bin_off;  // first sorted point of each bin
   const int *nsub;
   const float2 *vals;
   int64_t ips, ics;
@@ -43,61 +43,6 @@ __device__ __forceinline__ float prologue(const PointGeom &g, int id, const floa
   return sc * ctf_factor(ctf, ctfc, g, id);
 }
 
-constexpr int kLMin = -8;   // window corners relative to the bin lie in [kLMin, kLMin + 16)
-constexpr int kKeys = 256;  // sort key (l1 - kLMin) * 16 + (l0 - kLMin)
-constexpr int kFoldRanges = 3;  // window-corner rows l1 summed in FP32 between compensated folds
-
-// Per-point record staged once per block, in elements of float2 (each weight twice, the operand
-// of a packed multiply: spread_kernel) or float (each weight once, splatted in a register:
-// spread_rows_kernel, where the bytes shared memory returns per visit are the bound): the
-// axis-0 weights by tile plane and the axis-2 weights by tile column, zero
-// outside the point's window (the column slot T is always zero, for idle lanes), and the W
-// axis-1 weights with ROWS - 1 zeros before them and max(ROWS - 1, 1) after.  A lane's weight
-// for tile row b of a point with window corner l1 is then
-// rec[plane] * rec[W1 + b - l1] * rec[W2 + column], with no corner arithmetic and no select:
-// lanes outside the window read zeros.
-template <int W, int ROWS>
-struct PointRec {
-  static constexpr int T = kBin + W - 1;
-  static constexpr int W1 = T + ROWS - 1;            // axis-1 weight o1 at W1 + o1
-  static constexpr int Z1 = ROWS > 1 ? ROWS - 1 : 1;  // zeros after the axis-1 weights
-  static constexpr int W2 = W1 + W + Z1;             // axis-2 weights by column
-  static constexpr int F2 = (W2 + T + 2) / 2 * 2;    // float2 per record (even)
-};
-
-// Shared memory after the staged channel values: tile row offsets, point records, sort keys,
-// point ids, prologue factors, key counters and offsets, column offsets, the task counter.
-struct StageSmem {
-  long long *rowoff;  // T * T
-  void *rec;          // max_sub * F2 record elements (float2, or float for scalar weights)
-  int *key;           // max_sub
-  unsigned *pid;      // max_sub: the record's id with kPairBit and kConjBit
-  float *sc, *scm;    // max_sub each: factors of the id and of its mirror pixel
-  int *cnt, *off;     // kKeys, kKeys + 1
-  int *coloff;        // T
-  int *task;          // 1
-};
-
-__host__ __device__ constexpr size_t stage_bytes(int max_sub, int T, int F2, size_t esize) {
-  return (size_t)T * T * sizeof(long long) + (size_t)max_sub * (F2 * esize + 4 * sizeof(int)) +
-         (size_t)(2 * kKeys + 2 + T) * sizeof(int);
-}
-
-__device__ __forceinline__ StageSmem carve(void *base, int max_sub, int T, int F2, int esize) {
-  StageSmem s;
-  s.rowoff = static_cast<long long *>(base);
-  s.rec = s.rowoff + T * T;
-  s.key = reinterpret_cast<int *>(static_cast<char *>(s.rec) + (size_t)max_sub * F2 * esize);
-  s.pid = reinterpret_cast<unsigned *>(s.key + max_sub);
-  s.sc = reinterpret_cast<float *>(s.pid + max_sub);
-  s.scm = s.sc + max_sub;
-  s.cnt = reinterpret_cast<int *>(s.scm + max_sub);
-  s.off = s.cnt + kKeys;
-  s.coloff = s.off + kKeys + 1;
-  s.task = s.coloff + T;
-  return s;
-}
-
 // A subproblem: its points [first, first + cnt) of the sorted order and the tile origin.
 struct SubTile {
   int first, cnt, ts0, ts1, ts2;
@@ -115,311 +60,127 @@ __device__ __forceinline__ SubTile sub_tile(const SpreadParams &a, int sub) {
   return t;
 }
 
-// Stage 1 of both spreading kernels: the block counting-sorts its points by the (axis-1,
-// axis-0) corner (l1, l0) of their window and stages, in that order, each point's record, id
-// and prologue factor (im_backward's Nyquist zeroing, CTF and scale), then the global offsets
-// of the tile's rows and columns.  The caller synchronises before reading them.
-// a weight as a record element: twice (a packed-multiply operand) or once
-__device__ __forceinline__ void put_weight(float2 *e, float x) { *e = make_float2(x, x); }
-__device__ __forceinline__ void put_weight(float *e, float x) { *e = x; }
-
-template <int KT, int W, int ROWS, typename E, bool HALF>
-__device__ __forceinline__ void stage_subproblem(const SpreadParams &a, const StageSmem &s, const SubTile &st) {
-  using Rec = PointRec<W, ROWS>;
-  constexpr int T = Rec::T;
-  constexpr int F2 = Rec::F2;
-  const int n = a.g.n;
-  const int tid = threadIdx.x;
-  for (int e = tid; e < kKeys; e += blockDim.x) s.cnt[e] = 0;
-  __syncthreads();
-  // sort keys and ranks
-  for (int k = tid; k < st.cnt; k += blockDim.x) {
-    const SortedPoint sp = a.pts[st.first + k];
-    int c0 = record_cell<KT, W, HALF>(sp.t0, a.g.frac), c1 = record_cell<KT, W, HALF>(sp.t1, a.g.frac);
-    if (KT == COV3D_KERNEL_ES) {
-      c0 = wrap1(c0, n);
-      c1 = wrap1(c1, n);
-    }
-    const int key = (min(max(c1 - st.ts1 - kLMin, 0), 15) << 4) | min(max(c0 - st.ts0 - kLMin, 0), 15);
-    s.key[k] = key | (atomicAdd(s.cnt + key, 1) << 8);
-  }
-  __syncthreads();
-  if (tid < 32) {  // exclusive scan of the 256 counters by one warp, 8 per lane
-    int v[kKeys / 32], sum = 0;
-#pragma unroll
-    for (int u = 0; u < kKeys / 32; ++u) {
-      v[u] = s.cnt[tid * (kKeys / 32) + u];
-      sum += v[u];
-    }
-    int incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (tid >= o) incl += t;
-    }
-    int base = incl - sum;
-#pragma unroll
-    for (int u = 0; u < kKeys / 32; ++u) {
-      s.off[tid * (kKeys / 32) + u] = base;
-      base += v[u];
-    }
-    if (tid == 31) s.off[kKeys] = incl;
-  }
-  __syncthreads();
-  // records, point ids and prologue factors in sorted order
-  for (int k = tid; k < st.cnt; k += blockDim.x) {
-    const SortedPoint sp = a.pts[st.first + k];
-    const int kr = s.key[k];
-    const int slot = s.off[kr & 255] + (kr >> 8);
-    float w0[W], w1[W], w2[W];
-    int c0 = taps<KT, W, HALF>(sp.t0, a.g.frac, a.k.beta, w0);
-    taps<KT, W, HALF>(sp.t1, a.g.frac, a.k.beta, w1);
-    int c2 = taps<KT, W, HALF>(sp.t2, a.g.frac, a.k.beta, w2);
-    if (KT == COV3D_KERNEL_ES) {
-      c0 = wrap1(c0, n);
-      c2 = wrap1(c2, n);
-    }
-    E *rec = static_cast<E *>(s.rec) + slot * F2;
-    const int l0 = c0 - st.ts0, l2 = c2 - st.ts2;  // bin-local corners, >= 1 - W (zero padding below)
-    const float z = 0.0f;
-#pragma unroll
-    for (int e = 0; e < T; ++e) {
-      put_weight(rec + e, z);
-      put_weight(rec + Rec::W2 + e, z);
-    }
-    put_weight(rec + Rec::W2 + T, z);
-#pragma unroll
-    for (int e = T; e < Rec::W1; ++e) put_weight(rec + e, z);
-#pragma unroll
-    for (int e = Rec::W1 + W; e < Rec::W2; ++e) put_weight(rec + e, z);
-#pragma unroll
-    for (int r = 0; r < W; ++r) {
-      if (l0 + r >= 0 && l0 + r < T) put_weight(rec + l0 + r, w0[r]);
-      if (l2 + r >= 0 && l2 + r < T) put_weight(rec + Rec::W2 + l2 + r, w2[r]);
-      put_weight(rec + Rec::W1 + r, w1[r]);
-    }
-    const int id = sp_id<HALF>(sp.idf);
-    float sc = (a.nyquist && sp_nyquist(sp.idf)) ? 0.0f : a.scale;
-    sc *= ctf_factor(a.ctf, a.ctfc, a.g, id);
-    s.pid[slot] = sp.idf & ~kNyquistBit;
-    s.sc[slot] = sc;
-    if (sp_pair<HALF>(sp.idf)) s.scm[slot] = a.scale * ctf_factor(a.ctf, a.ctfc, a.g, mirror_id(a.g, id));
-  }
-  // global offsets of the tile's rows (axes 0, 1) and columns (axis 2)
-  for (int e = tid; e < T * T; e += blockDim.x) {
-    const int ra = e / T, rb = e - (e / T) * T;
-    int m0 = st.ts0 + ra, m1 = st.ts1 + rb;
-    bool ok = true;
-    if (KT == COV3D_KERNEL_ES) {
-      m0 = m0 >= n ? m0 - n : m0;
-      m1 = m1 >= n ? m1 - n : m1;
-    } else {
-      ok = m0 < n && m1 < n;
-    }
-    m0 += a.shift;
-    m1 += a.shift;
-    m0 = m0 >= n ? m0 - n : m0;
-    m1 = m1 >= n ? m1 - n : m1;
-    s.rowoff[e] = ok ? ((int64_t)m0 * n + m1) * n : -1;
-  }
-  for (int e = tid; e < T; e += blockDim.x) {
-    int m2 = st.ts2 + e;
-    bool ok = true;
-    if (KT == COV3D_KERNEL_ES) {
-      m2 = m2 >= n ? m2 - n : m2;
-    } else {
-      ok = m2 < n;
-    }
-    m2 += a.shift;
-    m2 = m2 >= n ? m2 - n : m2;
-    s.coloff[e] = ok ? m2 : -1;
-  }
+// TwoSum (Knuth): s + d = s' + e exactly, e added to the error sum err.
+__device__ __forceinline__ void two_sum(float &s, float &err, float d) {
+  const float t = __fadd_rn(s, d), b = __fsub_rn(t, s);
+  err = __fadd_rn(err, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(d, b)));
+  s = t;
 }
 
-// The scaled value of one channel of a staged record: src = values + channel * channel stride.  A
-// record of kSortHalf that stands for a pair of mirror pixels takes the sum of the one's value
-// and the conjugate of the other's, which has the same real part after the inverse transform.
-template <bool HALF>
-__device__ __forceinline__ float2 record_value(const SpreadParams &a, const StageSmem &s, int slot, const float2 *src) {
-  const unsigned pid = s.pid[slot];
-  const float sc = s.sc[slot];
-  const int id = sp_id<HALF>(pid);
-  const float2 x = __ldg(src + (int64_t)id * a.ips);
-  float2 v = make_float2(x.x * sc, sp_conj<HALF>(pid) ? -(x.y * sc) : x.y * sc);
-  if (sp_pair<HALF>(pid)) {
-    const float sm = s.scm[slot];
-    const float2 m = __ldg(src + (int64_t)mirror_id(a.g, id) * a.ips);
-    v.x = fmaf(m.x, sm, v.x);
-    v.y = fmaf(-m.y, sm, v.y);
+// Values of the mean's backprojection (mean_cg.cu): channel 0 = y * exp(-i (gx sx + gy sy)) * c * ctf
+// (the image phase-shifted by -offset, mean.py:201-204), channel 1 = (c * ctf)^2 / L (the kernel,
+// real, whose extra 1/L is mean.py:215).
+struct MeanValue {
+  MeanSource s;
+  __device__ __forceinline__ void operator()(const PointGeom &g, int id, float2 &v0, float2 &v1) const {
+    mean_value(s, id, g.P, g.Lp, v0, v1.x);
+    v1.y = 0.0f;
   }
-  return v;
-}
-
-// TwoSum (Knuth) on both lanes of a float2: s + d = s' + e exactly, e added to the error sum
-// err.  Differences are fused multiply-adds with -1, which round exactly like a subtraction.
-__device__ __forceinline__ void two_sum2(float2 &s, float2 &err, const float2 d) {
-  const float2 m1 = make_float2(-1.0f, -1.0f);
-  const float2 s2 = __fadd2_rn(s, d);
-  const float2 bb = __ffma2_rn(s, m1, s2);   // s2 - s
-  const float2 sb = __ffma2_rn(bb, m1, s2);  // s2 - bb
-  const float2 e1 = __ffma2_rn(sb, m1, s);   // s - (s2 - bb)
-  const float2 e2 = __ffma2_rn(bb, m1, d);   // d - bb
-  err = __fadd2_rn(err, __fadd2_rn(e1, e2));
-  s = s2;
-}
-
-// Lane layout of the row tasks: lane = g * T + c owns tile column c (T = 8 + W - 1 columns)
-// and the channel pairs g, g + G, ..., G = 32 / T lane groups.
-template <int W>
-struct SpreadLanes {
-  static constexpr int T = kBin + W - 1;
-  static constexpr int G = 32 / T;
+};
+// Two channels of an array of point values
+struct ArrayValue {
+  const float2 *vals;
+  int64_t ips, ics;
+  int nch;
+  __device__ __forceinline__ void operator()(const PointGeom &, int id, float2 &v0, float2 &v1) const {
+    v0 = __ldg(vals + (int64_t)id * ips);
+    v1 = nch > 1 ? __ldg(vals + (int64_t)id * ips + ics) : make_float2(0.f, 0.f);
+  }
 };
 
-// Row tasks, for few channels.  One block per subproblem (a bin of 8^3 cells and at most
-// max_sub of its points); the cells it can reach form a tile of the bin and a (W-1)-cell halo,
-// T^3 cells.  After stage_subproblem, a task is one tile row: plane a, row b.  The points whose
-// window covers it are the W contiguous ranges {l1 = b - o1, l0 in [a - W + 1, a]},
-// o1 = 0 .. W-1, of the sorted order.  Lane (g, c) keeps the sums of cell (a, b, c) for its
-// channel pairs in registers: each group of kFoldRanges ranges is summed in FP32 and, with COMP,
-// added to the cell's (hi, lo) pair by a TwoSum, so the error of the cell's accumulation is that
-// of one short FP32 sum per group.  The finished row goes to the global grid with one complex
-// atomic per cell and channel.  Warps take tasks from a shared counter.  The block needs no
-// shared-memory tile: its shared memory is the staged points only.
-template <int KT, int W, int CPL, bool COMP, bool HALF>
-__global__ void __launch_bounds__(kSpreadWarps * 32, W < 8 ? 2 : 1) spread_kernel(const SpreadParams a) {
-  constexpr int T = SpreadLanes<W>::T;
-  constexpr int G = SpreadLanes<W>::G;  // lane groups over channel pairs
-  constexpr int NP = G * CPL;           // channel pairs staged per group
-  using Rec = PointRec<W, 1>;
-  constexpr int F2 = Rec::F2;
-  extern __shared__ float4 smem4[];
-  float4 *s_val = smem4;  // max_sub * NP
-  const StageSmem s = carve(s_val + a.max_sub * NP, a.max_sub, T, F2, sizeof(float2));
-  const float2 *recs = static_cast<const float2 *>(s.rec);
+// Nearest-cell spreading of one or two channels.  A bin's cells belong to its points alone, so one
+// block takes the bin (up to kNearestSubs subproblems of it), thread t the bin's cell t: the block
+// counting-sorts its points by cell, kNearestThreads at a time, computes their values in that order
+// into shared memory, and every thread adds its cell's values in registers (with COMP by TwoSum).
+// A bin that fits one block is added to the grid without atomics.  The mean's batch of 1024 images of
+// 128^2: 1.75 + 0.11 ms (row tasks over staged values, values made by a kernel of their own) -> 0.63 ms;
+// what bounds it is the gather of the points' pixels and the barriers of the sort.
+constexpr int kNearestThreads = kBin * kBin * kBin;
+constexpr int kNearestSubs = 16;
+
+template <bool COMP, typename Value>
+__global__ void __launch_bounds__(kNearestThreads) spread_nearest_kernel(const SpreadParams a, const Value value) {
+  __shared__ int s_cnt[kNearestThreads], s_off[kNearestThreads + 1], s_warp[kNearestThreads / 32];
+  __shared__ float2 s_v0[kNearestThreads], s_v1[kNearestThreads];
   const int sub = blockIdx.x;
   if (sub >= *a.nsub) return;
+  const int bin = a.sub_bin[sub], first = a.sub_first[sub];
+  const int begin = a.bin_off[bin], end = a.bin_off[bin + 1];
+  if ((first - begin) % (kNearestSubs * a.max_sub) != 0) return;
+  const int last = min(end, first + kNearestSubs * a.max_sub);
+  const bool alone = first == begin && last == end;
   const SubTile st = sub_tile(a, sub);
-  stage_subproblem<KT, W, 1, float2, HALF>(a, s, st);
-
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int g = lane / T, c = lane - (lane / T) * T;
-  const bool lane_live = g < G;
-  const int gv = lane_live ? g : 0;  // idle lanes compute pair 0 and drop it
-  const int npairs = (a.nch + 1) / 2;
-  for (int p0 = 0; p0 < npairs; p0 += NP) {  // channel groups of NP pairs
-    __syncthreads();
-    // this group's scaled channel pairs, in sorted order
-    for (int e = tid; e < st.cnt * NP; e += blockDim.x) {
-      const int slot = e / NP, pp = p0 + (e - (e / NP) * NP);
-      const float2 *src = a.vals + (int64_t)(a.ch0 + 2 * pp) * a.ics;
-      const float2 v0 = 2 * pp < a.nch ? record_value<HALF>(a, s, slot, src) : make_float2(0.f, 0.f);
-      const float2 v1 = 2 * pp + 1 < a.nch ? record_value<HALF>(a, s, slot, src + a.ics) : make_float2(0.f, 0.f);
-      s_val[e] = make_float4(v0.x, v0.y, v1.x, v1.y);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float2 h0 = make_float2(0.f, 0.f), h1 = h0, l0 = h0, l1 = h0;
+  bool any = false;
+  for (int base = first; base < last; base += kNearestThreads) {
+    s_cnt[tid] = 0;
+    __syncthreads();  // also: the previous chunk's values have been read
+    const bool live = base + tid < last;
+    int key = 0, rank = 0;
+    float2 v0, v1;
+    if (live) {
+      const SortedPoint sp = a.pts[base + tid];
+      key = (((int)rintf(sp.t0) - st.ts0) * kBin + (int)rintf(sp.t1) - st.ts1) * kBin + (int)rintf(sp.t2) - st.ts2;
+      rank = atomicAdd(s_cnt + key, 1);
+      const int id = sp_id<false>(sp.idf);
+      value(a.g, id, v0, v1);
+      float sc = (a.nyquist && sp_nyquist(sp.idf)) ? 0.0f : a.scale;
+      sc *= ctf_factor(a.ctf, a.ctfc, a.g, id);
+      v0 = make_float2(v0.x * sc, v0.y * sc);
+      v1 = make_float2(v1.x * sc, v1.y * sc);
     }
-    if (tid == 0) *s.task = 0;
     __syncthreads();
-
-    for (;;) {
-      int task = 0;
-      if (lane == 0) task = atomicAdd(s.task, 1);
-      task = __shfl_sync(0xffffffffu, task, 0);
-      if (task >= T * T) break;
-      const int pa = task / T;
-      const int rb = task - pa * T;  // the task's row
-      const int b0lo = max(pa - W + 1 - kLMin, 0), b0hi = min(pa - kLMin, 15);
-      // cell sums of channel pairs (0, 1) and (2, 3) of each pair group, and their TwoSum errors
-      float2 hi01[CPL], hi23[CPL], lo01[CPL], lo23[CPL];
+    const int c = s_cnt[tid];
+    int incl = c;
 #pragma unroll
-      for (int u = 0; u < CPL; ++u) {
-        hi01[u] = hi23[u] = lo01[u] = lo23[u] = make_float2(0.f, 0.f);
-      }
-      bool any = false;
-      const float2 *w2c = recs + Rec::W2 + c;  // this lane's column weight, record 0
-      for (int l1g = rb; l1g > rb - W; l1g -= kFoldRanges) {
-        float2 part01[CPL], part23[CPL];  // packed FP32 (FFMA2), same rounding as fmaf
-#pragma unroll
-        for (int u = 0; u < CPL; ++u) {
-          part01[u] = make_float2(0.f, 0.f);
-          part23[u] = make_float2(0.f, 0.f);
-        }
-        bool in = false;
-#pragma unroll
-        for (int sr = 0; sr < kFoldRanges; ++sr) {
-          const int l1 = l1g - sr;
-          const int b1 = l1 - kLMin;
-          if (l1 <= rb - W || b1 < 0 || b1 > 15 || b0lo > b0hi) continue;
-          const int ibeg = s.off[(b1 << 4) | b0lo], iend = s.off[((b1 << 4) | b0hi) + 1];
-          in |= lane_live && ibeg < iend;
-          const int k1 = Rec::W1 + (lane_live ? rb - l1 : W);  // a zero slot for idle lanes
-          // two points per iteration; a lane whose column is outside a point's window
-          // multiplies by a zero weight
-          int i = ibeg;
-          for (; i + 1 < iend; i += 2) {
-            const float2 *ra = recs + i * F2, *rb2 = ra + F2;
-            const float2 wa = __fmul2_rn(__fmul2_rn(ra[pa], ra[k1]), w2c[i * F2]);
-            const float2 wb = __fmul2_rn(__fmul2_rn(rb2[pa], rb2[k1]), w2c[(i + 1) * F2]);
-#pragma unroll
-            for (int u = 0; u < CPL; ++u) {
-              const float4 xa = s_val[i * NP + gv + G * u];
-              const float4 xb = s_val[(i + 1) * NP + gv + G * u];
-              part01[u] = __ffma2_rn(wa, make_float2(xa.x, xa.y), part01[u]);
-              part23[u] = __ffma2_rn(wa, make_float2(xa.z, xa.w), part23[u]);
-              part01[u] = __ffma2_rn(wb, make_float2(xb.x, xb.y), part01[u]);
-              part23[u] = __ffma2_rn(wb, make_float2(xb.z, xb.w), part23[u]);
-            }
-          }
-          if (i < iend) {
-            const float2 *ra = recs + i * F2;
-            const float2 wa = __fmul2_rn(__fmul2_rn(ra[pa], ra[k1]), w2c[i * F2]);
-#pragma unroll
-            for (int u = 0; u < CPL; ++u) {
-              const float4 xa = s_val[i * NP + gv + G * u];
-              part01[u] = __ffma2_rn(wa, make_float2(xa.x, xa.y), part01[u]);
-              part23[u] = __ffma2_rn(wa, make_float2(xa.z, xa.w), part23[u]);
-            }
-          }
-        }
-        if (!in) continue;
-        if (!any) {  // the first group: its fold, TwoSum(0, sum), is (sum, 0) exactly
-#pragma unroll
-          for (int u = 0; u < CPL; ++u) {
-            hi01[u] = part01[u];
-            hi23[u] = part23[u];
-          }
-        } else {
-#pragma unroll
-          for (int u = 0; u < CPL; ++u) {
-            if (!COMP) {
-              hi01[u] = __fadd2_rn(hi01[u], part01[u]);
-              hi23[u] = __fadd2_rn(hi23[u], part23[u]);
-            } else {
-              two_sum2(hi01[u], lo01[u], part01[u]);
-              two_sum2(hi23[u], lo23[u], part23[u]);
-            }
-          }
-        }
-        any = true;
-      }
-      // the finished cell goes to the global grid
-      if (!any) continue;
-      const long long ro = s.rowoff[pa * T + rb];
-      const int co = s.coloff[c];
-      if (ro < 0 || co < 0) continue;
-#pragma unroll
-      for (int u = 0; u < CPL; ++u) {
-        const int pp = p0 + gv + G * u;
-        const float2 x01 = COMP ? __fadd2_rn(hi01[u], lo01[u]) : hi01[u];
-        const float2 x23 = COMP ? __fadd2_rn(hi23[u], lo23[u]) : hi23[u];
-        float2 *dst = a.grid + (ro + co) * a.cs + (int64_t)(a.ch0 + 2 * pp) * a.chs;
-        if (2 * pp < a.nch && (x01.x != 0.0f || x01.y != 0.0f)) atomicAdd(dst, x01);
-        if (2 * pp + 1 < a.nch && (x23.x != 0.0f || x23.y != 0.0f)) atomicAdd(dst + a.chs, x23);
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += x;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    int before = 0;
+    for (int w = 0; w < warp; ++w) before += s_warp[w];
+    const int off = before + incl - c;
+    s_off[tid] = off;
+    __syncthreads();
+    if (live) {
+      const int slot = s_off[key] + rank;
+      s_v0[slot] = v0;
+      s_v1[slot] = v1;
+    }
+    __syncthreads();
+    any = any || c > 0;
+    for (int i = off; i < off + c; ++i) {
+      const float2 x = s_v0[i], y = s_v1[i];
+      if (COMP) {
+        two_sum(h0.x, l0.x, x.x);
+        two_sum(h0.y, l0.y, x.y);
+        two_sum(h1.x, l1.x, y.x);
+        two_sum(h1.y, l1.y, y.y);
+      } else {
+        h0 = __fadd2_rn(h0, x);
+        h1 = __fadd2_rn(h1, y);
       }
     }
   }
+  if (!any) return;
+  const int m0 = st.ts0 + tid / (kBin * kBin), m1 = st.ts1 + (tid / kBin) % kBin, m2 = st.ts2 + tid % kBin;
+  const int n = a.g.n;  // a cell with points lies in the grid
+  const int64_t cell = ((int64_t)wrap1(m0 + a.shift, n) * n + wrap1(m1 + a.shift, n)) * n + wrap1(m2 + a.shift, n);
+  float2 *dst = a.grid + cell * a.cs + (int64_t)a.ch0 * a.chs;
+  const float2 x0 = __fadd2_rn(h0, l0), x1 = __fadd2_rn(h1, l1);
+  if (alone) {
+    *dst = __fadd2_rn(*dst, x0);
+    if (a.nch > 1) dst[a.chs] = __fadd2_rn(dst[a.chs], x1);
+  } else {
+    atomicAdd(dst, x0);
+    if (a.nch > 1) atomicAdd(dst + a.chs, x1);
+  }
 }
 
-// Spreading for the ES windows (W = 4 .. 8), any number of channels.  One block per subproblem (a bin
+// Spreading for the ES windows (W = 4 .. 8) and the linear one (W = 2), any number of channels.  One block per subproblem (a bin
 // of 8^3 cells and at most max_sub of its points); the cells it can reach are a tile of T^3,
 // T = 8 + W - 1.  The block sorts its points by (axis-2 group, l1, l0), l the bin-local corner of
 // their window and a group GS = 9 - W neighbouring l2, so that the windows of a group lie in the
@@ -765,7 +526,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 2) spread_tile_kernel(const S
 
 template <typename Kernel>
 int launch_spread_kernel(Kernel kernel, const char *name, size_t smem, const SpreadParams &a, int64_t max_blocks,
-                         cudaStream_t st, int warps = kSpreadWarps) {
+                         cudaStream_t st, int warps) {
   if (smem > 227 * 1024) {
     set_error("spreading stage of %zu bytes exceeds shared memory", smem);
     return COV3D_EINVAL;
@@ -778,27 +539,11 @@ int launch_spread_kernel(Kernel kernel, const char *name, size_t smem, const Spr
   return launched(name);
 }
 
-// One launch for all channels: the block sorts and stages its points once.  With three or more
-// channel pairs a lane group takes two pairs of a row task (bilinear step: 4.6 against 7.4 ms with
-// tasks of three rows over two lane halves), otherwise the (at most two, G >= 2) pairs are spread
-// over the lane groups.
-template <int KT, int W, bool COMP, bool HALF>
-int launch_wc(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
-  constexpr int T = kBin + W - 1;
-  constexpr int G = SpreadLanes<W>::G;
-  a.ch0 = 0;
-  a.nch = nchan;
-  const int npairs = (nchan + 1) / 2;
-  if (npairs >= 3) {
-    constexpr int CPL = 2;
-    const size_t smem = (size_t)a.max_sub * G * CPL * sizeof(float4) +
-                        stage_bytes(a.max_sub, T, PointRec<W, 1>::F2, sizeof(float2));
-    return launch_spread_kernel(spread_kernel<KT, W, CPL, COMP, HALF>, "spread_kernel", smem, a, max_blocks, st);
-  }
-  static_assert(2 * G >= 2, "at most two channel pairs spread over the lane groups");
-  const size_t smem =
-      (size_t)a.max_sub * G * sizeof(float4) + stage_bytes(a.max_sub, T, PointRec<W, 1>::F2, sizeof(float2));
-  return launch_spread_kernel(spread_kernel<KT, W, 1, COMP, HALF>, "spread_kernel", smem, a, max_blocks, st);
+template <typename Value>
+int launch_nearest(const SpreadParams &a, const Value &value, bool comp, int64_t max_blocks, cudaStream_t st) {
+  if (comp) spread_nearest_kernel<true, Value><<<(unsigned)max_blocks, kNearestThreads, 0, st>>>(a, value);
+  else spread_nearest_kernel<false, Value><<<(unsigned)max_blocks, kNearestThreads, 0, st>>>(a, value);
+  return launched("spread_nearest_kernel");
 }
 
 template <int KT, int W, int F, int NQ, int PP, bool HALF>
@@ -827,14 +572,19 @@ int launch_tile_channels(SpreadParams a, int nchan, int64_t max_blocks, cudaStre
 }
 
 template <int KT, int W>
-int launch_w(SpreadParams a, int nchan, bool comp, int64_t max_blocks, cudaStream_t st) {
-  if constexpr (KT != COV3D_KERNEL_NEAREST) {
-    return a.half ? launch_tile_channels<KT, W, true>(a, nchan, max_blocks, st)
-                  : launch_tile_channels<KT, W, false>(a, nchan, max_blocks, st);
-  } else {
-    return comp ? launch_wc<KT, W, true, false>(a, nchan, max_blocks, st)
-                : launch_wc<KT, W, false, false>(a, nchan, max_blocks, st);
+int launch_w(const SpreadParams &a, int nchan, int64_t max_blocks, cudaStream_t st) {
+  return a.half ? launch_tile_channels<KT, W, true>(a, nchan, max_blocks, st)
+                : launch_tile_channels<KT, W, false>(a, nchan, max_blocks, st);
+}
+
+// Channels of an array two at a time
+int launch_nearest_channels(SpreadParams a, int nchan, bool comp, int64_t max_blocks, cudaStream_t st) {
+  for (int c = 0; c < nchan; c += 2) {
+    a.ch0 = c;
+    a.nch = min(2, nchan - c);
+    COV3D_TRY(launch_nearest(a, ArrayValue{a.vals + (int64_t)c * a.ics, a.ips, a.ics, a.nch}, comp, max_blocks, st));
   }
+  return COV3D_OK;
 }
 
 // Per-image adjoint (no sum over images): direct global atomics, one thread per point.
@@ -880,15 +630,20 @@ __global__ void spread_unagg_kernel(PointGeom g, KernelSpec k, int64_t M, const 
 
 }  // namespace
 
-int launch_spread(cov3d_plan *p, const void *values, int64_t in_ps, int64_t in_cs, int nchan, const EpilogueArgs &e,
-                  void *grid, int64_t cell_stride, int64_t chan_stride, int shift, SortMode mode) {
+// What every spreading launch of a plan's points shares.
+static int spread_params(cov3d_plan *p, const EpilogueArgs &e, void *grid, int64_t cell_stride, int64_t chan_stride,
+                         int shift, SortMode mode, SpreadParams &a, int64_t &max_blocks) {
   if (p->point_kind == kPointsNone || p->n_points == 0) {
     set_error("no points set");
     return COV3D_ESTATE;
   }
+  if (p->bins.bs[0] != kBin || p->bins.bs[1] != kBin || p->bins.bs[2] != kBin) {
+    set_error("spreading requires %d^3-cell bins", kBin);
+    return COV3D_EINVAL;
+  }
   COV3D_TRY(need_sorted(p, 1u << mode));
   const SortSet &ss = p->sets[mode];
-  SpreadParams a{};
+  a = SpreadParams{};
   a.g = make_geom(p);
   a.k = make_kernel(p);
   a.bins = p->bins;
@@ -896,10 +651,8 @@ int launch_spread(cov3d_plan *p, const void *values, int64_t in_ps, int64_t in_c
   a.sub_bin = ss.sub_bin;
   a.sub_first = ss.sub_first;
   a.sub_count = ss.sub_count;
+  a.bin_off = ss.bin_off;
   a.nsub = ss.nsub;
-  a.vals = static_cast<const float2 *>(values);
-  a.ips = in_ps;
-  a.ics = in_cs;
   a.ctf = e.ctf;
   a.ctfc = e.ctfc;
   a.nyquist = e.nyquist;
@@ -910,25 +663,40 @@ int launch_spread(cov3d_plan *p, const void *values, int64_t in_ps, int64_t in_c
   a.shift = shift;
   a.max_sub = p->max_sub;
   a.half = mode == kSortHalf;
-  if (p->bins.bs[0] != kBin || p->bins.bs[1] != kBin || p->bins.bs[2] != kBin) {
-    set_error("spreading requires %d^3-cell bins", kBin);
-    return COV3D_EINVAL;
-  }
-  const int64_t max_blocks = p->bins.nbins + p->n_points / p->max_sub + 1;
-  const bool comp = p->compensated != 0;
+  max_blocks = p->bins.nbins + p->n_points / p->max_sub + 1;
+  return COV3D_OK;
+}
+
+int launch_spread(cov3d_plan *p, const void *values, int64_t in_ps, int64_t in_cs, int nchan, const EpilogueArgs &e,
+                  void *grid, int64_t cell_stride, int64_t chan_stride, int shift, SortMode mode) {
+  SpreadParams a;
+  int64_t mb;
+  COV3D_TRY(spread_params(p, e, grid, cell_stride, chan_stride, shift, mode, a, mb));
+  a.vals = static_cast<const float2 *>(values);
+  a.ips = in_ps;
+  a.ics = in_cs;
   switch (p->kernel) {
-    case COV3D_KERNEL_NEAREST: return launch_w<COV3D_KERNEL_NEAREST, 1>(a, nchan, comp, max_blocks, p->stream);
-    case COV3D_KERNEL_LINEAR: return launch_w<COV3D_KERNEL_LINEAR, 2>(a, nchan, comp, max_blocks, p->stream);
+    case COV3D_KERNEL_NEAREST: return launch_nearest_channels(a, nchan, p->compensated != 0, mb, p->stream);
+    case COV3D_KERNEL_LINEAR: return launch_w<COV3D_KERNEL_LINEAR, 2>(a, nchan, mb, p->stream);
     default:
       switch (p->width) {
-        case 4: return launch_w<COV3D_KERNEL_ES, 4>(a, nchan, comp, max_blocks, p->stream);
-        case 5: return launch_w<COV3D_KERNEL_ES, 5>(a, nchan, comp, max_blocks, p->stream);
-        case 6: return launch_w<COV3D_KERNEL_ES, 6>(a, nchan, comp, max_blocks, p->stream);
-        case 7: return launch_w<COV3D_KERNEL_ES, 7>(a, nchan, comp, max_blocks, p->stream);
-        case 8: return launch_w<COV3D_KERNEL_ES, 8>(a, nchan, comp, max_blocks, p->stream);
+        case 4: return launch_w<COV3D_KERNEL_ES, 4>(a, nchan, mb, p->stream);
+        case 5: return launch_w<COV3D_KERNEL_ES, 5>(a, nchan, mb, p->stream);
+        case 6: return launch_w<COV3D_KERNEL_ES, 6>(a, nchan, mb, p->stream);
+        case 7: return launch_w<COV3D_KERNEL_ES, 7>(a, nchan, mb, p->stream);
+        case 8: return launch_w<COV3D_KERNEL_ES, 8>(a, nchan, mb, p->stream);
         default: set_error("unsupported ES width %d (supported: 4..8)", p->width); return COV3D_EINVAL;
       }
   }
+}
+
+int launch_spread_mean_nearest(cov3d_plan *p, const MeanSource &src, const EpilogueArgs &e, void *grids,
+                               int64_t chan_stride) {
+  SpreadParams a;
+  int64_t mb;
+  COV3D_TRY(spread_params(p, e, grids, 1, chan_stride, 0, kSortFull, a, mb));
+  a.nch = 2;
+  return launch_nearest(a, MeanValue{src}, p->compensated != 0, mb, p->stream);
 }
 
 int launch_spread_unaggregated(cov3d_plan *p, const void *values, int64_t in_ps, const EpilogueArgs &e,
