@@ -10,7 +10,7 @@
 //   C = (conj(m^-1) + conj(z) z^T) / (2 s2),  u = -conj(z) / (2 s2)
 // LS objective (raw_cost_fourier_domain, covar_sgd.py:1320-1347), M = conj(gram), t = conj(h):
 //   cost_b = -2 |t|^2 + ||M||_F^2 + 2 s2 tr M,  C = 2 M + 2 s2 I,  u = -2 t
-// The r x r factorisations run in FP64 (one thread per image).
+// The r x r factorisations run in FP64 (a few threads per image).
 #include "cov3d_device.cuh"
 
 namespace cov3d {
@@ -292,28 +292,7 @@ __device__ __forceinline__ cd cmul(cd a, cd b) { return {a.x * b.x - a.y * b.y, 
 __device__ __forceinline__ cd cconj(cd a) { return {a.x, -a.y}; }
 __device__ __forceinline__ cd csub(cd a, cd b) { return {a.x - b.x, a.y - b.y}; }
 
-// In-place Cholesky m = L L^H (lower triangle); returns log det m, NaN if m is not positive
-// definite.  The diagonal entry (k, k) holds {L_kk, 1 / L_kk}, so the triangular solves
-// multiply instead of dividing.
-__device__ double chol_logdet(cd *m, int r) {
-  double logdet = 0.0;
-  for (int k = 0; k < r; ++k) {
-    double d = m[k * r + k].x;
-    for (int j = 0; j < k; ++j) d -= m[k * r + j].x * m[k * r + j].x + m[k * r + j].y * m[k * r + j].y;
-    if (!(d > 0.0)) return __longlong_as_double(0x7ff8000000000000ULL);
-    const double lkk = sqrt(d), inv = 1.0 / lkk;
-    m[k * r + k] = {lkk, inv};
-    logdet += 2.0 * log(lkk);
-    for (int i = k + 1; i < r; ++i) {
-      cd s = m[i * r + k];
-      for (int j = 0; j < k; ++j) s = csub(s, cmul(m[i * r + j], cconj(m[k * r + j])));
-      m[i * r + k] = {s.x * inv, s.y * inv};
-    }
-  }
-  return logdet;
-}
-
-// Solve (L L^H) x = rhs in place, L from chol_logdet.
+// Solve (L L^H) x = rhs in place; the diagonal entry (k, k) of Lm holds {L_kk, 1 / L_kk}.
 __device__ void chol_solve(const cd *Lm, int r, cd *x) {
   for (int i = 0; i < r; ++i) {
     cd s = x[i];
@@ -348,122 +327,139 @@ struct SolveArgs {
   int *bad;            // set to 1 if a factorisation failed
 };
 
-// Thread kc of image b.  Every one of the image's r threads factors m (the same arithmetic,
-// so the same bits) and solves for z; thread kc then writes column kc of C from column kc of
-// m^-1, and thread 0 the per-image outputs (cost, z, m, u).  RMAX sizes the per-thread
-// working arrays (local memory): the smallest class that holds r keeps them in L1.
-// *glog receives the image's d cost / d log s_kc (the projections' channel kc scaled by s_kc):
-// 2 Re sum_p conj(W_pk) Q_pk, which m z = b and m^-1 gram / s2 = I - m^-1 (identity prior) turn into
+constexpr int kSolveThreads = 128;
+
+// r + 1 threads per image, kSolveThreads / (r + 1) images per block, each image's matrix in shared
+// memory.  ML: thread i < r computes row i of the Cholesky factor column by column (left-looking,
+// one barrier per column; every thread of the image forms the pivot itself), then solves for column i
+// of m^-1 while thread r solves for z; RMAX sizes the threads' right-hand sides.  Latency is the
+// bound, so each image is factored once by all its threads (each of r threads used to factor it alone
+// in local memory: 204 -> 84 us at r = 10, B = 1024, 879 -> 235 us at r = 20, B = 300, 64 -> 34 us at r = 10, B = 64); the
+// operations and their order are those of one thread's factorisation.
+// glog receives d cost / d log s_k (the projections' channel k scaled by s_k), 2 Re sum_p conj(W_pk)
+// Q_pk, which m z = b and m^-1 gram / s2 = I - m^-1 (identity prior) turn into
 // wscale (1 - (m^-1)_kk - |z_k|^2) for ML -- no cancellation -- and
 // wscale (4 sum_i |gram_ik|^2 + 4 s2 gram_kk - 4 |h_k|^2) for LS.
 template <int RMAX>
-__device__ double solve_one(const SolveArgs &a, const int b, const int kc, double *glog) {
-  const int r = a.r;
-  cd m[RMAX * RMAX];
-  cd z[RMAX];
-  cd bb[RMAX];
+__global__ void __launch_bounds__(kSolveThreads) solve_kernel(const SolveArgs a) {
+  extern __shared__ double2 solve_smem[];
+  __shared__ double s_glog[kSolveThreads], wsum[kSolveThreads / 32];
+  const int r = a.r, ipb = kSolveThreads / (r + 1);
+  const int im = threadIdx.x / (r + 1), kc = threadIdx.x - im * (r + 1);
+  const int b = blockIdx.x * ipb + im;
+  const bool live = im < ipb && b < a.B;
+  cd *m = reinterpret_cast<cd *>(solve_smem) + (size_t)(im < ipb ? im : 0) * (r * r + 2 * r);  // r * r
+  cd *s_z = m + r * r, *s_b = s_z + r;                                                           // r each
   const float2 *G = a.gram + (int64_t)b * r * r;
   const float2 *hb = a.h + (int64_t)b * r;
-  double cost = 0.0;
+  double cost = 0.0, glog = 0.0;
   if (a.objective == 0) {
-    for (int i = 0; i < r; ++i) {
-      for (int j = 0; j < r; ++j) {
-        const float2 g = G[i * r + j];
-        double add = a.linv ? a.linv[i * r + j] : (i == j ? 1.0 : 0.0);
-        m[i * r + j] = {g.x / a.s2 + add, g.y / a.s2};
+    if (live) {
+      for (int e = kc; e < r * r; e += r + 1) {
+        const int i = e / r, j = e - i * r;
+        const float2 g = G[e];
+        const double add = a.linv ? a.linv[e] : (i == j ? 1.0 : 0.0);
+        m[e] = {g.x / a.s2 + add, g.y / a.s2};
+        if (a.m_out) a.m_out[(int64_t)b * r * r + e] = make_float2((float)m[e].x, (float)m[e].y);
       }
-      bb[i] = {hb[i].x / a.s2, hb[i].y / a.s2};
+      if (kc < r) s_b[kc] = {hb[kc].x / a.s2, hb[kc].y / a.s2};
     }
-    if (a.m_out && kc == 0) {
-      for (int i = 0; i < r * r; ++i) a.m_out[(int64_t)b * r * r + i] = make_float2((float)m[i].x, (float)m[i].y);
+    __syncthreads();
+    double logdet = 0.0;
+    bool ok = true;
+    for (int k = 0; k < r; ++k) {
+      cd lik = {0.0, 0.0};
+      if (live && ok) {
+        double d = m[k * r + k].x;
+        for (int j = 0; j < k; ++j) d -= m[k * r + j].x * m[k * r + j].x + m[k * r + j].y * m[k * r + j].y;
+        if (!(d > 0.0)) {
+          ok = false;  // the same for every thread of the image
+          if (kc == 0) atomicExch(a.bad, 1);
+        } else {
+          const double lkk = sqrt(d), inv = 1.0 / lkk;
+          if (kc == r) logdet += 2.0 * log(lkk);
+          if (kc == k) {
+            lik = {lkk, inv};
+          } else if (kc > k && kc < r) {
+            cd s = m[kc * r + k];
+            for (int j = 0; j < k; ++j) s = csub(s, cmul(m[kc * r + j], cconj(m[k * r + j])));
+            lik = {s.x * inv, s.y * inv};
+          }
+        }
+      }
+      __syncthreads();  // (k, k) has been read as the pivot's own entry
+      if (live && ok && kc >= k && kc < r) m[kc * r + k] = lik;
+      __syncthreads();
     }
-    const double logdet = chol_logdet(m, r);
-    if (!(logdet == logdet)) {
-      atomicExch(a.bad, 1);
-      return 0.0;
+    cd x[RMAX];
+    const bool solves = live && ok;
+    if (solves && (kc == r || a.C)) {
+      for (int i = 0; i < r; ++i) x[i] = kc == r ? s_b[i] : cd{i == kc ? 1.0 : 0.0, 0.0};
+      chol_solve(m, r, x);
     }
-    for (int i = 0; i < r; ++i) z[i] = bb[i];
-    chol_solve(m, r, z);
-    double bz = 0.0;
-    for (int i = 0; i < r; ++i) bz += bb[i].x * z[i].x + bb[i].y * z[i].y;
-    cost = 0.5 * (-bz + logdet);
-    if (a.z_out && kc == 0) {
-      for (int i = 0; i < r; ++i) a.z_out[(int64_t)b * r + i] = make_float2((float)z[i].x, (float)z[i].y);
-    }
-    if (a.C) {
-      // column kc of m^-1: solve m x = e_kc; C_ij = (conj(minv_ij) + conj(z_i) z_j) / (2 s2)
-      const double f = a.wscale / (2.0 * a.s2);
-      cd col[RMAX];
-      for (int i = 0; i < r; ++i) col[i] = {i == kc ? 1.0 : 0.0, 0.0};
-      chol_solve(m, r, col);
-      *glog = a.wscale * (1.0 - col[kc].x - (z[kc].x * z[kc].x + z[kc].y * z[kc].y));
+    if (solves && kc == r) {
+      double bz = 0.0;
       for (int i = 0; i < r; ++i) {
-        const cd zz = cmul(cconj(z[i]), z[kc]);
-        a.C[((int64_t)b * r + i) * r + kc] = make_float2((float)((col[i].x + zz.x) * f), (float)((-col[i].y + zz.y) * f));
+        bz += s_b[i].x * x[i].x + s_b[i].y * x[i].y;
+        s_z[i] = x[i];
+        if (a.z_out) a.z_out[(int64_t)b * r + i] = make_float2((float)x[i].x, (float)x[i].y);
       }
-      if (kc == 0) {
-        for (int i = 0; i < r; ++i) a.u[(int64_t)b * r + i] = make_float2((float)(-z[i].x * f), (float)(z[i].y * f));
+      cost = 0.5 * (-bz + logdet);
+    }
+    __syncthreads();
+    if (solves && a.C) {
+      // C_ij = (conj(minv_ij) + conj(z_i) z_j) / (2 s2), column kc
+      const double f = a.wscale / (2.0 * a.s2);
+      if (kc < r) {
+        const cd zk = s_z[kc];
+        glog = a.wscale * (1.0 - x[kc].x - (zk.x * zk.x + zk.y * zk.y));
+        for (int i = 0; i < r; ++i) {
+          const cd zz = cmul(cconj(s_z[i]), zk);
+          a.C[((int64_t)b * r + i) * r + kc] = make_float2((float)((x[i].x + zz.x) * f), (float)((-x[i].y + zz.y) * f));
+        }
+        a.u[(int64_t)b * r + kc] = make_float2((float)(-zk.x * f), (float)(zk.y * f));
       }
     }
-  } else {
-    if (a.C) {
-      double g2 = 0.0;
-      for (int i = 0; i < r; ++i) g2 += (double)G[i * r + kc].x * G[i * r + kc].x + (double)G[i * r + kc].y * G[i * r + kc].y;
-      const double h2 = (double)hb[kc].x * hb[kc].x + (double)hb[kc].y * hb[kc].y;
-      *glog = 4.0 * a.wscale * (g2 + a.s2 * G[kc * r + kc].x - h2);
-    }
-    // the rest: thread 0 of the image
-    if (kc != 0) return 0.0;
-    double t2 = 0.0, fro = 0.0, tr = 0.0;
-    for (int i = 0; i < r; ++i) {
-      t2 += (double)hb[i].x * hb[i].x + (double)hb[i].y * hb[i].y;
-      tr += G[i * r + i].x;
-      for (int j = 0; j < r; ++j) fro += (double)G[i * r + j].x * G[i * r + j].x + (double)G[i * r + j].y * G[i * r + j].y;
-    }
-    cost = -2.0 * t2 + fro + 2.0 * a.s2 * tr;
+  } else if (live && kc < r) {  // least squares: M = conj(gram), t = conj(h)
+    double g2 = 0.0;
+    for (int i = 0; i < r; ++i) g2 += (double)G[i * r + kc].x * G[i * r + kc].x + (double)G[i * r + kc].y * G[i * r + kc].y;
+    const double h2 = (double)hb[kc].x * hb[kc].x + (double)hb[kc].y * hb[kc].y;
     if (a.C) {
       const double f = a.wscale;
+      glog = 4.0 * f * (g2 + a.s2 * G[kc * r + kc].x - h2);
       for (int i = 0; i < r; ++i) {
-        for (int j = 0; j < r; ++j) {
-          const float2 g = G[i * r + j];  // M_ij = conj(gram_ij)
-          a.C[((int64_t)b * r + i) * r + j] =
-              make_float2((float)((2.0 * g.x + (i == j ? 2.0 * a.s2 : 0.0)) * f), (float)(-2.0 * g.y * f));
-        }
-        // u_i = -2 t_i = -2 conj(h_i)
-        a.u[(int64_t)b * r + i] = make_float2((float)(-2.0 * hb[i].x * f), (float)(2.0 * hb[i].y * f));
+        const float2 g = G[i * r + kc];  // M_ij = conj(gram_ij)
+        a.C[((int64_t)b * r + i) * r + kc] =
+            make_float2((float)((2.0 * g.x + (i == kc ? 2.0 * a.s2 : 0.0)) * f), (float)(-2.0 * g.y * f));
       }
+      a.u[(int64_t)b * r + kc] = make_float2((float)(-2.0 * hb[kc].x * f), (float)(2.0 * hb[kc].y * f));
+    }
+    if (kc == 0) {
+      double t2 = 0.0, fro = 0.0, tr = 0.0;
+      for (int i = 0; i < r; ++i) {
+        t2 += (double)hb[i].x * hb[i].x + (double)hb[i].y * hb[i].y;
+        tr += G[i * r + i].x;
+        for (int j = 0; j < r; ++j) fro += (double)G[i * r + j].x * G[i * r + j].x + (double)G[i * r + j].y * G[i * r + j].y;
+      }
+      cost = -2.0 * t2 + fro + 2.0 * a.s2 * tr;
     }
   }
-  if (kc != 0) return 0.0;
-  cost *= a.cscale;
-  if (a.cost_b) a.cost_b[b] = cost;
-  return cost;
-}
-
-constexpr int kSolveThreads = 128;
-
-// r threads per image, kSolveThreads / r images per block; the images' costs are summed per
-// block (one FP64 atomic per block instead of one per image on the same address)
-template <int RMAX>
-__global__ void __launch_bounds__(kSolveThreads) solve_kernel(const SolveArgs a) {
-  const int ipb = kSolveThreads / a.r;
-  const int b = blockIdx.x * ipb + threadIdx.x / a.r;
-  const int kc = threadIdx.x - (threadIdx.x / a.r) * a.r;
-  double glog = 0.0;
-  double cost = (threadIdx.x < ipb * a.r && b < a.B) ? solve_one<RMAX>(a, b, kc, &glog) : 0.0;
+  // the image's cost is with one thread: z's, or the first in least squares
+  const bool teller = live && kc == (a.objective == 0 ? r : 0);
+  cost = teller ? cost * a.cscale : 0.0;
+  if (teller && a.cost_b) a.cost_b[b] = cost;
   if (!a.cost_sum) return;
   if (a.glog) {  // the block's images summed per channel
-    __shared__ double s_gl[kSolveThreads];
-    s_gl[threadIdx.x] = glog;
+    s_glog[threadIdx.x] = glog;
     __syncthreads();
-    if ((int)threadIdx.x < a.r) {
+    if ((int)threadIdx.x < r) {
       double t = 0.0;
-      for (int i = 0; i < ipb; ++i) t += s_gl[i * a.r + threadIdx.x];
+      for (int i = 0; i < ipb; ++i) t += s_glog[i * (r + 1) + threadIdx.x];
       atomicAdd(a.glog + threadIdx.x, t);
     }
   }
+  // the images' costs summed per block (one FP64 atomic per block)
   for (int o = 16; o > 0; o >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, o);
-  __shared__ double wsum[kSolveThreads / 32];
   if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = cost;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -638,18 +634,20 @@ int launch_solve(cudaStream_t st, int B, int r, int objective, const void *gram,
   sa.z_out = static_cast<float2 *>(z);
   sa.m_out = static_cast<float2 *>(m);
   sa.bad = bad;
-  static_assert(kMaxRank <= kSolveThreads, "one thread per column of every image");
-  const int ipb = kSolveThreads / r;
+  static_assert(kMaxRank + 1 <= kSolveThreads, "a thread per column of every image and one for z");
+  const int ipb = kSolveThreads / (r + 1);
   const unsigned blocks = (unsigned)((B + ipb - 1) / ipb);
-  if (r <= 10) {
-    solve_kernel<10><<<blocks, kSolveThreads, 0, st>>>(sa);
-  } else if (r <= 16) {
-    solve_kernel<16><<<blocks, kSolveThreads, 0, st>>>(sa);
-  } else if (r <= 20) {
-    solve_kernel<20><<<blocks, kSolveThreads, 0, st>>>(sa);
-  } else {
-    solve_kernel<kMaxRank><<<blocks, kSolveThreads, 0, st>>>(sa);
-  }
+  const size_t smem = objective == 0 ? (size_t)ipb * (r * r + 2 * r) * sizeof(cd) : 0;
+  auto launch = [&](auto kernel) -> int {
+    if (smem > 40 * 1024)
+      COV3D_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<blocks, kSolveThreads, smem, st>>>(sa);
+    return COV3D_OK;
+  };
+  if (r <= 10) COV3D_TRY(launch(solve_kernel<10>));
+  else if (r <= 16) COV3D_TRY(launch(solve_kernel<16>));
+  else if (r <= 20) COV3D_TRY(launch(solve_kernel<20>));
+  else COV3D_TRY(launch(solve_kernel<kMaxRank>));
   return launched("solve_kernel");
 }
 

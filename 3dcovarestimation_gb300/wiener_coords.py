@@ -1,7 +1,7 @@
 """Per-image Wiener / latent-MAP coordinates (drop-in for ``cov3d.wiener_coords``).
 
 ``compute_latentMAP_batch`` runs the per-image Gram contractions in FP32 on the GPU and the
-r x r Hermitian solve (Cholesky) in FP64, one thread per image (reference
+r x r Hermitian solve (Cholesky) in FP64, r + 1 threads per image (reference
 ``wiener_coords.py:168-203``).  ``latentMAP`` loops over the dataset in batches like
 ``wiener_coords.py:85-165``; ``wiener_coords`` (``wiener_coords.py:13-82``) gives the same
 posterior mean through the same two kernels (see its docstring).

@@ -379,7 +379,7 @@ int cov3d_resample3d(void *stream, const float *d_in, int64_t NC, int d, int D, 
  * file-scope device array that each GPU loading the library keeps until exit; the call
  * allocates nothing (no cudaMalloc / cudaFree / allocating library routine).  Two caveats:
  * the first launch of the solve kernel at a given rank may make the driver enlarge its
- * per-thread local-memory reservation (the kernel's r x r working arrays), so warm up once
+ * per-thread local-memory reservation (the kernel's working vectors), so warm up once
  * at the largest rank you will use; and the array's device address is looked up once per
  * device and kept, which assumes the runtime's primary context on that device for the life
  * of the process (after cudaDeviceReset, or with another context current, the kept address
