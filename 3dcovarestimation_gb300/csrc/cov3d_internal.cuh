@@ -187,6 +187,11 @@ PointGeom make_geom(const cov3d_plan *p);
 KernelSpec make_kernel(const cov3d_plan *p);
 int get_fft(cov3d_plan *p, int nchan, cufftHandle *out);
 int get_fft_planes(cov3d_plan *p, cufftHandle *out);
+int get_fft_all_planes(cov3d_plan *p, int nchan, cufftHandle *out);
+bool fft_ready(cov3d_plan *p, int key);
+int grid_fft(cov3d_plan *p, float2 *grid, int nchan, int dir);
+int volume_to_grid(cov3d_plan *p, const float *vr, const void *vc, int nchan, float2 *grid);
+int grid_to_volume(cov3d_plan *p, float2 *grid, int nchan, void *out);
 int get_fft_axis0(cov3d_plan *p, cufftHandle *out);
 int fft2(cufftHandle h, const float2 *in, float2 *out, int dir);
 
@@ -216,7 +221,14 @@ int cg_operator_lines(cov3d_plan *p, const float2 *in, float2 *fine, float2 *out
                       const float2 *z = nullptr, float2 *pdir = nullptr, CgState *st = nullptr);
 int step_forward_lines(cov3d_plan *p, const float *vec, const float *logs, const float *gc, int r, float2 *stage,
                        float2 *grid, const float *fr, int64_t fr_stride, double coef, double *cost, double *glog);
-int step_inverse_lines(cov3d_plan *p, float2 *grad_grid, const float *logs, const float *gc, int r, float *gvec);
+bool grid_lines_apply(const cov3d_plan *p);
+// (nchan, L^3) volumes, real (vr) or complex (vc), to their transforms, n = 64, 128, 256
+int grid_forward_lines(cov3d_plan *p, const float *vr, const float2 *vc, const float *gc, int nchan, float2 *grid);
+// The grid's inverse transform, cropped: the step's gradient (gvec), or with `out` the volumes
+int inverse_lines(cov3d_plan *p, float2 *grid, const float *logs, const float *gc, int r, float *gvec, float2 *out);
+// Fine grids on which a transform's launches cost more than its zero planes: see grid_fft
+constexpr int kSmallGrid = 160;
+constexpr int kAllPlanesKey = -100;  // FFT plans of all planes of nchan channels: key -100 - nchan
 inline bool prunable(const cov3d_plan *p) { return p->L % 2 == 0 && p->n >= p->L + 2; }
 
 // points_sort.cu

@@ -702,18 +702,24 @@ int covar_cost_grad(cov3d_plan *p, const cov3d_cost_args *a, double *h_cost, dou
   // forward one up to n = 256: at 512 its 32 x 16 split idles half the threads in one stage and
   // measured slower than pack + cuFFT + regulariser (19.0 against 15.4 ms at L = 256, r = 10);
   // the inverse is faster at every size (8.8 against 11.1 ms there).
-  const bool lines_inv = pruned && line_transforms_apply(p);
-  const bool lines_fwd = lines_inv && p->n <= 256;
+  // n = 64 has the inverse only: its forward transform keeps cuFFT's rounding, on which the 64-bit
+  // cost depends.
+  const bool lines_inv = grid_lines_apply(p);
+  const bool lines_fwd = lines_inv && line_transforms_apply(p) && p->n <= 256;
   const bool with_reg = a->d_fourier_reg && a->reg_scale != 0.0;
   const bool ml_reg = with_reg && a->objective == 0;  // sum fr |G|^2: fused into the transforms
   const bool ls_reg = with_reg && a->objective != 0;  // |X X^H|^2: GEMMs before the spread (ls_reg.cu)
   const int64_t fr_stride = a->fourier_reg_per_channel ? n3 : 0;
   const float *gcp = a->use_grid_correction ? p->gc1d.as<float>() : nullptr;
   cufftHandle fft = 0, fplanes = 0, faxis0 = 0;
+  // Small grids: one launch for all planes of all channels instead of two per channel (the same
+  // transforms of each plane, to the bit; 5 channels of 64^3: 103 -> 33 us with axis 0, of 160^3:
+  // 226 -> 215; of 200^3 the planes outside the support cost more: 441 against 505).
+  const bool all_planes = pruned && !lines_fwd && p->n <= kSmallGrid && fft_ready(p, kAllPlanesKey - r);
   if (pruned) {
-    COV3D_TRY(grow(p->fine2, n3 * r * 8));
     if (!lines_fwd) {  // the forward transform on cuFFT
-      COV3D_TRY(get_fft_planes(p, &fplanes));
+      if (all_planes) COV3D_TRY(get_fft_all_planes(p, r, &fplanes));
+      else COV3D_TRY(get_fft_planes(p, &fplanes));
       COV3D_TRY(get_fft_axis0(p, &faxis0));
     }
   } else {
@@ -733,10 +739,13 @@ int covar_cost_grad(cov3d_plan *p, const cov3d_cost_args *a, double *h_cost, dou
   if (!lines_fwd) {
     PhaseScope ps(p, kPhaseFftFwd);
     if (pruned) {
+      if (all_planes) COV3D_TRY(fft2(fplanes, p->fine2.as<float2>(), p->fine2.as<float2>(), CUFFT_FORWARD));
       for (int c = 0; c < r; ++c) {
         float2 *src = p->fine2.as<float2>() + c * n3;
-        COV3D_TRY(fft2(fplanes, src, src, CUFFT_FORWARD));
-        COV3D_TRY(fft2(fplanes, src + half_off, src + half_off, CUFFT_FORWARD));
+        if (!all_planes) {
+          COV3D_TRY(fft2(fplanes, src, src, CUFFT_FORWARD));
+          COV3D_TRY(fft2(fplanes, src + half_off, src + half_off, CUFFT_FORWARD));
+        }
         COV3D_TRY(fft2(faxis0, src, p->fine.as<float2>() + c * n3, CUFFT_FORWARD));
       }
     } else {
@@ -797,20 +806,10 @@ int covar_cost_grad(cov3d_plan *p, const cov3d_cost_args *a, double *h_cost, dou
   // 9. adjoint FFT, 10. crop + deapodise + chain rule to the Covar parameters
   if (lines_inv) {
     PhaseScope ps(p, kPhaseFftInv);
-    COV3D_TRY(step_inverse_lines(p, p->fine2.as<float2>(), a->d_log_sqrt, gcp, r, d_grad_vectors));
+    COV3D_TRY(inverse_lines(p, p->fine2.as<float2>(), a->d_log_sqrt, gcp, r, d_grad_vectors, nullptr));
   } else {
     PhaseScope ps(p, kPhaseFftInv);
-    if (pruned) {  // axis 0 over all lines, then 2D only on the support planes the crop reads
-      for (int c = 0; c < r; ++c) {
-        float2 *g = p->fine2.as<float2>() + c * n3;
-        COV3D_TRY(fft2(faxis0, g, g, CUFFT_INVERSE));
-        COV3D_TRY(fft2(fplanes, g, g, CUFFT_INVERSE));
-        COV3D_TRY(fft2(fplanes, g + half_off, g + half_off, CUFFT_INVERSE));
-      }
-    } else {
-      COV3D_TRY(check_cufft(cufftExecC2C(fft, p->fine2.as<cufftComplex>(), p->fine2.as<cufftComplex>(), CUFFT_INVERSE),
-                            "cufftExecC2C(inverse)"));
-    }
+    COV3D_TRY(grid_fft(p, p->fine2.as<float2>(), r, CUFFT_INVERSE));
   }
   if (!lines_inv) {
     PhaseScope ps(p, kPhaseUnpack);

@@ -251,9 +251,9 @@ int launch_zero(cov3d_plan *p, void *ptr, int64_t bytes) {
   return check_cuda(cudaMemsetAsync(ptr, 0, (size_t)bytes, p->stream), "cudaMemsetAsync");
 }
 
-// Pruned transforms (even L): the zero-padded volume has L nonzero planes of n (the first and
+// Pruned transforms: the zero-padded volume has L nonzero planes of n (the first L - L/2 and the
 // last L/2 in FFT-native order) and only those planes of an inverse transform are cropped, so a
-// 3D transform is a batched 2D FFT over the L/2 support planes of each half (key -2) and a 1D FFT
+// 3D transform is a batched 2D FFT over (L + 1) / 2 planes at each end (key -2) and a 1D FFT
 // along axis 0 over all n^2 lines (key -3).
 int get_fft_planes(cov3d_plan *p, cufftHandle *out) {
   auto it = p->ffts->find(-2);
@@ -261,7 +261,7 @@ int get_fft_planes(cov3d_plan *p, cufftHandle *out) {
     cufftHandle h;
     int dims[2] = {p->n, p->n};
     COV3D_TRY(check_cufft(cufftPlanMany(&h, 2, dims, nullptr, 1, p->n * p->n, nullptr, 1, p->n * p->n, CUFFT_C2C,
-                                        p->L / 2),
+                                        (p->L + 1) / 2),
                           "cufftPlanMany(planes)"));
     it = p->ffts->emplace(-2, h).first;
   }
@@ -280,6 +280,28 @@ int get_fft_axis0(cov3d_plan *p, cufftHandle *out) {
   }
   *out = it->second;
   return check_cufft(cufftSetStream(it->second, p->stream), "cufftSetStream");
+}
+
+// 2D transforms of every plane of nchan channels
+int get_fft_all_planes(cov3d_plan *p, int nchan, cufftHandle *out) {
+  auto it = p->ffts->find(kAllPlanesKey - nchan);
+  if (it == p->ffts->end()) {
+    cufftHandle h;
+    int dims[2] = {p->n, p->n};
+    const int nn = p->n * p->n;
+    COV3D_TRY(check_cufft(cufftPlanMany(&h, 2, dims, nullptr, 1, nn, nullptr, 1, nn, CUFFT_C2C, nchan * p->n),
+                          "cufftPlanMany(all planes)"));
+    it = p->ffts->emplace(kAllPlanesKey - nchan, h).first;
+  }
+  *out = it->second;
+  return check_cufft(cufftSetStream(it->second, p->stream), "cufftSetStream");
+}
+
+// Whether the FFT plan under `key` exists or can be made now (not while the stream is capturing).
+bool fft_ready(cov3d_plan *p, int key) {
+  if (p->ffts->count(key)) return true;
+  cudaStreamCaptureStatus cap;
+  return cudaStreamIsCapturing(p->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
 }
 
 int fft2(cufftHandle h, const float2 *in, float2 *out, int dir) {
@@ -302,6 +324,50 @@ int get_fft(cov3d_plan *p, int nchan, cufftHandle *out) {
   (*p->ffts)[nchan] = h;
   *out = h;
   return check_cufft(cufftSetStream(h, p->stream), "cufftSetStream");
+}
+
+// 3D transform in place of nchan channels whose volumes occupy the support planes (forward), or of
+// which only the support planes are wanted (inverse).  Above kSmallGrid channel by channel: the
+// channel's passes meet in the L2 cache, and the 2D transforms skip the other planes (5 channels of
+// 200^3: 441 against 509 us for one batched 3D transform, of 240^3: 669 against 881).  Up to it the
+// three launches per channel cost more than they save (5 channels of 64^3: 103 against 19 us, of
+// 100^3: 114 against 45, of 160^3: 226 against 206).
+int grid_fft(cov3d_plan *p, float2 *grid, int nchan, int dir) {
+  const int n = p->n, H = (p->L + 1) / 2;
+  cufftHandle h = 0, h0 = 0;
+  if (n < p->L + 2 || (n <= kSmallGrid && fft_ready(p, nchan))) {
+    COV3D_TRY(get_fft(p, nchan, &h));
+    return fft2(h, grid, grid, dir);
+  }
+  COV3D_TRY(get_fft_planes(p, &h));
+  COV3D_TRY(get_fft_axis0(p, &h0));
+  const int64_t nn = (int64_t)n * n;
+  for (int c = 0; c < nchan; ++c) {
+    float2 *g = grid + c * nn * n, *g2 = g + (n - H) * nn;
+    if (dir == CUFFT_INVERSE) COV3D_TRY(fft2(h0, g, g, dir));
+    COV3D_TRY(fft2(h, g, g, dir));
+    COV3D_TRY(fft2(h, g2, g2, dir));
+    if (dir == CUFFT_FORWARD) COV3D_TRY(fft2(h0, g, g, dir));
+  }
+  return COV3D_OK;
+}
+
+// (nchan, L^3) volumes, real or complex, deapodised and zero-padded, to their transforms.  The line
+// kernels up to n = 256, where they read and write the least; at 512 cuFFT is the faster forward
+// transform (15.4 against 19.0 ms at L = 256, 10 channels).
+int volume_to_grid(cov3d_plan *p, const float *vr, const void *vc, int nchan, float2 *grid) {
+  if (grid_lines_apply(p) && p->n <= 256)
+    return grid_forward_lines(p, vr, vr ? nullptr : static_cast<const float2 *>(vc), p->gc1d.as<float>(), nchan, grid);
+  COV3D_TRY(launch_pack(p, vr, vc, nullptr, 1, nchan, grid));
+  return grid_fft(p, grid, nchan, CUFFT_FORWARD);
+}
+
+// The adjoint: the grid's inverse transform (in place), cropped and deapodised.
+int grid_to_volume(cov3d_plan *p, float2 *grid, int nchan, void *out) {
+  if (grid_lines_apply(p))
+    return inverse_lines(p, grid, nullptr, p->gc1d.as<float>(), nchan, nullptr, static_cast<float2 *>(out));
+  COV3D_TRY(grid_fft(p, grid, nchan, CUFFT_INVERSE));
+  return launch_unpack_complex(p, grid, nchan, 1, out);
 }
 
 }  // namespace cov3d

@@ -232,20 +232,21 @@ __device__ void block_add_pairs(FloatPair x, FloatPair y, double *a, double *b) 
 // next one reads, so no grid is ever zeroed.
 //   kRowFwd    CG: the volume row zero-padded (pad fused), forward along axis 2, whole row out; with
 //              z, the row is the new search direction p = z + (rz_new / rz) p, which it also stores
-//   kPackRows  step: eigenvector row * exp(log_sqrt) / grid correction, zero-padded, forward
+//   kPackRows  volume row (real or complex) * exp(log_sqrt) / grid correction, zero-padded, forward
 //   kColFwd    forward along axis 1 over the support entries of a support plane, whole column out; in
 //              the CG one thread also rolls the iteration's scalars (after kRowFwd has used them)
 //   kColInv    inverse along axis 1, support entries out
 //   kRowInv    CG: inverse along axis 2, the L support entries / n^3 to the volume (crop fused),
 //              <p, out> accumulated
-//   kUnpackRows step: inverse along axis 2, then d cost / d eigenvectors (2 Re(.) / grid
-//              correction * exp(log_sqrt))
+//   kUnpackRows inverse along axis 2; step: d cost / d eigenvectors (2 Re(.) / grid correction *
+//              exp(log_sqrt)); with out, the complex volume (. / grid correction)
 //   kAxisFwd   step: forward along axis 0 over the support rows; G written whole to gout, and the
 //              gradient grid initialised in place: coef * fr * G (the Fourier regulariser's
 //              derivative) with its value coef * sum fr |G|^2 and, twice that per channel, its
 //              derivative with respect to log_sqrt accumulated, or zero without fr
-//   kAxisInv   step: inverse along axis 0, support rows out
-enum { kRowFwd, kPackRows, kColFwd, kColInv, kRowInv, kUnpackRows, kAxisFwd, kAxisInv };
+//   kAxisFwdIn forward along axis 0 over the support rows, in place
+//   kAxisInv   inverse along axis 0, support rows out
+enum { kRowFwd, kPackRows, kColFwd, kColInv, kRowInv, kUnpackRows, kAxisFwd, kAxisFwdIn, kAxisInv };
 
 struct LineArgs {
   int L;
@@ -253,11 +254,11 @@ struct LineArgs {
   const int *stop;   // the CG's done flag (every kernel returns once it is set) or null
   float2 *g;         // fine grid, channel stride cs
   int64_t cs;
-  const float2 *vol;  // kRowFwd: L^3 input
+  const float2 *vol;  // kRowFwd: L^3 input; kPackRows: (r, L^3) complex volumes, or null
   const float2 *z;    // kRowFwd: preconditioned residual, or null
   float2 *pdir;       // kRowFwd: search direction, updated
   CgState *st;        // kRowFwd, kColFwd: scalars, or null
-  float2 *out;        // kRowInv: L^3 output
+  float2 *out;        // kRowInv: L^3 output; kUnpackRows: (r, L^3) complex volumes, or null
   const float2 *p;    // kRowInv: <p, out> operand or null
   double *dot;        // kRowInv: <p, out> (2 doubles)
   const float *vec;   // kPackRows: (r, L^3) eigenvectors
@@ -324,7 +325,8 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
           },
           [&](int k, float2 v) { row[k] = v; });
     } else if (KIND == kPackRows) {
-      const float *src = a.vec + c * L3 + vrow;
+      const float *src = a.vec ? a.vec + c * L3 + vrow : nullptr;
+      const float2 *csrc = a.vec ? nullptr : a.vol + c * L3 + vrow;
       const float es = a.logs ? expf(__ldg(a.logs + c)) : 1.0f;
       const float g01 = a.gc ? __ldg(a.gc + j0) * __ldg(a.gc + j1) : 1.0f;
       line_dft<N1, N2, false>(
@@ -333,7 +335,9 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
             const int j = pad_voxel(i, L, n);
             if (j < 0) return zero;
             const float gi = a.gc ? 1.0f / (g01 * __ldg(a.gc + j)) : 1.0f;
-            return make_float2(__ldg(src + j) * (gi * es), 0.f);
+            if (src) return make_float2(__ldg(src + j) * (gi * es), 0.f);
+            const float2 v = csrc[j];
+            return make_float2(v.x * (gi * es), v.y * (gi * es));
           },
           [&](int k, float2 v) { row[k] = v; });
     } else if (KIND == kRowInv) {
@@ -360,13 +364,18 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
     } else {  // kUnpackRows
       const float es = a.logs ? expf(__ldg(a.logs + c)) : 1.0f;
       const float g01 = a.gc ? 1.0f / (__ldg(a.gc + j0) * __ldg(a.gc + j1)) : 1.0f;
-      float *gdst = a.gvec + c * L3 + vrow;
+      float *gdst = a.out ? nullptr : a.gvec + c * L3 + vrow;
+      float2 *cdst = a.out ? a.out + c * L3 + vrow : nullptr;
       line_dft<N1, N2, true>(
           ex, s_tw, role, [&](int i) { return row[i]; },
           [&](int k, float2 v) {
             const int j = pad_voxel(k, L, n);
             if (j < 0) return;
             const float gj = a.gc ? g01 / __ldg(a.gc + j) : 1.0f;
+            if (cdst) {
+              cdst[j] = make_float2(v.x * gj, v.y * gj);
+              return;
+            }
             const float dV = 2.0f * v.x * gj;
             gdst[j] = dV * es;
           });
@@ -406,6 +415,10 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
             ax[(int64_t)k * nn] = y;
           });
       if (a.fr) block_add_twice((double)part * a.coef, a.cost, a.glog + c);
+    } else if (KIND == kAxisFwdIn) {
+      line_dft<N1, N2, false>(
+          ex, s_tw, role, [&](int i) { return in_support(i, L, n) ? ax[(int64_t)i * nn] : zero; },
+          [&](int k, float2 v) { ax[(int64_t)k * nn] = v; });
     } else {  // kAxisInv
       line_dft<N1, N2, true>(
           ex, s_tw, role, [&](int i) { return ax[(int64_t)i * nn]; },
@@ -479,6 +492,7 @@ int step_forward_n(cov3d_plan *p, const LineArgs &a, int r) {
   constexpr int n = N1 * N2;
   COV3D_TRY((launch_lines<N1, N2, kPackRows>(p, a, (int64_t)a.L * a.L, r)));
   COV3D_TRY((launch_lines<N1, N2, kColFwd>(p, a, (int64_t)a.L * n, r)));
+  if (!a.gout) return launch_lines<N1, N2, kAxisFwdIn>(p, a, (int64_t)n * n, r);
   return launch_lines<N1, N2, kAxisFwd>(p, a, (int64_t)n * n, r);
 }
 
@@ -493,7 +507,7 @@ int step_inverse_n(cov3d_plan *p, const LineArgs &a, int r) {
 // The plan's twiddles for its fine size n; line transforms need the table of exactly n.
 int line_args(cov3d_plan *p, LineArgs &a) {
   COV3D_TRY(ensure_twiddles(p, p->n));
-  if (!line_transform_size(p->n) || p->fftw_n != p->n || p->L % 2 != 0 || p->n < p->L + 2) {
+  if ((!line_transform_size(p->n) && p->n != 64) || p->fftw_n != p->n || p->L % 2 != 0 || p->n < p->L + 2) {
     set_error("no line transform for L = %d, n = %d", p->L, p->n);
     return COV3D_EINVAL;
   }
@@ -507,6 +521,12 @@ int line_args(cov3d_plan *p, LineArgs &a) {
 
 bool line_transforms_apply(const cov3d_plan *p) {
   return line_transform_size(p->n) && p->L % 2 == 0 && p->n >= p->L + 2;
+}
+
+// 64 is left out of line_transforms_apply, whose other users keep cuFFT's rounding there (the covariance
+// step's G, from which its 64-bit cost follows, and the CG's iterates); L >= 4 fills a block with rows.
+bool grid_lines_apply(const cov3d_plan *p) {
+  return (line_transform_size(p->n) || p->n == 64) && p->L % 4 == 0 && p->n >= p->L + 2;
 }
 
 int cg_operator_lines(cov3d_plan *p, const float2 *in, float2 *fine, float2 *out, const float2 *dotp,
@@ -554,15 +574,32 @@ int step_forward_lines(cov3d_plan *p, const float *vec, const float *logs, const
   }
 }
 
-int step_inverse_lines(cov3d_plan *p, float2 *grad_grid, const float *logs, const float *gc, int r, float *gvec) {
+int grid_forward_lines(cov3d_plan *p, const float *vr, const float2 *vc, const float *gc, int nchan, float2 *grid) {
   LineArgs a;
   COV3D_TRY(line_args(p, a));
-  a.g = grad_grid;
+  a.g = grid;
+  a.cs = (int64_t)p->n * p->n * p->n;
+  a.vec = vr;
+  a.vol = vc;
+  a.gc = gc;
+  switch (p->n) {
+    case 64: return step_forward_n<16, 4>(p, a, nchan);
+    case 128: return step_forward_n<16, 8>(p, a, nchan);
+    default: return step_forward_n<16, 16>(p, a, nchan);
+  }
+}
+
+int inverse_lines(cov3d_plan *p, float2 *grid, const float *logs, const float *gc, int r, float *gvec, float2 *out) {
+  LineArgs a;
+  COV3D_TRY(line_args(p, a));
+  a.g = grid;
   a.cs = (int64_t)p->n * p->n * p->n;
   a.logs = logs;
   a.gc = gc;
   a.gvec = gvec;
+  a.out = out;
   switch (p->n) {
+    case 64: return step_inverse_n<16, 4>(p, a, r);
     case 128: return step_inverse_n<16, 8>(p, a, r);
     case 256: return step_inverse_n<16, 16>(p, a, r);
     default: return step_inverse_n<32, 16>(p, a, r);

@@ -345,17 +345,18 @@ int cov3d_plan_reserve(cov3d_plan *p, int64_t max_images, int points_L, int ncha
   COV3D_TRY(grow(p->q, M * nchan * 8));
   COV3D_TRY(grow(p->small, max_images * (nchan * nchan * 8 * 2 + nchan * 8 * 2 + 8 + 8) + 64));
   COV3D_TRY(grow(p->ctfc, max_images * (int64_t)sizeof(CtfCoef)));
-  if (line_transforms_apply(p)) COV3D_TRY(ensure_twiddles(p, p->n));
-  // the cuFFT plans (and their work areas) of the step's transforms where the line DFTs do not
-  // apply: the pruned 2D + axis-0 pair for even L, the full 3D transform of nchan channels else
+  if (grid_lines_apply(p)) COV3D_TRY(ensure_twiddles(p, p->n));
+  // the cuFFT plans (and their work areas) of the step's transforms where the line DFTs do not apply
+  // in both directions: the pruned 2D + axis-0 pair and, on small grids or odd L, batched ones
   cufftHandle h = 0;
-  if (prunable(p)) {
-    if (!(line_transforms_apply(p) && p->n <= 256)) {
+  const bool lines = grid_lines_apply(p), small = p->n <= kSmallGrid;
+  if (!(lines && line_transforms_apply(p) && p->n <= 256)) {
+    if (p->n >= p->L + 2) {
       COV3D_TRY(get_fft_planes(p, &h));
       COV3D_TRY(get_fft_axis0(p, &h));
     }
-  } else {
-    COV3D_TRY(get_fft(p, nchan, &h));
+    if (prunable(p) && small) COV3D_TRY(get_fft_all_planes(p, nchan, &h));
+    if (!prunable(p) || (small && !lines)) COV3D_TRY(get_fft(p, nchan, &h));
   }
   if (flags & COV3D_RESERVE_GRAM_BF16) COV3D_TRY(reserve_gram_bf16(p, (int)max_images, (int)P, nchan));
   if (flags & COV3D_RESERVE_LS_REG) COV3D_TRY(reserve_ls_reg(p, nchan));
@@ -524,11 +525,7 @@ static int type2(cov3d_plan *p, const float *d_vol_real, const void *d_vol_compl
   }
   const int64_t n3 = (int64_t)p->n * p->n * p->n;
   COV3D_TRY(grow(p->fine, n3 * nchan * 8));
-  COV3D_TRY(launch_pack(p, d_vol_real, d_vol_complex, nullptr, 1, nchan, p->fine.ptr));
-  cufftHandle fft;
-  COV3D_TRY(get_fft(p, nchan, &fft));
-  COV3D_TRY(check_cufft(cufftExecC2C(fft, p->fine.as<cufftComplex>(), p->fine.as<cufftComplex>(), CUFFT_FORWARD),
-                        "cufftExecC2C(forward)"));
+  COV3D_TRY(volume_to_grid(p, d_vol_real, d_vol_complex, nchan, p->fine.as<float2>()));
   GridArgs g{p->fine.ptr, 1, n3, p->n - p->n / 2};
   // a real volume's transform is Hermitian
   return launch_interp(p, g, nchan, d_out, ops, ocs, e, d_vol_real ? hermitian_mode(p) : kSortFull);
@@ -539,12 +536,7 @@ int cov3d_fine_grid(cov3d_plan *p, const float *d_vol_real, const void *d_vol_co
     set_error("invalid fine-grid arguments (nchan must be in 1..n_trans)");
     return COV3D_EINVAL;
   }
-  COV3D_TRY(launch_pack(p, d_vol_real, d_vol_complex, nullptr, 1, nchan, d_grid));
-  cufftHandle fft;
-  COV3D_TRY(get_fft(p, nchan, &fft));
-  return check_cufft(cufftExecC2C(fft, static_cast<cufftComplex *>(d_grid), static_cast<cufftComplex *>(d_grid),
-                                  CUFFT_FORWARD),
-                     "cufftExecC2C(forward)");
+  return volume_to_grid(p, d_vol_real, d_vol_complex, nchan, static_cast<float2 *>(d_grid));
 }
 
 int cov3d_execute_type2(cov3d_plan *p, const float *d_vol_real, const void *d_vol_complex, int nchan, void *d_out) {
@@ -578,11 +570,7 @@ static int type1(cov3d_plan *p, const void *d_values, int64_t ips, int64_t ics, 
   COV3D_TRY(grow(p->fine, n3 * nchan * 8));
   COV3D_TRY(launch_zero(p, p->fine.ptr, n3 * nchan * 8));
   COV3D_TRY(launch_spread(p, d_values, ips, ics, nchan, e, p->fine.ptr, 1, n3, p->n - p->n / 2, mode));
-  cufftHandle fft;
-  COV3D_TRY(get_fft(p, nchan, &fft));
-  COV3D_TRY(check_cufft(cufftExecC2C(fft, p->fine.as<cufftComplex>(), p->fine.as<cufftComplex>(), CUFFT_INVERSE),
-                        "cufftExecC2C(inverse)"));
-  return launch_unpack_complex(p, p->fine.ptr, nchan, 1, d_vol_out);
+  return grid_to_volume(p, p->fine.as<float2>(), nchan, d_vol_out);
 }
 
 int cov3d_execute_type1(cov3d_plan *p, const void *d_values, int nchan, void *d_vol_out) {
