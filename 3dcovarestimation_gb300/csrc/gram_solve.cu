@@ -20,171 +20,196 @@ namespace {
 constexpr int kMaxRank = 32;
 constexpr int kGramChunk = 128;
 
-// One block per image: chunks of pixels are staged in shared memory; every thread owns one
-// (job, pixel-group) pair where a job is one entry of the upper triangle of gram, one h_i,
-// or |y|^2.  Partial sums per chunk are added to a Kahan-compensated running total.
+constexpr int kGramTile = 3;       // products are summed in 3 x 3 register tiles
+constexpr int kGramStage = 88000;  // bytes of staged pixels per block: two blocks per SM
+
+// Per-image Gram at any rank and layout: v = (q_0 .. q_{r-1}, y) of a pixel, products conj(v_i) v_j, i <= j.
+// One block per image; chunks of kGramChunk pixels are staged in shared memory, nc at a time.  A chunk's
+// pixels p = grp, grp + groups, ... make one sum per product, Kahan-added to the totals of that grp over
+// the chunks in order, and the totals of the groups are added in order.  The chunk sums are independent:
+// a work item is a 3 x 3 tile of products of one chunk and group, which reads 6 staged values for 36 FMAs
+// (a thread per product read 2 for 4, and shared memory bound it: r = 20, 300 images of 128^2:
+// 1.91 -> 0.43 ms, 0.79 GB; r = 8, 512 of 64^2, channel-major: 172 -> 58 us, 0.13 GB).
 __global__ void __launch_bounds__(1024) gram_kernel(const float2 *__restrict__ Q, int64_t q_is, int64_t q_ps,
                                                     int64_t q_cs, const float2 *__restrict__ Y, int P, int r,
-                                                    float2 *__restrict__ gram, float2 *__restrict__ h,
-                                                    float *__restrict__ yy) {
-  extern __shared__ float2 sq[];  // kGramChunk * (r + 1)
-  const int b = blockIdx.x;
-  const int ntri = r * (r + 1) / 2;
-  const int J = ntri + r + 1;
-  const int groups = max(1, (int)blockDim.x / J);
-  const int tid = threadIdx.x;
-  const int job = tid % J;
-  const int grp = tid / J;
-  const bool active = grp < groups;
-  int ji = 0, jj = 0, kind = 0;
-  if (job < ntri) {
-    int q = job, i = 0;
-    while (q >= r - i) {
-      q -= r - i;
-      ++i;
-    }
-    ji = i;
-    jj = i + q;
-    kind = 0;
-  } else if (job < ntri + r) {
-    ji = job - ntri;
-    kind = 1;
-  } else {
-    kind = 2;
-  }
-  float2 sum = make_float2(0.f, 0.f), comp = make_float2(0.f, 0.f);
+                                                    int groups, int nc, int rs, float2 *__restrict__ gram,
+                                                    float2 *__restrict__ h, float *__restrict__ yy) {
+  constexpr int T = kGramTile;
+  extern __shared__ float2 sq[];  // nc chunks of kGramChunk rows of rs values, then nc * groups * J sums
+  const int b = blockIdx.x, tid = threadIdx.x;
+  const int R1 = r + 1, J = R1 * (R1 + 1) / 2;
+  const int nt = (R1 + T - 1) / T, ntile = nt * (nt + 1) / 2;
+  const int cstride = kGramChunk * rs + 3;  // (chunks apart in the banks)
+  float2 *s_part = sq + nc * cstride;
   const float2 *Qb = Q + (int64_t)b * q_is;
   const float2 *Yb = Y + (int64_t)b * P;
-  float2 *sy = sq + kGramChunk * r;
-  for (int p0 = 0; p0 < P; p0 += kGramChunk) {
-    const int np = min(kGramChunk, P - p0);
+  float2 sum = make_float2(0.f, 0.f), comp = make_float2(0.f, 0.f);
+  const bool keeps = tid < groups * J;  // thread grp * J + job holds the totals
+  for (int p0 = 0; p0 < P; p0 += nc * kGramChunk) {
+    const int np = min(nc * kGramChunk, P - p0);
+    auto row = [&](int p) { return sq + (p / kGramChunk) * cstride + (p % kGramChunk) * rs; };
+    auto copy = [&](float2 *d, const float2 *s) {
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(d)), "l"(s)
+                   : "memory");
+    };
     __syncthreads();
     if (q_cs == 1) {
-      for (int e = tid; e < np * r; e += blockDim.x) {
-        const int pp = e / r, i = e - pp * r;
-        sq[e] = Qb[(int64_t)(p0 + pp) * q_ps + i];
+      const int di = blockDim.x % r, dp = blockDim.x / r;
+      for (int i = tid % r, p = tid / r; p < np;) {
+        copy(row(p) + i, Qb + (int64_t)(p0 + p) * q_ps + i);
+        i += di;
+        p += dp;
+        if (i >= r) {
+          i -= r;
+          ++p;
+        }
       }
     } else {
-      for (int e = tid; e < np * r; e += blockDim.x) {
-        const int i = e / np, pp = e - i * np;
-        sq[pp * r + i] = Qb[(int64_t)(p0 + pp) * q_ps + (int64_t)i * q_cs];
-      }
+      for (int i = tid >> 5; i < r; i += blockDim.x >> 5)
+        for (int p = tid & 31; p < np; p += 32)
+          copy(row(p) + i, Qb + (int64_t)(p0 + p) * q_ps + (int64_t)i * q_cs);
     }
-    for (int e = tid; e < np; e += blockDim.x) sy[e] = Yb[p0 + e];
+    for (int p = tid; p < np; p += blockDim.x) copy(row(p) + r, Yb + p0 + p);
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
-    if (!active) continue;
-    float2 part = make_float2(0.f, 0.f);
-    for (int p = grp; p < np; p += groups) {
-      float2 a, c;
-      if (kind == 2) {
-        a = sy[p];
-        c = a;
-      } else {
-        a = sq[p * r + ji];
-        c = kind == 0 ? sq[p * r + jj] : sy[p];
+    const int chunks = (np + kGramChunk - 1) / kGramChunk;
+    for (int item = tid; item < chunks * groups * ntile; item += blockDim.x) {
+      const int tile = item % ntile, cg = item / ntile, grp = cg % groups, c = cg / groups;
+      int ti = 0, tj = tile;
+      while (tj >= nt - ti) {
+        tj -= nt - ti;
+        ++ti;
       }
-      // conj(a) * c
-      part.x = fmaf(a.x, c.x, fmaf(a.y, c.y, part.x));
-      part.y = fmaf(a.x, c.y, fmaf(-a.y, c.x, part.y));
+      const int i0 = ti * T, j0 = (ti + tj) * T;
+      const int pe = min(kGramChunk, np - c * kGramChunk);
+      const float2 *rows = sq + c * cstride;
+      float2 part[T][T];
+#pragma unroll
+      for (int i = 0; i < T; ++i)
+#pragma unroll
+        for (int j = 0; j < T; ++j) part[i][j] = make_float2(0.f, 0.f);
+#pragma unroll 2
+      for (int p = grp; p < pe; p += groups) {
+        float2 x[T], y[T];
+#pragma unroll
+        for (int i = 0; i < T; ++i) {
+          x[i] = rows[p * rs + i0 + i];
+          y[i] = rows[p * rs + j0 + i];
+        }
+#pragma unroll
+        for (int i = 0; i < T; ++i)
+#pragma unroll
+          for (int j = 0; j < T; ++j) {
+            part[i][j].x = fmaf(x[i].x, y[j].x, fmaf(x[i].y, y[j].y, part[i][j].x));
+            part[i][j].y = fmaf(x[i].x, y[j].y, fmaf(-x[i].y, y[j].x, part[i][j].y));
+          }
+      }
+#pragma unroll
+      for (int i = 0; i < T; ++i)
+#pragma unroll
+        for (int j = 0; j < T; ++j) {
+          const int vi = i0 + i, vj = j0 + j;
+          if (vi <= vj && vj < R1) s_part[cg * J + vi * R1 - vi * (vi - 1) / 2 + vj - vi] = part[i][j];
+        }
     }
-    // Kahan update of the running total
-    float yx = part.x - comp.x, tx = sum.x + yx;
-    comp.x = (tx - sum.x) - yx;
-    sum.x = tx;
-    float yyv = part.y - comp.y, ty = sum.y + yyv;
-    comp.y = (ty - sum.y) - yyv;
-    sum.y = ty;
+    __syncthreads();
+    if (keeps) {
+      for (int c = 0; c < chunks; ++c) {  // Kahan updates of the running totals
+        const float2 part = s_part[c * groups * J + tid];
+        float yx = part.x - comp.x, tx = sum.x + yx;
+        comp.x = (tx - sum.x) - yx;
+        sum.x = tx;
+        float yyv = part.y - comp.y, ty = sum.y + yyv;
+        comp.y = (ty - sum.y) - yyv;
+        sum.y = ty;
+      }
+    }
   }
   __syncthreads();
   // reduce over pixel groups
-  float2 *red = sq;
-  if (active) red[grp * J + job] = sum;
+  if (keeps) s_part[tid] = sum;
   __syncthreads();
-  if (active && grp == 0) {
+  if (tid < J) {
     float2 tot = sum;
     for (int g = 1; g < groups; ++g) {
-      tot.x += red[g * J + job].x;
-      tot.y += red[g * J + job].y;
+      tot.x += s_part[g * J + tid].x;
+      tot.y += s_part[g * J + tid].y;
     }
-    if (kind == 0) {
-      gram[((int64_t)b * r + ji) * r + jj] = tot;
-      if (ji != jj) gram[((int64_t)b * r + jj) * r + ji] = make_float2(tot.x, -tot.y);
-    } else if (kind == 1) {
-      h[(int64_t)b * r + ji] = tot;
+    int i = 0, k = tid;
+    while (k >= R1 - i) {
+      k -= R1 - i;
+      ++i;
+    }
+    const int j = i + k;
+    if (j < r) {
+      gram[((int64_t)b * r + i) * r + j] = tot;
+      if (i != j) gram[((int64_t)b * r + j) * r + i] = make_float2(tot.x, -tot.y);
+    } else if (i < r) {
+      h[(int64_t)b * r + i] = tot;
     } else {
       yy[b] = tot.x;
     }
   }
 }
 
-// (i, j) of product k of the upper triangle (0 <= i <= j < R1), row-major
-template <int R1>
-__host__ __device__ constexpr int tri_i(int k) {
-  int i = 0;
-  while (k >= R1 - i) {
-    k -= R1 - i;
-    ++i;
-  }
-  return i;
-}
-template <int R1>
-__host__ __device__ constexpr int tri_j(int k) {
-  int i = 0;
-  while (k >= R1 - i) {
-    k -= R1 - i;
-    ++i;
-  }
-  return i + k;
-}
+constexpr int kGramLanes = 64;      // threads per tile of products, striding over the pixels
+constexpr int kGramChunkPx = 512;   // pixels staged per chunk
+constexpr int kGramBufs = 2;        // staging buffers (a third measured no faster)
 
-constexpr int kGramSubsets = 8;   // product subsets per image (2 warps each)
-constexpr int kGramLanes = 64;    // threads per subset, striding over the pixels
-
-// part[KK] += conj(v[i]) * v[j] for product k = S + kGramSubsets * KK, indices fixed at
-// compile time so the pixel stays in registers
-template <int R1, int S, int KK, int PER>
-struct GramAcc {
-  __device__ __forceinline__ static void run(const float2 (&v)[R1], float2 (&part)[PER]) {
-    constexpr int k = S + kGramSubsets * KK;
-    if constexpr (k < R1 * (R1 + 1) / 2) {
-      constexpr int i = tri_i<R1>(k), j = tri_j<R1>(k);
-      const float2 a = v[i], c = v[j];
-      part[KK].x = fmaf(a.x, c.x, fmaf(a.y, c.y, part[KK].x));
-      part[KK].y = fmaf(a.x, c.y, fmaf(-a.y, c.x, part[KK].y));
-    }
-    if constexpr (KK + 1 < PER) GramAcc<R1, S, KK + 1, PER>::run(v, part);
-  }
-};
-
-// One staged chunk of pixels for the products k = S, S + kGramSubsets, ... of this subset:
-// part[kk] += conj(v[i]) * v[j] with v a pixel's r projections and y (row of R + 1 in shared
-// memory, read into registers)
-template <int R, int S, int PER>
-__device__ __forceinline__ void gram_chunk(const float2 *rows, int np, int lane, float2 (&part)[PER]) {
-  constexpr int R1 = R + 1;
+// One staged chunk of pixels for the products conj(v_i) v_j of tile (TI, TJ), v a pixel's R projections
+// and y (a row of R + 1 in shared memory): part[i * T + j] += ... for i <= j < R + 1
+template <int R, int TI, int TJ>
+__device__ __forceinline__ void gram_chunk(const float2 *rows, int np, int lane,
+                                           float2 (&part)[kGramTile * kGramTile]) {
+  constexpr int R1 = R + 1, T = kGramTile;
   for (int p = lane; p < np; p += kGramLanes) {
-    float2 v[R1];
+    float2 x[T], y[T];
 #pragma unroll
-    for (int i = 0; i < R1; ++i) v[i] = rows[p * R1 + i];
-    GramAcc<R1, S, 0, PER>::run(v, part);
+    for (int i = 0; i < T; ++i) {
+      if (TI * T + i < R1) x[i] = rows[p * R1 + TI * T + i];
+      if (TI != TJ && TJ * T + i < R1) y[i] = rows[p * R1 + TJ * T + i];
+    }
+#pragma unroll
+    for (int i = 0; i < T; ++i)
+#pragma unroll
+      for (int j = 0; j < T; ++j) {
+        if (TI * T + i > TJ * T + j || TJ * T + j >= R1) continue;
+        const float2 a = x[i], c = TI == TJ ? x[j] : y[j];
+        float2 &t = part[i * T + j];
+        t.x = fmaf(a.x, c.x, fmaf(a.y, c.y, t.x));
+        t.y = fmaf(a.x, c.y, fmaf(-a.y, c.x, t.y));
+      }
   }
 }
 
-constexpr int kGramChunkPx = kGramSubsets * kGramLanes;  // pixels staged per chunk
-constexpr int kGramBufs = 2;  // staging buffers (a third measured no faster)
+template <int R>
+constexpr int kGramSide = (R + kGramTile) / kGramTile;  // tiles of a side
+template <int R>
+constexpr int kGramTiles = kGramSide<R> * (kGramSide<R> + 1) / 2;
+
+// gram_chunk of tile number `sub` counted from (TI, TJ) along the upper triangle's rows
+template <int R, int TI, int TJ>
+__device__ __forceinline__ void gram_tile(int sub, const float2 *rows, int np, int lane,
+                                          float2 (&part)[kGramTile * kGramTile]) {
+  if (sub == 0) gram_chunk<R, TI, TJ>(rows, np, lane, part);
+  else if constexpr (TJ + 1 < kGramSide<R>) gram_tile<R, TI, TJ + 1>(sub - 1, rows, np, lane, part);
+  else if constexpr (TI + 1 < kGramSide<R>) gram_tile<R, TI + 1, TI + 1>(sub - 1, rows, np, lane, part);
+}
 
 // Per-image Gram for the fused step's layout (point-major Q with r contiguous projections per
-// pixel): one block per image, eight product subsets of two warps.  Chunks of kGramChunkPx
+// pixel): one block per image, two warps for each 3 x 3 tile of products.  Chunks of kGramChunkPx
 // pixels are staged in shared memory by coalesced 8-byte asynchronous copies (double-buffered)
-// as rows of r projections and y, 88 bytes apart at r = 10 so the subsets' 8-byte reads are
-// free of bank conflicts; every subset reads every pixel of the chunk from there, and each
-// thread adds its chunk sums to Kahan-compensated totals.
+// as rows of r projections and y, 88 bytes apart at r = 10 so the tiles' 8-byte reads are
+// free of bank conflicts; every tile reads every pixel of the chunk from there, and each
+// thread adds its chunk sums to Kahan-compensated totals.  Reads of shared memory bound it: a
+// tile reads 6 values (3 on the diagonal) for 9 products, 48 per pixel at r = 10 where eight
+// subsets of 9 products that each read the whole row took 88 (0.61 -> 0.46 ms at 1024 images of
+// 128^2, 1.5 GB).
 template <int R>
-__global__ void __launch_bounds__(kGramSubsets * kGramLanes, 1) gram_pixel_kernel(
+__global__ void __launch_bounds__(kGramTiles<R> * kGramLanes, 1) gram_pixel_kernel(
     const float2 *__restrict__ Q, int64_t q_is, const float2 *__restrict__ Y, int P, float2 *__restrict__ gram,
     float2 *__restrict__ h, float *__restrict__ yy) {
-  constexpr int R1 = R + 1, NPR = R1 * (R1 + 1) / 2, PER = (NPR + kGramSubsets - 1) / kGramSubsets;
-  constexpr int NT = kGramSubsets * kGramLanes;
+  constexpr int R1 = R + 1, T = kGramTile, PER = T * T, NT = kGramTiles<R> * kGramLanes;
   extern __shared__ float2 srows[];  // kGramBufs * kGramChunkPx * R1
   const int b = blockIdx.x;
   const int sub = threadIdx.x / kGramLanes, lane = threadIdx.x % kGramLanes;
@@ -228,16 +253,7 @@ __global__ void __launch_bounds__(kGramSubsets * kGramLanes, 1) gram_pixel_kerne
     float2 part[PER];
 #pragma unroll
     for (int kk = 0; kk < PER; ++kk) part[kk] = make_float2(0.f, 0.f);
-    switch (sub) {
-      case 0: gram_chunk<R, 0, PER>(cur, np, lane, part); break;
-      case 1: gram_chunk<R, 1, PER>(cur, np, lane, part); break;
-      case 2: gram_chunk<R, 2, PER>(cur, np, lane, part); break;
-      case 3: gram_chunk<R, 3, PER>(cur, np, lane, part); break;
-      case 4: gram_chunk<R, 4, PER>(cur, np, lane, part); break;
-      case 5: gram_chunk<R, 5, PER>(cur, np, lane, part); break;
-      case 6: gram_chunk<R, 6, PER>(cur, np, lane, part); break;
-      default: gram_chunk<R, 7, PER>(cur, np, lane, part); break;
-    }
+    gram_tile<R, 0, 0>(sub, cur, np, lane, part);
 #pragma unroll
     for (int kk = 0; kk < PER; ++kk) {  // Kahan update of the running totals
       float yx = part[kk].x - comp[kk].x, tx = sum[kk].x + yx;
@@ -249,8 +265,8 @@ __global__ void __launch_bounds__(kGramSubsets * kGramLanes, 1) gram_pixel_kerne
     }
     __syncthreads();  // the buffer is refilled next
   }
-  // reduce over the 64 lanes of the subset: shuffles within each warp, then the two warps
-  __shared__ float2 red[kGramSubsets][2][PER];
+  // reduce over the 64 lanes of the tile: shuffles within each warp, then the two warps
+  __shared__ float2 red[kGramTiles<R>][2][PER];
   const int w = lane >> 5;
 #pragma unroll
   for (int kk = 0; kk < PER; ++kk) {
@@ -264,15 +280,14 @@ __global__ void __launch_bounds__(kGramSubsets * kGramLanes, 1) gram_pixel_kerne
   __syncthreads();
   if (lane < PER) {
     const int kk = lane;
-    const int k = sub + kGramSubsets * kk;
-    if (k < NPR) {
+    int ti = 0, tj = sub;
+    while (tj >= kGramSide<R> - ti) {
+      tj -= kGramSide<R> - ti;
+      ++ti;
+    }
+    const int i = ti * T + kk / T, j = (ti + tj) * T + kk % T;
+    if (i <= j && j < R1) {
       const float2 t = make_float2(red[sub][0][kk].x + red[sub][1][kk].x, red[sub][0][kk].y + red[sub][1][kk].y);
-      int i = 0, kr = k;
-      while (kr >= R1 - i) {
-        kr -= R1 - i;
-        ++i;
-      }
-      const int j = i + kr;
       if (j < R) {
         gram[((int64_t)b * R + i) * R + j] = t;
         if (i != j) gram[((int64_t)b * R + j) * R + i] = make_float2(t.x, -t.y);
@@ -510,6 +525,45 @@ __global__ void __launch_bounds__(256) wpass_kernel(const float2 *Q, int64_t q_i
   }
 }
 
+// W = C Q + u y for channel-major Q and W (a channel's pixels adjacent): one thread per pixel with its r
+// projections in registers, C and u broadcast from shared memory.  Memory bounds it; staging the chunk
+// for the transposed reads of the kernel above cost 205 us where this takes 46 (r = 8, 512 images of
+// 64^2, 0.27 GB).  RMAX is the smallest class that holds r.
+template <int RMAX>
+__global__ void __launch_bounds__(256) wpass_channel_kernel(const float2 *Q, int64_t q_is, int64_t q_cs,
+                                                            const float2 *__restrict__ Y, const float2 *__restrict__ C,
+                                                            const float2 *__restrict__ u, int P, int r, float2 *W,
+                                                            int64_t w_is, int64_t w_cs) {
+  __shared__ float2 sC[RMAX * RMAX], su[RMAX];
+  const int b = blockIdx.y;
+  for (int e = threadIdx.x; e < r * r; e += blockDim.x) sC[e / r * RMAX + e % r] = C[(int64_t)b * r * r + e];
+  for (int e = threadIdx.x; e < r; e += blockDim.x) su[e] = u[(int64_t)b * r + e];
+  __syncthreads();
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= P) return;
+  const float2 *qp = Q + (int64_t)b * q_is + p;
+  float2 *wp = W + (int64_t)b * w_is + p;
+  const float2 yv = Y[(int64_t)b * P + p];
+  float2 q[RMAX];
+#pragma unroll
+  for (int j = 0; j < RMAX; ++j) q[j] = j < r ? qp[j * q_cs] : make_float2(0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < RMAX; ++i) {
+    if (i >= r) break;
+    const float2 ui = su[i];
+    float2 acc = make_float2(ui.x * yv.x - ui.y * yv.y, ui.x * yv.y + ui.y * yv.x);
+#pragma unroll
+    for (int j = 0; j < RMAX; ++j) {
+      if (j < r) {
+        const float2 c = sC[i * RMAX + j];
+        acc.x = fmaf(c.x, q[j].x, fmaf(-c.y, q[j].y, acc.x));
+        acc.y = fmaf(c.x, q[j].y, fmaf(c.y, q[j].x, acc.y));
+      }
+    }
+    wp[i * w_cs] = acc;
+  }
+}
+
 // wpass for the fused step's layout (point-major, channel stride 1, W over Q in place): one
 // thread per pixel holds its r projections and y in registers (16-byte loads), C and u are
 // broadcast from shared memory, the r outputs are written back over the pixel's Q (16-byte
@@ -572,16 +626,23 @@ int launch_gram(cudaStream_t st, int B, int P, int r, const void *q, int64_t is,
     const size_t smem = kGramBufs * (size_t)kGramChunkPx * (10 + 1) * sizeof(float2);
     cudaError_t e = cudaFuncSetAttribute(gram_pixel_kernel<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(gram_pixel_kernel)");
-    gram_pixel_kernel<10><<<B, kGramSubsets * kGramLanes, smem, st>>>(
+    gram_pixel_kernel<10><<<B, kGramTiles<10> * kGramLanes, smem, st>>>(
         static_cast<const float2 *>(q), is, static_cast<const float2 *>(images), P, static_cast<float2 *>(gram),
         static_cast<float2 *>(h), yy);
     return launched("gram_pixel_kernel");
   }
-  const int J = r * (r + 1) / 2 + r + 1;
+  const int J = (r + 1) * (r + 2) / 2;
   const int threads = J > 256 ? ((J + 31) / 32) * 32 : 256;
-  const size_t smem = (size_t)kGramChunk * (r + 1) * sizeof(float2);
+  const int groups = threads / J;
+  const int rs = (r + kGramTile) / kGramTile * kGramTile;
+  const int cbytes = (kGramChunk * rs + 3) * (int)sizeof(float2);
+  int nc = kGramStage / cbytes;
+  nc = std::max(1, std::min(std::min(nc, 8), (P + kGramChunk - 1) / kGramChunk));
+  const size_t smem = (size_t)nc * (cbytes + groups * J * sizeof(float2));
+  COV3D_CUDA(cudaFuncSetAttribute(gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   gram_kernel<<<B, threads, smem, st>>>(static_cast<const float2 *>(q), is, ps, cs, static_cast<const float2 *>(images),
-                                        P, r, static_cast<float2 *>(gram), static_cast<float2 *>(h), yy);
+                                        P, r, groups, nc, rs, static_cast<float2 *>(gram), static_cast<float2 *>(h),
+                                        yy);
   return launched("gram_kernel");
 }
 
@@ -599,6 +660,21 @@ int launch_wpass(cudaStream_t st, int B, int P, int r, const void *q, int64_t is
       wpass_pixel_kernel<20><<<g, 256, 0, st>>>(qw, is, ps, y, cc, uu, P);
     }
     return launched("wpass_pixel_kernel");
+  }
+  if (ps == 1 && wps == 1) {
+    dim3 g((P + 255) / 256, B);
+    auto launch = [&](auto kernel) {
+      kernel<<<g, 256, 0, st>>>(static_cast<const float2 *>(q), is, cs, static_cast<const float2 *>(images),
+                                static_cast<const float2 *>(C), static_cast<const float2 *>(u), P, r,
+                                static_cast<float2 *>(w), wis, wcs);
+      return launched("wpass_channel_kernel");
+    };
+    if (r <= 4) return launch(wpass_channel_kernel<4>);
+    if (r <= 8) return launch(wpass_channel_kernel<8>);
+    if (r <= 12) return launch(wpass_channel_kernel<12>);
+    if (r <= 16) return launch(wpass_channel_kernel<16>);
+    if (r <= 20) return launch(wpass_channel_kernel<20>);
+    return launch(wpass_channel_kernel<kMaxRank>);
   }
   const size_t smem = (size_t)(r * r + r + kGramChunk * (r + 1)) * sizeof(float2);
   dim3 grid((P + kGramChunk - 1) / kGramChunk, B);
