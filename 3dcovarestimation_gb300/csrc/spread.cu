@@ -287,9 +287,9 @@ struct TileRows {
   }
 };
 
-// F / 2 channels per lane in NQ parts: 2 x 5 channels per pass, or one part of 5, 2 or 1.
+// F / 2 channels per lane in NQ parts.
 template <int KT, int W, int F, int NQ, int PP, bool HALF>
-__global__ void __launch_bounds__(kTileWarps * 32, 2) spread_tile_kernel(const SpreadParams a) {
+__global__ void __launch_bounds__(kTileWarps * 32, W == 2 ? 4 : 2) spread_tile_kernel(const SpreadParams a) {
   constexpr bool ES = KT == COV3D_KERNEL_ES;
   using G = TileGroups<W>;
   using Rec = TileRec<W>;
@@ -554,7 +554,31 @@ int launch_tile(const SpreadParams &a, int64_t max_blocks, cudaStream_t st) {
                               kTileWarps);
 }
 
-// Passes of ten channels in one launch, then the rest in the layout that holds it.
+// Linear windows: few enough FMAs per point that staging and waiting bound the kernel, so the layouts
+// hold at most 3 channels x 9 rows in a lane's registers and four blocks fit an SM (with
+// subproblems of 208 points; 10 channels, 1024 images of 128^2: 1.96 ms against 2.20 with 5 channels a
+// lane and two blocks of 384 points).  Twelve channels in a pass, then the layout that holds the rest
+// (5 channels, 256 images of 32^2: 51 us at two blocks, 41 at four).
+template <int KT, int W, bool HALF>
+int launch_linear_channels(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
+  const int rest = nchan % 12, whole = rest > 8 ? nchan : nchan - rest;
+  if (whole > 0) {
+    a.ch0 = 0;
+    a.nch = whole;
+    COV3D_TRY((launch_tile<KT, W, 6, 4, 1, HALF>(a, max_blocks, st)));
+  }
+  a.ch0 = whole;
+  a.nch = nchan - whole;
+  if (a.nch >= 7) return launch_tile<KT, W, 4, 4, 1, HALF>(a, max_blocks, st);
+  if (a.nch >= 3) return launch_tile<KT, W, 6, 2, 1, HALF>(a, max_blocks, st);
+  if (a.nch == 2) return launch_tile<KT, W, 4, 1, 1, HALF>(a, max_blocks, st);
+  if (a.nch == 1) return launch_tile<KT, W, 2, 1, 2, HALF>(a, max_blocks, st);
+  return COV3D_OK;
+}
+
+// Passes of ten channels in one launch, then the rest in the layout that holds it (3 channels a lane
+// and three blocks of 256 points per SM, as for linear windows: 5.58 ms against 4.74, and 1.07 against
+// 0.44 for 5 channels: here the FMAs bound).
 template <int KT, int W, bool HALF>
 int launch_tile_channels(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
   const int rest = nchan % 10, whole = rest > 5 ? nchan : nchan - rest;
@@ -573,8 +597,13 @@ int launch_tile_channels(SpreadParams a, int nchan, int64_t max_blocks, cudaStre
 
 template <int KT, int W>
 int launch_w(const SpreadParams &a, int nchan, int64_t max_blocks, cudaStream_t st) {
-  return a.half ? launch_tile_channels<KT, W, true>(a, nchan, max_blocks, st)
-                : launch_tile_channels<KT, W, false>(a, nchan, max_blocks, st);
+  if constexpr (W == 2) {
+    return a.half ? launch_linear_channels<KT, W, true>(a, nchan, max_blocks, st)
+                  : launch_linear_channels<KT, W, false>(a, nchan, max_blocks, st);
+  } else {
+    return a.half ? launch_tile_channels<KT, W, true>(a, nchan, max_blocks, st)
+                  : launch_tile_channels<KT, W, false>(a, nchan, max_blocks, st);
+  }
 }
 
 // Channels of an array two at a time
