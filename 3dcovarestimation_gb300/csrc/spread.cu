@@ -288,8 +288,13 @@ struct TileRows {
 };
 
 // F / 2 channels per lane in NQ parts.
+// Warps per block: two blocks fit an SM either way (the staged records), and one channel's accumulators
+// (one plane and up to 15 rows a lane) leave registers for 14 warps in each, with a point per thread
+// and smaller tasks (512 images of 128^2, W = 7: 1.26 -> 1.00 ms against 6 warps and two planes a lane).
+__host__ __device__ constexpr int tile_warps(int W, int F) { return W > 2 && F == 2 ? 14 : kTileWarps; }
+
 template <int KT, int W, int F, int NQ, int PP, bool HALF>
-__global__ void __launch_bounds__(kTileWarps * 32, W == 2 ? 4 : 2) spread_tile_kernel(const SpreadParams a) {
+__global__ void __launch_bounds__(tile_warps(W, F) * 32, W == 2 ? 4 : 2) spread_tile_kernel(const SpreadParams a) {
   constexpr bool ES = KT == COV3D_KERNEL_ES;
   using G = TileGroups<W>;
   using Rec = TileRec<W>;
@@ -323,18 +328,18 @@ __global__ void __launch_bounds__(kTileWarps * 32, W == 2 ? 4 : 2) spread_tile_k
   };
   // each thread keeps its points until their place in the sorted order is known, and asks for their
   // values (point-major ones) ahead of the gather
-  constexpr int PPT = (kTileMaxSub + kTileWarps * 32 - 1) / (kTileWarps * 32);
+  constexpr int PPT = (kTileMaxSub + tile_warps(W, F) * 32 - 1) / (tile_warps(W, F) * 32);
   SortedPoint pt[PPT];
   int pkey[PPT];
 #pragma unroll
   for (int u = 0; u < PPT; ++u) {
-    const int k = tid + u * kTileWarps * 32;
+    const int k = tid + u * tile_warps(W, F) * 32;
     pkey[u] = -1;
     if (k < st.cnt) pt[u] = a.pts[st.first + k];
   }
 #pragma unroll
   for (int u = 0; u < PPT; ++u) {
-    if (tid + u * kTileWarps * 32 >= st.cnt) continue;
+    if (tid + u * tile_warps(W, F) * 32 >= st.cnt) continue;
     const int key = (corner(pt[u].t2, st.ts2) / G::GS) * 64 + corner(pt[u].t1, st.ts1) * 8 + corner(pt[u].t0, st.ts0);
     pkey[u] = key | (atomicAdd(s_cnt + key, 1) << 9);
     if (a.ics == 1) {
@@ -442,12 +447,12 @@ __global__ void __launch_bounds__(kTileWarps * 32, W == 2 ? 4 : 2) spread_tile_k
     // Four elements' loads in flight per thread: the gathers' latency is most of the staging.
     constexpr int GU = 4;
     const int total = st.cnt * CH;
-    for (int e0 = tid; e0 < total; e0 += GU * kTileWarps * 32) {
+    for (int e0 = tid; e0 < total; e0 += GU * tile_warps(W, F) * 32) {
       float2 x[GU], m[GU];
       int sl[GU];
 #pragma unroll
       for (int u = 0; u < GU; ++u) {
-        const int e = e0 + u * kTileWarps * 32;
+        const int e = e0 + u * tile_warps(W, F) * 32;
         const int slot = e / CH, ch = e - slot * CH;
         sl[u] = e < total ? slot : -1;
         x[u] = m[u] = make_float2(0.f, 0.f);
@@ -465,7 +470,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, W == 2 ? 4 : 2) spread_tile_k
       for (int u = 0; u < GU; ++u) {
         const int slot = sl[u];
         if (slot < 0) continue;
-        const int ch = e0 + u * kTileWarps * 32 - slot * CH;
+        const int ch = e0 + u * tile_warps(W, F) * 32 - slot * CH;
         const float sc = s_sc[slot];
         float2 v = make_float2(x[u].x * sc, HALF && s_id[slot] < 0 ? -(x[u].y * sc) : x[u].y * sc);
         if (HALF && s_mid[slot] >= 0) {
@@ -551,7 +556,7 @@ int launch_tile(const SpreadParams &a, int64_t max_blocks, cudaStream_t st) {
   const size_t smem = (size_t)a.max_sub * tile_point_bytes<W, F>(NQ) + 8 +
                       tile_fixed_bytes(TileGroups<W>::T, TileGroups<W>::NG);
   return launch_spread_kernel(spread_tile_kernel<KT, W, F, NQ, PP, HALF>, "spread_tile_kernel", smem, a, max_blocks, st,
-                              kTileWarps);
+                              tile_warps(W, F));
 }
 
 // Linear windows: few enough FMAs per point that staging and waiting bound the kernel, so the layouts
@@ -591,7 +596,7 @@ int launch_tile_channels(SpreadParams a, int nchan, int64_t max_blocks, cudaStre
   a.nch = nchan - whole;
   if (a.nch >= 3) return launch_tile<KT, W, 10, 1, 1, HALF>(a, max_blocks, st);
   if (a.nch == 2) return launch_tile<KT, W, 4, 1, 1, HALF>(a, max_blocks, st);
-  if (a.nch == 1) return launch_tile<KT, W, 2, 1, 2, HALF>(a, max_blocks, st);
+  if (a.nch == 1) return launch_tile<KT, W, 2, 1, 1, HALF>(a, max_blocks, st);
   return COV3D_OK;
 }
 
