@@ -1,6 +1,7 @@
 // Spreading ("type-1" half of the NUFFT; exact adjoint of interp.cu, replacing the
 // reference's grid_sample backward with FP32 global atomics, nufft_plan.py:171-242), over the
-// bin-sorted point records of points_sort.cu.  See spread_kernel for the decomposition.
+// bin-sorted point records of points_sort.cu.  See spread_tile_kernel (ES and linear windows) and
+// spread_nearest_kernel for the decompositions.
 
 #include "cov3d_device.cuh"
 
@@ -180,9 +181,9 @@ __global__ void __launch_bounds__(kNearestThreads) spread_nearest_kernel(const S
   }
 }
 
-// Spreading for the ES windows (W = 4 .. 8) and the linear one (W = 2), any number of channels.  One block per subproblem (a bin
-// of 8^3 cells and at most max_sub of its points); the cells it can reach are a tile of T^3,
-// T = 8 + W - 1.  The block sorts its points by (axis-2 group, l1, l0), l the bin-local corner of
+// Spreading for the ES windows (W = 4 .. 8) and the linear one (W = 2), any number of channels.  One
+// block per subproblem (a bin of 8^3 cells and at most max_sub of its points); the cells it can reach
+// are a tile of T^3, T = 8 + W - 1.  The block sorts its points by (axis-2 group, l1, l0), l the bin-local corner of
 // their window and a group GS = 9 - W neighbouring l2, so that the windows of a group lie in the
 // same 8 tile columns, and stages a record per point (weights) and its channel values.
 //
@@ -196,9 +197,10 @@ __global__ void __launch_bounds__(kNearestThreads) spread_nearest_kernel(const S
 // What bounds it: latency at twelve warps per SM (issue 47 %, FP32 pipe 32 %, shared wavefronts
 // 17 % of their peaks on the B = 256 capture).  At the covariance step's 10 channels, W = 6, a visit
 // is some 50 instructions and a point has 3.5 of them.  Its predecessor, lanes owning all 13 tile
-// columns of three rows of one plane, had 16 visits and 2.2x the multiply-adds.  Measured on the step at L = 128, B = 1024, r = 10: 8.6 -> 5.3 ms, of which staging
-// (sort, weights, gathered values) about 2.0, the flush 0.9; one channel at W = 7, 512 images of
-// 128^2: 6.2 -> 1.2 ms.
+// columns of three rows of one plane, had 16 visits and 2.2x the multiply-adds.  Measured on the step at
+// L = 128, B = 1024, r = 10: 8.6 -> 5.3 ms, of which staging (sort, weights, gathered values) about
+// 2.0 and the flush 0.9; 4.7 with the points in registers, their values asked for ahead and four
+// gathers in flight.  One channel at W = 7, 512 images of 128^2: 6.2 -> 1.0 ms.
 //
 // Each cell's sum is plain FP32 over the points of one group of one subproblem (some 30 terms at
 // one point per cell, a third of what the predecessor summed before its first TwoSum fold; two or

@@ -333,7 +333,7 @@ class NufftPlanDiscretized(BaseNufftPlan):
 
     ``execute_forward`` expects the volume already in the (upsampled, centered) Fourier domain,
     as ``NufftSpec.input_in_fourier`` says.  Extra keyword ``compensated`` selects TwoSum
-    compensated spreading (default True)."""
+    sums in nearest-cell spreading (default True)."""
 
     def __init__(self, sz: Tuple[int, ...], upsample_factor: int = 1, mode: str = "bilinear",
                  use_half_grid: bool = False, compensated: bool = True) -> None:

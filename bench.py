@@ -6,7 +6,7 @@ One step = one covariance-SGD iteration over a batch of 1024 synthetic L=128 ima
 r=10 eigenvolumes (the config of the GPU drop-in workload: ES kernel width 6 at tol 1e-6,
 upsampling 2, ML objective): on-the-fly points + bin sort, deapodise/pad + FFT3, ES
 interpolation with the fused projection epilogue, per-image Gram + FP64 solve, hand-written
-adjoint, compensated spreading, inverse FFT3, crop, Adam update.  Prints one JSON line.
+adjoint, spreading, inverse FFT3, crop, Adam update.  Prints one JSON line.
 
 ``--impl reference`` times the reference's own step on the host cores: its
 ``CovarTrainer.run_batch`` on ``NufftPlanDiscretized`` bilinear (the command line's default;
@@ -33,7 +33,7 @@ WORKLOAD = ("cov-SGD step, GPU drop-in plain FP32 config: L=128, pixel 1.5 A, r=
             "batch 1024, uniform SO(3) poses, CTF 300 kV / Cs 2.7 mm / AC 0.1 / defocus U[1,3] um (from per-image "
             "parameters), SNR 0.05, "
             "NUFFT upsampling 2, ML objective + Fourier regulariser, Adam")
-GPU_INTERP = "ES kernel width 6 (tol 1e-6), periodic, compensated FP32 spreading"
+GPU_INTERP = "ES kernel width 6 (tol 1e-6), periodic, FP32 spreading"
 REF_INTERP = ("reference NufftPlanDiscretized bilinear (grid_sample), the reference command line's default; its ES "
               "plan (cuFINUFFT) is not installed")
 
@@ -65,7 +65,7 @@ def parse():
                     help="seconds of timed reference steps in --impl reference (whole steps, at least one)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--seed", type=int, default=2000)
-    ap.add_argument("--uncompensated", action="store_true", help="plain FP32 spreading (no TwoSum error terms)")
+    ap.add_argument("--uncompensated", action="store_true", help="plans without TwoSum sums (only nearest-cell spreading has them)")
     ap.add_argument("--mean-images", type=int, default=300000, help="images backprojected for the mean-CG solve")
     ap.add_argument("--mean-L", type=int, default=128)
     ap.add_argument("--mean-rtol", type=float, default=1e-5)
@@ -736,14 +736,14 @@ def run_gb300(args):
     flops = M * (args.width**3) * r * 4
     sm_mhz = clocks.get("sm_mhz") or 1900.0
     fp32_peak = 152 * 128 * 2 * sm_mhz * 1e6 / 1e12
-    kernel_name = "interp_kernel" if dom == "interp" else ("spread_rows_kernel" if r >= 5 else "spread_kernel")
+    kernel_name = "interp_group_kernel" if dom == "interp" else "spread_tile_kernel"
     line = {
         "metric": METRIC, "value": value, "unit": "images/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": shared_config(args, world),
         "interpolation": GPU_INTERP, "resident_images": nb * B,
-        "spreading": "fp32" if args.uncompensated else "fp32 + TwoSum compensation",
+        "spreading": "fp32",
         "roofline": {"bound": "hbm", "kernel": kernel_name, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind, "traffic": load_traffic(kernel_name),
                      "algorithmic_bytes_per_launch": alg[dom], "ms_per_launch": dom_ms,
