@@ -639,7 +639,13 @@ int launch_gram(cudaStream_t st, int B, int P, int r, const void *q, int64_t is,
   int nc = kGramStage / cbytes;
   nc = std::max(1, std::min(std::min(nc, 8), (P + kGramChunk - 1) / kGramChunk));
   const size_t smem = (size_t)nc * (cbytes + groups * J * sizeof(float2));
-  COV3D_CUDA(cudaFuncSetAttribute(gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // one limit for every rank: calls of several threads set the same
+  constexpr int kMost = kGramStage + 8 * 255 * (int)sizeof(float2) + (1 << 14);
+  if (smem > (size_t)kMost) {
+    set_error("Gram stage of %zu bytes", smem);
+    return COV3D_EINVAL;
+  }
+  COV3D_CUDA(cudaFuncSetAttribute(gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
   gram_kernel<<<B, threads, smem, st>>>(static_cast<const float2 *>(q), is, ps, cs, static_cast<const float2 *>(images),
                                         P, r, groups, nc, rs, static_cast<float2 *>(gram), static_cast<float2 *>(h),
                                         yy);
@@ -715,8 +721,9 @@ int launch_solve(cudaStream_t st, int B, int r, int objective, const void *gram,
   const unsigned blocks = (unsigned)((B + ipb - 1) / ipb);
   const size_t smem = objective == 0 ? (size_t)ipb * (r * r + 2 * r) * sizeof(cd) : 0;
   auto launch = [&](auto kernel) -> int {
+    // (one limit for every rank: calls of several threads set the same)
     if (smem > 40 * 1024)
-      COV3D_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      COV3D_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
     kernel<<<blocks, kSolveThreads, smem, st>>>(sa);
     return COV3D_OK;
   };

@@ -2,7 +2,8 @@
 // decomposition, one shared-memory exchange per transform.  They carry the pruned 3D
 // transforms of the mean CG's padding operator and of the covariance step (pack, forward
 // transform and regulariser; inverse transform and unpack), each fused with the elementwise
-// work around it, for fine grids of n = 128, 256, 512 (and the axis-0 CG kernel also for 64).
+// work around it, for fine grids of n = 128, 256, 512; the transforms of the plans' volumes, the step's
+// inverse one and the axis-0 CG kernel also for 64.
 // Twiddles exp(-2 pi i j / n) are computed on the host in double precision.
 
 #include <cmath>
