@@ -234,27 +234,40 @@ __device__ __forceinline__ void scatter_half(const PointGeom &g, int64_t M, cons
 }
 
 // Exclusive scans over a view's bin counts, one block per view: point offsets, and subproblem
-// offsets (ceil(count / max_sub) subproblems per live bin).  Each pass takes four bins per thread
-// from one 16-byte load (a scan of contiguous per-thread chunks loaded 128 bytes apart took 53 us
-// for 32768 bins, this one 32 at 1024 images of 128^2).
+// offsets (ceil(count / max_sub) subproblems per live bin).  A chain of passes bounds it, so a pass
+// takes eight bins per thread, in 16-byte loads and stores, and the next pass's loads are in flight
+// meanwhile (32768 bins, 1024 images of 128^2: 53 us with contiguous chunks per thread, loaded 128
+// bytes apart, 32 with four bins and scalar stores, now 22).
+constexpr int kScanBins = 8;
+
 __global__ void __launch_bounds__(1024) bin_scan_kernel(int64_t nbins, int max_sub, SortViews views) {
   const SortView &v = views.v[blockIdx.x];
   __shared__ int s_pts[32], s_sub[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t total = nbins + 1;  // includes the dead bin
   int carry_p = 0, carry_s = 0;
-  for (int64_t base = 0; base < total; base += 4 * 1024) {
-    const int64_t i0 = base + 4 * tid;
-    int c[4] = {0, 0, 0, 0}, sp = 0, ss = 0, sub[4];
-    if (i0 + 4 <= total) {
-      const int4 x = *reinterpret_cast<const int4 *>(v.count + i0);
-      c[0] = x.x; c[1] = x.y; c[2] = x.z; c[3] = x.w;
-    } else {
-      for (int k = 0; k < 4; ++k)
-        if (i0 + k < total) c[k] = v.count[i0 + k];
-    }
+  int next[kScanBins];
+  auto load = [&](int64_t i0) {
+    if (i0 + kScanBins <= total) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+      for (int u = 0; u < kScanBins; u += 4) {
+        const int4 x = *reinterpret_cast<const int4 *>(v.count + i0 + u);
+        next[u] = x.x; next[u + 1] = x.y; next[u + 2] = x.z; next[u + 3] = x.w;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kScanBins; ++k) next[k] = i0 + k < total ? v.count[i0 + k] : 0;
+    }
+  };
+  load((int64_t)kScanBins * tid);
+  for (int64_t base = 0; base < total; base += kScanBins * 1024) {
+    const int64_t i0 = base + kScanBins * tid;
+    int c[kScanBins], sp = 0, ss = 0, sub[kScanBins];
+#pragma unroll
+    for (int k = 0; k < kScanBins; ++k) c[k] = next[k];
+    if (base + kScanBins * 1024 < total) load(i0 + kScanBins * 1024);
+#pragma unroll
+    for (int k = 0; k < kScanBins; ++k) {
       sub[k] = i0 + k < nbins ? (c[k] + max_sub - 1) / max_sub : 0;
       sp += c[k];
       ss += sub[k];
@@ -285,12 +298,26 @@ __global__ void __launch_bounds__(1024) bin_scan_kernel(int64_t nbins, int max_s
     }
     const int before_p = __shfl_sync(0xffffffffu, wp, (warp + 31) & 31), before_s = __shfl_sync(0xffffffffu, ws, (warp + 31) & 31);
     int rp = carry_p + (warp ? before_p : 0) + ip - sp, rs = carry_s + (warp ? before_s : 0) + is - ss;
+    int off[kScanBins];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (i0 + k < total) v.off[i0 + k] = rp;
-      if (i0 + k < nbins) v.sub_off[i0 + k] = rs;
+    for (int k = 0; k < kScanBins; ++k) {
+      off[k] = rp;
       rp += c[k];
+      c[k] = rs;  // the subproblem offset
       rs += sub[k];
+    }
+    if (i0 + kScanBins <= nbins) {
+#pragma unroll
+      for (int u = 0; u < kScanBins; u += 4) {
+        *reinterpret_cast<int4 *>(v.off + i0 + u) = make_int4(off[u], off[u + 1], off[u + 2], off[u + 3]);
+        *reinterpret_cast<int4 *>(v.sub_off + i0 + u) = make_int4(c[u], c[u + 1], c[u + 2], c[u + 3]);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kScanBins; ++k) {
+        if (i0 + k < total) v.off[i0 + k] = off[k];
+        if (i0 + k < nbins) v.sub_off[i0 + k] = c[k];
+      }
     }
     carry_p += __shfl_sync(0xffffffffu, wp, 31);
     carry_s += __shfl_sync(0xffffffffu, ws, 31);
