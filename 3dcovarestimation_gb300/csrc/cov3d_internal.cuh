@@ -93,7 +93,7 @@ void release(DevBuf &b);
 // Which records the sort makes of the plan's points.  kSortFull: one per point.  kSortHalf: for a
 // Hermitian grid G(-k) = conj G(k) (the transform of a real volume), one record per pair of
 // mirror pixels (k, -k) of an image, so interpolation, and spreading of which only the real part
-// of the inverse transform is kept, do half the work (points_sort.cu, half_point).
+// of the inverse transform is kept, do half the work (points_sort.cu, pair_record).
 enum SortMode { kSortFull = 0, kSortHalf = 1, kSortModes = 2 };
 
 // One sorted view of the plan's points: records in bin order and the subproblem table, in one
@@ -111,7 +111,6 @@ struct SortSet {
   int *nsub = nullptr;  // scalar
   bool used = false;    // some operator has asked for it: sorted with every new point set
   bool valid = false;   // holds the current points
-  bool every_use = false;  // points may change by the replay of a graph that does not sort this view
 };
 }  // namespace cov3d
 
@@ -140,6 +139,9 @@ struct cov3d_plan {
   cov3d::Bins bins{};
   int max_sub = 288;
   cov3d::SortSet sets[cov3d::kSortModes];     // bin-sorted records by SortMode
+  cudaStream_t sort_stream = nullptr;  // first uses of a view are sorted here (need_sorted) ...
+  cudaEvent_t points_set = nullptr;    // ... after the points
+  bool pairs_off = false;              // no operator uses kSortHalf any more (new_points)
 
   // workspaces
   cov3d::DevBuf fine, fine2;   // complex fine grids (n^3 * channels)
@@ -236,10 +238,8 @@ int new_points(cov3d_plan *p);
 int need_sorted(cov3d_plan *p, unsigned modes);
 int reserve_sort(cov3d_plan *p, int64_t M, SortMode mode);
 // The records an operator uses on a grid (or volume) it knows to be Hermitian (real): half of them
-// where the plan's kernel and point count allow.
-inline SortMode hermitian_mode(const cov3d_plan *p) {
-  return p->kernel != COV3D_KERNEL_NEAREST && p->n_points < (int64_t(1) << 29) ? kSortHalf : kSortFull;
-}
+// where the plan's kernel, point count and buffers allow.
+SortMode hermitian_mode(const cov3d_plan *p);
 // gram_tc.cu: the BF16 Gram's operand and sum buffers for B images of P pixels at rank r
 int reserve_gram_bf16(cov3d_plan *p, int B, int P, int r);
 

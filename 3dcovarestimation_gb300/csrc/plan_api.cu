@@ -199,7 +199,9 @@ void grid_correction_1d(const cov3d_plan *p, std::vector<double> &g) {
 int finish_points(cov3d_plan *p) {
   p->n_points = p->n_images * (int64_t)p->points_L * p->points_L;
   PhaseScope ps(p, kPhaseSort);
-  return new_points(p);
+  const int rc = new_points(p);
+  if (rc != COV3D_OK) p->point_kind = kPointsNone;
+  return rc;
 }
 
 bool valid(const cov3d_plan *p) { return p != nullptr && p->n > 0; }
@@ -373,6 +375,8 @@ int cov3d_plan_destroy(cov3d_plan *p) {
                     &p->small, &p->acc, &p->cgw, &p->xbf, &p->gsum, &p->fftw, &p->ctfc, &p->lsw};
   for (DevBuf *b : bufs) release(*b);
   for (SortSet &ss : p->sets) release(ss.mem);
+  if (p->points_set) cudaEventDestroy(p->points_set);
+  if (p->sort_stream) cudaStreamDestroy(p->sort_stream);
   release_blas(p);
   if (p->h_acc) cudaFreeHost(p->h_acc);
   if (p->ev_pool) {
@@ -416,6 +420,7 @@ int cov3d_setpts(cov3d_plan *p, const float *d_pts, int64_t n_images, int points
     set_error("points must have contiguous rows (row_stride == L^2) and img_stride >= 3 L^2");
     return COV3D_EINVAL;
   }
+  p->point_kind = kPointsNone;  // until the new ones are in place
   COV3D_TRY(grow(p->pts, n_images * 3 * P * 4));
   COV3D_CUDA(cudaMemcpy2DAsync(p->pts.ptr, (size_t)(3 * P * 4), d_pts, (size_t)(img_stride * 4), (size_t)(3 * P * 4),
                                (size_t)n_images, cudaMemcpyDeviceToDevice, p->stream));
@@ -431,6 +436,7 @@ int cov3d_setrot(cov3d_plan *p, const float *d_rot, int64_t n_images, int points
     set_error("invalid setrot arguments");
     return COV3D_EINVAL;
   }
+  p->point_kind = kPointsNone;
   COV3D_TRY(grow(p->rot, n_images * 9 * 4));
   COV3D_CUDA(cudaMemcpyAsync(p->rot.ptr, d_rot, (size_t)(n_images * 9 * 4), cudaMemcpyDeviceToDevice, p->stream));
   p->point_kind = kPointsRotations;

@@ -481,10 +481,38 @@ int reserve_sort(cov3d_plan *p, int64_t M, SortMode mode) {
   return COV3D_OK;
 }
 
-// The plan's points have changed: the views that operators have used so far are sorted now (so a
-// captured call that reads one finds the new points in it), the others on their first use.  Inside
-// a stream capture the others are sorted too where their buffers are large enough already; where
-// not, a replay of that graph would change the points unseen, so such a view is sorted on every use.
+// Pair records need a linear or ES window and ids below 2^29.
+static bool pairs_apply(const cov3d_plan *p) {
+  return p->kernel != COV3D_KERNEL_NEAREST && p->n_points < (int64_t(1) << 29);
+}
+
+// Whether the pairs' view of the current points fits the buffers that it has.
+static bool pairs_fit(const cov3d_plan *p) {
+  return p->sets[kSortHalf].cap >= p->n_points &&
+         (p->point_kind != kPointsRotations || p->rotc.cap >= p->n_images * 6 * 8);
+}
+
+static int capturing(const cov3d_plan *p, bool *yes) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  COV3D_CUDA(cudaStreamIsCapturing(p->stream, &cap));
+  *yes = cap != cudaStreamCaptureStatusNone;
+  return COV3D_OK;
+}
+
+SortMode hermitian_mode(const cov3d_plan *p) {
+  if (!pairs_apply(p) || p->pairs_off) return kSortFull;
+  bool cap = false;
+  // a capture cannot allocate the view
+  if (!p->sets[kSortHalf].valid && !pairs_fit(p) && (capturing(p, &cap) != COV3D_OK || cap)) return kSortFull;
+  return kSortHalf;
+}
+
+// The plan's points have changed: the views that operators have used so far are sorted now, on the
+// stream that sets the points (so an operator ordered after this call, and a captured one that reads
+// the view, find the new points in it); the others on their first use (need_sorted).  Points set
+// inside a stream capture reach every view by the replay, also those that nothing has used yet; where
+// the pairs' view has no room to be sorted there, the replay would change the points unseen by it, so
+// no operator of this plan uses pair records from then on (graphs made before still find theirs).
 int new_points(cov3d_plan *p) {
   for (SortSet &ss : p->sets) ss.valid = false;
   const int64_t M = p->n_points;
@@ -493,37 +521,61 @@ int new_points(cov3d_plan *p) {
     set_error("too many points (%lld); the limit is 2^30-1 per plan", (long long)M);
     return COV3D_EINVAL;
   }
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  COV3D_CUDA(cudaStreamIsCapturing(p->stream, &cap));
-  const bool capturing = cap != cudaStreamCaptureStatusNone;
-  unsigned modes = 0;
-  for (int m = 0; m < kSortModes; ++m) {
-    SortSet &ss = p->sets[m];
-    if (m != kSortFull && hermitian_mode(p) != m) continue;  // no operator reads it
-    if (capturing && !ss.used) {
-      const bool fits = ss.cap >= M &&
-                        (m == kSortFull || p->point_kind != kPointsRotations || p->rotc.cap >= p->n_images * 6 * 8);
-      if (fits) ss.used = true;
-      else ss.every_use = true;
+  COV3D_TRY(reserve_sort(p, M, kSortFull));  // a first use inside a capture needs its buffers
+  bool cap = false;
+  COV3D_TRY(capturing(p, &cap));
+  if (cap) {
+    p->sets[kSortFull].used = true;
+    if (pairs_apply(p)) {
+      if (pairs_fit(p)) p->sets[kSortHalf].used = true;
+      else p->pairs_off = true;
     }
-    if (ss.used) modes |= 1u << m;
   }
-  return sort_points(p, modes);
+  unsigned modes = 0;
+  bool later = false;
+  for (int m = 0; m < kSortModes; ++m) {
+    if (m == kSortHalf && !(pairs_apply(p) && (!p->pairs_off || (p->sets[m].used && pairs_fit(p))))) continue;
+    if (p->sets[m].used) modes |= 1u << m;
+    else later = true;
+  }
+  COV3D_TRY(sort_points(p, modes));
+  if (!later) return COV3D_OK;
+  // first uses wait for this event
+  if (!p->sort_stream) COV3D_CUDA(cudaStreamCreateWithFlags(&p->sort_stream, cudaStreamNonBlocking));
+  if (!p->points_set) COV3D_CUDA(cudaEventCreateWithFlags(&p->points_set, cudaEventDisableTiming));
+  return check_cuda(cudaEventRecord(p->points_set, p->stream), "points event");
 }
 
-// The views in `modes` (bits 1 << SortMode) hold the current points, sorted in one launch sequence
-// where they do not yet.
+// The views in `modes` (bits 1 << SortMode) hold the current points.  A view's first use (once per
+// plan and view) sorts it on a stream of the plan's own, after the points, and waits for it: the view
+// is then complete for the operators of every stream, and when the caller's stream is capturing the
+// sort has run and is no part of the graph (as if it had been sorted when the points were set).
 int need_sorted(cov3d_plan *p, unsigned modes) {
   unsigned todo = 0;
   for (int m = 0; m < kSortModes; ++m) {
     if (!(modes >> m & 1)) continue;
     SortSet &ss = p->sets[m];
     ss.used = true;
-    if (!ss.valid || ss.every_use) todo |= 1u << m;
+    if (!ss.valid) todo |= 1u << m;
   }
   if (!todo) return COV3D_OK;
-  PhaseScope ps(p, kPhaseSort);
-  return sort_points(p, todo);
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // this thread may wait while a stream captures
+  COV3D_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+  const cudaStream_t caller = p->stream;
+  p->stream = p->sort_stream;
+  int rc = check_cuda(cudaStreamWaitEvent(p->sort_stream, p->points_set, 0), "points event");
+  if (rc == COV3D_OK) {
+    PhaseScope ps(p, kPhaseSort);
+    rc = sort_points(p, todo);
+  }
+  const int done = check_cuda(cudaStreamSynchronize(p->sort_stream), "sort");
+  p->stream = caller;
+  const int back = check_cuda(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
+  if (rc == COV3D_OK) rc = done != COV3D_OK ? done : back;
+  if (rc != COV3D_OK)
+    for (int m = 0; m < kSortModes; ++m)
+      if (todo >> m & 1) p->sets[m].valid = false;
+  return rc;
 }
 
 }  // namespace cov3d
