@@ -288,14 +288,14 @@ int cov3d_plan_create(int L, int n_trans, double eps, const cov3d_opts *opts, co
     p->beta = o.beta > 0.0 ? o.beta : 0.97 * kPi * (1.0 - 1.0 / (2.0 * o.upsample)) * w;
     // subproblems of up to 416 points: the most whose staged records keep two blocks of the
     // spreading on an SM; fewer subproblems flush fewer tiles
-    p->max_sub = 416;
+    p->max_sub = kSubPointsES;
   } else {
     p->width = o.kernel == COV3D_KERNEL_LINEAR ? 2 : 1;
     p->beta = 0.0;
     // 208 points are the most that keep four blocks of the linear windows' spreading on an SM (10
     // channels, 1024 images of 128^2: spread 2.20 -> 1.96 ms, interpolation 1.59 -> 1.66, against 384
     // points and two blocks); the nearest cells' spreading stages none
-    p->max_sub = o.kernel == COV3D_KERNEL_LINEAR ? 208 : 384;
+    p->max_sub = o.kernel == COV3D_KERNEL_LINEAR ? kSubPointsLinear : kSubPointsNearest;
   }
   const int bs = 8;
   if (o.bin_size != 0 && o.bin_size != 8) {

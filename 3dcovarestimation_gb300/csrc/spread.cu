@@ -209,7 +209,6 @@ __global__ void __launch_bounds__(kNearestThreads) spread_nearest_kernel(const S
 // per block, two blocks per SM (168 registers); 5 or 4 warps measured 5.8 and 6.8 ms against 5.3 (a
 // unrolled point loop is slower too: the ranges hold some ten points), 7 spill
 constexpr int kTileWarps = 6;
-constexpr int kTileMaxSub = 448;  // largest subproblem of an ES plan (three points per thread)
 
 // A point's record in floats: the W axis-1 weights twice each (operands of packed multiplies), the
 // axis-2 weights of the group's 8 columns, the axis-0 weights of up to 16 planes; a stride that keeps
@@ -555,6 +554,10 @@ int launch_nearest(const SpreadParams &a, const Value &value, bool comp, int64_t
 
 template <int KT, int W, int F, int NQ, int PP, bool HALF>
 int launch_tile(const SpreadParams &a, int64_t max_blocks, cudaStream_t st) {
+  if (a.max_sub > kTileMaxSub) {
+    set_error("subproblems of %d points; the spreading holds %d", a.max_sub, kTileMaxSub);
+    return COV3D_EINVAL;
+  }
   const size_t smem = (size_t)a.max_sub * tile_point_bytes<W, F>(NQ) + 8 +
                       tile_fixed_bytes(TileGroups<W>::T, TileGroups<W>::NG);
   return launch_spread_kernel(spread_tile_kernel<KT, W, F, NQ, PP, HALF>, "spread_tile_kernel", smem, a, max_blocks, st,
