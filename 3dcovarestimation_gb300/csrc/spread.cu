@@ -93,7 +93,7 @@ struct ArrayValue {
 // block takes the bin (up to kNearestSubs subproblems of it), thread t the bin's cell t: the block
 // counting-sorts its points by cell, kNearestThreads at a time, computes their values in that order
 // into shared memory, and every thread adds its cell's values in registers (with COMP by TwoSum).
-// A bin that fits one block is added to the grid without atomics.  The mean's batch of 1024 images of
+// The mean's batch of 1024 images of
 // 128^2: 1.75 + 0.11 ms (row tasks over staged values, values made by a kernel of their own) -> 0.63 ms;
 // what bounds it is the gather of the points' pixels and the barriers of the sort.
 constexpr int kNearestThreads = kBin * kBin * kBin;
@@ -109,7 +109,6 @@ __global__ void __launch_bounds__(kNearestThreads) spread_nearest_kernel(const S
   const int begin = a.bin_off[bin], end = a.bin_off[bin + 1];
   if ((first - begin) % (kNearestSubs * a.max_sub) != 0) return;
   const int last = min(end, first + kNearestSubs * a.max_sub);
-  const bool alone = first == begin && last == end;
   const SubTile st = sub_tile(a, sub);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float2 h0 = make_float2(0.f, 0.f), h1 = h0, l0 = h0, l1 = h0;
@@ -171,14 +170,9 @@ __global__ void __launch_bounds__(kNearestThreads) spread_nearest_kernel(const S
   const int n = a.g.n;  // a cell with points lies in the grid
   const int64_t cell = ((int64_t)wrap1(m0 + a.shift, n) * n + wrap1(m1 + a.shift, n)) * n + wrap1(m2 + a.shift, n);
   float2 *dst = a.grid + cell * a.cs + (int64_t)a.ch0 * a.chs;
-  const float2 x0 = __fadd2_rn(h0, l0), x1 = __fadd2_rn(h1, l1);
-  if (alone) {
-    *dst = __fadd2_rn(*dst, x0);
-    if (a.nch > 1) dst[a.chs] = __fadd2_rn(dst[a.chs], x1);
-  } else {
-    atomicAdd(dst, x0);
-    if (a.nch > 1) atomicAdd(dst + a.chs, x1);
-  }
+  // (atomics also where one block has the whole bin: several plans may add to one grid at a time)
+  atomicAdd(dst, __fadd2_rn(h0, l0));
+  if (a.nch > 1) atomicAdd(dst + a.chs, __fadd2_rn(h1, l1));
 }
 
 // Spreading for the ES windows (W = 4 .. 8) and the linear one (W = 2), any number of channels.  One
