@@ -73,37 +73,43 @@ __device__ __forceinline__ void two_sum(float &s, float &err, float d) {
 // real, whose extra 1/L is mean.py:215).
 struct MeanValue {
   MeanSource s;
-  __device__ __forceinline__ void operator()(const PointGeom &g, int id, float2 &v0, float2 &v1) const {
+  __device__ __forceinline__ void operator()(const PointGeom &g, int id, int, float2 &v0, float2 &v1) const {
     mean_value(s, id, g.P, g.Lp, v0, v1.x);
     v1.y = 0.0f;
   }
 };
-// Two channels of an array of point values
+// Channels 2 pair and 2 pair + 1 of an array of point values
 struct ArrayValue {
   const float2 *vals;
   int64_t ips, ics;
   int nch;
-  __device__ __forceinline__ void operator()(const PointGeom &, int id, float2 &v0, float2 &v1) const {
-    v0 = __ldg(vals + (int64_t)id * ips);
-    v1 = nch > 1 ? __ldg(vals + (int64_t)id * ips + ics) : make_float2(0.f, 0.f);
+  __device__ __forceinline__ void operator()(const PointGeom &, int id, int pair, float2 &v0, float2 &v1) const {
+    const float2 *v = vals + (int64_t)id * ips + 2 * pair * ics;
+    v0 = __ldg(v);
+    v1 = 2 * pair + 1 < nch ? __ldg(v + ics) : make_float2(0.f, 0.f);
   }
 };
 
-// Nearest-cell spreading of one or two channels.  A bin's cells belong to its points alone, so one
-// block takes the bin (up to kNearestSubs subproblems of it), thread t the bin's cell t: the block
-// counting-sorts its points by cell, kNearestThreads at a time, computes their values in that order
-// into shared memory, and every thread adds its cell's values in registers (with COMP by TwoSum).
-// The mean's batch of 1024 images of
-// 128^2: 1.75 + 0.11 ms (row tasks over staged values, values made by a kernel of their own) -> 0.63 ms;
-// what bounds it is the gather of the points' pixels and the barriers of the sort.
+// Nearest-cell spreading, NC pairs of channels per block (blockIdx.y).  A bin's cells belong to its points alone, so
+// one block takes the bin (up to kNearestSubs subproblems of it), thread t the bin's cell t: the block
+// counting-sorts its points by cell, kNearestThreads at a time, puts a channel pair's values in that
+// order into shared memory (two buffers in turn), and every thread adds its cell's values in registers
+// (with COMP by TwoSum).  What bounds it is the gather of the points' values and the barriers.  The
+// mean's batch of 1024 images of 128^2: 1.75 + 0.11 ms (row tasks over staged values, values made by a
+// kernel of their own) -> 0.57 ms.  The points are sorted once for up to five channel pairs, against a
+// sort and a launch per pair: 4.17 -> 3.2 ms for 10 channels of 1024 images of 128^2, 77 -> 53 us for 5
+// of 256 of 32^2, 111 -> 51 for 20 of 64 of 32^2.
 constexpr int kNearestThreads = kBin * kBin * kBin;
 constexpr int kNearestSubs = 16;
+constexpr int kNearestPairs = 5;
 
-template <bool COMP, typename Value>
-__global__ void __launch_bounds__(kNearestThreads) spread_nearest_kernel(const SpreadParams a, const Value value) {
+template <bool COMP, int NC, typename Value>
+__global__ void __launch_bounds__(kNearestThreads, NC <= 2 ? 2 : 1) spread_nearest_kernel(const SpreadParams a,
+                                                                                         const Value value) {
+  constexpr int NB = NC > 1 ? 2 : 1;
   __shared__ int s_cnt[kNearestThreads], s_off[kNearestThreads + 1], s_warp[kNearestThreads / 32];
-  __shared__ float2 s_v0[kNearestThreads], s_v1[kNearestThreads];
-  const int sub = blockIdx.x;
+  __shared__ float2 s_v[NB][2][kNearestThreads];
+  const int sub = blockIdx.x, pair0 = blockIdx.y * NC, nch = min(2 * NC, a.nch - 2 * pair0);
   if (sub >= *a.nsub) return;
   const int bin = a.sub_bin[sub], first = a.sub_first[sub];
   const int begin = a.bin_off[bin], end = a.bin_off[bin + 1];
@@ -111,24 +117,30 @@ __global__ void __launch_bounds__(kNearestThreads) spread_nearest_kernel(const S
   const int last = min(end, first + kNearestSubs * a.max_sub);
   const SubTile st = sub_tile(a, sub);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  float2 h0 = make_float2(0.f, 0.f), h1 = h0, l0 = h0, l1 = h0;
+  float2 h[NC][2], l[NC][2];
+#pragma unroll
+  for (int k = 0; k < NC; ++k) h[k][0] = h[k][1] = l[k][0] = l[k][1] = make_float2(0.f, 0.f);
   bool any = false;
   for (int base = first; base < last; base += kNearestThreads) {
     s_cnt[tid] = 0;
     __syncthreads();  // also: the previous chunk's values have been read
     const bool live = base + tid < last;
-    int key = 0, rank = 0;
+    int key = 0, rank = 0, id = 0;
+    float sc = 0.0f;
     float2 v0, v1;
+    auto load = [&](int pair) {
+      value(a.g, id, pair0 + pair, v0, v1);
+      v0 = make_float2(v0.x * sc, v0.y * sc);
+      v1 = make_float2(v1.x * sc, v1.y * sc);
+    };
     if (live) {
       const SortedPoint sp = a.pts[base + tid];
       key = (((int)rintf(sp.t0) - st.ts0) * kBin + (int)rintf(sp.t1) - st.ts1) * kBin + (int)rintf(sp.t2) - st.ts2;
       rank = atomicAdd(s_cnt + key, 1);
-      const int id = sp_id<false>(sp.idf);
-      value(a.g, id, v0, v1);
-      float sc = (a.nyquist && sp_nyquist(sp.idf)) ? 0.0f : a.scale;
+      id = sp_id<false>(sp.idf);
+      sc = (a.nyquist && sp_nyquist(sp.idf)) ? 0.0f : a.scale;
       sc *= ctf_factor(a.ctf, a.ctfc, a.g, id);
-      v0 = make_float2(v0.x * sc, v0.y * sc);
-      v1 = make_float2(v1.x * sc, v1.y * sc);
+      load(0);
     }
     __syncthreads();
     const int c = s_cnt[tid];
@@ -145,23 +157,29 @@ __global__ void __launch_bounds__(kNearestThreads) spread_nearest_kernel(const S
     const int off = before + incl - c;
     s_off[tid] = off;
     __syncthreads();
-    if (live) {
-      const int slot = s_off[key] + rank;
-      s_v0[slot] = v0;
-      s_v1[slot] = v1;
-    }
-    __syncthreads();
+    const int slot = live ? s_off[key] + rank : 0;
     any = any || c > 0;
-    for (int i = off; i < off + c; ++i) {
-      const float2 x = s_v0[i], y = s_v1[i];
-      if (COMP) {
-        two_sum(h0.x, l0.x, x.x);
-        two_sum(h0.y, l0.y, x.y);
-        two_sum(h1.x, l1.x, y.x);
-        two_sum(h1.y, l1.y, y.y);
-      } else {
-        h0 = __fadd2_rn(h0, x);
-        h1 = __fadd2_rn(h1, y);
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      if (2 * k >= nch) break;
+      float2(&s_v0)[kNearestThreads] = s_v[k & (NB - 1)][0], (&s_v1)[kNearestThreads] = s_v[k & (NB - 1)][1];
+      if (live) {
+        s_v0[slot] = v0;
+        s_v1[slot] = v1;
+        if (k + 1 < NC && 2 * k + 2 < nch) load(k + 1);
+      }
+      __syncthreads();  // (the buffer written next was read before the last one)
+      for (int i = off; i < off + c; ++i) {
+        const float2 x = s_v0[i], y = s_v1[i];
+        if (COMP) {
+          two_sum(h[k][0].x, l[k][0].x, x.x);
+          two_sum(h[k][0].y, l[k][0].y, x.y);
+          two_sum(h[k][1].x, l[k][1].x, y.x);
+          two_sum(h[k][1].y, l[k][1].y, y.y);
+        } else {
+          h[k][0] = __fadd2_rn(h[k][0], x);
+          h[k][1] = __fadd2_rn(h[k][1], y);
+        }
       }
     }
   }
@@ -169,10 +187,11 @@ __global__ void __launch_bounds__(kNearestThreads) spread_nearest_kernel(const S
   const int m0 = st.ts0 + tid / (kBin * kBin), m1 = st.ts1 + (tid / kBin) % kBin, m2 = st.ts2 + tid % kBin;
   const int n = a.g.n;  // a cell with points lies in the grid
   const int64_t cell = ((int64_t)wrap1(m0 + a.shift, n) * n + wrap1(m1 + a.shift, n)) * n + wrap1(m2 + a.shift, n);
-  float2 *dst = a.grid + cell * a.cs + (int64_t)a.ch0 * a.chs;
+  float2 *dst = a.grid + cell * a.cs + (int64_t)(2 * pair0) * a.chs;
   // (atomics also where one block has the whole bin: several plans may add to one grid at a time)
-  atomicAdd(dst, __fadd2_rn(h0, l0));
-  if (a.nch > 1) atomicAdd(dst + a.chs, __fadd2_rn(h1, l1));
+#pragma unroll
+  for (int ch = 0; ch < 2 * NC; ++ch)
+    if (ch < nch) atomicAdd(dst + ch * a.chs, __fadd2_rn(h[ch / 2][ch % 2], l[ch / 2][ch % 2]));
 }
 
 // Spreading for the ES windows (W = 4 .. 8) and the linear one (W = 2), any number of channels.  One
@@ -539,10 +558,11 @@ int launch_spread_kernel(Kernel kernel, const char *name, size_t smem, const Spr
   return launched(name);
 }
 
-template <typename Value>
+template <int NC, typename Value>
 int launch_nearest(const SpreadParams &a, const Value &value, bool comp, int64_t max_blocks, cudaStream_t st) {
-  if (comp) spread_nearest_kernel<true, Value><<<(unsigned)max_blocks, kNearestThreads, 0, st>>>(a, value);
-  else spread_nearest_kernel<false, Value><<<(unsigned)max_blocks, kNearestThreads, 0, st>>>(a, value);
+  const dim3 grid((unsigned)max_blocks, (unsigned)((a.nch + 2 * NC - 1) / (2 * NC)));
+  if (comp) spread_nearest_kernel<true, NC, Value><<<grid, kNearestThreads, 0, st>>>(a, value);
+  else spread_nearest_kernel<false, NC, Value><<<grid, kNearestThreads, 0, st>>>(a, value);
   return launched("spread_nearest_kernel");
 }
 
@@ -610,14 +630,15 @@ int launch_w(const SpreadParams &a, int nchan, int64_t max_blocks, cudaStream_t 
   }
 }
 
-// Channels of an array two at a time
 int launch_nearest_channels(SpreadParams a, int nchan, bool comp, int64_t max_blocks, cudaStream_t st) {
-  for (int c = 0; c < nchan; c += 2) {
-    a.ch0 = c;
-    a.nch = min(2, nchan - c);
-    COV3D_TRY(launch_nearest(a, ArrayValue{a.vals + (int64_t)c * a.ics, a.ips, a.ics, a.nch}, comp, max_blocks, st));
+  a.nch = nchan;
+  const ArrayValue v{a.vals, a.ips, a.ics, nchan};
+  switch ((nchan + 1) / 2) {
+    case 1: return launch_nearest<1>(a, v, comp, max_blocks, st);
+    case 2: return launch_nearest<2>(a, v, comp, max_blocks, st);
+    case 3: return launch_nearest<3>(a, v, comp, max_blocks, st);
+    default: return launch_nearest<kNearestPairs>(a, v, comp, max_blocks, st);
   }
-  return COV3D_OK;
 }
 
 // Per-image adjoint (no sum over images): direct global atomics, one thread per point.
@@ -729,7 +750,7 @@ int launch_spread_mean_nearest(cov3d_plan *p, const MeanSource &src, const Epilo
   int64_t mb;
   COV3D_TRY(spread_params(p, e, grids, 1, chan_stride, 0, kSortFull, a, mb));
   a.nch = 2;
-  return launch_nearest(a, MeanValue{src}, p->compensated != 0, mb, p->stream);
+  return launch_nearest<1>(a, MeanValue{src}, p->compensated != 0, mb, p->stream);
 }
 
 int launch_spread_unaggregated(cov3d_plan *p, const void *values, int64_t in_ps, const EpilogueArgs &e,
