@@ -253,18 +253,24 @@ __device__ __forceinline__ int taps(float t, int frac, float beta, float *wt) {
   return c0;
 }
 
-// Groups of neighbouring window corners along axis 2 for the ES windows (W = 4 .. 8): the windows of
-// the GS = 9 - W corners of a group lie in the same eight columns of a bin's tile (8 + W - 1 cells
-// per axis).
-template <int W>
+// Groups of neighbouring window corners along axis 2: the windows of the GS corners of a group lie in
+// the same COLS (8, or all) of the T = 8 + W - 1 columns of a bin's tile.
+template <int W, int COLUMNS = 8>
 struct TileGroups {
   static constexpr int T = 8 + W - 1;
-  static constexpr int GS = 9 - W;           // corners per group
+  static constexpr int COLS = COLUMNS;
+  static constexpr int GS = COLS + 1 - W < 8 ? COLS + 1 - W : 8;  // corners per group
   static constexpr int NG = (8 + GS - 1) / GS;
-  __device__ static constexpr int base(int g) {  // first tile column of the group's eight
-    return g * GS < T - 8 ? g * GS : T - 8;
+  __device__ static constexpr int base(int g) {  // first tile column of the group's
+    return g * GS < T - COLS ? g * GS : T - COLS;
   }
 };
+
+// Adds x to a cell of a grid.  (Spelled out: with its result unused, atomicAdd on a float2 took up to
+// twice the kernel's time, depending on the code around it.)
+__device__ __forceinline__ void add_cell(float2 *cell, float2 x) {
+  asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};" ::"l"(__cvta_generic_to_global(cell)), "f"(x.x), "f"(x.y) : "memory");
+}
 
 // CTF at pixel offsets (ka, kb) (row, column) from the image centre: sqrt(1 - w^2) sin(gamma) -
 // w cos(gamma) with gamma = c0 K + c1 D + c2 X + d K^2 - ps (see CtfCoef).  gamma reaches a few

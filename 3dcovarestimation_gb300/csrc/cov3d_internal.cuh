@@ -98,7 +98,7 @@ enum SortMode { kSortFull = 0, kSortHalf = 1, kSortModes = 2 };
 
 // Points of a subproblem by kernel (chosen in cov3d_plan_create); the spreading kernels give each
 // thread a fixed number of points, so theirs are bounded by kTileMaxSub.
-constexpr int kSubPointsES = 416, kSubPointsLinear = 208, kSubPointsNearest = 384;
+constexpr int kSubPointsES = 416, kSubPointsLinear = 384, kSubPointsNearest = 384;
 constexpr int kTileMaxSub = 448;
 static_assert(kSubPointsES <= kTileMaxSub && kSubPointsLinear <= kTileMaxSub, "points per thread of spread_tile_kernel");
 

@@ -292,9 +292,8 @@ int cov3d_plan_create(int L, int n_trans, double eps, const cov3d_opts *opts, co
   } else {
     p->width = o.kernel == COV3D_KERNEL_LINEAR ? 2 : 1;
     p->beta = 0.0;
-    // 208 points are the most that keep four blocks of the linear windows' spreading on an SM (10
-    // channels, 1024 images of 128^2: spread 2.20 -> 1.96 ms, interpolation 1.59 -> 1.66, against 384
-    // points and two blocks); the nearest cells' spreading stages none
+    // 384 points are the most that keep two blocks of the linear windows' spreading on an SM; the nearest
+    // cells' stages none
     p->max_sub = o.kernel == COV3D_KERNEL_LINEAR ? kSubPointsLinear : kSubPointsNearest;
   }
   const int bs = 8;

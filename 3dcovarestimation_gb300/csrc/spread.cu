@@ -191,137 +191,203 @@ __global__ void __launch_bounds__(kNearestThreads, NC <= 2 ? 2 : 1) spread_neare
   // (atomics also where one block has the whole bin: several plans may add to one grid at a time)
 #pragma unroll
   for (int ch = 0; ch < 2 * NC; ++ch)
-    if (ch < nch) atomicAdd(dst + ch * a.chs, __fadd2_rn(h[ch / 2][ch % 2], l[ch / 2][ch % 2]));
+    if (ch < nch) add_cell(dst + ch * a.chs, __fadd2_rn(h[ch / 2][ch % 2], l[ch / 2][ch % 2]));
 }
 
 // Spreading for the ES windows (W = 4 .. 8) and the linear one (W = 2), any number of channels.  One
 // block per subproblem (a bin of 8^3 cells and at most max_sub of its points); the cells it can reach
-// are a tile of T^3, T = 8 + W - 1.  The block sorts its points by (axis-2 group, l1, l0), l the bin-local corner of
-// their window and a group GS = 9 - W neighbouring l2, so that the windows of a group lie in the
-// same 8 tile columns, and stages a record per point (weights) and its channel values.
+// are a tile of T^3, T = 8 + W - 1.  The block sorts its points by (axis-2 group, l1, l0), l the
+// bin-local corner of their window and a group the neighbouring l2 whose windows lie in the same COLS
+// tile columns (8, or with ONE all T in one group), and stages a record per point: its weights and its
+// channel values.
 //
-// A warp task is NPL tile planes of one group, all T rows: lane (q, c) owns column c of the group,
-// part q % NQ of the channels (F floats) and part q / NQ of the planes (PP of them), with
-// acc[PP][T][F / 2] in registers.  The points whose windows meet the planes are for each l1 the
-// contiguous range l0 in [first plane - W + 1, last plane] of the sorted order, and with l1 a
-// compile-time constant in the unrolled loop their W rows are fixed registers: a point costs a lane
-// F values, W + PP + 1 weights and PP * W * F multiply-adds.
+// A warp task is one tile plane, all T rows: lane (h, part, c) owns column c modulo COLS, a part of the
+// channels (F floats) and every NH-th point, with acc[T][F / 2] in registers.  The points of a group
+// whose windows meet the plane are for each l1 the contiguous range l0 in [plane - W + 1, plane] of the
+// sorted order, and with l1 a compile-time constant in the unrolled loop their W rows are fixed
+// registers: a point costs a lane F values, W + 2 weights and W * F multiply-adds.  The groups follow
+// one another; a column goes to the grid after the last group that reaches it, and its lane takes the
+// column COLS further on.
 //
-// What bounds it: latency at twelve warps per SM (issue 47 %, FP32 pipe 32 %, shared wavefronts
-// 17 % of their peaks on the B = 256 capture).  At the covariance step's 10 channels, W = 6, a visit
-// is some 50 instructions and a point has 3.5 of them.  Its predecessor, lanes owning all 13 tile
-// columns of three rows of one plane, had 16 visits and 2.2x the multiply-adds.  Measured on the step at
-// L = 128, B = 1024, r = 10: 8.6 -> 5.3 ms, of which staging (sort, weights, gathered values) about
-// 2.0 and the flush 0.9; 4.7 with the points in registers, their values asked for ahead and four
-// gathers in flight.  One channel at W = 7, 512 images of 128^2: 6.2 -> 1.0 ms.
+// Every cell is added to the grid once per subproblem, from folded sums: the NH lanes' sums meet in
+// shuffles, and the ES windows' points are added in pairs.  So a cell's error is that of about half as
+// many FP32 additions as it has points in a subproblem and of one atomic addition per subproblem,
+// whether the plan asks for `compensated` sums or not.  That is no more than the compensated row sums
+// of this kernel's predecessor had (one atomic addition per subproblem of as many points, two or three
+// FP32 sums folded by TwoSum).  Relative error of 1024 central slices of 64^2 on 128^3 against 64-bit
+// sums, all cells and the 9^3 around the origin, where up to 416 points of a subproblem meet in a cell
+// and some 500 subproblems follow one another: values of one sign 1.08e-7 and 1.89e-7 then, 1.06e-7
+// and 1.8e-7 here (W = 6, ten channels); noise 1.68e-7 and 2.53e-7, here 1.64e-7 and 2.45e-7; linear
+// windows 6.0e-8 and 9.6e-8, here 5.6e-8 to 6.1e-8 and 7.7e-8 to 9.6e-8.  A task per plane pair and group,
+// each group's columns added to the grid apart, took 8.6 ms where this takes 10.5 (below), but its 1.85 additions
+// per cell and subproblem cost 1.36e-7 and 2.58e-7.
 //
-// Each cell's sum is plain FP32 over the points of one group of one subproblem (some 30 terms at
-// one point per cell, a third of what the predecessor summed before its first TwoSum fold; two or
-// three partial sums folded by TwoSum round to the float sum of the partials), and the partial sums
-// meet in FP32 global atomics, so `compensated` changes nothing here.
-// per block, two blocks per SM (168 registers); 5 or 4 warps measured 5.8 and 6.8 ms against 5.3 (a
-// unrolled point loop is slower too: the ranges hold some ten points), 7 spill
-constexpr int kTileWarps = 6;
+// What bounds it: latency at sixteen warps per SM (some 38 instructions for a point's visit to a plane,
+// of which it has W), then the flush, W + 7 times W + 7 rows in NG steps, for subproblems of few points.
+// 10 channels, W = 6, 1024 images of 128^2 (full records): 15.8 ms the predecessor, 10.5 here; W = 7, one
+// channel, 512 images: 11.2 and 2.2; W = 7, 10 channels, 100 images: 3.46 and 3.73.  Bilinear, 10 channels of
+// 1024 images: 4.24 and 3.06.
+template <int W, int F, int NQ, bool ONE>
+struct TileShape {
+  using G = TileGroups<W, ONE ? 8 + W - 1 : 8>;
+  static constexpr int T = G::T, COLS = G::COLS, NG = G::NG;
+  static constexpr int NH = 32 / COLS / NQ;     // subsets of the points
+  static constexpr int RH = (T + NH - 1) / NH;  // rows that each of them flushes
+  // How a lane folds its sums: the points of a range summed apart (wide windows, of which a cell sees the
+  // most points, which in pairs are 1.5e-7 off near the origin against 1.24e-7; the registers leave six
+  // warps, 11.2 ms against 10.5 at W = 6), or points added in pairs.
+  static constexpr bool RANGES = W >= 7 && NH == 1 && F > 2;
+  static constexpr bool PAIRS = W > 2 && !RANGES && (NH == 1 || F == 2);
+  static constexpr int WARPS = W == 2 ? 9 : F == 2 ? 14 : RANGES ? 6 : 8;
+  static_assert(NH >= 1 && NH <= 3 && T <= 16, "lanes; plane weights of a record");
 
-// A point's record in floats: the W axis-1 weights twice each (operands of packed multiplies), the
-// axis-2 weights of the group's 8 columns, the axis-0 weights of up to 16 planes; a stride that keeps
-// 16-byte stores of consecutive records free of bank conflicts (4 modulo 8 words).
-template <int W>
-struct TileRec {
-  static constexpr int W2 = (2 * W + 3) / 4 * 4;
-  static constexpr int W0 = W2 + 8;
-  static constexpr int STRIDE = W <= 2 ? 28 : W <= 6 ? 36 : 44;
-  static_assert(W0 + 16 <= STRIDE && STRIDE % 8 == 4, "plane weights; conflict-free stores");
-};
-
-template <int F>
-struct TileVals {  // floats of a channel part's values, padded to 16 bytes where loads are
-  static constexpr int STRIDE = F <= 2 ? F : (F + 3) / 4 * 4;
-};
-
-template <int W, int F>
-__host__ __device__ constexpr size_t tile_point_bytes(int NQ) {
-  return (TileRec<W>::STRIDE + NQ * TileVals<F>::STRIDE + 4) * 4;  // ... id, mirror id, two factors
-}
-__host__ __device__ constexpr size_t tile_fixed_bytes(int T, int NG) {
-  return (size_t)T * T * sizeof(long long) + (size_t)(2 * NG * 64 + 1 + T + 2) * sizeof(int);
-}
-
-// The points of corner row l1 = L1 .. 7 added to the lane's cells
-template <int W, int F, int NQ, int PP, int L1>
-struct TileRows {
-  template <typename Range>
-  __device__ __forceinline__ static void run(const Range &range, const float *recs, const float *vals, int cp, int col,
-                                             int plane, float2 (&acc)[PP][TileGroups<W>::T][F / 2]) {
-    using Rec = TileRec<W>;
-    int i, iend;
-    range(L1, i, iend);
-    const float *rec = recs + i * Rec::STRIDE;
-    const float *vp = vals + (i * NQ + cp) * TileVals<F>::STRIDE;
-#pragma unroll 1
-    for (; i < iend; ++i, rec += Rec::STRIDE, vp += NQ * TileVals<F>::STRIDE) {
-      const float w2 = rec[Rec::W2 + col];
-      float w0[PP];
-      if constexpr (PP == 2) {
-        const float2 x = *reinterpret_cast<const float2 *>(rec + Rec::W0 + plane);
-        w0[0] = x.x;
-        w0[1] = x.y;
-      } else {
-        w0[0] = rec[Rec::W0 + plane];
-      }
-      float2 w1[W];
+  // A point's record in floats: the W axis-1 weights twice each (operands of packed multiplies), the
+  // axis-2 weights of the group's columns, the axis-0 weights of the T planes; a stride that keeps
+  // 16-byte stores of consecutive records free of bank conflicts (4 modulo 8 words).
+  static constexpr int W2 = 2 * W, W0 = W2 + COLS, REC = (W0 + T + 3) / 8 * 8 + 4;
+  static_assert(W0 + T <= REC, "a record's weights");
+  // Its staged channel values: NQ parts of F / 2 channels next to each other.
+  static constexpr int VALS = F * NQ;
+  __device__ __forceinline__ static void load_values(const float *vp, float2 (&v)[F / 2]) {
+    if constexpr (F % 4 == 0) {
 #pragma unroll
-      for (int j = 0; j + 1 < W; j += 2) {
-        const float4 x = *reinterpret_cast<const float4 *>(rec + 2 * j);
-        w1[j] = make_float2(x.x, x.y);
-        w1[j + 1] = make_float2(x.z, x.w);
-      }
-      if constexpr (W & 1) w1[W - 1] = *reinterpret_cast<const float2 *>(rec + 2 * (W - 1));
-      float2 v[F / 2];
-#pragma unroll
-      for (int f = 0; f + 1 < F / 2; f += 2) {
+      for (int f = 0; f < F / 2; f += 2) {
         const float4 x = *reinterpret_cast<const float4 *>(vp + 2 * f);
         v[f] = make_float2(x.x, x.y);
         v[f + 1] = make_float2(x.z, x.w);
       }
-      if constexpr ((F / 2) & 1) v[F / 2 - 1] = *reinterpret_cast<const float2 *>(vp + F - 2);
+    } else {
 #pragma unroll
-      for (int k = 0; k < PP; ++k) {
-        const float w02 = w0[k] * w2;
-        const float2 ww = make_float2(w02, w02);
+      for (int f = 0; f < F / 2; ++f) v[f] = *reinterpret_cast<const float2 *>(vp + 2 * f);
+    }
+  }
+  // bytes of shared memory: a point's (record, values, id, mirror id, two factors), and the rest
+  static constexpr size_t POINT = (REC + VALS + 4) * sizeof(float);
+  static constexpr size_t FIXED = T * T * sizeof(long long) + (2 * NG * 64 + 1 + T + 1) * sizeof(int) + 8;
+};
+
+// The points of corner row l1 = L1 .. 7 of the lane's subset added to its cells
+template <int W, int F, int NQ, bool ONE, int L1>
+struct TileRows {
+  using S = TileShape<W, F, NQ, ONE>;
+  // axis-1 weights (twice each) and the product of the other axes' weights
+  __device__ __forceinline__ static float2 weights(const float *rec, int col, int plane, float2 (&w)[W]) {
+    const float w02 = rec[S::W0 + plane] * rec[S::W2 + col];
+#pragma unroll
+    for (int j = 0; j + 1 < W; j += 2) {
+      const float4 x = *reinterpret_cast<const float4 *>(rec + 2 * j);
+      w[j] = make_float2(x.x, x.y);
+      w[j + 1] = make_float2(x.z, x.w);
+    }
+    if constexpr (W & 1) w[W - 1] = *reinterpret_cast<const float2 *>(rec + 2 * (W - 1));
+    return make_float2(w02, w02);
+  }
+  template <typename Range>
+  __device__ __forceinline__ static void run(const Range &range, const float *recs, const float *vals, int cp, int h,
+                                             int col, int plane, float2 (&acc)[S::T][F / 2]) {
+    constexpr int NH = S::NH;
+    int i, iend;
+    range(L1, i, iend);
+    i += h;
+    const float *rec = recs + i * S::REC;
+    const float *vp = vals + i * S::VALS + F * cp;
+    float2 wa[W], va[F / 2];
+    if constexpr (S::RANGES) {
+      if (i < iend) {
+        float2 t[W][F / 2];
+        const float2 sa = weights(rec, col, plane, wa);
+        S::load_values(vp, va);
 #pragma unroll
         for (int j = 0; j < W; ++j) {
-          const float2 w = __fmul2_rn(ww, w1[j]);
+          const float2 x = __fmul2_rn(sa, wa[j]);
 #pragma unroll
-          for (int f = 0; f < F / 2; ++f) acc[k][L1 + j][f] = __ffma2_rn(w, v[f], acc[k][L1 + j][f]);
+          for (int f = 0; f < F / 2; ++f) t[j][f] = __fmul2_rn(x, va[f]);
+        }
+#pragma unroll 1
+        for (i += NH; i < iend; i += NH) {
+          rec += NH * S::REC, vp += NH * S::VALS;
+          const float2 sb = weights(rec, col, plane, wa);
+          S::load_values(vp, va);
+#pragma unroll
+          for (int j = 0; j < W; ++j) {
+            const float2 x = __fmul2_rn(sb, wa[j]);
+#pragma unroll
+            for (int f = 0; f < F / 2; ++f) t[j][f] = __ffma2_rn(x, va[f], t[j][f]);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+#pragma unroll
+          for (int f = 0; f < F / 2; ++f) acc[L1 + j][f] = __fadd2_rn(acc[L1 + j][f], t[j][f]);
+      }
+    }
+    if constexpr (S::PAIRS) {
+#pragma unroll 1
+      for (; i + NH < iend; i += 2 * NH, rec += 2 * NH * S::REC, vp += 2 * NH * S::VALS) {
+        float2 wb[W], vb[F / 2];
+        const float2 sa = weights(rec, col, plane, wa);
+        S::load_values(vp, va);
+        const float2 sb = weights(rec + NH * S::REC, col, plane, wb);
+        S::load_values(vp + NH * S::VALS, vb);
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+          const float2 x = __fmul2_rn(sa, wa[j]), y = __fmul2_rn(sb, wb[j]);
+#pragma unroll
+          for (int f = 0; f < F / 2; ++f)
+            acc[L1 + j][f] = __fadd2_rn(acc[L1 + j][f], __ffma2_rn(y, vb[f], __fmul2_rn(x, va[f])));
         }
       }
     }
-    if constexpr (L1 + 1 < kBin) TileRows<W, F, NQ, PP, L1 + 1>::run(range, recs, vals, cp, col, plane, acc);
+#pragma unroll 1
+    for (; !S::RANGES && i < iend; i += NH, rec += NH * S::REC, vp += NH * S::VALS) {
+      const float2 sa = weights(rec, col, plane, wa);
+      S::load_values(vp, va);
+#pragma unroll
+      for (int j = 0; j < W; ++j) {
+        const float2 x = __fmul2_rn(sa, wa[j]);
+#pragma unroll
+        for (int f = 0; f < F / 2; ++f) acc[L1 + j][f] = __ffma2_rn(x, va[f], acc[L1 + j][f]);
+      }
+      if (S::PAIRS) break;  // at most one is left
+    }
+    if constexpr (L1 + 1 < kBin) TileRows<W, F, NQ, ONE, L1 + 1>::run(range, recs, vals, cp, h, col, plane, acc);
   }
 };
 
-// F / 2 channels per lane in NQ parts.
-// Warps per block: two blocks fit an SM either way (the staged records), and one channel's accumulators
-// (one plane and up to 15 rows a lane) leave registers for 14 warps in each, with a point per thread
-// and smaller tasks (512 images of 128^2, W = 7: 1.26 -> 1.00 ms against 6 warps and two planes a lane).
-__host__ __device__ constexpr int tile_warps(int W, int F) { return W > 2 && F == 2 ? 14 : kTileWarps; }
+// The sum over the NH lane subsets of channel f of row k + RH h, in subset h; LANES lanes in a subset.
+template <int NH, int LANES, int T, int FH>
+__device__ __forceinline__ float2 subset_sum(const float2 (&acc)[T][FH], int k, int f, int h, int lane) {
+  constexpr int RH = (T + NH - 1) / NH;
+  auto row = [&](int r) { return r < T ? acc[r][f] : make_float2(0.f, 0.f); };
+  auto pick = [](bool p, float2 a, float2 b) { return make_float2(p ? a.x : b.x, p ? a.y : b.y); };
+  auto from = [](float2 x, int l) {
+    return make_float2(__shfl_sync(0xffffffffu, x.x, l), __shfl_sync(0xffffffffu, x.y, l));
+  };
+  if constexpr (NH == 1) {
+    return row(k);
+  } else if constexpr (NH == 2) {
+    const bool up = h != 0;
+    return __fadd2_rn(pick(up, row(k + RH), row(k)), from(pick(up, row(k), row(k + RH)), up ? lane - LANES : lane + LANES));
+  } else {  // the rows of the next subset go to it, those of the one before to that
+    const int next = h < 2 ? lane + LANES : lane - 2 * LANES, prev = h > 0 ? lane - LANES : lane + 2 * LANES;
+    auto of = [&](int s) { return pick(s == 0, row(k), pick(s == 1, row(k + RH), row(k + 2 * RH))); };
+    const int h1 = h < 2 ? h + 1 : 0, h2 = h > 0 ? h - 1 : 2;
+    return __fadd2_rn(of(h), __fadd2_rn(from(of(h1), prev), from(of(h2), next)));
+  }
+}
 
-template <int KT, int W, int F, int NQ, int PP, bool HALF>
-__global__ void __launch_bounds__(tile_warps(W, F) * 32, W == 2 ? 4 : 2) spread_tile_kernel(const SpreadParams a) {
+template <int KT, int W, int F, int NQ, bool ONE, bool HALF>
+__global__ void __launch_bounds__(TileShape<W, F, NQ, ONE>::WARPS * 32, 2) spread_tile_kernel(const SpreadParams a) {
   constexpr bool ES = KT == COV3D_KERNEL_ES;
-  using G = TileGroups<W>;
-  using Rec = TileRec<W>;
-  constexpr int VS = TileVals<F>::STRIDE;
-  constexpr int T = G::T, NG = G::NG, NK = NG * 64;
-  constexpr int CH = NQ * F / 2;                 // channels per pass
-  constexpr int NPL = PP * (4 / NQ);             // planes per task
-  constexpr int PGS = (T + NPL - 1) / NPL;       // plane groups
-  static_assert(PGS * NPL <= 16, "plane weights of a record");
+  using S = TileShape<W, F, NQ, ONE>;
+  using G = typename S::G;
+  constexpr int T = G::T, NG = G::NG, NK = NG * 64, COLS = G::COLS, NH = S::NH, RH = S::RH;
+  constexpr int FH = F / 2, CH = NQ * FH, VS = S::VALS;  // channels of a lane, of a pass; values of a point
+  constexpr int THREADS = S::WARPS * 32;
   extern __shared__ float4 smem4[];
-  float *recs = reinterpret_cast<float *>(smem4);                // max_sub * record stride
-  float *vals = recs + (size_t)a.max_sub * Rec::STRIDE;          // max_sub * NQ * VS
-  int *s_id = reinterpret_cast<int *>(vals + (size_t)a.max_sub * NQ * VS);
+  float *recs = reinterpret_cast<float *>(smem4);                // max_sub * record
+  float *vals = recs + (size_t)a.max_sub * S::REC;               // max_sub * VS
+  int *s_id = reinterpret_cast<int *>(vals + (size_t)a.max_sub * VS);
   int *s_mid = s_id + a.max_sub;      // ids; mirror ids or -1
   float *s_sc = reinterpret_cast<float *>(s_mid + a.max_sub), *s_scm = s_sc + a.max_sub;
   long long *s_row = reinterpret_cast<long long *>((reinterpret_cast<uintptr_t>(s_scm + a.max_sub) + 7) & ~(uintptr_t)7);
@@ -342,18 +408,18 @@ __global__ void __launch_bounds__(tile_warps(W, F) * 32, W == 2 ? 4 : 2) spread_
   };
   // each thread keeps its points until their place in the sorted order is known, and asks for their
   // values (point-major ones) ahead of the gather
-  constexpr int PPT = (kTileMaxSub + tile_warps(W, F) * 32 - 1) / (tile_warps(W, F) * 32);
+  constexpr int PPT = (kTileMaxSub + THREADS - 1) / (THREADS);
   SortedPoint pt[PPT];
   int pkey[PPT];
 #pragma unroll
   for (int u = 0; u < PPT; ++u) {
-    const int k = tid + u * tile_warps(W, F) * 32;
+    const int k = tid + u * THREADS;
     pkey[u] = -1;
     if (k < st.cnt) pt[u] = a.pts[st.first + k];
   }
 #pragma unroll
   for (int u = 0; u < PPT; ++u) {
-    if (tid + u * tile_warps(W, F) * 32 >= st.cnt) continue;
+    if (tid + u * THREADS >= st.cnt) continue;
     const int key = (corner(pt[u].t2, st.ts2) / G::GS) * 64 + corner(pt[u].t1, st.ts1) * 8 + corner(pt[u].t0, st.ts0);
     pkey[u] = key | (atomicAdd(s_cnt + key, 1) << 9);
     if (a.ics == 1) {
@@ -390,7 +456,7 @@ __global__ void __launch_bounds__(tile_warps(W, F) * 32, W == 2 ? 4 : 2) spread_
   for (int e = tid; e < T * T; e += blockDim.x) {
     const int ra = e / T, rb = e - (e / T) * T;
     const int m0 = wrap1(wrap1(st.ts0 + ra, n) + a.shift, n), m1 = wrap1(wrap1(st.ts1 + rb, n) + a.shift, n);
-    s_row[e] = ES || (st.ts0 + ra < n && st.ts1 + rb < n) ? ((int64_t)m0 * n + m1) * n : -1;
+    s_row[e] = ES || (st.ts0 + ra < n && st.ts1 + rb < n) ? ((int64_t)m0 * n + m1) * n * a.cs : -1;
   }
   for (int e = tid; e < T; e += blockDim.x) s_col[e] = ES || st.ts2 + e < n ? wrap1(wrap1(st.ts2 + e, n) + a.shift, n) : -1;
   __syncthreads();
@@ -405,7 +471,7 @@ __global__ void __launch_bounds__(tile_warps(W, F) * 32, W == 2 ? 4 : 2) spread_
               c2 = record_cell<KT, W, HALF>(sp.t2, a.g.frac);
     const int l0 = (ES ? wrap1(c0, n) : c0) - st.ts0, l2 = (ES ? wrap1(c2, n) : c2) - st.ts2;
     const int b2 = G::base((kr & 511) >> 6);
-    float4 *rec = reinterpret_cast<float4 *>(recs + slot * Rec::STRIDE);
+    float4 *rec = reinterpret_cast<float4 *>(recs + slot * S::REC);
     // the axes' weights at offset i from the window's first cell, zero outside the window
     float x0, x1, x2, y0 = 0.f, y1 = 0.f, y2 = 0.f;
     if (ES) {
@@ -427,21 +493,17 @@ __global__ void __launch_bounds__(tile_warps(W, F) * 32, W == 2 ? 4 : 2) spread_
     auto weight = [&](float x, float y, int i) {
       return ES ? es_weight<W>(x - (float)i, a.k.beta) : i == 0 ? x : i == 1 ? y : 0.0f;
     };
-    float w[8];
+    float w[S::REC];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) w[j] = j < W ? weight(x1, y1, j) : 0.0f;
+    for (int j = 0; j < W; ++j) w[2 * j] = w[2 * j + 1] = weight(x1, y1, j);
 #pragma unroll
-    for (int u = 0; u < Rec::W2 / 4; ++u) rec[u] = make_float4(w[2 * u], w[2 * u], w[2 * u + 1], w[2 * u + 1]);
+    for (int j = 0; j < COLS; ++j) w[S::W2 + j] = weight(x2, y2, b2 + j - l2);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) w[j] = weight(x2, y2, b2 + j - l2);
-    rec[Rec::W2 / 4] = make_float4(w[0], w[1], w[2], w[3]);
-    rec[Rec::W2 / 4 + 1] = make_float4(w[4], w[5], w[6], w[7]);
+    for (int j = 0; j < T; ++j) w[S::W0 + j] = weight(x0, y0, j - l0);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int j = S::W0 + T; j < S::REC; ++j) w[j] = 0.0f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = 4 * u + j < T ? weight(x0, y0, 4 * u + j - l0) : 0.0f;
-      rec[Rec::W0 / 4 + u] = make_float4(w[0], w[1], w[2], w[3]);
-    }
+    for (int u = 0; u < S::REC / 4; ++u) rec[u] = make_float4(w[4 * u], w[4 * u + 1], w[4 * u + 2], w[4 * u + 3]);
     const int id = sp_id<HALF>(sp.idf);
     const float sc = ((a.nyquist && sp_nyquist(sp.idf)) ? 0.0f : a.scale) * ctf_factor(a.ctf, a.ctfc, a.g, id);
     const int mid = sp_pair<HALF>(sp.idf) ? mirror_id(a.g, id) : -1;
@@ -451,8 +513,11 @@ __global__ void __launch_bounds__(tile_warps(W, F) * 32, W == 2 ? 4 : 2) spread_
     if (mid >= 0) s_scm[slot] = a.scale * ctf_factor(a.ctf, a.ctfc, a.g, mid);
   }
 
-  const int q = lane >> 3, c = lane & 7;
-  const int cp = q % NQ;  // channel part
+  // (lanes past the columns repeat the first one's work and keep it)
+  constexpr int LANES = COLS * NQ;  // of a subset
+  const bool lane_live = lane < LANES * NH;
+  const int q = lane_live ? lane / COLS : 0, c = lane_live ? lane - q * COLS : 0;
+  const int cp = q % NQ, h = q / NQ;  // channel part, subset of the points
   for (int p0 = 0; p0 < a.nch; p0 += CH) {
     __syncthreads();
     // this pass's channel values in sorted order.  A record of kSortHalf that stands for a pair of
@@ -461,12 +526,12 @@ __global__ void __launch_bounds__(tile_warps(W, F) * 32, W == 2 ? 4 : 2) spread_
     // Four elements' loads in flight per thread: the gathers' latency is most of the staging.
     constexpr int GU = 4;
     const int total = st.cnt * CH;
-    for (int e0 = tid; e0 < total; e0 += GU * tile_warps(W, F) * 32) {
+    for (int e0 = tid; e0 < total; e0 += GU * THREADS) {
       float2 x[GU], m[GU];
       int sl[GU];
 #pragma unroll
       for (int u = 0; u < GU; ++u) {
-        const int e = e0 + u * tile_warps(W, F) * 32;
+        const int e = e0 + u * THREADS;
         const int slot = e / CH, ch = e - slot * CH;
         sl[u] = e < total ? slot : -1;
         x[u] = m[u] = make_float2(0.f, 0.f);
@@ -484,7 +549,7 @@ __global__ void __launch_bounds__(tile_warps(W, F) * 32, W == 2 ? 4 : 2) spread_
       for (int u = 0; u < GU; ++u) {
         const int slot = sl[u];
         if (slot < 0) continue;
-        const int ch = e0 + u * tile_warps(W, F) * 32 - slot * CH;
+        const int ch = e0 + u * THREADS - slot * CH;
         const float sc = s_sc[slot];
         float2 v = make_float2(x[u].x * sc, HALF && s_id[slot] < 0 ? -(x[u].y * sc) : x[u].y * sc);
         if (HALF && s_mid[slot] >= 0) {
@@ -492,8 +557,7 @@ __global__ void __launch_bounds__(tile_warps(W, F) * 32, W == 2 ? 4 : 2) spread_
           v.x = fmaf(m[u].x, sm, v.x);
           v.y = fmaf(-m[u].y, sm, v.y);
         }
-        const int part = ch / (F / 2);
-        *reinterpret_cast<float2 *>(vals + (slot * NQ + part) * VS + 2 * (ch - part * (F / 2))) = v;
+        *reinterpret_cast<float2 *>(vals + slot * VS + 2 * ch) = v;
       }
     }
     if (tid == 0) *s_task = 0;
@@ -503,41 +567,50 @@ __global__ void __launch_bounds__(tile_warps(W, F) * 32, W == 2 ? 4 : 2) spread_
       int task = 0;
       if (lane == 0) task = atomicAdd(s_task, 1);
       task = __shfl_sync(0xffffffffu, task, 0);
-      if (task >= PGS * NG) break;
-      const int g = task / PGS, pa0 = (task - g * PGS) * NPL;
-      const int plane = pa0 + (q / NQ) * PP;  // this lane's first plane
-      const int lo = max(pa0 - W + 1, 0), hi = min(pa0 + NPL - 1, kBin - 1);
-      if (lo > hi || s_off[g * 64] == s_off[g * 64 + 64]) continue;
-      float2 acc[PP][T][F / 2];
+      if (task >= T) break;
+      const int plane = T / 2 + (task & 1 ? -((task + 1) / 2) : task / 2);  // the fullest first
+      const int lo = max(plane - W + 1, 0), hi = min(plane, kBin - 1);
+      float2 acc[T][FH];
 #pragma unroll
-      for (int k = 0; k < PP; ++k)
+      for (int r = 0; r < T; ++r)
+#pragma unroll
+        for (int f = 0; f < FH; ++f) acc[r][f] = make_float2(0.f, 0.f);
+      bool any = false;
+#pragma unroll 1
+      for (int g = 0; g < NG; ++g) {
+        // the lane's column in the group and in the tile
+        const int col = NG == 1 ? c : (c - G::base(g)) & (COLS - 1), tc = G::base(g) + col;
+        if (s_off[g * 64] != s_off[g * 64 + 64]) {
+          any = true;
+          auto range = [&](int l1, int &i, int &iend) {
+            i = s_off[g * 64 + l1 * 8 + lo];
+            iend = s_off[g * 64 + l1 * 8 + hi + 1];
+          };
+          TileRows<W, F, NQ, ONE, 0>::run(range, recs, vals, cp, h, col, plane, acc);
+        }
+        if (!any) continue;
+        // the columns that no later group reaches go to the global grid
+        const bool last = g + 1 == NG, done = last || tc < G::base(g + 1);
+        const int co = done && lane_live ? s_col[tc] : -1, ch0 = p0 + cp * FH;
+        const int nf = co < 0 ? 0 : a.nch - ch0;  // channels to write
+        float2 *const dst0 = a.grid + (int64_t)co * a.cs + (int64_t)(a.ch0 + ch0) * a.chs;
+#pragma unroll
+        for (int k = 0; k < RH; ++k) {
+          const int r = k + RH * h;
+          const long long ro = r < T ? s_row[plane * T + r] : -1;
+          float2 *dst = dst0 + ro;
+#pragma unroll
+          for (int f = 0; f < FH; ++f) {
+            const float2 x = subset_sum<NH, LANES>(acc, k, f, h, lane);
+            if (f < nf && (ro >= 0 || (ES && RH * NH == T)) && (x.x != 0.0f || x.y != 0.0f)) add_cell(dst + f * a.chs, x);
+          }
+        }
+        if (last) break;
 #pragma unroll
         for (int r = 0; r < T; ++r)
 #pragma unroll
-          for (int f = 0; f < F / 2; ++f) acc[k][r][f] = make_float2(0.f, 0.f);
-      auto range = [&](int l1, int &i, int &iend) {
-        i = s_off[g * 64 + l1 * 8 + lo];
-        iend = s_off[g * 64 + l1 * 8 + hi + 1];
-      };
-      TileRows<W, F, NQ, PP, 0>::run(range, recs, vals, cp, c, plane, acc);
-      // the finished cells go to the global grid
-      const int co = s_col[G::base(g) + c];
-      if (!ES && co < 0) continue;
-      const int ch0 = p0 + cp * (F / 2);  // this lane's first channel
-#pragma unroll
-      for (int k = 0; k < PP; ++k) {
-        if (plane + k >= T) break;
-#pragma unroll
-        for (int r = 0; r < T; ++r) {
-          const long long ro = s_row[(plane + k) * T + r];
-          if (!ES && ro < 0) continue;
-          float2 *dst = a.grid + (ro + co) * a.cs + (int64_t)(a.ch0 + ch0) * a.chs;
-#pragma unroll
-          for (int f = 0; f < F / 2; ++f) {
-            const float2 x = acc[k][r][f];
-            if (ch0 + f < a.nch && (x.x != 0.0f || x.y != 0.0f)) atomicAdd(dst + f * a.chs, x);
-          }
-        }
+          for (int f = 0; f < FH; ++f)
+            if (done) acc[r][f] = make_float2(0.f, 0.f);
       }
     }
   }
@@ -566,68 +639,57 @@ int launch_nearest(const SpreadParams &a, const Value &value, bool comp, int64_t
   return launched("spread_nearest_kernel");
 }
 
-template <int KT, int W, int F, int NQ, int PP, bool HALF>
+template <int KT, int W, int F, int NQ, bool ONE, bool HALF>
 int launch_tile(const SpreadParams &a, int64_t max_blocks, cudaStream_t st) {
+  using S = TileShape<W, F, NQ, ONE>;
   if (a.max_sub > kTileMaxSub) {
     set_error("subproblems of %d points; the spreading holds %d", a.max_sub, kTileMaxSub);
     return COV3D_EINVAL;
   }
-  const size_t smem = (size_t)a.max_sub * tile_point_bytes<W, F>(NQ) + 8 +
-                      tile_fixed_bytes(TileGroups<W>::T, TileGroups<W>::NG);
-  return launch_spread_kernel(spread_tile_kernel<KT, W, F, NQ, PP, HALF>, "spread_tile_kernel", smem, a, max_blocks, st,
-                              tile_warps(W, F));
+  return launch_spread_kernel(spread_tile_kernel<KT, W, F, NQ, ONE, HALF>, "spread_tile_kernel",
+                              a.max_sub * S::POINT + S::FIXED, a, max_blocks, st, S::WARPS);
 }
 
-// Linear windows: few enough FMAs per point that staging and waiting bound the kernel, so the layouts
-// hold at most 3 channels x 9 rows in a lane's registers and four blocks fit an SM (with
-// subproblems of 208 points; 10 channels, 1024 images of 128^2: 1.96 ms against 2.20 with 5 channels a
-// lane and two blocks of 384 points).  Twelve channels in a pass, then the layout that holds the rest
-// (5 channels, 256 images of 32^2: 51 us at two blocks, 41 at four).
+// Channels in passes of twelve in one launch, then the rest in the layout that holds it.  The linear
+// windows' FMAs are few, so all their columns fit one group; the ES windows' bound their time, and eight
+// columns waste fewer of them, except for one channel, where the flush of the groups costs more.  Microseconds of
+// the layouts tried, ES W = 6: 4 channels of 256 images of 64^2: 422 with one channel a part, 443 with two and
+// two subsets, 544 with three; 2 of 256 of 128^2: 1565, 1635 with all columns and two channels a lane; 1 of 64
+// of 128^2: 699, 853 with eight columns and four subsets; 10 of 1024 of 128^2: 10519, 12121 with two
+// parts of five channels and two subsets.  Linear, 8 channels of 512 images of 64^2: 324, 386 with four
+// channels a part.
 template <int KT, int W, bool HALF>
-int launch_linear_channels(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
-  const int rest = nchan % 12, whole = rest > 8 ? nchan : nchan - rest;
-  if (whole > 0) {
-    a.ch0 = 0;
-    a.nch = whole;
-    COV3D_TRY((launch_tile<KT, W, 6, 4, 1, HALF>(a, max_blocks, st)));
+int launch_channels(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
+  constexpr bool linear = W == 2;
+  const int rest = nchan % 12, whole = rest > 6 ? nchan : nchan - rest;
+  a.ch0 = 0;
+  a.nch = whole;
+  if constexpr (linear) {
+    if (whole > 9) COV3D_TRY((launch_tile<KT, W, 8, 3, true, HALF>(a, max_blocks, st)));
+    else if (whole > 0) return launch_tile<KT, W, 6, 3, true, HALF>(a, max_blocks, st);
+  } else {
+    if (whole > 0) COV3D_TRY((launch_tile<KT, W, 6, 4, false, HALF>(a, max_blocks, st)));
   }
   a.ch0 = whole;
   a.nch = nchan - whole;
-  if (a.nch >= 7) return launch_tile<KT, W, 4, 4, 1, HALF>(a, max_blocks, st);
-  if (a.nch >= 3) return launch_tile<KT, W, 6, 2, 1, HALF>(a, max_blocks, st);
-  if (a.nch == 2) return launch_tile<KT, W, 4, 1, 1, HALF>(a, max_blocks, st);
-  if (a.nch == 1) return launch_tile<KT, W, 2, 1, 2, HALF>(a, max_blocks, st);
-  return COV3D_OK;
-}
-
-// Passes of ten channels in one launch, then the rest in the layout that holds it (3 channels a lane
-// and three blocks of 256 points per SM, as for linear windows: 5.58 ms against 4.74, and 1.07 against
-// 0.44 for 5 channels: here the FMAs bound).
-template <int KT, int W, bool HALF>
-int launch_tile_channels(SpreadParams a, int nchan, int64_t max_blocks, cudaStream_t st) {
-  const int rest = nchan % 10, whole = rest > 5 ? nchan : nchan - rest;
-  if (whole > 0) {
-    a.ch0 = 0;
-    a.nch = whole;
-    COV3D_TRY((launch_tile<KT, W, 10, 2, 1, HALF>(a, max_blocks, st)));
+  if constexpr (linear) {
+    if (a.nch > 3) return launch_tile<KT, W, 4, 3, true, HALF>(a, max_blocks, st);
+    if (a.nch > 2) return launch_tile<KT, W, 2, 3, true, HALF>(a, max_blocks, st);
+    if (a.nch > 1) return launch_tile<KT, W, 4, 1, true, HALF>(a, max_blocks, st);
+    if (a.nch > 0) return launch_tile<KT, W, 2, 1, true, HALF>(a, max_blocks, st);
+  } else {
+    if (a.nch > 4) return launch_tile<KT, W, 6, 2, false, HALF>(a, max_blocks, st);
+    if (a.nch > 2) return launch_tile<KT, W, 2, 4, false, HALF>(a, max_blocks, st);
+    if (a.nch > 1) return launch_tile<KT, W, 2, 2, false, HALF>(a, max_blocks, st);
+    if (a.nch > 0) return launch_tile<KT, W, 2, 1, true, HALF>(a, max_blocks, st);
   }
-  a.ch0 = whole;
-  a.nch = nchan - whole;
-  if (a.nch >= 3) return launch_tile<KT, W, 10, 1, 1, HALF>(a, max_blocks, st);
-  if (a.nch == 2) return launch_tile<KT, W, 4, 1, 1, HALF>(a, max_blocks, st);
-  if (a.nch == 1) return launch_tile<KT, W, 2, 1, 1, HALF>(a, max_blocks, st);
   return COV3D_OK;
 }
 
 template <int KT, int W>
 int launch_w(const SpreadParams &a, int nchan, int64_t max_blocks, cudaStream_t st) {
-  if constexpr (W == 2) {
-    return a.half ? launch_linear_channels<KT, W, true>(a, nchan, max_blocks, st)
-                  : launch_linear_channels<KT, W, false>(a, nchan, max_blocks, st);
-  } else {
-    return a.half ? launch_tile_channels<KT, W, true>(a, nchan, max_blocks, st)
-                  : launch_tile_channels<KT, W, false>(a, nchan, max_blocks, st);
-  }
+  return a.half ? launch_channels<KT, W, true>(a, nchan, max_blocks, st)
+                : launch_channels<KT, W, false>(a, nchan, max_blocks, st);
 }
 
 int launch_nearest_channels(SpreadParams a, int nchan, bool comp, int64_t max_blocks, cudaStream_t st) {

@@ -60,8 +60,8 @@ typedef struct {
   int upsample;      /* sigma; fine grid n = upsample * L (>= 1) */
   int width;         /* ES width w in [2, 16]; 0 = from eps: ceil(-log10(eps/10)) */
   double beta;       /* ES shape; 0 = 0.97*pi*(1 - 1/(2 sigma))*w */
-  int compensated;   /* 1 = TwoSum sums in nearest-cell spreading; the other windows sum few points per cell
-                        in FP32 before they meet in the grid, either way */
+  int compensated;   /* 1 = TwoSum sums in nearest-cell spreading; the other windows fold their FP32 sums either
+                        way, to the accuracy of compensated ones (one atomic addition per cell and up to 416 points) */
   int bin_size;      /* spatial bin edge in fine-grid cells (0 or 8; spreading tiles are 8^3 bins) */
   void *stream;      /* cudaStream_t for all work of this plan (NULL = legacy default) */
 } cov3d_opts;
