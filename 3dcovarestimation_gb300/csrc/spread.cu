@@ -104,7 +104,7 @@ constexpr int kNearestSubs = 16;
 constexpr int kNearestPairs = 5;
 
 template <bool COMP, int NC, typename Value>
-__global__ void __launch_bounds__(kNearestThreads, NC <= 2 ? 2 : 1) spread_nearest_kernel(const SpreadParams a,
+__global__ void __launch_bounds__(kNearestThreads, NC == 1 ? 3 : NC <= 3 ? 2 : 1) spread_nearest_kernel(const SpreadParams a,
                                                                                          const Value value) {
   constexpr int NB = NC > 1 ? 2 : 1;
   __shared__ int s_cnt[kNearestThreads], s_off[kNearestThreads + 1], s_warp[kNearestThreads / 32];
