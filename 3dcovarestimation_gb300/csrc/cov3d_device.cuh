@@ -335,31 +335,45 @@ __device__ __forceinline__ void mean_value(const MeanSource &s, int id, int P, i
   v1 = f * f / (float)L;
 }
 
-// Sums of products of floats in a float pair (about 46 bits: the products' rounding errors and those
-// of the leading sum are carried along): a thread's few terms and a warp's partial sums of the CG's
-// inner products before they are added in FP64, whose pipe (two operations per clock and SM) took
-// most of the kernels that formed every term there.
-struct FloatPair {
-  float h = 0.0f, l = 0.0f;
-  __device__ __forceinline__ void add(float x) {  // TwoSum
-    const float s = __fadd_rn(h, x), b = __fsub_rn(s, h);
-    l = __fadd_rn(l, __fadd_rn(__fsub_rn(h, __fsub_rn(s, b)), __fsub_rn(x, b)));
-    h = s;
+// Sums of products of floats, no less precise than FP64 and of its range: exact products and their exact
+// sum's leading 70 bits in three floats (TwoProd, TwoSum), and the products that floats cannot hold
+// exactly, outside 2^-96 .. 2^100, in FP64.  (The FP64 pipe takes two operations per clock and SM: an
+// iteration of the mean's CG at L = 128 takes 236 us with every term formed there, 210 here; 191 in pairs of
+// floats, 46 bits, whose products lose the range as well.)
+struct WideSum {
+  float h = 0.0f, m = 0.0f, l = 0.0f;
+  double w = 0.0;
+  __device__ __forceinline__ static float two_sum(float &s, float x) {  // s + x = s' + the result
+    const float t = __fadd_rn(s, x), b = __fsub_rn(t, s);
+    const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(x, b));
+    s = t;
+    return e;
   }
   __device__ __forceinline__ void add_product(float a, float b) {
     const float p = __fmul_rn(a, b);
-    const float e = __fmaf_rn(a, b, -p);
-    add(p);
-    l = __fadd_rn(l, e);
+    if (!(fabsf(p) > 1.2621774e-29f && fabsf(p) < 1.2676506e30f) && a != 0.0f && b != 0.0f) {
+      w += (double)a * (double)b;
+      return;
+    }
+    const float e = two_sum(m, __fmaf_rn(a, b, -p)), t = two_sum(h, p);
+    l = __fadd_rn(l, __fadd_rn(e, two_sum(m, t)));
   }
   __device__ __forceinline__ double warp_sum() {  // every lane
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      const float xh = __shfl_xor_sync(0xffffffffu, h, o), xl = __shfl_xor_sync(0xffffffffu, l, o);
-      add(xh);
-      l = __fadd_rn(l, xl);
+      const float xh = __shfl_xor_sync(0xffffffffu, h, o), xm = __shfl_xor_sync(0xffffffffu, m, o);
+      const float xl = __shfl_xor_sync(0xffffffffu, l, o);
+      const float t = two_sum(h, xh), e = two_sum(m, xm);
+      l = __fadd_rn(__fadd_rn(l, xl), __fadd_rn(e, two_sum(m, t)));
     }
-    return (double)h + (double)l;
+    double v = (double)h + ((double)m + (double)l);
+    if (__any_sync(0xffffffffu, w != 0.0)) {  // (also NaN)
+      double x = w;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+      v += x;
+    }
+    return v;
   }
 };
 

@@ -205,8 +205,8 @@ __device__ void block_add_twice(double x, double *a, double *b) {
   }
 }
 
-// Block sums of two float pairs added to a and b; every thread calls it.
-__device__ void block_add_pairs(FloatPair x, FloatPair y, double *a, double *b) {
+// Block sums of x and y added to a and b; every thread calls it.
+__device__ void block_add_two(WideSum x, WideSum y, double *a, double *b) {
   __shared__ double sx[8], sy[8];
   const double wx = x.warp_sum(), wy = y.warp_sum();
   if ((threadIdx.x & 31) == 0) {
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
       float2 *dst = a.out + vrow;
       const float2 *pr = a.p ? a.p + vrow : nullptr;
       const float inv = 1.0f / ((float)n * (float)n * (float)n);
-      FloatPair re, im;
+      WideSum re, im;
       line_dft<N1, N2, true>(
           ex, s_tw, role, [&](int i) { return row[i]; },
           [&](int k, float2 v) {
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(256) line_kernel(const LineArgs a) {
               im.add_product(-q.y, y.x);
             }
           });
-      if (a.p) block_add_pairs(re, im, a.dot, a.dot + 1);
+      if (a.p) block_add_two(re, im, a.dot, a.dot + 1);
     } else {  // kUnpackRows
       const float es = a.logs ? expf(__ldg(a.logs + c)) : 1.0f;
       const float g01 = a.gc ? 1.0f / (__ldg(a.gc + j0) * __ldg(a.gc + j1)) : 1.0f;

@@ -10,10 +10,10 @@
 // DFTs of line_fft.cu (pad, crop and the diagonal fused in); at n = 64 the axis-0 transform
 // and the diagonal are fused between cuFFT 2D transforms of the support planes; otherwise it is
 // pad + cuFFT + diagonal multiply + inverse cuFFT + crop.  The vector updates
-// are fused with their inner products: exact products summed in float pairs within a warp, FP64 from
-// there.  The iteration scalars stay in device memory and a convergence flag turns every kernel of
-// later iterations into a no-op, so the host polls the flag only every few iterations, one poll
-// behind the launches.  Preconditioners:
+// are fused with their inner products, which have the precision and range of FP64 (WideSum).  The
+// iteration scalars stay in device memory and a convergence flag turns every kernel of later iterations
+// into a no-op, so the host polls the flag only every few iterations, one poll behind the launches.
+// Preconditioners:
 //   1: M r = crop(ifft3(fft3(pad r) / lhs))              (the Fourier-diagonal solve on the
 //      fine grid, the operator the reference uses for its starting point, mean.py:238-239)
 //   2: M r = ifft3_L(fft3_L(r) / s)                      (a Fourier diagonal on the L^3 grid:
@@ -182,8 +182,8 @@ __global__ void residual_kernel(const float2 *__restrict__ b, float2 *__restrict
   block_add2(rr, bb, &st->rr, &st->b2);
 }
 
-// Block sum of a float pair added to a global accumulator
-__device__ void block_add_pair(FloatPair v, double *out) {
+// Block sum of v added to a global accumulator
+__device__ void block_add(WideSum v, double *out) {
   __shared__ double sv[32];
   const double w = v.warp_sum();
   if ((threadIdx.x & 31) == 0) sv[threadIdx.x >> 5] = w;
@@ -198,13 +198,13 @@ __device__ void block_add_pair(FloatPair v, double *out) {
 // Re <r, z> into st->rz_new
 __global__ void dot_rz_kernel(const float2 *__restrict__ r, const float2 *__restrict__ z, int64_t N, CgState *st) {
   if (stopped(st)) return;
-  FloatPair acc;
+  WideSum acc;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
     const float2 a = r[i], c = z[i];
     acc.add_product(a.x, c.x);
     acc.add_product(a.y, c.y);
   }
-  block_add_pair(acc, &st->rz_new);
+  block_add(acc, &st->rz_new);
 }
 
 // convergence test of loop index `running` (||r|| < rtol ||b||, mean.py:80-81)
@@ -234,7 +234,7 @@ __global__ void update_kernel(float2 *__restrict__ x, float2 *__restrict__ r, co
   const double pr = st->pap[0], pi = st->pap[1];
   const double den = pr * pr + pi * pi;
   const float ar = (float)(st->rz * pr / den), ai = (float)(-st->rz * pi / den);
-  FloatPair rr;
+  WideSum rr;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
     const float2 pv = p[i], av = ap[i];
     float2 xv = x[i], rv = r[i];
@@ -247,7 +247,7 @@ __global__ void update_kernel(float2 *__restrict__ x, float2 *__restrict__ r, co
     rr.add_product(rv.x, rv.x);
     rr.add_product(rv.y, rv.y);
   }
-  block_add_pair(rr, &st->rr_new);
+  block_add(rr, &st->rr_new);
   if (threadIdx.x == 0) {
     __threadfence();
     if (atomicInc(&st->ticket, gridDim.x - 1) == gridDim.x - 1) {
