@@ -90,14 +90,14 @@ __global__ void unpack_grad_kernel(const float2 *__restrict__ fine, const float 
 // ML Fourier regulariser reg_scale * sum |G|^2 fr / (2 s2) (covar_sgd.py:1373-1376): adds its
 // conjugate-Wirtinger derivative coef * fr * G to the fine-grid gradient (or, with `init`,
 // writes it there, so the grid needs no zeroing before the spread), accumulates its value and, twice
-// that per channel, its derivative with respect to log_sqrt (each thread's terms of a channel in
+// that per channel, its derivative with respect to log_sqrt (each thread's FP64 sums, one per channel, in
 // shared memory).
 __global__ void ml_reg_kernel(const float2 *__restrict__ grid, float2 *__restrict__ gg, const float *__restrict__ fr,
                               int64_t frs, int nchan, int n, double coef, double *__restrict__ cost,
                               double *__restrict__ glog, int init) {
-  extern __shared__ float s_gl[];  // nchan * blockDim.x
-  float *gl = s_gl + threadIdx.x;
-  for (int c = 0; c < nchan; ++c) gl[c * blockDim.x] = 0.0f;
+  extern __shared__ double s_gl[];  // nchan * blockDim.x
+  double *gl = s_gl + threadIdx.x;
+  for (int c = 0; c < nchan; ++c) gl[c * blockDim.x] = 0.0;
   // capped grid walking whole rows (no per-element division); the channel sum of one cell is
   // FP32, the running sum over cells FP64, one FP64 atomic per block
   const int64_t n3 = (int64_t)n * n * n;
@@ -137,7 +137,8 @@ __global__ void ml_reg_kernel(const float2 *__restrict__ grid, float2 *__restric
                                                fmaf(cfb, x[u].z, y[u].z), fmaf(cfb, x[u].w, y[u].w));
             pa = fmaf(x[u].x, x[u].x, fmaf(x[u].y, x[u].y, pa));
             pb = fmaf(x[u].z, x[u].z, fmaf(x[u].w, x[u].w, pb));
-            gl[(c + u) * blockDim.x] += wa * (x[u].x * x[u].x + x[u].y * x[u].y) + wb * (x[u].z * x[u].z + x[u].w * x[u].w);
+            gl[(c + u) * blockDim.x] +=
+                (double)(wa * (x[u].x * x[u].x + x[u].y * x[u].y) + wb * (x[u].z * x[u].z + x[u].w * x[u].w));
           }
         }
         for (; c < nchan; ++c) {
@@ -146,7 +147,7 @@ __global__ void ml_reg_kernel(const float2 *__restrict__ grid, float2 *__restric
           dst[c * cstep] = make_float4(fmaf(cfa, x.x, y.x), fmaf(cfa, x.y, y.y), fmaf(cfb, x.z, y.z), fmaf(cfb, x.w, y.w));
           pa = fmaf(x.x, x.x, fmaf(x.y, x.y, pa));
           pb = fmaf(x.z, x.z, fmaf(x.w, x.w, pb));
-          gl[c * blockDim.x] += wa * (x.x * x.x + x.y * x.y) + wb * (x.z * x.z + x.w * x.w);
+          gl[c * blockDim.x] += (double)(wa * (x.x * x.x + x.y * x.y) + wb * (x.z * x.z + x.w * x.w));
         }
         part += (double)(wa * pa) + (double)(wb * pb);
       }
@@ -165,7 +166,7 @@ __global__ void ml_reg_kernel(const float2 *__restrict__ grid, float2 *__restric
         y.y = fmaf(cf, x.y, y.y);
         gg[c * n3 + cell] = y;
         p32 = fmaf(w, fmaf(x.x, x.x, x.y * x.y), p32);
-        gl[c * blockDim.x] += w * (x.x * x.x + x.y * x.y);
+        gl[c * blockDim.x] += (double)(w * (x.x * x.x + x.y * x.y));
       }
       part += (double)p32;
     }
@@ -184,7 +185,7 @@ __global__ void ml_reg_kernel(const float2 *__restrict__ grid, float2 *__restric
   const int lane = threadIdx.x & 31, nw = (int)(blockDim.x >> 5);
   for (int c = threadIdx.x >> 5; c < nchan; c += nw) {  // a warp per channel
     double t = 0.0;
-    for (int i = lane; i < (int)blockDim.x; i += 32) t += (double)s_gl[c * blockDim.x + i];
+    for (int i = lane; i < (int)blockDim.x; i += 32) t += s_gl[c * blockDim.x + i];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (lane == 0 && t != 0.0) atomicAdd(glog + c, 2.0 * t * coef);
@@ -236,8 +237,8 @@ int launch_ml_reg(cov3d_plan *p, const void *grid, void *ggrid, const float *fr,
   const int64_t rows = (int64_t)p->n * p->n;
   const unsigned blocks = (unsigned)(rows < 2432 ? rows : 2432);  // 16 blocks of 4 warps per SM
   (void)n3;
-  ml_reg_kernel<<<blocks, 128, (size_t)nchan * 128 * sizeof(float), p->stream>>>(static_cast<const float2 *>(grid), static_cast<float2 *>(ggrid), fr,
-                                               fr_stride, nchan, p->n, coef, cost_acc, glog, init);
+  ml_reg_kernel<<<blocks, 128, (size_t)nchan * 128 * sizeof(double), p->stream>>>(
+      static_cast<const float2 *>(grid), static_cast<float2 *>(ggrid), fr, fr_stride, nchan, p->n, coef, cost_acc, glog, init);
   return launched("ml_reg_kernel");
 }
 

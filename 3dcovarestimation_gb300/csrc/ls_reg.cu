@@ -52,7 +52,6 @@ __global__ void ls_scatter_kernel(const float2 *__restrict__ y, const float2 *__
   const int c = blockIdx.y;
   double part = 0.0;
   for (int64_t rr = blockIdx.x; rr < n2; rr += gridDim.x) {
-    float dot = 0.0f;  // a thread's terms of one row in FP32
     const int s0 = (int)(rr / n), s1 = (int)(rr - (int64_t)s0 * n);
     const int64_t crow = ((int64_t)native_to_centered(s0, n) * n + native_to_centered(s1, n)) * n;
     const float2 *src = y + c * n3 + crow;
@@ -65,9 +64,8 @@ __global__ void ls_scatter_kernel(const float2 *__restrict__ y, const float2 *__
       const float2 v = src[c2];
       const float2 o = dst[s2], x = gr[s2];
       dst[s2] = make_float2(fmaf(w, v.x, o.x), fmaf(w, v.y, o.y));
-      dot = fmaf(w, fmaf(v.x, x.x, v.y * x.y), dot);
+      part += (double)(w * fmaf(v.x, x.x, v.y * x.y));
     }
-    part += (double)dot;
   }
   for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
   __shared__ double wsum[32];
