@@ -336,9 +336,16 @@ int cov3d_plan_reserve(cov3d_plan *p, int64_t max_images, int points_L, int ncha
   const int64_t P = (int64_t)points_L * points_L;
   const int64_t M = max_images * P;
   const int64_t n3 = (int64_t)p->n * p->n * p->n;
-  for (int m = 0; m < kSortModes; ++m) COV3D_TRY(reserve_sort(p, M, (SortMode)m));
+  // the records of the step's interpolation and spreading, which every new point set is sorted into
+  // from now on (need_sorted's first use would wait for them); nearest cells have no pairs
+  COV3D_TRY(reserve_sort(p, M, kSortFull));
+  p->sets[kSortFull].used = true;
   COV3D_TRY(grow(p->rot, max_images * 9 * 4));
-  COV3D_TRY(grow(p->rotc, max_images * 6 * 8));
+  if (p->kernel != COV3D_KERNEL_NEAREST && M < (int64_t(1) << 29)) {
+    COV3D_TRY(reserve_sort(p, M, kSortHalf));
+    COV3D_TRY(grow(p->rotc, max_images * 6 * 8));
+    p->sets[kSortHalf].used = true;
+  }
   if (flags & COV3D_RESERVE_POINTS) COV3D_TRY(grow(p->pts, max_images * 3 * P * 4));
   // the covariance step: fine grid and its gradient, projections, per-image matrices
   COV3D_TRY(grow(p->fine, n3 * nchan * 8));
