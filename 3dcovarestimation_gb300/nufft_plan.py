@@ -306,8 +306,8 @@ class _BackprojectFn(torch.autograd.Function):
     def forward(ctx, values, plan, ctf, flags, scale, real=False):
         ctx.plan, ctx.ctf, ctx.flags, ctx.scale = plan, ctf, flags, scale
         ctx.complex_input = values.is_complex()
-        if real:
-            return plan.backproject(values, ctf, flags | _lib.REAL_OUTPUT, scale).real
+        if real:  # (a copy: autograd refuses in-place changes of a view made here)
+            return plan.backproject(values, ctf, flags | _lib.REAL_OUTPUT, scale).real.contiguous()
         return plan.backproject(values, ctf, flags, scale)
 
     @staticmethod
