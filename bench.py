@@ -115,6 +115,17 @@ def cpu_baseline_reference(args, batch, steps, warmup, budget_s):
                        f"torch CPU threads={det['threads']}, {det['seconds']:.1f} s timed")}, det
 
 
+def cpu_baselines(args):
+    """The GPU line's CPU baselines: the reference's own trainer, with a null value and the reason where it
+    is not installed or does not run on this host, and the ES port."""
+    try:
+        ref, _ = cpu_baseline_reference(args, args.ref_batch, 1, 1, 1e9)
+    except Exception as e:
+        why = f"{type(e).__name__}: {e}".splitlines()[0]
+        ref = {"value": None, "unit": "images/s", "kind": "reference", "unavailable": why}
+    return {"cpu_baseline": ref, "cpu_baseline_es_port": cpu_baseline_port(args)}
+
+
 def run_reference(args):
     rank, world, _ = dist_env()
     if rank != 0:
@@ -337,12 +348,14 @@ def run_small_epoch(pkg, args, dev, with_reference):
     if with_reference:
         from oracle import ref_step
 
-        if ref_step.available():
+        try:
             ips, det = ref_step.time_steps(L, r, B, 8, 1, seed=args.seed, budget_s=60.0)
             out["reference_images_per_s"] = ips
             out["reference_epoch_s_estimate"] = N / ips
             out["reference_sample"] = (f"{det['steps']} whole run_batch step(s) of {B} images after {det['warmup']} "
                                        f"warm-up, torch CPU threads={det['threads']}")
+        except Exception as e:  # not installed, or does not run on this host: the GPU's figures stand
+            out["reference_unavailable"] = f"{type(e).__name__}: {e}".splitlines()[0]
     return out
 
 
@@ -736,7 +749,9 @@ def run_gb300(args):
     flops = M * (args.width**3) * r * 4
     sm_mhz = clocks.get("sm_mhz") or 1900.0
     fp32_peak = 152 * 128 * 2 * sm_mhz * 1e6 / 1e12
-    kernel_name = "interp_group_kernel" if dom == "interp" else "spread_tile_kernel"
+    # more than five channels share tile loads where there are points enough per cell (group_pass, interp.cu)
+    grouped = args.width <= 6 and r > 5 and M >= (0.75 if args.width == 6 else 0.5) * n3
+    kernel_name = "spread_tile_kernel" if dom == "spread" else "interp_group_kernel" if grouped else "interp_kernel"
     line = {
         "metric": METRIC, "value": value, "unit": "images/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
@@ -770,9 +785,7 @@ def run_gb300(args):
     if bilinear is not None:
         line["bilinear_step"] = bilinear
     if not args.no_cpu_baseline:
-        cb, _ = cpu_baseline_reference(args, args.ref_batch, 1, 1, 1e9)
-        line["cpu_baseline"] = cb
-        line["cpu_baseline_es_port"] = cpu_baseline_port(args)
+        line.update(cpu_baselines(args))
     print(json.dumps(line), flush=True)
     if world > 1:
         import torch.distributed as dist
