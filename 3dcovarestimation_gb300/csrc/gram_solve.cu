@@ -861,7 +861,9 @@ int covar_cost_grad(cov3d_plan *p, const cov3d_cost_args *a, double *h_cost, dou
                            a->objective == 0 ? 1.0 / B : 1.0 / (B * L4), a->objective == 0 ? 1.0 : 1.0 / L4, C, u,
                            d_per_image_cost, acc, nullptr, nullptr, bad, acc + 8));
   }
-  // 6. dcost/dconj(Q) in place, 7. spread through the exact adjoint (CTF, Nyquist, 1/L prologue)
+  // 6. dcost/dconj(Q) in place, 7. spread through the adjoint (CTF, Nyquist, 1/L prologue): exact for
+  // nearest cells; the other windows' pair records sit up to 6e-5 cells from the 32-bit indices that
+  // the projections were taken at, and are the finer ones
   {
     PhaseScope ps(p, kPhaseWpass);
     COV3D_TRY(launch_wpass(p->stream, B, P, r, p->q.ptr, (int64_t)P * r, r, 1, a->d_images, C, u, p->q.ptr,

@@ -1,6 +1,6 @@
-// Spreading ("type-1" half of the NUFFT; exact adjoint of interp.cu, replacing the
-// reference's grid_sample backward with FP32 global atomics, nufft_plan.py:171-242), over the
-// bin-sorted point records of points_sort.cu.  See spread_tile_kernel (ES and linear windows) and
+// Spreading ("type-1" half of the NUFFT; the exact adjoint of interp.cu over the same records,
+// replacing the reference's grid_sample backward with FP32 global atomics, nufft_plan.py:171-242), over
+// the bin-sorted point records of points_sort.cu, whose two views differ by up to 6e-5 cells.  See spread_tile_kernel (ES and linear windows) and
 // spread_nearest_kernel for the decompositions.
 
 #include "cov3d_device.cuh"

@@ -58,7 +58,7 @@ typedef struct cov3d_plan cov3d_plan;
 typedef struct {
   int kernel;        /* cov3d_kernel */
   int upsample;      /* sigma; fine grid n = upsample * L (>= 1) */
-  int width;         /* ES width w in [2, 16]; 0 = from eps: ceil(-log10(eps/10)) */
+  int width;         /* ES width w in [4, 8]; 0 = from eps: ceil(-log10(eps/10)) */
   double beta;       /* ES shape; 0 = 0.97*pi*(1 - 1/(2 sigma))*w */
   int compensated;   /* 1 = TwoSum sums in nearest-cell spreading; the other windows fold their FP32 sums either
                         way, to the accuracy of compensated ones (one atomic addition per cell and up to 416 points) */
@@ -151,7 +151,7 @@ int cov3d_setrot(cov3d_plan *plan, const float *d_rot, int64_t n_images, int poi
 int cov3d_interp(cov3d_plan *plan, const void *d_grid, const cov3d_grid_layout *layout, int nchan, void *d_out,
                  int64_t out_point_stride, int64_t out_chan_stride, const float *d_ctf, int flags, float scale);
 
-/* Exact adjoint of cov3d_interp: spread nchan channels of point values into a fine grid
+/* Exact adjoint of cov3d_interp (without COV3D_GRID_HERMITIAN): spread nchan channels of point values into a fine grid
  * (the reference's grid_sample backward, execute_adjoint nufft_plan.py:171-200).  The grid is
  * zeroed first unless accumulate != 0.  flags / scale as in cov3d_interp (im_backward's
  * CTF multiply, Nyquist zeroing and 1/L, projection_funcs.py:385-399). */
@@ -169,8 +169,9 @@ int cov3d_spread_unaggregated(cov3d_plan *plan, const void *d_values, int64_t in
  * (nchan, n_points) complex64 (NufftPlan.execute_forward, nufft_plan.py:338-364). */
 int cov3d_execute_type2(cov3d_plan *plan, const float *d_vol_real, const void *d_vol_complex, int nchan, void *d_out);
 
-/* Type-1 NUFFT (exact adjoint of type 2): (nchan, n_points) complex64 -> (nchan, L^3)
- * complex64 (NufftPlan.execute_adjoint, nufft_plan.py:366-392). */
+/* Type-1 NUFFT (exact adjoint of type 2 of complex volumes; a real volume's mirror pixels are taken at
+ * one position, up to 6e-5 cells from each of theirs): (nchan, n_points) complex64 -> (nchan, L^3) complex64
+ * (NufftPlan.execute_adjoint, nufft_plan.py:366-392). */
 int cov3d_execute_type1(cov3d_plan *plan, const void *d_values, int nchan, void *d_vol_out);
 
 /* CTF images (n_images, L, L) float32 from per-image parameters (n_images, COV3D_CTF_NPARAMS):
@@ -193,7 +194,8 @@ int cov3d_project(cov3d_plan *plan, const float *d_vol_real, const void *d_vol_c
  * its plan on the same eigenvolumes for every batch (wiener_coords.py:131-139). */
 int cov3d_fine_grid(cov3d_plan *plan, const float *d_vol_real, const void *d_vol_complex, int nchan, void *d_grid);
 
-/* Its exact adjoint: cov3d_execute_type1 with im_backward's prologue fused into the spreading
+/* The exact adjoint of cov3d_project of complex volumes or, with COV3D_REAL_OUTPUT, of real ones:
+ * cov3d_execute_type1 with im_backward's prologue fused into the spreading
  * (projection_funcs.py:373-399); (point, channel) input at d_values[point*in_point_stride +
  * ch*in_chan_stride], (nchan, L^3) complex64 output. */
 int cov3d_backproject(cov3d_plan *plan, const void *d_values, int64_t in_point_stride, int64_t in_chan_stride,
@@ -210,7 +212,9 @@ int cov3d_grid_correction(const cov3d_plan *plan, float *d_out);
  * (covar_sgd.py:1350-1399) / cost_fourier_domain (:1290-1347) + autograd backward as driven
  * by CovarTrainer.run_batch (covar_sgd.py:199-229).  The gradient is the hand-written adjoint:
  * per-image r x r Gram + FP64 Hermitian solve, then backprojection of the cost's derivative
- * with respect to the projections through the exact adjoint of the interpolation.
+ * with respect to the projections through the adjoint of the interpolation.  ES and linear windows
+ * interpolate at each pixel's 32-bit index and spread mirror pixels at one finer position, up to
+ * 6e-5 cells away at n = 256.
  * Points must be set (setpts/setrot) for n_images = B images of L^2 pixels. */
 typedef struct {
   int objective;            /* 0 = maximum likelihood (default objective), 1 = least squares */
