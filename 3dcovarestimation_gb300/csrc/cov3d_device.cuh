@@ -232,7 +232,7 @@ __device__ __forceinline__ float record_offset(float t, int c, int frac) {
 template <int KT, int W, bool HALF>
 __device__ __forceinline__ float record_weight(float t, int c0, int q, int frac, float beta) {
   if (KT == COV3D_KERNEL_NEAREST) return 1.0f;
-  if (HALF) {  // the offset is exact
+  if (HALF) {  // the offset, of at most W / 2 cells, is exact from n = 256 on and rounded to 24 bits on smaller grids
     const float x = record_offset<true>(t, c0, frac);
     if (KT == COV3D_KERNEL_LINEAR) return q == 0 ? 1.0f - x : x;
     return es_weight<W>(x - (float)q, beta);

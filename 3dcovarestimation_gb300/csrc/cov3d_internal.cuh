@@ -143,7 +143,7 @@ struct cov3d_plan {
 
   // sort / subproblems
   cov3d::Bins bins{};
-  int max_sub = 288;
+  int max_sub = cov3d::kSubPointsES;
   cov3d::SortSet sets[cov3d::kSortModes];     // bin-sorted records by SortMode
   cudaStream_t sort_stream = nullptr;  // first uses of a view are sorted here (need_sorted) ...
   cudaEvent_t points_set = nullptr;    // ... after the points

@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(InterpWarps<W, CP>::value * 32) interp_kernel(
   const int first = a.sub_first[sub];
   // one block per bin: the block of the bin's first subproblem takes all of the bin's points,
   // kInterpChunk at a time, so the tile is staged once per bin (512 points per bin on average
-  // at the cov-SGD workload, which 288-point subproblems split 2.8 ways; 14.1 -> 12.6 ms)
+  // at the cov-SGD workload, two subproblems; 14.1 -> 12.6 ms when they were of 288 points)
   if (first != a.bin_off[bin]) return;
   const int last = a.bin_off[bin + 1];
   int cnt = min(kInterpChunk, last - first);

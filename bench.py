@@ -33,7 +33,7 @@ WORKLOAD = ("cov-SGD step, GPU drop-in plain FP32 config: L=128, pixel 1.5 A, r=
             "batch 1024, uniform SO(3) poses, CTF 300 kV / Cs 2.7 mm / AC 0.1 / defocus U[1,3] um (from per-image "
             "parameters), SNR 0.05, "
             "NUFFT upsampling 2, ML objective + Fourier regulariser, Adam")
-GPU_INTERP = "ES kernel width 6 (tol 1e-6), periodic, FP32 spreading"
+GPU_INTERP = "ES kernel width 6 (tol 1e-6), periodic, FP32 spreading with folded sums"
 REF_INTERP = ("reference NufftPlanDiscretized bilinear (grid_sample), the reference command line's default; its ES "
               "plan (cuFINUFFT) is not installed")
 
@@ -758,7 +758,7 @@ def run_gb300(args):
         "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": shared_config(args, world),
         "interpolation": GPU_INTERP, "resident_images": nb * B,
-        "spreading": "fp32",
+        "spreading": "fp32, folded sums",
         "roofline": {"bound": "hbm", "kernel": kernel_name, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind, "traffic": load_traffic(kernel_name),
                      "algorithmic_bytes_per_launch": alg[dom], "ms_per_launch": dom_ms,
