@@ -116,7 +116,9 @@ struct SortSet {
   int *sub_bin = nullptr, *sub_first = nullptr, *sub_count = nullptr;  // (max subproblems)
   int *nsub = nullptr;  // scalar
   bool used = false;    // some operator has asked for it: sorted with every new point set
-  bool valid = false;   // holds the current points
+  bool valid = false;   // holds the current points, or will once ...
+  bool pending = false;          // ... the first use's sort is done, on whatever stream:
+  cudaEvent_t done = nullptr;    // operators wait for this meanwhile
 };
 }  // namespace cov3d
 
@@ -145,8 +147,8 @@ struct cov3d_plan {
   cov3d::Bins bins{};
   int max_sub = cov3d::kSubPointsES;
   cov3d::SortSet sets[cov3d::kSortModes];     // bin-sorted records by SortMode
-  cudaStream_t sort_stream = nullptr;  // first uses of a view are sorted here (need_sorted) ...
-  cudaEvent_t points_set = nullptr;    // ... after the points
+  cudaStream_t sort_stream = nullptr;  // first uses inside a capture are sorted here (need_sorted)
+  cudaEvent_t points_set = nullptr;    // first uses wait for it
   bool pairs_off = false;              // no operator uses kSortHalf any more (new_points)
 
   // workspaces

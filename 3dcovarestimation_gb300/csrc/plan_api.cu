@@ -381,6 +381,8 @@ int cov3d_plan_destroy(cov3d_plan *p) {
                     &p->small, &p->acc, &p->cgw, &p->xbf, &p->gsum, &p->fftw, &p->ctfc, &p->lsw};
   for (DevBuf *b : bufs) release(*b);
   for (SortSet &ss : p->sets) release(ss.mem);
+  for (SortSet &ss : p->sets)
+    if (ss.done) cudaEventDestroy(ss.done);
   if (p->points_set) cudaEventDestroy(p->points_set);
   if (p->sort_stream) cudaStreamDestroy(p->sort_stream);
   release_blas(p);

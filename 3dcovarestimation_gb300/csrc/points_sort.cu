@@ -514,68 +514,119 @@ SortMode hermitian_mode(const cov3d_plan *p) {
 // the pairs' view has no room to be sorted there, the replay would change the points unseen by it, so
 // no operator of this plan uses pair records from then on (graphs made before still find theirs).
 int new_points(cov3d_plan *p) {
-  for (SortSet &ss : p->sets) ss.valid = false;
+  for (SortSet &ss : p->sets) ss.valid = ss.pending = false;
   const int64_t M = p->n_points;
   if (M <= 0) return COV3D_OK;
   if (M >= (int64_t)(1 << 30)) {
     set_error("too many points (%lld); the limit is 2^30-1 per plan", (long long)M);
     return COV3D_EINVAL;
   }
-  COV3D_TRY(reserve_sort(p, M, kSortFull));  // a first use inside a capture needs its buffers
   bool cap = false;
   COV3D_TRY(capturing(p, &cap));
   if (cap) {
     p->sets[kSortFull].used = true;
+    if (!p->sets[kSortFull].mem.ptr) {  // a first allocation is possible here, in the relaxed mode
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      COV3D_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+      const int rc = reserve_sort(p, M, kSortFull);
+      COV3D_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+      COV3D_TRY(rc);
+    }
     if (pairs_apply(p)) {
       if (pairs_fit(p)) p->sets[kSortHalf].used = true;
       else p->pairs_off = true;
     }
   }
   unsigned modes = 0;
-  bool later = false;
   for (int m = 0; m < kSortModes; ++m) {
     if (m == kSortHalf && !(pairs_apply(p) && (!p->pairs_off || (p->sets[m].used && pairs_fit(p))))) continue;
     if (p->sets[m].used) modes |= 1u << m;
-    else later = true;
   }
   COV3D_TRY(sort_points(p, modes));
-  if (!later) return COV3D_OK;
-  // first uses wait for this event
-  if (!p->sort_stream) COV3D_CUDA(cudaStreamCreateWithFlags(&p->sort_stream, cudaStreamNonBlocking));
+  if (cap) return COV3D_OK;
   if (!p->points_set) COV3D_CUDA(cudaEventCreateWithFlags(&p->points_set, cudaEventDisableTiming));
   return check_cuda(cudaEventRecord(p->points_set, p->stream), "points event");
 }
 
-// The views in `modes` (bits 1 << SortMode) hold the current points.  A view's first use (once per
-// plan and view) sorts it on a stream of the plan's own, after the points, and waits for it: the view
-// is then complete for the operators of every stream, and when the caller's stream is capturing the
-// sort has run and is no part of the graph (as if it had been sorted when the points were set).
-int need_sorted(cov3d_plan *p, unsigned modes) {
-  unsigned todo = 0;
-  for (int m = 0; m < kSortModes; ++m) {
-    if (!(modes >> m & 1)) continue;
-    SortSet &ss = p->sets[m];
-    ss.used = true;
-    if (!ss.valid) todo |= 1u << m;
+// A first use outside a capture: the views in `todo` sorted on the caller's stream, after the points.
+// Operators of other streams wait for the views' events until they have completed.
+static int first_use(cov3d_plan *p, unsigned todo) {
+  if (p->points_set) COV3D_CUDA(cudaStreamWaitEvent(p->stream, p->points_set, 0));
+  {
+    PhaseScope ps(p, kPhaseSort);
+    COV3D_TRY(sort_points(p, todo));
   }
-  if (!todo) return COV3D_OK;
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // this thread may wait while a stream captures
-  COV3D_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+  for (int m = 0; m < kSortModes; ++m) {
+    if (!(todo >> m & 1)) continue;
+    SortSet &ss = p->sets[m];
+    ss.valid = false;  // until operators can wait for it
+    if (!ss.done) COV3D_CUDA(cudaEventCreateWithFlags(&ss.done, cudaEventDisableTiming));
+    COV3D_CUDA(cudaEventRecord(ss.done, p->stream));
+    ss.valid = ss.pending = true;
+  }
+  return COV3D_OK;
+}
+
+// A first use inside a capture: sorted on a stream of the plan's own and waited for, so that the sort
+// has run and is no part of the graph (as if the view had been sorted when the points were set).  It may
+// allocate the view's buffers (in the relaxed mode); it never frees any: a view that nothing has used yet
+// has none, or those that cov3d_plan_reserve made.
+static int first_use_in_capture(cov3d_plan *p, unsigned todo) {
+  if (!p->sort_stream) COV3D_CUDA(cudaStreamCreateWithFlags(&p->sort_stream, cudaStreamNonBlocking));
+  if (p->points_set) COV3D_CUDA(cudaStreamWaitEvent(p->sort_stream, p->points_set, 0));
   const cudaStream_t caller = p->stream;
   p->stream = p->sort_stream;
-  int rc = check_cuda(cudaStreamWaitEvent(p->sort_stream, p->points_set, 0), "points event");
-  if (rc == COV3D_OK) {
+  int rc;
+  {
     PhaseScope ps(p, kPhaseSort);
     rc = sort_points(p, todo);
   }
   const int done = check_cuda(cudaStreamSynchronize(p->sort_stream), "sort");
   p->stream = caller;
+  return rc != COV3D_OK ? rc : done;
+}
+
+// The caller's stream comes after a pending first use of the view; a capture, whose graph may be replayed
+// at any time, waits for it here.
+static int after_first_use(cov3d_plan *p, SortSet &ss, bool cap) {
+  const cudaError_t q = cudaEventQuery(ss.done);
+  if (q != cudaSuccess && q != cudaErrorNotReady) return check_cuda(q, "sort event");
+  if (q == cudaErrorNotReady) {
+    (void)cudaGetLastError();
+    if (!cap) return check_cuda(cudaStreamWaitEvent(p->stream, ss.done, 0), "sort event");
+    COV3D_CUDA(cudaEventSynchronize(ss.done));
+  }
+  ss.pending = false;
+  return COV3D_OK;
+}
+
+// The views in `modes` (bits 1 << SortMode) hold the current points for the caller's stream.
+int need_sorted(cov3d_plan *p, unsigned modes) {
+  unsigned todo = 0;
+  bool wait = false;
+  for (int m = 0; m < kSortModes; ++m) {
+    if (!(modes >> m & 1)) continue;
+    SortSet &ss = p->sets[m];
+    ss.used = true;
+    if (!ss.valid) todo |= 1u << m;
+    else wait = wait || ss.pending;
+  }
+  if (!todo && !wait) return COV3D_OK;
+  bool cap = false;
+  COV3D_TRY(capturing(p, &cap));
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // this thread may allocate, ask and wait in a capture
+  COV3D_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+  int rc = COV3D_OK;
+  for (int m = 0; m < kSortModes && rc == COV3D_OK; ++m)
+    if ((modes >> m & 1) && p->sets[m].valid && p->sets[m].pending) rc = after_first_use(p, p->sets[m], cap);
+  if (rc == COV3D_OK && todo) {
+    rc = cap ? first_use_in_capture(p, todo) : first_use(p, todo);
+    if (rc != COV3D_OK)
+      for (int m = 0; m < kSortModes; ++m)
+        if (todo >> m & 1) p->sets[m].valid = false;
+  }
   const int back = check_cuda(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
-  if (rc == COV3D_OK) rc = done != COV3D_OK ? done : back;
-  if (rc != COV3D_OK)
-    for (int m = 0; m < kSortModes; ++m)
-      if (todo >> m & 1) p->sets[m].valid = false;
-  return rc;
+  return rc != COV3D_OK ? rc : back;
 }
 
 }  // namespace cov3d

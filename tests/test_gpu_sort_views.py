@@ -109,6 +109,32 @@ def test_capture_as_the_first_use(pkg, dev, kernel, reserved, hermitian):
 
 
 @pytest.mark.parametrize("kernel", [0, 1])
+@pytest.mark.parametrize("hermitian", [False, True])
+def test_capture_right_after_the_first_use(pkg, dev, kernel, hermitian):
+    """The first operator is launched on one stream and the next one captured on another that does not wait
+    for it."""
+    grid = _grid(_plan(pkg, kernel, dev), dev)
+    rot = _rotations(dev, 2)
+    want = _want(pkg, kernel, dev, rot, grid)[1 if hermitian else 0]
+    flags = pkg._lib.GRID_HERMITIAN if hermitian else 0
+    p = _plan(pkg, kernel, dev)
+    a, b, c = (torch.cuda.Stream() for _ in range(3))
+    torch.cuda.synchronize()
+    with torch.cuda.stream(a):
+        p.setrot(rot, L)
+    with torch.cuda.stream(b):
+        first = p.interp_native(grid, None, flags)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(c):
+        graph.capture_begin()
+        out = p.interp_native(grid, None, flags)
+        graph.capture_end()
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(first, want) and torch.equal(out, want)
+
+
+@pytest.mark.parametrize("kernel", [0, 1])
 @pytest.mark.parametrize("used", ["none", "full"])
 def test_points_set_by_a_replay_reach_every_view(pkg, dev, kernel, used):
     """Poses set inside a graph: a plan that has no room for the pairs' records there leaves them out."""
