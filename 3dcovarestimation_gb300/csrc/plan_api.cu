@@ -337,7 +337,7 @@ int cov3d_plan_reserve(cov3d_plan *p, int64_t max_images, int points_L, int ncha
   const int64_t M = max_images * P;
   const int64_t n3 = (int64_t)p->n * p->n * p->n;
   // the records of the step's interpolation and spreading, which every new point set is sorted into
-  // from now on (a captured step finds them sorted by each replay); nearest cells have no pairs
+  // from now on, inside a capture too; nearest cells have no pairs
   COV3D_TRY(reserve_sort(p, M, kSortFull));
   p->sets[kSortFull].used = true;
   COV3D_TRY(grow(p->rot, max_images * 9 * 4));
